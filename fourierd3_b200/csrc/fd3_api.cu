@@ -680,6 +680,7 @@ void carve(const fd3_plan* p, int64_t N, int64_t K_in, Carver& c, Work& w, int64
   w.ei.kd = c.take<int>(E);
   w.ei.ord_s = c.take<int>(E);
   w.ei.ord_d = c.take<int>(E);
+  w.ei.arrival = c.take<int>(E);
   w.ei.cnt = c.take<int>(N);
   w.ei.st_s = c.take<int>(N + 1);
   w.ei.st_d = c.take<int>(N + 1);
@@ -752,7 +753,8 @@ static int mesh_sort(fd3_plan* p, int N, const double* pos, double ps, const int
   const MeshGeom& mg = p->mg;
   const int Kmesh = mg.nt[0] * mg.nt[1] * mg.nt[2] * p->S;
   FD3_TRY(launch_mesh_keys(mg, N, pos, ps, species, w.ci, w.mkeys, s));
-  return counting_sort(w.mkeys, N, Kmesh, w.mcount, w.mstart, w.morder, s);
+  // the stencil nodes are written after the sort: until then they are its scratch
+  return counting_sort(w.mkeys, N, Kmesh, w.mcount, w.mstart, w.morder, reinterpret_cast<int*>(w.rec.b), s);
 }
 
 // The position-only preparation of the mesh stage that can run beside the cell list and the CN

@@ -114,69 +114,56 @@ int scan_exclusive(const int* in, int n, int* out, cudaStream_t s) {
   return FD3_OK;
 }
 
-__global__ void __launch_bounds__(256) k_hist(const int* __restrict__ keys, int n, int* __restrict__ counts) {
+// Counting sort of the ids 0..n-1 by key, ids ascending within a key. The atomic that counts a key
+// also hands the id its arrival slot, so one scatter fills the segments in arrival order; the last
+// kernel then gives every id its final place by its rank in its segment (the number of smaller ids
+// there), which makes the order independent of the atomics. Its threads walk the segments in
+// position order, so the lanes of a warp scan the same few segments (broadcast loads): m compares
+// per id for a segment of m ids, all ids at once. (Sorting each segment in one warp, longer ones by
+// insertion in one lane, took 62 us at 12,000 HCNO atoms in 343 bins of 35; this takes 4 us.)
+__global__ void __launch_bounds__(256) k_key_slots(const int* __restrict__ keys, int n, int* __restrict__ counts,
+                                                  int* __restrict__ slot) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) atomicAdd(&counts[keys[i]], 1);
+  if (i < n) slot[i] = atomicAdd(&counts[keys[i]], 1);
 }
 
 __global__ void __launch_bounds__(256) k_scatter(const int* __restrict__ keys, int n, const int* __restrict__ starts,
-                          int* __restrict__ fill, int* __restrict__ order) {
+                                                const int* __restrict__ slot, int* __restrict__ arrival) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
-    const int k = keys[i];
-    order[starts[k] + atomicAdd(&fill[k], 1)] = i;
-  }
+  if (i < n) arrival[starts[keys[i]] + slot[i]] = i;
 }
 
-// Sort each key segment by atom id: makes the order (and every sum taken in that order)
-// independent of the atomic slot assignment above. One warp per segment: a segment of at most
-// 32 ids is ranked in registers (rank = number of smaller ids, the ids being distinct) and
-// written back in one step; a longer one is insertion-sorted by lane 0.
-__global__ void __launch_bounds__(256) k_sort_segments(const int* __restrict__ starts, int K, int* __restrict__ order) {
-  const int lane = threadIdx.x & 31;
-  const int k = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (k >= K) return;
-  const int a = starts[k], b = starts[k + 1], m = b - a;
-  if (m <= 1) return;
-  if (m <= 32) {
-    const int v = lane < m ? order[a + lane] : 0x7fffffff;
-    int rank = 0;
-#pragma unroll 8
-    for (int j = 0; j < 32; ++j) {
-      const int u = __shfl_sync(0xffffffffu, v, j);
-      rank += (j < m && u < v) ? 1 : 0;
-    }
-    __syncwarp();
-    if (lane < m) order[a + rank] = v;
-    return;
-  }
-  if (lane != 0) return;
-  for (int u = a + 1; u < b; ++u) {
-    const int v = order[u];
-    int w = u - 1;
-    while (w >= a && order[w] > v) {
-      order[w + 1] = order[w];
-      --w;
-    }
-    order[w + 1] = v;
-  }
+// Place of the id at position p of the arrival-ordered segments once its segment is sorted.
+__device__ __forceinline__ int ranked_place(const int* __restrict__ arrival, int id, int a, int b) {
+  int rank = 0;
+#pragma unroll 4
+  for (int q = a; q < b; ++q) rank += arrival[q] < id ? 1 : 0;
+  return a + rank;
 }
 
-int counting_sort(const int* keys, int n, int K, int* counts, int* starts, int* order, cudaStream_t s) {
-  const int tb = 256;
+__global__ void __launch_bounds__(256) k_rank_segments(const int* __restrict__ keys, int n,
+                                                      const int* __restrict__ starts,
+                                                      const int* __restrict__ arrival, int* __restrict__ order) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= n) return;
+  const int i = arrival[p], k = keys[i];
+  order[ranked_place(arrival, i, starts[k], starts[k + 1])] = i;
+}
+
+// arrival: scratch of n ints; order also holds the arrival slots until the last kernel writes it.
+int counting_sort(const int* keys, int n, int K, int* counts, int* starts, int* order, int* arrival,
+                  cudaStream_t s) {
+  const int tb = 256, nb = (n + tb - 1) / tb;
   FD3_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * K, s));
   if (n > 0) {
-    k_hist<<<(n + tb - 1) / tb, tb, 0, s>>>(keys, n, counts);
+    k_key_slots<<<nb, tb, 0, s>>>(keys, n, counts, order);
     FD3_LAUNCHED();
   }
   int rc = scan_exclusive(counts, K, starts, s);
-  if (rc) return rc;
-  FD3_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * K, s));
-  if (n > 0) {
-    k_scatter<<<(n + tb - 1) / tb, tb, 0, s>>>(keys, n, starts, counts, order);
-    FD3_LAUNCHED();
-  }
-  k_sort_segments<<<(K + tb / 32 - 1) / (tb / 32), tb, 0, s>>>(starts, K, order);
+  if (rc || n <= 0) return rc;
+  k_scatter<<<nb, tb, 0, s>>>(keys, n, starts, order, arrival);
+  FD3_LAUNCHED();
+  k_rank_segments<<<nb, tb, 0, s>>>(keys, n, starts, arrival, order);
   FD3_LAUNCHED();
   return FD3_OK;
 }
@@ -239,7 +226,8 @@ int build_cell_list(const CellGrid& g, int n, const double* pos_ang, const int32
     k_bin_atoms<<<(n + tb - 1) / tb, tb, 0, s>>>(to_dev(g), n, pos_ang, cl.bin_of, cl.off);
     FD3_LAUNCHED();
   }
-  int rc = counting_sort(cl.bin_of, n, K, cl.bin_count, cl.bin_start, cl.order, s);
+  // meta is written after the sort: until then it is the sort's scratch
+  int rc = counting_sort(cl.bin_of, n, K, cl.bin_count, cl.bin_start, cl.order, reinterpret_cast<int*>(cl.meta), s);
   if (rc) return rc;
   if (n > 0) {
     k_gather_sorted<<<(n + tb - 1) / tb, tb, 0, s>>>(n, cl.order, pos_ang, species, cl.off, cl.xs, cl.meta);
@@ -793,9 +781,9 @@ int launch_edge_index(int64_t n_edges, int n, const int64_t* src, const int64_t*
     k_edge_keys<<<(unsigned)((n_edges + tb - 1) / tb), tb, 0, s>>>(n_edges, n, src, dst, ei.ks, ei.kd, ei.bad);
     FD3_LAUNCHED();
   }
-  int rc = counting_sort(ei.ks, (int)n_edges, n, ei.cnt, ei.st_s, ei.ord_s, s);
+  int rc = counting_sort(ei.ks, (int)n_edges, n, ei.cnt, ei.st_s, ei.ord_s, ei.arrival, s);
   if (rc) return rc;
-  return counting_sort(ei.kd, (int)n_edges, n, ei.cnt, ei.st_d, ei.ord_d, s);
+  return counting_sort(ei.kd, (int)n_edges, n, ei.cnt, ei.st_d, ei.ord_d, ei.arrival, s);
 }
 
 // CN of atom a: the sum of the smooth-cutoff function over its source edges in edge order

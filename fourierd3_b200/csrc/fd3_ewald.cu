@@ -287,7 +287,7 @@ int launch_ewald(const EwaldGeom& eg, int n, const double* pos, double ps, const
   // species-sorted atom order
   k_species_keys<<<(n + tb - 1) / tb, tb, 0, s>>>(n, species, w.keys);
   FD3_LAUNCHED();
-  int rc = counting_sort(w.keys, n, e.S, w.counts, w.sp_start, w.order, s);
+  int rc = counting_sort(w.keys, n, e.S, w.counts, w.sp_start, w.order, reinterpret_cast<int*>(w.sp_of), s);
   if (rc) return rc;
   k_species_of_slot<<<(n + tb - 1) / tb, tb, 0, s>>>(n, w.order, species, w.sp_of);
   FD3_LAUNCHED();

@@ -53,8 +53,9 @@ struct CellList {
 };
 
 // counting sort of keys[N] in [0, K): out order sorted by key then by index.
-// counts[K] and starts[K+1] are workspace; counts must be zeroed by the caller.
-int counting_sort(const int* keys, int n, int K, int* counts, int* starts, int* order, cudaStream_t s);
+// counts[K], starts[K+1] and arrival[N] are workspace (counts is zeroed here).
+int counting_sort(const int* keys, int n, int K, int* counts, int* starts, int* order, int* arrival,
+                  cudaStream_t s);
 int scan_exclusive(const int* in, int n, int* out, cudaStream_t s);   // out[n] = total
 
 int build_cell_list(const CellGrid& g, int n, const double* pos_ang, const int32_t* species, CellList& cl,
@@ -102,6 +103,7 @@ int launch_direct_finalize(const double* pair_part, int n_pair, const double* ta
 struct EdgeIndex {
   int *ks, *kd;         // [E] source / destination keys
   int *ord_s, *ord_d;   // [E] edge ids by source / by destination
+  int* arrival;         // [E] counting-sort scratch
   int* cnt;             // [N] counting-sort scratch
   int *st_s, *st_d;     // [N+1] segment starts
   int* bad;             // [1] set when an edge index is outside 0..N-1
