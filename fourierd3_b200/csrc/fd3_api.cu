@@ -609,8 +609,9 @@ void carve(const fd3_plan* p, int64_t N, int64_t K_in, Carver& c, Work& w, int64
   const int64_t K = fused ? K_in : 1;
   const size_t es = p->precision == FD3_PREC_FP64 ? sizeof(double) : sizeof(float);
   const int R = p->R;
-  // per-block partials: per-atom kernels use ceil(N/8) blocks, the bin kernels one per bin
-  const int64_t nblk = (2 * ((N + 7) / 8) > K ? 2 * ((N + 7) / 8) : K) + 1;
+  // per-block partials: per-atom kernels use ceil(N/8) blocks, the CN kernel cn_max_blocks
+  const int64_t ncnb = cn_max_blocks(K);
+  const int64_t nblk = (2 * ((N + 7) / 8) > ncnb ? 2 * ((N + 7) / 8) : ncnb) + 1;
   w.ci = c.take<CellInfo>(1);
   w.cn = c.take<double>(N);
   w.c6 = c.take<double>(N * R);
@@ -656,7 +657,6 @@ void carve(const fd3_plan* p, int64_t N, int64_t K_in, Carver& c, Work& w, int64
   w.hits.j = c.take<int>(hn * kHitCap);
   w.hits.ad = c.take<char>(hn * kHitCap * 4 * es);
   w.hits.n = c.take<int>(N);
-  w.hits.ovf = c.take<int>(1);
   const size_t C = (size_t)p->S * p->R;
   w.rho = c.take<char>(mesh ? C * M * es : 1);
   // the mixed form's spectrum may carry one pad slot per ky row (16-byte rows for the fused
@@ -1055,19 +1055,18 @@ extern "C" int fd3_energy_forces_stress(fd3_plan* p, int64_t n_atoms, const doub
   FD3_TRY(build_cell_list(g, N, d_pos_ang, d_species, w.cl, s));
   prof_mark(p, s, "cell_list");
   int n_self = 0, n_kspc = 0, n_mcell = 0, n_cnv = 0;
-  FD3_TRY(launch_cn_c6_cells(g, N, w.cl, d_pos_ang, d_species, p->d_tab, p->d_eigvecs, p->R, w.cn, w.c6, w.dc6,
+  FD3_TRY(launch_cn_c6_cells(g, N, w.cl, d_species, p->d_tab, p->d_eigvecs, p->R, w.cn, w.c6, w.dc6,
                              w.self_part, &n_self, w.hits, s));
   prof_mark(p, s, "cn_c6");
   if (fork) FD3_CUDA(cudaStreamWaitEvent(s, p->ev_join, 0));
   // the mesh gradient (Hartree/Bohr) is staged in d_forces, then finished by the CN adjoint
   FD3_TRY(run_mesh(p, N, d_pos_ang, kAngToBohr, d_species, w, true, d_forces, nullptr, &n_kspc, &n_mcell, s,
                    fork, fork));
-  FD3_TRY(launch_cn_adjoint_cells(g, N, w.cl, d_pos_ang, d_species, p->d_tab, w.gcn, d_forces,
+  FD3_TRY(launch_cn_adjoint_cells(g, N, w.cl, p->d_tab, w.ci, w.gcn, d_forces,
                                   -kHartreeToEv * kAngToBohr, w.cnv_part, &n_cnv, w.hits, s));
   prof_mark(p, s, "cn_adjoint");
   Partials pa{w.self_part, n_self, w.kspc_part, n_kspc, w.cnv_part, n_cnv, nullptr, 0};
   FD3_TRY(launch_finalize(pa, w.ci, 1, kHartreeToEv, d_energy, d_stress, s));
-  FD3_TRY(launch_poison_if_stale(w.ci, N, d_energy, d_forces, d_stress, s));
   prof_mark(p, s, "finalize");
   return FD3_OK;
 }
@@ -1155,7 +1154,7 @@ extern "C" int fd3_direct_energy_forces_stress(fd3_plan* p, int64_t n_atoms, con
   FD3_TRY(launch_cellinfo(d_cell_ang, kAngToBohr, w.ci, s, h_cell_ang));
   FD3_TRY(build_cell_list(g, N, d_pos_ang, d_species, w.cl, s));
   int n_self = 0, n_pair = 0, n_cnv = 0;
-  FD3_TRY(launch_cn_c6_cells(g, N, w.cl, d_pos_ang, d_species, p->d_tab, p->d_eigvecs, p->R, w.cn, w.c6, w.dc6,
+  FD3_TRY(launch_cn_c6_cells(g, N, w.cl, d_species, p->d_tab, p->d_eigvecs, p->R, w.cn, w.c6, w.dc6,
                              w.self_part, &n_self, w.hits, s));
   FD3_TRY(build_cell_list(g2, N, d_pos_ang, d_species, d.cl, s));
   // pair gradient (Hartree/Bohr) staged in d_forces, finished by the CN adjoint
@@ -1164,7 +1163,7 @@ extern "C" int fd3_direct_energy_forces_stress(fd3_plan* p, int64_t n_atoms, con
   FD3_TRY(launch_direct_tail_gcn(N, d_species, w.c6, w.dc6, d.dEdc, p->d_tab, p->d_green, p->S, p->R,
                                  r_direct_ang * kAngToBohr, w.ci, d.sp_part, kDirSpBlocks, d.A, d.tail, d.scratch,
                                  w.gcn, s));
-  FD3_TRY(launch_cn_adjoint_cells(g, N, w.cl, d_pos_ang, d_species, p->d_tab, w.gcn, d_forces,
+  FD3_TRY(launch_cn_adjoint_cells(g, N, w.cl, p->d_tab, w.ci, w.gcn, d_forces,
                                   -kHartreeToEv * kAngToBohr, w.cnv_part, &n_cnv, w.hits, s));
   FD3_TRY(launch_direct_finalize(d.pair_part, n_pair, d.tail, w.cnv_part, n_cnv, w.ci, d_energy, d_stress, s));
   FD3_TRY(launch_poison_if_stale(w.ci, N, d_energy, d_forces, d_stress, s));

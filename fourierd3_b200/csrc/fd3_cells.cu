@@ -301,7 +301,7 @@ constexpr int kWarpsPerBlock = 8;
 
 // Per-atom traversal straight from global memory: the path for bins whose neighbourhood does not
 // fit the shared-memory stage (dense clusters, cells much narrower than the cutoff).
-__device__ __forceinline__ double cn_atom_global(const GridDev& g, const int* __restrict__ bin_start,
+__device__ __noinline__ double cn_atom_global(const GridDev& g, const int* __restrict__ bin_start,
                                                  const double4* __restrict__ xs, const int4* __restrict__ meta,
                                                  const int4* __restrict__ off, const Tables* __restrict__ tab,
                                                  int t) {
@@ -321,16 +321,21 @@ __device__ __forceinline__ double cn_atom_global(const GridDev& g, const int* __
   return warp_sum(acc);
 }
 
-__device__ __forceinline__ void cn_adjoint_atom_global(const GridDev& g, const int* __restrict__ bin_start,
-                                                       const double4* __restrict__ xs,
-                                                       const int4* __restrict__ meta, const int4* __restrict__ off,
-                                                       const Tables* __restrict__ tab, const double* __restrict__ gcn,
-                                                       int t, double* f, double* v) {
+// Sums of one atom's pairs, this lane's share: the CN force and the six virial components.
+struct PairSums {
+  double f0, f1, f2, xx, xy, xz, yy, yz, zz;
+};
+__device__ __noinline__ PairSums cn_adjoint_atom_global(const GridDev& g, const int* __restrict__ bin_start,
+                                                        const double4* __restrict__ xs,
+                                                        const int4* __restrict__ meta, const int4* __restrict__ off,
+                                                        const Tables* __restrict__ tab, const double* __restrict__ gcn,
+                                                        int t) {
   const double4 xi = xs[t];
   const int i = meta[t].w;
   const int4 offi = off[i];
   const double rci = tab->rcov[(int)xi.w];
   const double gi = gcn[i];
+  PairSums p{0, 0, 0, 0, 0, 0, 0, 0, 0};
   visit_neighbors(g, bin_start, xs, meta, i, xi.x, xi.y, xi.z, offi,
                   [&](bool hit, int u, int j, int, int, int, double d0, double d1, double d2) {
                     if (!hit) return;
@@ -341,55 +346,40 @@ __device__ __forceinline__ void cn_adjoint_atom_global(const GridDev& g, const i
                     if (r > 1e-6) {
                       const double a = df / r;
                       const double w = (gi + gcn[j]) * a;
-                      f[0] -= w * v0;
-                      f[1] -= w * v1;
-                      f[2] -= w * v2;
+                      p.f0 -= w * v0;
+                      p.f1 -= w * v1;
+                      p.f2 -= w * v2;
                       const double b = gi * a;
-                      v[0] += b * v0 * v0; v[1] += b * v0 * v1; v[2] += b * v0 * v2;
-                      v[4] += b * v1 * v1; v[5] += b * v1 * v2; v[8] += b * v2 * v2;
+                      p.xx += b * v0 * v0; p.xy += b * v0 * v1; p.xz += b * v0 * v2;
+                      p.yy += b * v1 * v1; p.yz += b * v1 * v2; p.zz += b * v2 * v2;
                     }
                   });
+  return p;
 }
 
 // ------------------------------------------------------------------ bin-staged CN
-// One CTA per bin: the atoms of the (2 reach + 1)^3 neighbour bins are staged once in shared
-// memory as image positions p_j = x_j + (S' - off_j) . cell, and the warps of the CTA run the
-// bin's own atoms against that stage (d = p_j - (x_i - off_i . cell)). The same stage and the
-// same arithmetic serve the CN and its adjoint, so both see the same pairs.
-constexpr int kBinCap = 768;
+// The candidates of a bin are the atoms of its (2 reach + 1)^3 neighbour bins, numbered through the
+// neighbour bins in a fixed order. A CTA stages up to `cap` of them at a time in shared memory as
+// image positions p_j = x_j + (S' - off_j) . cell, and its warps run the bin's own atoms against
+// that stage (d = p_j - (x_i - off_i . cell)).
 constexpr int kMaxNbrBins = 343;
 
 // P4 = double4: absolute image positions (the plain form, and the exact pair predicate);
 // P4 = float4 (mixed form): positions relative to the bin's own corner, so that float keeps
 // ~1e-6 A over the few bins a stage spans.
-template <typename P4>
-struct BinStage {
-  P4 p[kBinCap];   // image position (A), species in .w
-  int j[kBinCap];
+struct NbrBins {
   int a0[kMaxNbrBins];
   int pref[kMaxNbrBins + 1];
   int img[kMaxNbrBins][3];
 };
 
-// Returns the number of staged candidates, or -1 when the neighbourhood does not fit; org is the
-// origin subtracted from the staged positions (zero for double4).
-// rcov: when given, the staged w component is the candidate's covalent radius rcov[species]
-// (the CN kernel's only use of the species) instead of the species index.
-template <typename P4>
-__device__ int stage_bin(const GridDev& g, int b, const int* __restrict__ bin_start,
-                         const double4* __restrict__ xs, const int4* __restrict__ meta, BinStage<P4>& st,
-                         double* __restrict__ s_g, const double* __restrict__ gcn, double (&org)[3],
-                         const double* __restrict__ rcov = nullptr) {
+// Table of the neighbour bins of bin b. Returns the number of candidates, or -1 when the
+// neighbourhood has more than kMaxNbrBins bins (a cell much narrower than the cutoff).
+__device__ __forceinline__ int nbr_bins(const GridDev& g, int b, const int* __restrict__ bin_start, NbrBins& st) {
   const int nx = 2 * g.reach[0] + 1, ny = 2 * g.reach[1] + 1, nz = 2 * g.reach[2] + 1;
   const int nnb = nx * ny * nz;
   if (nnb > kMaxNbrBins) return -1;
   const int bz = b % g.nb[2], by = (b / g.nb[2]) % g.nb[1], bx = b / (g.nb[2] * g.nb[1]);
-#pragma unroll
-  for (int c = 0; c < 3; ++c)
-    org[c] = sizeof(P4) == sizeof(double4)
-                 ? 0.0
-                 : ((double)bx / g.nb[0]) * g.cell[c] + ((double)by / g.nb[1]) * g.cell[3 + c] +
-                       ((double)bz / g.nb[2]) * g.cell[6 + c];
   for (int e = threadIdx.x; e < nnb; e += blockDim.x) {
     const int dz = e % nz - g.reach[2], dy = (e / nz) % ny - g.reach[1], dx = e / (nz * ny) - g.reach[0];
     const int cx = bx + dx, cy = by + dy, cz = bz + dz;
@@ -403,25 +393,35 @@ __device__ int stage_bin(const GridDev& g, int b, const int* __restrict__ bin_st
     st.img[e][2] = sz;
   }
   __syncthreads();
-  if (nnb <= 32) {   // one warp scans the bin sizes (27 bins at reach 1)
-    if (threadIdx.x < 32) {
-      int v = threadIdx.x < nnb ? st.pref[threadIdx.x + 1] : 0;
+  if (threadIdx.x < 32) {   // one warp scans the bin sizes (27 bins at reach 1: one round)
+    int carry = 0;
+    for (int e0 = 0; e0 < nnb; e0 += 32) {
+      const int e = e0 + (int)threadIdx.x;
+      int v = e < nnb ? st.pref[e + 1] : 0;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const int u = __shfl_up_sync(0xffffffffu, v, o);
         if ((int)threadIdx.x >= o) v += u;
       }
-      if ((int)threadIdx.x < nnb) st.pref[threadIdx.x + 1] = v;
-      if (threadIdx.x == 0) st.pref[0] = 0;
+      v += carry;
+      if (e < nnb) st.pref[e + 1] = v;
+      carry = __shfl_sync(0xffffffffu, v, 31);
     }
-  } else if (threadIdx.x == 0) {
-    st.pref[0] = 0;
-    for (int e = 0; e < nnb; ++e) st.pref[e + 1] += st.pref[e];
+    if (threadIdx.x == 0) st.pref[0] = 0;
   }
   __syncthreads();
-  const int total = st.pref[nnb];
-  if (total > kBinCap) return -1;
-  for (int c = threadIdx.x; c < total; c += blockDim.x) {
+  return st.pref[nnb];
+}
+
+// Stage candidates [c0, c1); org is subtracted from the staged positions (zero for double4). The
+// staged w component is the candidate's covalent radius (the CN's only use of the species).
+template <typename P4>
+__device__ __forceinline__ void stage_candidates(const GridDev& g, const NbrBins& st, int c0, int c1,
+                                                 const double4* __restrict__ xs, const int4* __restrict__ meta,
+                                                 const double (&org)[3], const double* __restrict__ rcov, P4* p,
+                                                 int* j) {
+  const int nnb = (2 * g.reach[0] + 1) * (2 * g.reach[1] + 1) * (2 * g.reach[2] + 1);
+  for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
     int lo = 0, hi = nnb - 1;          // last entry with pref[e] <= c
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
@@ -434,16 +434,13 @@ __device__ int stage_bin(const GridDev& g, int b, const int* __restrict__ bin_st
     const double px = xj.x + S0 * g.cell[0] + S1 * g.cell[3] + S2 * g.cell[6];
     const double py = xj.y + S0 * g.cell[1] + S1 * g.cell[4] + S2 * g.cell[7];
     const double pz = xj.z + S0 * g.cell[2] + S1 * g.cell[5] + S2 * g.cell[8];
-    const double wv = rcov ? rcov[(int)xj.w] : xj.w;
+    const double wv = rcov[(int)xj.w];
     if constexpr (sizeof(P4) == sizeof(double4))
-      st.p[c] = make_double4(px, py, pz, wv);
+      p[c - c0] = make_double4(px, py, pz, wv);
     else
-      st.p[c] = make_float4((float)(px - org[0]), (float)(py - org[1]), (float)(pz - org[2]), (float)wv);
-    st.j[c] = mj.w;
-    if (s_g) s_g[c] = gcn[mj.w];
+      p[c - c0] = make_float4((float)(px - org[0]), (float)(py - org[1]), (float)(pz - org[2]), (float)wv);
+    j[c - c0] = mj.w;
   }
-  __syncthreads();
-  return total;
 }
 
 __device__ __forceinline__ void wrapped_pos(const GridDev& g, double4 x, int4 m, double& w0, double& w1,
@@ -470,9 +467,62 @@ struct HitList {
   int cap;
 };
 
-// CN of the atoms of one bin from the shared-memory stage (raw CN, before cncorr), plus the
-// pair records. Bins whose neighbourhood does not fit the stage mark their atoms n = -2 and
-// leave them to k_cn_global.
+// C6 weights and factors of one atom by a group of 8 lanes: softmax interpolation over the 7
+// reference CNs (one lane each), the rank-r factors c_r = sum_p w_p V[s, p, r] (core.py:449-478,
+// 525-532; ranks over the lanes), their CN derivative (times the cncorr slope) and the self term
+// sum_r lambda_r c_r^2 phi_ss(0) (core.py:545-550), of which each lane returns its ranks' share.
+// raw_cn is the CN before cncorr; cn receives the corrected one. Every lane of the warp takes part
+// (`on` false: an idle group). Eight lanes per atom: a thread per atom is a chain of seven float64
+// exponentials (6 us at any size), a warp per atom repeats the work 32-fold (+60 us at 139,968 atoms).
+__device__ __forceinline__ double c6_group(bool on, int i, int s, double raw_cn, const Tables* __restrict__ tab,
+                                           const double* __restrict__ V, int R, double* __restrict__ cn,
+                                           double* __restrict__ c6, double* __restrict__ dc6) {
+  const int lane = threadIdx.x & 7;
+  double cnv = raw_cn, slope = 1.0;
+  if (tab->has_cncorr) {
+    slope = tab->cncorr[2 * s + 1];
+    cnv = slope * cnv + tab->cncorr[2 * s + 0];
+  }
+  const double ref = lane < 7 ? tab->cnref[7 * s + lane] : -1.0;
+  const bool ok = ref != -1.0;
+  const double diff = cnv - ref;
+  double lg = ok ? -4.0 * (diff * diff) : -INFINITY;
+  const double dl = ok ? -8.0 * diff : 0.0;
+  double mx = lg;
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  lg = lg == -INFINITY ? 0.0 : exp(lg - mx);
+  double sum = lg;
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  const double w = lg * (1.0 / sum);   // softmax weight (0 in lane 7)
+  double dlbar = w * dl;
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) dlbar += __shfl_xor_sync(0xffffffffu, dlbar, o);
+  const double wd = w * (dl - dlbar);
+  double selfv = 0.0;
+  for (int r0 = 0; r0 < R; r0 += 8) {
+    const int r = r0 + lane;
+    double c = 0.0, d = 0.0;
+#pragma unroll
+    for (int p = 0; p < 7; ++p) {
+      const double wp = __shfl_sync(0xffffffffu, w, p, 8), wdp = __shfl_sync(0xffffffffu, wd, p, 8);
+      const double v = r < R ? V[(7 * s + p) * R + r] : 0.0;
+      c += wp * v;
+      d += wdp * v;
+    }
+    if (on && r < R) {
+      c6[(size_t)i * R + r] = c;
+      dc6[(size_t)i * R + r] = slope * d;
+      selfv += tab->eigs[r] * c * c * tab->selfcont[s];
+    }
+  }
+  if (on && lane == 0) cn[i] = cnv;
+  return selfv;
+}
+
+// CN and C6 factors of the atoms of one bin (split over nsplit CTAs when there are few bins), plus
+// the pair records.
 // Per atom (one warp) the staged candidates are first tested against the cutoff 32 at a time
 // (float64 distances in the plain form, float relative to the bin corner in the mixed form); the
 // indices of the pairs inside are compacted in order into a per-warp ring of 64, and whenever 32
@@ -480,17 +530,24 @@ struct HitList {
 // instead of on the ~15 % of lanes that hit in a given candidate batch.
 // A bin holds ~15 atoms at r_cut 6 A (SiO2 density): 4 warps per CTA leave fewer idle warps
 // waiting for a bin's last atom than 8 do, and more CTAs (bins) fit per SM.
+// The stage holds what the box's mean density fills, with half as much again; a bin with more candidates (a
+// dense cluster, or a tiny cell whose images are all candidates) restages them in pieces of `cap`
+// for each round of its warps. (With one fixed stage of 768 and a per-atom traversal of global
+// memory beyond it, every bin of an HCNO box, 936 candidates, took the traversal: CN 97 us and
+// adjoint 178 us at 12,000 atoms.)
 constexpr int kCnRing = 64;
 constexpr int kCnWarps = 4;
+constexpr int kCnSmem = 56 * 1024;   // stage bytes at most: three CTAs per SM (1,593 candidates in float64)
+constexpr int kCnSmemPlain = 38 * 1024;   // ... without the shared-memory opt-in (8 KB are static)
 
 template <typename TC> struct StagePos { using type = double4; };
 template <> struct StagePos<float> { using type = float4; };
 
-template <typename TE, typename TC>
-__device__ __forceinline__ void cn_hit(const BinStage<typename StagePos<TC>::type>& st, int c, TC w0, TC w1, TC w2,
-                                       TC rci, TC rc, const Tables* __restrict__ tab, HitList<TE>& hl, size_t hb,
-                                       int h, TC& acc) {
-  const auto pj = st.p[c];
+template <typename TE, typename TC, typename P4>
+__device__ __forceinline__ void cn_hit(const P4* __restrict__ sp, const int* __restrict__ sj, int c, TC w0, TC w1,
+                                       TC w2, TC rci, TC rc, const HitList<TE>& hl, size_t hb, int h,
+                                       TC& acc) {
+  const P4 pj = sp[c];
   const TC v0 = (TC)((pj.x - w0) * (TC)kAngToBohr);
   const TC v1 = (TC)((pj.y - w1) * (TC)kAngToBohr);
   const TC v2 = (TC)((pj.z - w2) * (TC)kAngToBohr);
@@ -501,133 +558,239 @@ __device__ __forceinline__ void cn_hit(const BinStage<typename StagePos<TC>::typ
     acc += f;
   }
   if (h < hl.cap) {
-    hl.j[hb + h] = st.j[c];
+    hl.j[hb + h] = sj[c];
     hl.ad[hb + h] = typename Vec4<TE>::type{(TE)a, (TE)v0, (TE)v1, (TE)v2};
   }
 }
 
-template <typename TE, typename TC>
-__global__ void __launch_bounds__(32 * kCnWarps) k_cn_bins(GridDev g, const int* __restrict__ bin_start,
-                                                const double4* __restrict__ xs, const int4* __restrict__ meta,
-                                                const Tables* __restrict__ tab, double* __restrict__ cn,
-                                                HitList<TE> hl, int* __restrict__ ovf) {
+// The atoms of bin b that this CTA takes (part of nsplit), in arithmetic TC: raw CN to cn[], records.
+// ONCE: the candidates fit the stage.
+template <typename TE, typename TC, bool ONCE>
+__device__ __forceinline__ void cn_bin(const GridDev& g, const NbrBins& st, int total, int cap, int b, int s0, int s1,
+                                       int part, int nsplit, const double4* __restrict__ xs,
+                                       const int4* __restrict__ meta, const Tables* __restrict__ tab,
+                                       double* __restrict__ cn, const HitList<TE>& hl, unsigned char* stage,
+                                       int* __restrict__ rg) {
   using P4 = typename StagePos<TC>::type;
-  __shared__ BinStage<P4> st;
-  __shared__ int ring[kCnWarps][kCnRing];
+  P4* sp = reinterpret_cast<P4*>(stage);
+  int* sj = reinterpret_cast<int*>(sp + cap);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int b = blockIdx.x;
+  const int bz = b % g.nb[2], by = (b / g.nb[2]) % g.nb[1], bx = b / (g.nb[2] * g.nb[1]);
   double org[3];
-  const int total = stage_bin<P4>(g, b, bin_start, xs, meta, st, nullptr, nullptr, org, tab->rcov);
-  const int s0 = bin_start[b], s1 = bin_start[b + 1];
-  if (total < 0) {
-    for (int t = s0 + threadIdx.x; t < s1; t += blockDim.x) hl.n[t] = -2;
-    if (threadIdx.x == 0 && s1 > s0) atomicAdd(ovf, 1);
-    return;
-  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+    org[c] = sizeof(P4) == sizeof(double4)
+                 ? 0.0
+                 : ((double)bx / g.nb[0]) * g.cell[c] + ((double)by / g.nb[1]) * g.cell[3 + c] +
+                       ((double)bz / g.nb[2]) * g.cell[6 + c];
   const unsigned lt = (1u << lane) - 1u;
   const TC rc = (TC)tab->r_cut;
   const TC rc2 = (TC)g.rc2;
-  int* rg = ring[wid];
-  for (int t = s0 + wid; t < s1; t += kCnWarps) {
-    const double4 xi = xs[t];
-    const int4 mi = meta[t];
-    double wd0, wd1, wd2;
-    wrapped_pos(g, xi, mi, wd0, wd1, wd2);
+  if (ONCE) {
+    stage_candidates<P4>(g, st, 0, total, xs, meta, org, tab->rcov, sp, sj);
+    __syncthreads();
+  }
+  // rounds of one atom per warp (the same number for every warp where restaging takes barriers)
+  for (int t0 = s0 + part * kCnWarps; t0 < s1; t0 += kCnWarps * nsplit) {
+    const int t = t0 + wid;
+    const bool on = t < s1;
+    if (ONCE && !on) break;
+    double wd0 = 0, wd1 = 0, wd2 = 0;
+    int i = 0, s = 0;
+    if (on) {
+      const double4 xi = xs[t];
+      const int4 mi = meta[t];
+      wrapped_pos(g, xi, mi, wd0, wd1, wd2);
+      i = mi.w;
+      s = (int)xi.w;
+    }
     const TC w0 = (TC)(wd0 - org[0]), w1 = (TC)(wd1 - org[1]), w2 = (TC)(wd2 - org[2]);
-    const TC rci = (TC)tab->rcov[(int)xi.w];
+    const TC rci = (TC)tab->rcov[s];
     TC acc = TC(0);
     int produced = 0, consumed = 0;
     const size_t hb = (size_t)t * hl.cap;
-    for (int c0 = 0; c0 < total; c0 += 32) {
-      const int c = c0 + lane;
-      bool hit = false;
-      if (c < total) {
-        const P4 pj = st.p[c];
-        const TC d0 = pj.x - w0, d1 = pj.y - w1, d2 = pj.z - w2;
-        hit = d0 * d0 + d1 * d1 + d2 * d2 < rc2;
+    for (int cb = 0; cb < (ONCE ? 1 : total); cb += cap) {
+      const int cnt = ONCE || total - cb < cap ? total - cb : cap;
+      if (!ONCE) {
+        __syncthreads();   // every warp has finished with the previous piece
+        stage_candidates<P4>(g, st, cb, cb + cnt, xs, meta, org, tab->rcov, sp, sj);
+        __syncthreads();
+        if (!on) continue;
       }
-      const unsigned m = __ballot_sync(0xffffffffu, hit);
-      if (hit) rg[(produced + __popc(m & lt)) & (kCnRing - 1)] = c;
-      produced += __popc(m);
-      __syncwarp();
-      if (produced - consumed >= 32) {
-        const int h = consumed + lane;
-        cn_hit<TE, TC>(st, rg[h & (kCnRing - 1)], w0, w1, w2, rci, rc, tab, hl, hb, h, acc);
-        consumed += 32;
+      for (int c0 = 0; c0 < cnt; c0 += 32) {
+        const int c = c0 + lane;
+        bool hit = false;
+        if (c < cnt) {
+          const P4 pj = sp[c];
+          const TC d0 = pj.x - w0, d1 = pj.y - w1, d2 = pj.z - w2;
+          hit = d0 * d0 + d1 * d1 + d2 * d2 < rc2;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, hit);
+        if (hit) rg[(produced + __popc(m & lt)) & (kCnRing - 1)] = c;
+        produced += __popc(m);
         __syncwarp();
+        if (produced - consumed >= 32) {
+          const int h = consumed + lane;
+          cn_hit<TE, TC>(sp, sj, rg[h & (kCnRing - 1)], w0, w1, w2, rci, rc, hl, hb, h, acc);
+          consumed += 32;
+          __syncwarp();
+        }
       }
+      // the ring holds indices into this piece: take the rest of it before the next
+      if (consumed + lane < produced) {
+        const int h = consumed + lane;
+        cn_hit<TE, TC>(sp, sj, rg[h & (kCnRing - 1)], w0, w1, w2, rci, rc, hl, hb, h, acc);
+      }
+      consumed = produced;
+      __syncwarp();
     }
-    if (consumed + lane < produced) {
-      const int h = consumed + lane;
-      cn_hit<TE, TC>(st, rg[h & (kCnRing - 1)], w0, w1, w2, rci, rc, tab, hl, hb, h, acc);
-    }
-    __syncwarp();
     const double cnv = warp_sum((double)acc);
-    if (lane == 0) {
+    if (on && lane == 0) {
       hl.n[t] = produced <= hl.cap ? produced : -1;
-      if (produced > hl.cap) atomicAdd(ovf, 1);
-      cn[mi.w] = cnv;
+      cn[i] = cnv;
     }
   }
 }
 
-constexpr int kFallbackBlocks = 148 * 4;
+// The mixed form (TE = float) takes bins of up to kCnFloat candidates in float and denser ones in
+// float64, so that the sums over more pairs keep the accuracy of the smaller ones.
+constexpr int kCnFloat = 768;
 
-// Raw CN of atoms whose bin overflowed the stage, straight from the cell list in global memory.
-// Returns at once when no bin overflowed (the counter is zero).
-__global__ void __launch_bounds__(256) k_cn_global(GridDev g, int n, const int* __restrict__ bin_start,
-                                                  const double4* __restrict__ xs, const int4* __restrict__ meta,
-                                                  const int4* __restrict__ off, const Tables* __restrict__ tab,
-                                                  double* __restrict__ cn, int* __restrict__ hit_n,
-                                                  const int* __restrict__ ovf) {
-  if (*ovf == 0) return;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int t = blockIdx.x * kWarpsPerBlock + wid; t < n; t += gridDim.x * kWarpsPerBlock) {
-    if (hit_n[t] != -2) continue;
-    const double v = cn_atom_global(g, bin_start, xs, meta, off, tab, t);
-    if (lane == 0) {
-      cn[meta[t].w] = v;
-      hit_n[t] = -1;
-    }
-  }
-}
-
-int launch_cn_c6_cells(const CellGrid& g, int n, const CellList& cl, const double* pos_ang,
-                       const int32_t* species, const Tables* tab, const double* eigvecs, int R, double* cn,
-                       double* c6, double* dc6, double* self_part, int* n_self_blocks, const HitStore& hs,
-                       cudaStream_t s) {
-  (void)pos_ang;
-  const int K = g.nb[0] * g.nb[1] * g.nb[2];
-  FD3_CUDA(cudaMemsetAsync(hs.ovf, 0, sizeof(int), s));
-  if (hs.is_double)
-    k_cn_bins<double, double><<<K, 32 * kCnWarps, 0, s>>>(
-        to_dev(g), cl.bin_start, cl.xs, cl.meta, tab, cn,
-        HitList<double>{hs.j, (double4*)hs.ad, hs.n, hs.cap}, hs.ovf);
+// The other cases, out of line so that the common one keeps its registers (nine CTAs per SM in float):
+// a bin whose candidates do not fit the stage, and the dense bins of the mixed form.
+template <typename TE>
+__device__ __noinline__ void cn_bin_dense(const GridDev& g, const NbrBins& st, int total, int stage_bytes, int b,
+                                          int s0, int s1, int part, int nsplit, const double4* __restrict__ xs,
+                                          const int4* __restrict__ meta, const Tables* __restrict__ tab,
+                                          double* __restrict__ cn, const HitList<TE>& hl, unsigned char* stage,
+                                          int* __restrict__ rg) {
+  if (sizeof(TE) == 4 && total <= kCnFloat)
+    cn_bin<TE, float, false>(g, st, total, stage_bytes / 20, b, s0, s1, part, nsplit, xs, meta, tab, cn, hl, stage,
+                             rg);
+  else if (sizeof(TE) == 4 && total <= stage_bytes / 36)
+    cn_bin<TE, double, true>(g, st, total, stage_bytes / 36, b, s0, s1, part, nsplit, xs, meta, tab, cn, hl, stage,
+                             rg);
   else
-    k_cn_bins<float, float><<<K, 32 * kCnWarps, 0, s>>>(
-        to_dev(g), cl.bin_start, cl.xs, cl.meta, tab, cn,
-        HitList<float>{hs.j, (float4*)hs.ad, hs.n, hs.cap}, hs.ovf);
-  FD3_LAUNCHED();
-  const int blocks = (n + kWarpsPerBlock - 1) / kWarpsPerBlock;
-  if (blocks > 0) {
-    const int fb = blocks < kFallbackBlocks ? blocks : kFallbackBlocks;
-    k_cn_global<<<fb, 32 * kWarpsPerBlock, 0, s>>>(to_dev(g), n, cl.bin_start, cl.xs, cl.meta, cl.off, tab, cn,
-                                                    hs.n, hs.ovf);
-    FD3_LAUNCHED();
+    cn_bin<TE, double, false>(g, st, total, stage_bytes / 36, b, s0, s1, part, nsplit, xs, meta, tab, cn, hl, stage,
+                              rg);
+}
+
+// C6: the factors too (c6_group, after the CTA's atoms); without it k_c6_atoms follows.
+template <typename TE, bool C6>
+__global__ void __launch_bounds__(32 * kCnWarps, sizeof(TE) == 4 ? 9 : 7) k_cn_bins(
+                                                const __grid_constant__ GridDev g, int stage_bytes,
+                                                int nsplit, const int* __restrict__ bin_start,
+                                                const double4* __restrict__ xs, const int4* __restrict__ meta,
+                                                const int4* __restrict__ off, const Tables* __restrict__ tab,
+                                                const double* __restrict__ V, int R, double* __restrict__ cn,
+                                                double* __restrict__ c6, double* __restrict__ dc6,
+                                                const __grid_constant__ HitList<TE> hl,
+                                                double* __restrict__ self_part) {
+  extern __shared__ __align__(16) unsigned char cn_raw[];
+  __shared__ NbrBins st;
+  __shared__ int ring[kCnWarps][kCnRing];
+  const int b = blockIdx.x / nsplit, part = blockIdx.x - b * nsplit;
+  const int s0 = bin_start[b], s1 = bin_start[b + 1];
+  double self[1] = {0.0};
+  if (s0 + part * kCnWarps < s1) {
+    int* rg = ring[threadIdx.x >> 5];
+    const int total = nbr_bins(g, b, bin_start, st);
+    if (total < 0) {
+      for (int t = s0 + part * kCnWarps + (threadIdx.x >> 5); t < s1; t += kCnWarps * nsplit) {
+        const double cnv = cn_atom_global(g, bin_start, xs, meta, off, tab, t);
+        if ((threadIdx.x & 31) == 0) {
+          hl.n[t] = -1;
+          cn[meta[t].w] = cnv;
+        }
+      }
+    } else {
+      constexpr int each = sizeof(TE) == 4 ? 20 : 36;   // staged bytes per candidate
+      if (total <= stage_bytes / each && (sizeof(TE) == 8 || total <= kCnFloat))
+        cn_bin<TE, TE, true>(g, st, total, stage_bytes / each, b, s0, s1, part, nsplit, xs, meta, tab, cn, hl, cn_raw,
+                             rg);
+      else
+        cn_bin_dense<TE>(g, st, total, stage_bytes, b, s0, s1, part, nsplit, xs, meta, tab, cn, hl, cn_raw, rg);
+    }
+    if constexpr (C6) {
+    __syncthreads();   // the raw CNs are written
+    constexpr int kGroups = 4 * kCnWarps;
+    const int grp = threadIdx.x >> 3;
+    const int rounds = (s1 - s0 - part * kCnWarps + kCnWarps * nsplit - 1) / (kCnWarps * nsplit);
+    for (int a0 = 0; a0 < rounds * kCnWarps; a0 += kGroups) {
+      const int a = a0 + grp;   // atom a of this CTA: warp a mod kCnWarps of round a / kCnWarps
+      const int t = s0 + part * kCnWarps + a / kCnWarps * (kCnWarps * nsplit) + a % kCnWarps;
+      const bool on = a < rounds * kCnWarps && t < s1;
+      const int i = on ? meta[t].w : 0, s = on ? (int)xs[t].w : 0;
+      self[0] += c6_group(on, i, s, on ? cn[i] : 0.0, tab, V, R, cn, c6, dc6);
+    }
+    }
   }
+  if constexpr (C6) block_sum_store<1>(self, self_part + blockIdx.x);
+}
+
+int64_t cn_max_blocks(int64_t bins) { return 4 * 148 + bins; }   // bins * ceil(4 * 148 / bins) at most
+
+int launch_cn_c6_cells(const CellGrid& g, int n, const CellList& cl, const int32_t* species, const Tables* tab,
+                       const double* eigvecs, int R, double* cn, double* c6, double* dc6, double* self_part, int* n_self_blocks,
+                       const HitStore& hs, cudaStream_t s) {
+  const int K = g.nb[0] * g.nb[1] * g.nb[2];
+  // stage: the mean number of candidates and half as much again, within kCnSmem
+  const double mean = (double)n / K * (2 * g.reach[0] + 1) * (2 * g.reach[1] + 1) * (2 * g.reach[2] + 1);
+  const double want = 1.5 * mean + 64;
+  const int each = !hs.is_double && mean + 32 <= kCnFloat ? 20 : 36;   // float4 or double4, and the id
+  int stage = want * each < kCnSmem ? ((int)want + 3) / 4 * 4 * each : kCnSmem / (4 * each) * (4 * each);
+  if (!hs.is_double && each == 20 && stage > kCnFloat * 20) stage = kCnFloat * 20;
+  // few bins: several CTAs share a bin's atoms (each stages the candidates) until the chip has four
+  // CTAs per SM or every warp one atom. 27 bins of 24 atoms (648 SiO2 atoms, float64): 40 -> 9 us.
+  const int per_bin = (n + K - 1) / K;
+  int nsplit = (4 * 148 + K - 1) / K;
+  const int most = (per_bin + kCnWarps - 1) / kCnWarps;
+  if (nsplit > most) nsplit = most;
+  if (nsplit < 1) nsplit = 1;
+  const int grid = K * nsplit;
+  // Where the bins alone fill the chip, the factors take a kernel of their own (8 us): the CN kernel
+  // runs more CTAs per SM without them (139,968 atoms, mixed, both: 226 us with, 189 us without).
+  const bool with_c6 = nsplit > 1 || K < 4 * 148;
+  auto launch = [&](auto kern, auto hl) -> int {
+    if (stage > kCnSmemPlain)
+      FD3_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kCnSmem));
+    kern<<<grid, 32 * kCnWarps, stage, s>>>(to_dev(g), stage, nsplit, cl.bin_start, cl.xs, cl.meta, cl.off, tab,
+                                            eigvecs, R, cn, c6, dc6, hl, self_part);
+    FD3_LAUNCHED();
+    return FD3_OK;
+  };
+  int rc;
+  if (hs.is_double) {
+    const HitList<double> hl{hs.j, (double4*)hs.ad, hs.n, hs.cap};
+    rc = with_c6 ? launch(k_cn_bins<double, true>, hl) : launch(k_cn_bins<double, false>, hl);
+  } else {
+    const HitList<float> hl{hs.j, (float4*)hs.ad, hs.n, hs.cap};
+    rc = with_c6 ? launch(k_cn_bins<float, true>, hl) : launch(k_cn_bins<float, false>, hl);
+  }
+  *n_self_blocks = grid;
+  if (rc || with_c6) return rc;
   return launch_c6_atoms(n, species, tab, eigvecs, R, cn, c6, dc6, self_part, n_self_blocks, s);
 }
 
 // CN adjoint: dE/dx_i = -sum_(j,S) (g_i + g_j) f'(r) d / r  (the list is symmetric), and the
 // strain virial W_ab = sum_i g_i sum_(j,S) f'(r) d_a d_b / r  (Bohr, Hartree). The force written
 // is out_scale * (mesh gradient already in grad + CN gradient). One warp per atom streams the
-// atom's recorded pairs; atoms without a record (n < 0) are left to k_cn_adjoint_global.
+// atom's recorded pairs; an atom without a record (n < 0) is traversed again from the cell list.
+// A stale cell (ci->stale, see k_cellinfo) makes every force NaN.
 // The kernel is bound by the latency of its dependent loads (count -> atom -> records -> g_j), so
 // a warp fetches the next atom's count and index while it works on this one, issues all of a
 // batch of 96 records' loads before the g_j loads that depend on them, and reads the atom's mesh
 // gradient at the start. Lane l still sums the records l, l + 32, ... in that order.
-template <typename TE>
-__global__ void __launch_bounds__(256, 4) k_cn_adjoint_hits(int n, const int4* __restrict__ meta,
+//
+// REST: the same kernel takes the unrecorded atoms, for the sizes where another launch costs more
+// than the registers of that path (up to kAdjointOne atoms; 5,184: 16 us against 19, 139,968: 104
+// against 78); otherwise k_cn_adjoint_rest follows.
+template <typename TE, bool REST>
+__global__ void __launch_bounds__(256, 4) k_cn_adjoint(const __grid_constant__ GridDev g, int n, const int* __restrict__ bin_start,
+                                                        const double4* __restrict__ xs,
+                                                        const int4* __restrict__ meta, const int4* __restrict__ off,
+                                                        const Tables* __restrict__ tab,
+                                                        const CellInfo* __restrict__ ci,
                                                         const double* __restrict__ gcn, double* __restrict__ grad,
                                                         double out_scale, double* __restrict__ vir_part,
                                                         HitList<TE> hl) {
@@ -639,14 +802,18 @@ __global__ void __launch_bounds__(256, 4) k_cn_adjoint_hits(int n, const int4* _
   int t = blockIdx.x * kWarpsPerBlock + wid;
   int nh_next = t < n ? hl.n[t] : -1;
   int i_next = t < n ? meta[t].w : 0;
+  if (ci->stale != 0.0) out_scale = __longlong_as_double(0x7ff8000000000000LL);
   // grid-stride over atoms: the block's virial is reduced once, after all its atoms
+  bool unrecorded = false;
   for (; t < n; t += stride) {
     const int nh = nh_next, i = i_next;
     if (t + stride < n) {
       nh_next = hl.n[t + stride];
       i_next = meta[t + stride].w;
     }
-    if (nh >= 0) {
+    if (nh < 0) {
+      unrecorded = true;
+    } else {
       const double gi = gcn[i];
       const double gq = lane < 3 ? grad[3 * i + lane] : 0.0;
       double f0 = 0, f1 = 0, f2 = 0;
@@ -693,34 +860,54 @@ __global__ void __launch_bounds__(256, 4) k_cn_adjoint_hits(int n, const int4* _
       }
     }
   }
+  // atoms without a record, in a loop of their own: the call would cost the loop above its registers
+  if (REST && unrecorded)
+    for (t = blockIdx.x * kWarpsPerBlock + wid; t < n; t += stride) {
+      if (hl.n[t] >= 0) continue;
+      const int i = meta[t].w;
+      const PairSums p = cn_adjoint_atom_global(g, bin_start, xs, meta, off, tab, gcn, t);
+      v[0] += p.xx; v[1] += p.xy; v[2] += p.xz;
+      v[4] += p.yy; v[5] += p.yz; v[8] += p.zz;
+      const double f0 = warp_sum(p.f0), f1 = warp_sum(p.f1), f2 = warp_sum(p.f2);
+      if (lane == 0) {
+        grad[3 * i] = out_scale * (grad[3 * i] + f0);
+        grad[3 * i + 1] = out_scale * (grad[3 * i + 1] + f1);
+        grad[3 * i + 2] = out_scale * (grad[3 * i + 2] + f2);
+      }
+    }
   v[3] = v[1];
   v[6] = v[2];
   v[7] = v[5];
   block_sum_store<9>(v, vir_part + 9 * blockIdx.x);
 }
 
-__global__ void __launch_bounds__(256) k_cn_adjoint_global(GridDev g, int n, const int* __restrict__ bin_start,
-                                                          const double4* __restrict__ xs,
-                                                          const int4* __restrict__ meta,
-                                                          const int4* __restrict__ off, const Tables* __restrict__ tab,
-                                                          const double* __restrict__ gcn, double* __restrict__ grad,
-                                                          double out_scale, double* __restrict__ vir_part,
-                                                          const int* __restrict__ hit_n, const int* __restrict__ ovf) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+// Atoms without a record, after k_cn_adjoint<TE, false>. A warp reads the counts of the 32 atoms that
+// are its own (a grid stride apart) at once: almost always none is unrecorded.
+__global__ void __launch_bounds__(256) k_cn_adjoint_rest(const __grid_constant__ GridDev g, int n,
+                                                        const int* __restrict__ bin_start,
+                                                        const double4* __restrict__ xs, const int4* __restrict__ meta,
+                                                        const int4* __restrict__ off, const Tables* __restrict__ tab,
+                                                        const CellInfo* __restrict__ ci,
+                                                        const double* __restrict__ gcn, double* __restrict__ grad,
+                                                        double out_scale, double* __restrict__ vir_part,
+                                                        const int* __restrict__ hit_n) {
+  const int lane = threadIdx.x & 31, stride = gridDim.x * kWarpsPerBlock;
   double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  const bool any = *ovf != 0;
-  for (int t = blockIdx.x * kWarpsPerBlock + wid; any && t < n; t += gridDim.x * kWarpsPerBlock) {
-    if (hit_n[t] >= 0) continue;
-    const int i = meta[t].w;
-    double f[3] = {0, 0, 0};
-    cn_adjoint_atom_global(g, bin_start, xs, meta, off, tab, gcn, t, f, v);
-    f[0] = warp_sum(f[0]);
-    f[1] = warp_sum(f[1]);
-    f[2] = warp_sum(f[2]);
-    if (lane == 0) {
-      grad[3 * i] = out_scale * (grad[3 * i] + f[0]);
-      grad[3 * i + 1] = out_scale * (grad[3 * i + 1] + f[1]);
-      grad[3 * i + 2] = out_scale * (grad[3 * i + 2] + f[2]);
+  if (ci->stale != 0.0) out_scale = __longlong_as_double(0x7ff8000000000000LL);
+  for (int64_t t0 = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); t0 < n; t0 += 32 * (int64_t)stride) {
+    const int64_t own = t0 + (int64_t)lane * stride;
+    unsigned todo = __ballot_sync(0xffffffffu, own < n && hit_n[own] < 0);
+    for (; todo; todo &= todo - 1) {
+      const int t = (int)(t0 + (int64_t)(__ffs(todo) - 1) * stride), i = meta[t].w;
+      const PairSums p = cn_adjoint_atom_global(g, bin_start, xs, meta, off, tab, gcn, t);
+      v[0] += p.xx; v[1] += p.xy; v[2] += p.xz;
+      v[4] += p.yy; v[5] += p.yz; v[8] += p.zz;
+      const double f0 = warp_sum(p.f0), f1 = warp_sum(p.f1), f2 = warp_sum(p.f2);
+      if (lane == 0) {
+        grad[3 * i] = out_scale * (grad[3 * i] + f0);
+        grad[3 * i + 1] = out_scale * (grad[3 * i + 1] + f1);
+        grad[3 * i + 2] = out_scale * (grad[3 * i + 2] + f2);
+      }
     }
   }
   v[3] = v[1];
@@ -729,29 +916,38 @@ __global__ void __launch_bounds__(256) k_cn_adjoint_global(GridDev g, int n, con
   block_sum_store<9>(v, vir_part + 9 * blockIdx.x);
 }
 
-int launch_cn_adjoint_cells(const CellGrid& g, int n, const CellList& cl, const double* pos_ang,
-                            const int32_t* species, const Tables* tab, const double* gcn, double* grad,
-                            double out_scale, double* vir_part, int* n_blocks, const HitStore& hs,
-                            cudaStream_t s) {
-  (void)pos_ang;
-  (void)species;
+constexpr int kAdjointOne = 16384;
+constexpr int kRestBlocks = 148 * 2;
+
+int launch_cn_adjoint_cells(const CellGrid& g, int n, const CellList& cl, const Tables* tab, const CellInfo* ci,
+                            const double* gcn, double* grad, double out_scale, double* vir_part, int* n_blocks,
+                            const HitStore& hs, cudaStream_t s) {
   const int need = (n + kWarpsPerBlock - 1) / kWarpsPerBlock;
   const int blocks = need < 148 * 8 ? need : 148 * 8;   // resident grid, grid-stride over atoms
-  const int fb = need < kFallbackBlocks ? need : kFallbackBlocks;
-  *n_blocks = blocks + fb;
+  *n_blocks = blocks;
   if (blocks == 0) return FD3_OK;
-  if (hs.is_double)
-    k_cn_adjoint_hits<double><<<blocks, 32 * kWarpsPerBlock, 0, s>>>(
-        n, cl.meta, gcn, grad, out_scale, vir_part,
-        HitList<double>{hs.j, (double4*)hs.ad, hs.n, hs.cap});
-  else
-    k_cn_adjoint_hits<float><<<blocks, 32 * kWarpsPerBlock, 0, s>>>(
-        n, cl.meta, gcn, grad, out_scale, vir_part, HitList<float>{hs.j, (float4*)hs.ad, hs.n, hs.cap});
+  const GridDev gd = to_dev(g);
+  const bool one = n <= kAdjointOne;
+  auto launch = [&](auto kern, auto hl) -> int {
+    kern<<<blocks, 32 * kWarpsPerBlock, 0, s>>>(gd, n, cl.bin_start, cl.xs, cl.meta, cl.off, tab, ci, gcn, grad,
+                                                out_scale, vir_part, hl);
+    FD3_LAUNCHED();
+    return FD3_OK;
+  };
+  int rc;
+  if (hs.is_double) {
+    const HitList<double> hl{hs.j, (double4*)hs.ad, hs.n, hs.cap};
+    rc = one ? launch(k_cn_adjoint<double, true>, hl) : launch(k_cn_adjoint<double, false>, hl);
+  } else {
+    const HitList<float> hl{hs.j, (float4*)hs.ad, hs.n, hs.cap};
+    rc = one ? launch(k_cn_adjoint<float, true>, hl) : launch(k_cn_adjoint<float, false>, hl);
+  }
+  if (rc || one) return rc;
+  k_cn_adjoint_rest<<<kRestBlocks, 32 * kWarpsPerBlock, 0, s>>>(gd, n, cl.bin_start, cl.xs, cl.meta, cl.off, tab, ci,
+                                                                gcn, grad, out_scale, vir_part + 9 * (size_t)blocks,
+                                                                hs.n);
   FD3_LAUNCHED();
-  k_cn_adjoint_global<<<fb, 32 * kWarpsPerBlock, 0, s>>>(to_dev(g), n, cl.bin_start, cl.xs, cl.meta, cl.off, tab,
-                                                          gcn, grad, out_scale, vir_part + 9 * (size_t)blocks, hs.n,
-                                                          hs.ovf);
-  FD3_LAUNCHED();
+  *n_blocks = blocks + kRestBlocks;
   return FD3_OK;
 }
 

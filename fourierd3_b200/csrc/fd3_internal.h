@@ -68,22 +68,20 @@ struct HitStore {
   int* j;
   void* ad;
   int* n;
-  int* ovf;     // count of bins / atoms that need the global-memory fallback (zeroed per call)
   int cap;
   bool is_double;
 };
 constexpr int kHitCap = 160;
 
-// fused CN + C6 factors over the cell list (one CTA per bin)
-int launch_cn_c6_cells(const CellGrid& g, int n, const CellList& cl, const double* pos_ang,
-                       const int32_t* species, const Tables* tab, const double* eigvecs, int R, double* cn,
-                       double* c6, double* dc6, double* self_part, int* n_self_blocks, const HitStore& hs,
-                       cudaStream_t s);
+// fused CN + C6 factors over the cell list (one CTA or a few per bin, cn_max_blocks at most)
+int64_t cn_max_blocks(int64_t bins);
+int launch_cn_c6_cells(const CellGrid& g, int n, const CellList& cl, const int32_t* species, const Tables* tab,
+                       const double* eigvecs, int R, double* cn, double* c6, double* dc6, double* self_part, int* n_self_blocks,
+                       const HitStore& hs, cudaStream_t s);
 // CN adjoint: grad = out_scale * (grad + dE/dx_CN) (Hartree/Bohr in); virial partials (9 per block)
-int launch_cn_adjoint_cells(const CellGrid& g, int n, const CellList& cl, const double* pos_ang,
-                            const int32_t* species, const Tables* tab, const double* gcn, double* grad,
-                            double out_scale, double* vir_part, int* n_blocks, const HitStore& hs,
-                            cudaStream_t s);
+int launch_cn_adjoint_cells(const CellGrid& g, int n, const CellList& cl, const Tables* tab, const CellInfo* ci,
+                            const double* gcn, double* grad, double out_scale, double* vir_part, int* n_blocks,
+                            const HitStore& hs, cudaStream_t s);
 
 // direct pairwise lattice sum (float64 accuracy oracle on the device)
 int launch_direct_pairs(const CellGrid& g, int n, const CellList& cl, const double* c6, const Tables* tab, int R,

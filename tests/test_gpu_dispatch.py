@@ -3,8 +3,9 @@ import numpy as np
 import pytest
 import torch
 
-from fourierd3_b200 import neighbour_list
+from fourierd3_b200 import D3Model, neighbour_list
 from oracle.neighbours import neighbour_list_cells
+from oracle.reference_port import OracleFourierD3
 
 pytestmark = pytest.mark.gpu
 
@@ -21,3 +22,33 @@ def test_neighbours_of_bins_from_one_to_hundreds_of_atoms(cuda_device, n_atoms):
     want = np.concatenate((ri[:, None], rj[:, None], rs), 1)
     assert np.all(np.diff(got[:, 0]) >= 0)
     assert np.array_equal(got[np.lexsort(got.T[::-1])], want[np.lexsort(want.T[::-1])])
+
+
+def _against_oracle(device, pos, cell, numbers, precision, tol, **kw):
+    o = OracleFourierD3(numbers, cell, **kw)
+    i, j, s = neighbour_list_cells(pos, cell, 6.0)
+    e_ref, f_ref, s_ref = o.calculate(pos, cell, edges=(np.stack([i, j]), s))
+    e, f, st = D3Model(numbers, cell, precision=precision, device=device, **kw)(pos, cell)
+    assert abs(float(e) - e_ref) <= tol[0] * abs(e_ref)
+    assert np.abs(f.cpu().numpy() - f_ref).max() <= tol[1]
+    assert np.abs(st.cpu().numpy() - s_ref).max() <= tol[2]
+
+
+# the tolerances of the two forms against the oracle (energy relative, eV/A, eV/A^3)
+TOL = {"fp64": (1e-10, 1e-8, 1e-9), "mixed": (1e-6, 1e-4, 1e-6)}
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("edge,n_atoms", [(1.9, 1), (2.9, 3), (5.2, 14), (12.2, 60), (12.2, 420), (19.0, 500)])
+def test_cn_stage_from_image_only_cells_to_bins_beyond_the_stage(cuda_device, edge, n_atoms, precision):
+    # 1.9 A: more neighbour bins than the table holds (traversal of global memory); 2.9 and 5.2 A: every
+    # candidate is an image of one bin; 420 atoms in 12.2 A: 27 bins of 52, pieces of the stage and
+    # atoms with more pairs than the record holds; 19 A: several CTAs per bin
+    rng = np.random.default_rng(n_atoms)
+    cell = np.diag([edge, edge, edge]) + np.triu(np.full((3, 3), 0.03 * edge), 1)
+    m = int(np.ceil(n_atoms ** (1 / 3)))
+    grid = rng.permutation(m ** 3)[:n_atoms]
+    frac = (np.stack(np.unravel_index(grid, (m, m, m)), 1) + rng.uniform(0.4, 0.6, (n_atoms, 3))) / m
+    numbers = rng.choice([1, 6, 8], n_atoms)
+    _against_oracle(cuda_device, frac @ cell, cell, numbers, precision, TOL[precision], method="spme",
+                    mesh_spacing=1.2, interpolation_nodes=4, c6tol=1.0, r_cut=6.0)
