@@ -6,7 +6,7 @@
 #include <atomic>
 #include <new>
 
-#include "fd3_internal.h"
+#include "fd3_prep_args.cuh"
 
 using namespace fd3;
 
@@ -32,10 +32,6 @@ struct fd3_plan {
   cufftHandle fwd2 = 0, inv2 = 0;   // (y, z) 2D transforms of the fused x-pass path
   bool has_fft2 = false;
   size_t fft_ws = 0;
-  // side stream of the fused entry: the mesh sort (positions only) runs beside the cell list and
-  // the CN stage, forked from and joined back to the caller's stream by events (also under capture)
-  cudaStream_t side = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   // optional per-stage CUDA-event timing (fd3_profile_enable / fd3_profile_read)
   static constexpr int kMaxMarks = 24;
   bool prof = false;
@@ -352,16 +348,6 @@ extern "C" int fd3_plan_create(const fd3_plan_desc* d, fd3_plan** out) {
           break;
         }
       }
-      // side stream and fork/join events of the fused entry (without them it runs on one stream)
-      if (cudaStreamCreateWithFlags(&p->side, cudaStreamNonBlocking) != cudaSuccess ||
-          cudaEventCreateWithFlags(&p->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-          cudaEventCreateWithFlags(&p->ev_join, cudaEventDisableTiming) != cudaSuccess) {
-        cudaGetLastError();
-        if (p->ev_fork) cudaEventDestroy(p->ev_fork);
-        if (p->side) cudaStreamDestroy(p->side);
-        p->side = nullptr;
-        p->ev_fork = p->ev_join = nullptr;
-      }
     }
   } while (0);
   delete[] gp;
@@ -559,9 +545,6 @@ extern "C" int fd3_plan_destroy(fd3_plan* p) {
   cudaFree(p->d_cnpair);
   cudaFree(p->d_cnself);
   if (p->inv2) cufftDestroy(p->inv2);
-  if (p->ev_fork) cudaEventDestroy(p->ev_fork);
-  if (p->ev_join) cudaEventDestroy(p->ev_join);
-  if (p->side) cudaStreamDestroy(p->side);
   cudaFree(p->d_tab);
   cudaFree(p->d_eigvecs);
   cudaFree(p->d_green);
@@ -590,7 +573,7 @@ struct Work {
   CellInfo* ci;
   double *cn, *c6, *dc6, *gcn;
   double *self_part, *kspc_part, *cnv_part, *mcell_part;
-  int *mkeys, *mcount, *mstart, *morder;
+  int *mkeys, *mcount, *mstart, *morder, *mslot, *mtmp;
   MeshRecords rec;
   CellList cl;
   HitStore hits;
@@ -640,11 +623,13 @@ void carve(const fd3_plan* p, int64_t N, int64_t K_in, Carver& c, Work& w, int64
   w.rec.w = c.take<char>(N * P3 * es);
   w.rec.dw = c.take<char>(N * P3 * es);
   w.rec.c = c.take<char>(N * p->R * es);
-  w.mcount = c.take<int>(Kmesh);
+  w.cl.bin_count = c.take<int>(K + Kmesh);   // one array: the preparation zeroes both in one go
+  w.mcount = w.cl.bin_count + K;
   w.mstart = c.take<int>(Kmesh + 1);
   w.morder = c.take<int>(N);
+  w.mslot = c.take<int>(N);
+  w.mtmp = c.take<int>(N);
   w.cl.bin_of = c.take<int>(N);
-  w.cl.bin_count = c.take<int>(K);
   w.cl.bin_start = c.take<int>(K + 1);
   w.cl.order = c.take<int>(N);
   w.cl.xs = c.take<double4>(N);
@@ -745,40 +730,82 @@ static int check_work(const fd3_plan* p, int64_t N, int64_t K, void* work, size_
   return FD3_OK;
 }
 
-// ------------------------------------------------------------------ shared mesh pipeline
-// spread -> forward FFT -> filter (energy, virial, H = G S) -> [inverse FFT -> gather]
-// atoms counting-sorted by (mesh tile, species): needs only the positions and the cell info
-static int mesh_sort(fd3_plan* p, int N, const double* pos, double ps, const int32_t* species, Work& w,
-                     cudaStream_t s) {
-  const MeshGeom& mg = p->mg;
-  const int Kmesh = mg.nt[0] * mg.nt[1] * mg.nt[2] * p->S;
-  FD3_TRY(launch_mesh_keys(mg, N, pos, ps, species, w.ci, w.mkeys, s));
-  // the stencil nodes are written after the sort: until then they are its scratch
-  return counting_sort(w.mkeys, N, Kmesh, w.mcount, w.mstart, w.morder, reinterpret_cast<int*>(w.rec.b), s);
+// ------------------------------------------------------------------ preparation
+// Cell-derived quantities of a host cell (as k_cellinfo computes them from a device cell).
+static CellInfo host_cellinfo(const double* cell, double scale) {
+  CellInfo ci{};
+  double m[9];
+  for (int k = 0; k < 9; ++k) ci.cell[k] = m[k] = cell[k] * scale;
+  const double adj[9] = {m[4] * m[8] - m[5] * m[7], m[2] * m[7] - m[1] * m[8], m[1] * m[5] - m[2] * m[4],
+                         m[5] * m[6] - m[3] * m[8], m[0] * m[8] - m[2] * m[6], m[2] * m[3] - m[0] * m[5],
+                         m[3] * m[7] - m[4] * m[6], m[1] * m[6] - m[0] * m[7], m[0] * m[4] - m[1] * m[3]};
+  const double det = m[0] * adj[0] + m[1] * adj[3] + m[2] * adj[6];
+  for (int k = 0; k < 9; ++k) ci.inv[k] = adj[k] / det;
+  for (int i = 0; i < 3; ++i)
+    for (int c = 0; c < 3; ++c) ci.recip[3 * i + c] = 2.0 * kPi * ci.inv[3 * c + i];
+  ci.volume = fabs(det);
+  return ci;
 }
 
-// The position-only preparation of the mesh stage that can run beside the cell list and the CN
-// stage: the stencil records' nodes and weights, and the mixed form's Green table.
-static int mesh_side_prep(fd3_plan* p, int N, const double* pos, double ps, const int32_t* species, Work& w,
-                          cudaStream_t s) {
+// Mesh sort, stencil records and (mixed form) Green table of a mesh plan; with g the cell list too,
+// the cell then being h_cell (compared with d_cell), otherwise the one in w.ci.
+static int prepare(fd3_plan* p, const CellGrid* g, int N, const double* pos, double ps, const int32_t* species,
+                   const double* h_cell, const double* d_cell, Work& w, cudaStream_t s) {
   const MeshGeom& mg = p->mg;
+  PrepDev a{};
+  a.n = N;
+  a.pos = pos;
+  a.ps = ps;
+  a.species = species;
+  if (g) {
+    a.g = to_dev(*g);
+    a.K = g->nb[0] * g->nb[1] * g->nb[2];
+    a.use_host = 1;
+    a.host = host_cellinfo(h_cell, ps);
+    a.d_cell = d_cell;
+    for (int k = 0; k < 9; ++k) a.host_cell[k] = h_cell[k];
+  }
+  a.xs = w.cl.xs;
+  a.meta = w.cl.meta;
+  a.off = w.cl.off;
+  a.bin_start = w.cl.bin_start;
+  a.bslot = w.cl.bin_of;
+  a.btmp = w.cl.order;
+  a.m = to_dev(mg);
+  a.P = mg.order;
+  a.Km = mg.nt[0] * mg.nt[1] * mg.nt[2] * p->S;
+  a.mkeys = w.mkeys;
+  a.mslot = w.mslot;
+  a.mtmp = w.mtmp;
+  a.mstart = w.mstart;
+  a.morder = w.morder;
+  a.rb = w.rec.b;
+  a.rw = w.rec.w;
+  a.rdw = w.rec.dw;
+  a.counts = g ? w.cl.bin_count : w.mcount;
+  a.ci = w.ci;
+  a.gp = p->d_green;
+  a.tab = p->d_tab;
   if (p->precision == FD3_PREC_FP64)
-    return launch_spread<double>(mg, N, pos, ps, species, nullptr, w.ci, w.mstart, w.morder, w.rec, (double*)w.rho,
-                                 s, kSpreadRecordsOnly);
-  FD3_TRY(launch_spread<float>(mg, N, pos, ps, species, nullptr, w.ci, w.mstart, w.morder, w.rec, (float*)w.rho, s,
-                               kSpreadRecordsOnly));
-  return launch_green_table(mg, w.ci, p->d_green, p->d_tab, w.gtab, s);
+    return mg.lagrange ? launch_prep<double, true>(a, s) : launch_prep<double, false>(a, s);
+  a.gtab = (float4*)w.gtab;
+  return mg.lagrange ? launch_prep<float, true>(a, s) : launch_prep<float, false>(a, s);
 }
 
+// rank factors of the stencil records, written by the C6 kernels
+static RankOut rank_out(const fd3_plan* p, const Work& w) {
+  if (p->method == FD3_METHOD_EWALD) return RankOut{nullptr, nullptr, 0};
+  return RankOut{w.rec.c, w.mslot, p->precision == FD3_PREC_FP64 ? 1 : 0};
+}
+
+// ------------------------------------------------------------------ shared mesh pipeline
+// spread -> forward FFT -> filter (energy, virial, H = G S) -> [inverse FFT -> gather], after
+// prepare() and the C6 kernels
 template <typename T>
 static int mesh_pipeline(fd3_plan* p, int N, const double* pos, double ps, const int32_t* species, Work& w,
-                         bool need_grad, double* gpos, double* mcell, int* n_kspc, int* n_mcell, bool presorted,
-                         cudaStream_t s, bool side_prep = false) {
+                         bool need_grad, double* gpos, double* mcell, int* n_kspc, int* n_mcell, cudaStream_t s) {
   const MeshGeom& mg = p->mg;
-  if (!presorted) FD3_TRY(mesh_sort(p, N, pos, ps, species, w, s));
-  prof_mark(p, s, "mesh_sort");
-  FD3_TRY(launch_spread<T>(mg, N, pos, ps, species, w.c6, w.ci, w.mstart, w.morder, w.rec, (T*)w.rho, s,
-                           side_prep ? 1 : 0));
+  FD3_TRY(launch_spread<T>(mg, N, nullptr, w.mstart, w.morder, w.rec, (T*)w.rho, s));
   prof_mark(p, s, "spread");
   const bool tma_x = sizeof(T) == 4 && xpass_on(p);
   if (tma_x || old_xpass_on(p)) {
@@ -800,7 +827,6 @@ static int mesh_pipeline(fd3_plan* p, int N, const double* pos, double ps, const
         FD3_CUFFT(cufftExecR2C(p->fwd2, (cufftReal*)w.rho, (cufftComplex*)w.spec));
     }
     prof_mark(p, s, "fft_r2c");
-    if (sizeof(T) == 4 && !side_prep) FD3_TRY(launch_green_table(mg, w.ci, p->d_green, p->d_tab, w.gtab, s));
     if (tma_x) {
       int Q, RG;
       xpass_shape(p, &Q, &RG);
@@ -837,7 +863,6 @@ static int mesh_pipeline(fd3_plan* p, int N, const double* pos, double ps, const
     FD3_CUFFT(cufftExecR2C(p->fwd, (cufftReal*)w.rho, (cufftComplex*)w.spec));
   prof_mark(p, s, "fft_r2c");
   void* hspec = w.spec;   // the filter overwrites the spectrum with H in place
-  if (sizeof(T) == 4 && !side_prep) FD3_TRY(launch_green_table(mg, w.ci, p->d_green, p->d_tab, w.gtab, s));
   FD3_TRY(launch_filter<T>(mg, w.ci, p->d_green, p->d_green_f, (const float4*)w.gtab, p->d_tab, p->d_deconv, p->method == FD3_METHOD_SPME, w.spec,
                            w.kspc_part, n_kspc, s));
   prof_mark(p, s, "filter");
@@ -857,8 +882,7 @@ static int mesh_pipeline(fd3_plan* p, int N, const double* pos, double ps, const
 }
 
 static int run_mesh(fd3_plan* p, int N, const double* pos, double ps, const int32_t* species, Work& w,
-                    bool need_grad, double* gpos, double* mcell, int* n_kspc, int* n_mcell, cudaStream_t s,
-                    bool presorted = false, bool side_prep = false) {
+                    bool need_grad, double* gpos, double* mcell, int* n_kspc, int* n_mcell, cudaStream_t s) {
   if (p->method == FD3_METHOD_EWALD) {
     EwaldGeom eg{{p->ens[0], p->ens[1], p->ens[2]}, p->S, p->R};
     int rc;
@@ -872,15 +896,13 @@ static int run_mesh(fd3_plan* p, int N, const double* pos, double ps, const int3
     return rc;
   }
   if (p->precision == FD3_PREC_FP64)
-    return mesh_pipeline<double>(p, N, pos, ps, species, w, need_grad, gpos, mcell, n_kspc, n_mcell, presorted, s,
-                                 side_prep);
-  return mesh_pipeline<float>(p, N, pos, ps, species, w, need_grad, gpos, mcell, n_kspc, n_mcell, presorted, s,
-                              side_prep);
+    return mesh_pipeline<double>(p, N, pos, ps, species, w, need_grad, gpos, mcell, n_kspc, n_mcell, s);
+  return mesh_pipeline<float>(p, N, pos, ps, species, w, need_grad, gpos, mcell, n_kspc, n_mcell, s);
 }
 
 // ------------------------------------------------------------------ D4 k-space CN stages
 // Forward: one-hot species density -> 3D R2C (spectrum kept for the adjoint) -> G^CN -> C2R ->
-// CN values (w.cn). Needs the mesh sort of this call (w.mstart, w.morder).
+// CN values (w.cn). Needs prepare() of this call.
 template <typename T>
 static int cn4_forward(fd3_plan* p, int N, const double* pos, double ps, const int32_t* species, Work& w,
                        cudaStream_t s) {
@@ -888,7 +910,7 @@ static int cn4_forward(fd3_plan* p, int N, const double* pos, double ps, const i
   m1.R = 1;
   const int spme = p->method == FD3_METHOD_SPME;
   FD3_TRY(launch_cn4_values(N, 0, nullptr, w.ci, w.cn4_vals, s));
-  FD3_TRY(launch_spread<T>(m1, N, pos, ps, species, w.cn4_vals, w.ci, w.mstart, w.morder, w.rec, (T*)w.cn4_rho, s));
+  FD3_TRY(launch_spread<T>(m1, N, w.cn4_vals, w.mstart, w.morder, w.rec, (T*)w.cn4_rho, s));
   FD3_CUFFT(cufftSetStream(p->fwd_cn, s));
   FD3_CUFFT(cufftSetWorkArea(p->fwd_cn, w.fftw));
   if (sizeof(T) == 8)
@@ -918,7 +940,7 @@ static int cn4_adjoint(fd3_plan* p, int N, const double* pos, double ps, const i
   m1.R = 1;
   const int spme = p->method == FD3_METHOD_SPME;
   FD3_TRY(launch_cn4_values(N, 1, w.gcn, w.ci, w.cn4_vals, s));
-  FD3_TRY(launch_spread<T>(m1, N, pos, ps, species, w.cn4_vals, w.ci, w.mstart, w.morder, w.rec, (T*)w.cn4_rho, s));
+  FD3_TRY(launch_spread<T>(m1, N, w.cn4_vals, w.mstart, w.morder, w.rec, (T*)w.cn4_rho, s));
   FD3_CUFFT(cufftSetStream(p->fwd_cn, s));
   FD3_CUFFT(cufftSetWorkArea(p->fwd_cn, w.fftw));
   if (sizeof(T) == 8)
@@ -971,12 +993,12 @@ extern "C" int fd3_energy_edges(fd3_plan* p, int64_t n_atoms, const double* d_po
   if (p->cnfunc == FD3_CN_D4) {
     // k-space D4 CN: no edges (the reference's forward ignores them, core.py:512-516)
     int n_self = 0, n_kspc = 0, n_mcell = 0, n_cnv = 0;
-    FD3_TRY(mesh_sort(p, N, d_pos, 1.0, d_species, w, s));
+    FD3_TRY(prepare(p, nullptr, N, d_pos, 1.0, d_species, nullptr, nullptr, w, s));
     FD3_TRY(cn4_forward_any(p, N, d_pos, 1.0, d_species, w, s));
-    FD3_TRY(launch_c6_atoms(N, d_species, p->d_tab, p->d_eigvecs, p->R, w.cn, w.c6, w.dc6, w.self_part, &n_self, s));
+    FD3_TRY(launch_c6_atoms(N, d_species, p->d_tab, p->d_eigvecs, p->R, w.cn, w.c6, w.dc6, rank_out(p, w),
+                            w.self_part, &n_self, s));
     prof_mark(p, s, "cn_c6");
-    FD3_TRY(run_mesh(p, N, d_pos, 1.0, d_species, w, need_grad != 0, d_gpos, w.mcell_part, &n_kspc, &n_mcell, s,
-                     true));
+    FD3_TRY(run_mesh(p, N, d_pos, 1.0, d_species, w, need_grad != 0, d_gpos, w.mcell_part, &n_kspc, &n_mcell, s));
     if (need_grad) {
       FD3_TRY(cn4_adjoint_any(p, N, d_pos, 1.0, d_species, w, d_gpos, 1.0, w.mcell_part + 9 * (size_t)n_mcell,
                               &n_cnv, s));
@@ -990,11 +1012,14 @@ extern "C" int fd3_energy_edges(fd3_plan* p, int64_t n_atoms, const double* d_po
   }
   // edges sorted by source and destination; the CN is summed per atom in edge order
   const double mask_r2 = p->edge_cutoff ? p->h_tab.r_cut * p->h_tab.r_cut : INFINITY;
+  if (p->method != FD3_METHOD_EWALD)
+    FD3_TRY(prepare(p, nullptr, N, d_pos, 1.0, d_species, nullptr, nullptr, w, s));
   FD3_TRY(launch_edge_index(n_edges, N, d_src, d_dst, w.ei, s));
   FD3_TRY(launch_cn_edges_seg(n_edges, N, d_pos, d_species, d_src, d_dst, d_shift, p->d_tab, mask_r2, w.ei, w.cn,
                               s));
   int n_self = 0, n_kspc = 0, n_mcell = 0;
-  FD3_TRY(launch_c6_atoms(N, d_species, p->d_tab, p->d_eigvecs, p->R, w.cn, w.c6, w.dc6, w.self_part, &n_self, s));
+  FD3_TRY(launch_c6_atoms(N, d_species, p->d_tab, p->d_eigvecs, p->R, w.cn, w.c6, w.dc6, rank_out(p, w),
+                            w.self_part, &n_self, s));
   prof_mark(p, s, "cn_c6");
   FD3_TRY(run_mesh(p, N, d_pos, 1.0, d_species, w, need_grad != 0, d_gpos, w.mcell_part, &n_kspc, &n_mcell, s));
   if (need_grad)
@@ -1024,18 +1049,16 @@ extern "C" int fd3_energy_forces_stress(fd3_plan* p, int64_t n_atoms, const doub
   Work w;
   FD3_TRY(check_work(p, N, K, d_work, work_bytes, w));
   prof_begin(p, s);
-  // the cell list below is built from the host cell: a device cell that differs (a captured graph
-  // replayed after a cell change) makes every output NaN instead of silently dropping pairs
-  FD3_TRY(launch_cellinfo(d_cell_ang, kAngToBohr, w.ci, s, p->cnfunc == FD3_CN_D4 ? nullptr : h_cell_ang));
   if (p->cnfunc == FD3_CN_D4) {
     // k-space D4 CN: no neighbour search (calculator.py:171-173)
+    FD3_TRY(launch_cellinfo(d_cell_ang, kAngToBohr, w.ci, s));
     int n_self = 0, n_kspc = 0, n_mcell = 0, n_cnv = 0;
-    FD3_TRY(mesh_sort(p, N, d_pos_ang, kAngToBohr, d_species, w, s));
+    FD3_TRY(prepare(p, nullptr, N, d_pos_ang, kAngToBohr, d_species, nullptr, nullptr, w, s));
     FD3_TRY(cn4_forward_any(p, N, d_pos_ang, kAngToBohr, d_species, w, s));
-    FD3_TRY(launch_c6_atoms(N, d_species, p->d_tab, p->d_eigvecs, p->R, w.cn, w.c6, w.dc6, w.self_part, &n_self, s));
+    FD3_TRY(launch_c6_atoms(N, d_species, p->d_tab, p->d_eigvecs, p->R, w.cn, w.c6, w.dc6, rank_out(p, w),
+                            w.self_part, &n_self, s));
     prof_mark(p, s, "cn_c6");
-    FD3_TRY(run_mesh(p, N, d_pos_ang, kAngToBohr, d_species, w, true, d_forces, nullptr, &n_kspc, &n_mcell, s,
-                     true));
+    FD3_TRY(run_mesh(p, N, d_pos_ang, kAngToBohr, d_species, w, true, d_forces, nullptr, &n_kspc, &n_mcell, s));
     FD3_TRY(cn4_adjoint_any(p, N, d_pos_ang, kAngToBohr, d_species, w, d_forces, -kHartreeToEv * kAngToBohr,
                             nullptr, &n_cnv, s));
     prof_mark(p, s, "cn_adjoint");
@@ -1044,24 +1067,21 @@ extern "C" int fd3_energy_forces_stress(fd3_plan* p, int64_t n_atoms, const doub
     prof_mark(p, s, "finalize");
     return FD3_OK;
   }
-  const bool fork = p->side != nullptr && p->method != FD3_METHOD_EWALD;
-  if (fork) {   // mesh sort, stencil records and Green table on the side stream, beside the cell list and CN
-    FD3_CUDA(cudaEventRecord(p->ev_fork, s));
-    FD3_CUDA(cudaStreamWaitEvent(p->side, p->ev_fork, 0));
-    FD3_TRY(mesh_sort(p, N, d_pos_ang, kAngToBohr, d_species, w, p->side));
-    FD3_TRY(mesh_side_prep(p, N, d_pos_ang, kAngToBohr, d_species, w, p->side));
-    FD3_CUDA(cudaEventRecord(p->ev_join, p->side));
+  // the cell list is built from the host cell: a device cell that differs (a captured graph replayed
+  // after a cell change) makes every output NaN instead of silently dropping pairs
+  if (p->method == FD3_METHOD_EWALD) {
+    FD3_TRY(launch_cellinfo(d_cell_ang, kAngToBohr, w.ci, s, h_cell_ang));
+    FD3_TRY(build_cell_list(g, N, d_pos_ang, d_species, w.cl, s));
+  } else {
+    FD3_TRY(prepare(p, &g, N, d_pos_ang, kAngToBohr, d_species, h_cell_ang, d_cell_ang, w, s));
   }
-  FD3_TRY(build_cell_list(g, N, d_pos_ang, d_species, w.cl, s));
   prof_mark(p, s, "cell_list");
   int n_self = 0, n_kspc = 0, n_mcell = 0, n_cnv = 0;
-  FD3_TRY(launch_cn_c6_cells(g, N, w.cl, d_species, p->d_tab, p->d_eigvecs, p->R, w.cn, w.c6, w.dc6,
+  FD3_TRY(launch_cn_c6_cells(g, N, w.cl, d_species, p->d_tab, p->d_eigvecs, p->R, w.cn, w.c6, w.dc6, rank_out(p, w),
                              w.self_part, &n_self, w.hits, s));
   prof_mark(p, s, "cn_c6");
-  if (fork) FD3_CUDA(cudaStreamWaitEvent(s, p->ev_join, 0));
   // the mesh gradient (Hartree/Bohr) is staged in d_forces, then finished by the CN adjoint
-  FD3_TRY(run_mesh(p, N, d_pos_ang, kAngToBohr, d_species, w, true, d_forces, nullptr, &n_kspc, &n_mcell, s,
-                   fork, fork));
+  FD3_TRY(run_mesh(p, N, d_pos_ang, kAngToBohr, d_species, w, true, d_forces, nullptr, &n_kspc, &n_mcell, s));
   FD3_TRY(launch_cn_adjoint_cells(g, N, w.cl, p->d_tab, w.ci, w.gcn, d_forces,
                                   -kHartreeToEv * kAngToBohr, w.cnv_part, &n_cnv, w.hits, s));
   prof_mark(p, s, "cn_adjoint");
@@ -1155,7 +1175,7 @@ extern "C" int fd3_direct_energy_forces_stress(fd3_plan* p, int64_t n_atoms, con
   FD3_TRY(build_cell_list(g, N, d_pos_ang, d_species, w.cl, s));
   int n_self = 0, n_pair = 0, n_cnv = 0;
   FD3_TRY(launch_cn_c6_cells(g, N, w.cl, d_species, p->d_tab, p->d_eigvecs, p->R, w.cn, w.c6, w.dc6,
-                             w.self_part, &n_self, w.hits, s));
+                             RankOut{nullptr, nullptr, 0}, w.self_part, &n_self, w.hits, s));
   FD3_TRY(build_cell_list(g2, N, d_pos_ang, d_species, d.cl, s));
   // pair gradient (Hartree/Bohr) staged in d_forces, finished by the CN adjoint
   FD3_TRY(launch_direct_pairs(g2, N, d.cl, w.c6, p->d_tab, p->R, p->S, p->d_green, d.dEdc, d_forces, d.pair_part,

@@ -10,7 +10,7 @@
 #include <math.h>
 #include <stdio.h>
 
-#include "fd3_internal.h"
+#include "fd3_sort.cuh"
 
 namespace fd3 {
 
@@ -58,54 +58,9 @@ int make_cell_grid(const double* h_cell, double r_cut, CellGrid* g) {
 }
 
 // ------------------------------------------------------------------ scan / sort
-constexpr int kScanThreads = 1024;
-constexpr int kScanItems = 4;
-
-__global__ void __launch_bounds__(1024) k_scan_exclusive(const int* __restrict__ in, int n, int* __restrict__ out) {
-  __shared__ int warp_tot[32];
-  __shared__ int carry_s;
-  if (threadIdx.x == 0) carry_s = 0;
-  __syncthreads();
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int base = 0; base < n; base += kScanThreads * kScanItems) {
-    int v[kScanItems];
-    int local = 0;
-    const int i0 = base + threadIdx.x * kScanItems;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-      v[k] = (i0 + k < n) ? in[i0 + k] : 0;
-      local += v[k];
-    }
-    int incl = local;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      int t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += t;
-    }
-    if (lane == 31) warp_tot[wid] = incl;
-    __syncthreads();
-    if (wid == 0) {
-      int w = warp_tot[lane];
-      int wi = w;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        int t = __shfl_up_sync(0xffffffffu, wi, o);
-        if (lane >= o) wi += t;
-      }
-      warp_tot[lane] = wi - w;   // exclusive warp offsets
-    }
-    __syncthreads();
-    int run = carry_s + warp_tot[wid] + incl - local;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-      if (i0 + k < n) out[i0 + k] = run;
-      run += v[k];
-    }
-    __syncthreads();
-    if (threadIdx.x == kScanThreads - 1) carry_s = run;
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[n] = carry_s;
+__global__ void __launch_bounds__(kScanThreads) k_scan_exclusive(const int* __restrict__ in, int n,
+                                                                int* __restrict__ out) {
+  scan_exclusive_block(in, n, out);
 }
 
 int scan_exclusive(const int* in, int n, int* out, cudaStream_t s) {
@@ -131,14 +86,6 @@ __global__ void __launch_bounds__(256) k_scatter(const int* __restrict__ keys, i
                                                 const int* __restrict__ slot, int* __restrict__ arrival) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) arrival[starts[keys[i]] + slot[i]] = i;
-}
-
-// Place of the id at position p of the arrival-ordered segments once its segment is sorted.
-__device__ __forceinline__ int ranked_place(const int* __restrict__ arrival, int id, int a, int b) {
-  int rank = 0;
-#pragma unroll 4
-  for (int q = a; q < b; ++q) rank += arrival[q] < id ? 1 : 0;
-  return a + rank;
 }
 
 __global__ void __launch_bounds__(256) k_rank_segments(const int* __restrict__ keys, int n,
@@ -169,25 +116,6 @@ int counting_sort(const int* keys, int n, int K, int* counts, int* starts, int* 
 }
 
 // ------------------------------------------------------------------ cell list
-struct GridDev {
-  int nb[3], reach[3];
-  double cell[9], inv[9];
-  double rc2;
-};
-static GridDev to_dev(const CellGrid& g) {
-  GridDev d;
-  for (int a = 0; a < 3; ++a) {
-    d.nb[a] = g.nb[a];
-    d.reach[a] = g.reach[a];
-  }
-  for (int k = 0; k < 9; ++k) {
-    d.cell[k] = g.cell[k];
-    d.inv[k] = g.inv[k];
-  }
-  d.rc2 = g.rc2;
-  return d;
-}
-
 __global__ void __launch_bounds__(256) k_bin_atoms(GridDev g, int n, const double* __restrict__ x, int* __restrict__ bin_of,
                             int4* __restrict__ off) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -476,7 +404,7 @@ struct HitList {
 // exponentials (6 us at any size), a warp per atom repeats the work 32-fold (+60 us at 139,968 atoms).
 __device__ __forceinline__ double c6_group(bool on, int i, int s, double raw_cn, const Tables* __restrict__ tab,
                                            const double* __restrict__ V, int R, double* __restrict__ cn,
-                                           double* __restrict__ c6, double* __restrict__ dc6) {
+                                           double* __restrict__ c6, double* __restrict__ dc6, const RankOut& ro) {
   const int lane = threadIdx.x & 7;
   double cnv = raw_cn, slope = 1.0;
   if (tab->has_cncorr) {
@@ -514,6 +442,7 @@ __device__ __forceinline__ double c6_group(bool on, int i, int s, double raw_cn,
     if (on && r < R) {
       c6[(size_t)i * R + r] = c;
       dc6[(size_t)i * R + r] = slope * d;
+      ro.put(i, r, R, c);
       selfv += tab->eigs[r] * c * c * tab->selfcont[s];
     }
   }
@@ -684,7 +613,7 @@ __global__ void __launch_bounds__(32 * kCnWarps, sizeof(TE) == 4 ? 9 : 7) k_cn_b
                                                 const int4* __restrict__ off, const Tables* __restrict__ tab,
                                                 const double* __restrict__ V, int R, double* __restrict__ cn,
                                                 double* __restrict__ c6, double* __restrict__ dc6,
-                                                const __grid_constant__ HitList<TE> hl,
+                                                const __grid_constant__ HitList<TE> hl, RankOut ro,
                                                 double* __restrict__ self_part) {
   extern __shared__ __align__(16) unsigned char cn_raw[];
   __shared__ NbrBins st;
@@ -721,7 +650,7 @@ __global__ void __launch_bounds__(32 * kCnWarps, sizeof(TE) == 4 ? 9 : 7) k_cn_b
       const int t = s0 + part * kCnWarps + a / kCnWarps * (kCnWarps * nsplit) + a % kCnWarps;
       const bool on = a < rounds * kCnWarps && t < s1;
       const int i = on ? meta[t].w : 0, s = on ? (int)xs[t].w : 0;
-      self[0] += c6_group(on, i, s, on ? cn[i] : 0.0, tab, V, R, cn, c6, dc6);
+      self[0] += c6_group(on, i, s, on ? cn[i] : 0.0, tab, V, R, cn, c6, dc6, ro);
     }
     }
   }
@@ -731,8 +660,8 @@ __global__ void __launch_bounds__(32 * kCnWarps, sizeof(TE) == 4 ? 9 : 7) k_cn_b
 int64_t cn_max_blocks(int64_t bins) { return 4 * 148 + bins; }   // bins * ceil(4 * 148 / bins) at most
 
 int launch_cn_c6_cells(const CellGrid& g, int n, const CellList& cl, const int32_t* species, const Tables* tab,
-                       const double* eigvecs, int R, double* cn, double* c6, double* dc6, double* self_part, int* n_self_blocks,
-                       const HitStore& hs, cudaStream_t s) {
+                       const double* eigvecs, int R, double* cn, double* c6, double* dc6,
+                       const RankOut& ro, double* self_part, int* n_self_blocks, const HitStore& hs, cudaStream_t s) {
   const int K = g.nb[0] * g.nb[1] * g.nb[2];
   // stage: the mean number of candidates and half as much again, within kCnSmem
   const double mean = (double)n / K * (2 * g.reach[0] + 1) * (2 * g.reach[1] + 1) * (2 * g.reach[2] + 1);
@@ -755,7 +684,7 @@ int launch_cn_c6_cells(const CellGrid& g, int n, const CellList& cl, const int32
     if (stage > kCnSmemPlain)
       FD3_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kCnSmem));
     kern<<<grid, 32 * kCnWarps, stage, s>>>(to_dev(g), stage, nsplit, cl.bin_start, cl.xs, cl.meta, cl.off, tab,
-                                            eigvecs, R, cn, c6, dc6, hl, self_part);
+                                            eigvecs, R, cn, c6, dc6, hl, ro, self_part);
     FD3_LAUNCHED();
     return FD3_OK;
   };
@@ -769,7 +698,7 @@ int launch_cn_c6_cells(const CellGrid& g, int n, const CellList& cl, const int32
   }
   *n_self_blocks = grid;
   if (rc || with_c6) return rc;
-  return launch_c6_atoms(n, species, tab, eigvecs, R, cn, c6, dc6, self_part, n_self_blocks, s);
+  return launch_c6_atoms(n, species, tab, eigvecs, R, cn, c6, dc6, ro, self_part, n_self_blocks, s);
 }
 
 // CN adjoint: dE/dx_i = -sum_(j,S) (g_i + g_j) f'(r) d / r  (the list is symmetric), and the
@@ -1107,7 +1036,8 @@ int launch_cn_adjoint_edges_seg(int64_t n_edges, int n, const double* pos, const
 __global__ void __launch_bounds__(256) k_c6_atoms(int n, const int32_t* __restrict__ species,
                                                  const Tables* __restrict__ tab, const double* __restrict__ V, int R,
                                                  double* __restrict__ cn, double* __restrict__ c6,
-                                                 double* __restrict__ dc6, double* __restrict__ self_part) {
+                                                 double* __restrict__ dc6, RankOut ro,
+                                                 double* __restrict__ self_part) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   double selfv = 0.0;
   if (i < n) {
@@ -1151,6 +1081,7 @@ __global__ void __launch_bounds__(256) k_c6_atoms(int n, const int32_t* __restri
       }
       c6[(size_t)i * R + r] = c;
       dc6[(size_t)i * R + r] = slope * d;
+      ro.put(i, r, R, c);
       selfv += tab->eigs[r] * c * c * tab->selfcont[s];
     }
     cn[i] = cnv;
@@ -1160,12 +1091,13 @@ __global__ void __launch_bounds__(256) k_c6_atoms(int n, const int32_t* __restri
 }
 
 int launch_c6_atoms(int n, const int32_t* species, const Tables* tab, const double* eigvecs, int R,
-                    const double* cn, double* c6, double* dc6, double* self_part, int* n_self_blocks,
-                    cudaStream_t s) {
+                    const double* cn, double* c6, double* dc6, const RankOut& ro, double* self_part,
+                    int* n_self_blocks, cudaStream_t s) {
   const int blocks = (n + 255) / 256;
   *n_self_blocks = blocks;
   if (blocks == 0) return FD3_OK;
-  k_c6_atoms<<<blocks, 256, 0, s>>>(n, species, tab, eigvecs, R, const_cast<double*>(cn), c6, dc6, self_part);
+  k_c6_atoms<<<blocks, 256, 0, s>>>(n, species, tab, eigvecs, R, const_cast<double*>(cn), c6, dc6, ro,
+                                     self_part);
   FD3_LAUNCHED();
   return FD3_OK;
 }

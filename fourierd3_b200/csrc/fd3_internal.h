@@ -73,11 +73,29 @@ struct HitStore {
 };
 constexpr int kHitCap = 160;
 
+// Where the C6 kernels put the rank factors a second time: in the mesh precision, in the order of the
+// mesh-sorted stencil records (slot = record of each atom; null: nowhere).
+struct RankOut {
+  void* c;
+  const int* slot;
+  int is_double;
+#ifdef __CUDACC__
+  __device__ __forceinline__ void put(int i, int r, int R, double v) const {
+    if (!slot) return;
+    const size_t k = (size_t)slot[i] * R + r;
+    if (is_double)
+      reinterpret_cast<double*>(c)[k] = v;
+    else
+      reinterpret_cast<float*>(c)[k] = (float)v;
+  }
+#endif
+};
+
 // fused CN + C6 factors over the cell list (one CTA or a few per bin, cn_max_blocks at most)
 int64_t cn_max_blocks(int64_t bins);
 int launch_cn_c6_cells(const CellGrid& g, int n, const CellList& cl, const int32_t* species, const Tables* tab,
-                       const double* eigvecs, int R, double* cn, double* c6, double* dc6, double* self_part, int* n_self_blocks,
-                       const HitStore& hs, cudaStream_t s);
+                       const double* eigvecs, int R, double* cn, double* c6, double* dc6, const RankOut& ro,
+                       double* self_part, int* n_self_blocks, const HitStore& hs, cudaStream_t s);
 // CN adjoint: grad = out_scale * (grad + dE/dx_CN) (Hartree/Bohr in); virial partials (9 per block)
 int launch_cn_adjoint_cells(const CellGrid& g, int n, const CellList& cl, const Tables* tab, const CellInfo* ci,
                             const double* gcn, double* grad, double out_scale, double* vir_part, int* n_blocks,
@@ -117,8 +135,8 @@ int launch_cn_adjoint_edges_seg(int64_t n_edges, int n, const double* pos, const
                                 double mask_r2, const double* gcn, const EdgeIndex& ei, double* gpos,
                                 double* gshift, cudaStream_t s);
 int launch_c6_atoms(int n, const int32_t* species, const Tables* tab, const double* eigvecs, int R,
-                    const double* cn, double* c6, double* dc6, double* self_part, int* n_self_blocks,
-                    cudaStream_t s);
+                    const double* cn, double* c6, double* dc6, const RankOut& ro, double* self_part,
+                    int* n_self_blocks, cudaStream_t s);
 
 // neighbour export
 int launch_nbr_count(const CellGrid& g, int n, const CellList& cl, const double* pos_ang, int* counts,
@@ -157,10 +175,12 @@ int launch_cellinfo(const double* cell, double scale, CellInfo* ci, cudaStream_t
 // energy, forces [n*3] and stress [9] made NaN when ci->stale is set
 int launch_poison_if_stale(const CellInfo* ci, int n, double* energy, double* forces, double* stress,
                            cudaStream_t s);
-int launch_mesh_keys(const MeshGeom& mg, int n, const double* pos, double pos_scale, const int32_t* species,
-                     const CellInfo* ci, int* keys, cudaStream_t s);
-// Per-atom stencil records in (tile, species)-sorted order, written by the spread launcher and
-// read again by the gather (T = mesh precision).
+// Per-atom stencil records in (tile, species)-sorted order, written by the preparation (the rank
+// factors by the C6 kernels) and read by the spread and the gather (T = mesh precision).
+struct PrepDev;
+// Cell list, mesh sort, stencil records and Green table of one call (fd3_prep.cuh)
+template <typename T, bool LAG>
+int launch_prep(const PrepDev& a, cudaStream_t s);
 struct MeshRecords {
   int4* b;      // [N] {base_x, base_y, base_z, species}
   void* w;      // [N][3][P] weights
@@ -178,15 +198,11 @@ int launch_yz_inverse(const MeshGeom& mg, int nchannels, int variant, const void
                       cudaStream_t s);
 // Whether the tile-staged (TMA) gather applies to this mesh for elements of `elem` bytes.
 bool gather_tile_applies(const MeshGeom& mg, size_t elem);
-// records: 0 = write the stencil records (with the rank factors) and spread; 1 = the records'
-// nodes and weights are written already (kSpreadRecordsOnly on another stream): write the rank
-// factors and spread; 2 (kSpreadRecordsOnly) = write the records' nodes and weights only (they
-// need the positions and the mesh sort, not C6).
-constexpr int kSpreadRecordsOnly = 2;
+// factors: the records' rank factors are written first, from these values per atom (null: they are
+// there already).
 template <typename T>
-int launch_spread(const MeshGeom& mg, int n, const double* pos, double pos_scale, const int32_t* species,
-                  const double* c6, const CellInfo* ci, const int* key_start, const int* order,
-                  const MeshRecords& rec, T* rho, cudaStream_t s, int records = 0);
+int launch_spread(const MeshGeom& mg, int n, const double* factors, const int* key_start, const int* order,
+                  const MeshRecords& rec, T* rho, cudaStream_t s);
 template <typename T>
 int launch_filter(const MeshGeom& mg, const CellInfo* ci, const GreenPair* gp, const GreenPairF* gpf,
                   const float4* gtab, const Tables* tab, const float* deconv, int spme, void* spec, double* part,
@@ -208,9 +224,6 @@ bool filter_mma_applies(const MeshGeom& mg);
 bool filter_mma_on(const MeshGeom& mg);
 int launch_filter_mma(const MeshGeom& mg, const CellInfo* ci, const float4* gtab, const Tables* tab,
                       const float* deconv, int spme, void* spec, double* part, int* n_blocks, cudaStream_t s);
-// mixed form: per-call table of G and its k-derivatives per species pair (gtab of the filter)
-int launch_green_table(const MeshGeom& mg, const CellInfo* ci, const GreenPair* gp, const Tables* tab, void* table,
-                       cudaStream_t s);
 size_t green_table_bytes(int S);
 int filter_max_blocks();
 int filter_default_kt(int S, int R, size_t tsize);

@@ -83,84 +83,6 @@ int launch_poison_if_stale(const CellInfo* ci, int n, double* energy, double* fo
   return FD3_OK;
 }
 
-__global__ void __launch_bounds__(256) k_mesh_keys(MeshDev g, int n, int P, const double* __restrict__ pos, double ps,
-                            const int32_t* __restrict__ species, const CellInfo* __restrict__ ci,
-                            int* __restrict__ keys) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  int base[3];
-  double xl[3];
-  mesh_locate<double>(pos, i, ps, ci, g.n[0], g.n[1], g.n[2], P, base, xl);
-  const int tx = base[0] / g.t[0], ty = base[1] / g.t[1], tz = base[2] / g.t[2];
-  keys[i] = ((tx * g.nt[1] + ty) * g.nt[2] + tz) * g.S + species[i];
-}
-
-int launch_mesh_keys(const MeshGeom& mg, int n, const double* pos, double pos_scale, const int32_t* species,
-                     const CellInfo* ci, int* keys, cudaStream_t s) {
-  if (n == 0) return FD3_OK;
-  const int tb = 256;
-  k_mesh_keys<<<(n + tb - 1) / tb, tb, 0, s>>>(to_dev(mg), n, mg.order, pos, pos_scale, species, ci, keys);
-  FD3_LAUNCHED();
-  return FD3_OK;
-}
-
-// ------------------------------------------------------------------ Green table (mixed form)
-// Thread per (pair X <= Y, knot j); pair index X S - X (X - 1) / 2 + (Y - X).
-__global__ void __launch_bounds__(256) k_green_table(MeshDev g, const CellInfo* __restrict__ ci,
-                                                     const GreenPair* __restrict__ gp,
-                                                     const Tables* __restrict__ tab, float4* __restrict__ out) {
-  const int S = g.S, NP = S * (S + 1) / 2;
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= NP * (kGreenKnots + 1)) return;
-  const int pi = e / (kGreenKnots + 1), j = e - pi * (kGreenKnots + 1);
-  int X = 0;
-  while ((X + 1) * S - (X + 1) * X / 2 <= pi) ++X;
-  const int Y = X + (pi - (X * S - X * (X - 1) / 2));
-  const GreenPair& q = gp[X * S + Y];
-  double rec[9];
-  for (int c = 0; c < 9; ++c) rec[c] = ci->recip[c];
-  const int n[3] = {g.n[0], g.n[1], g.n[2]};
-  const double h = green_kmax(rec, n) / kGreenKnots;
-  const double k = j * h;
-  const double s6 = tab->s6, s8 = tab->s8;
-  const double A6 = s6 * q.c6pre, A8 = 3.0 * s8 * q.qq * q.c8pre;
-  double G, G1, G2, G3;
-  if (k * q.R < 1e-15) {
-    // k = 0: the value of the reference's Taylor branch (pair_pot.py:146, G = a), and the
-    // derivatives of the closed form G = F(kR) / k there, G^(m)(0) = F^(m+1)(0) R^(m+1) / (m+1)
-    // with F'(0) = A6 - sqrt2 sin(pi/8) A8, F''(0) = 0, F'''(0) = -2 A6 + sqrt2 sin(pi/8) A8,
-    // F''''(0) = 3 A6. (The reference's k^2 coefficient of the C6 term, pair_pot.py:96, scales as
-    // R where the expansion of the closed form gives 2 pi^2 / (9 R); it multiplies k^2 = 0 there,
-    // so it never enters its results, but the interpolation between knots needs the true G''.)
-    const double a = s6 * q.c6s1 + 3.0 * s8 * q.qq * q.c8s1;
-    const double r2s8 = 0.54119610014619698440;   // sqrt(2) sin(pi/8)
-    const double R3 = q.R * q.R * q.R;
-    G = a;
-    G1 = 0.0;
-    G2 = (-2.0 * A6 + r2s8 * A8) * R3 / 3.0;
-    G3 = 3.0 * A6 * R3 * q.R / 4.0;
-  } else {
-    double n6[4], n8[4];
-    green_n(k * q.R, n6, n8);
-    double F[4];
-    for (int m = 0; m < 4; ++m) F[m] = A6 * n6[m] + A8 * n8[m];
-    G = F[0] / k;
-    G1 = (q.R * F[1] - G) / k;
-    G2 = (q.R * q.R * F[2] - 2.0 * G1) / k;
-    G3 = (q.R * q.R * q.R * F[3] - 3.0 * G2) / k;
-  }
-  out[e] = make_float4((float)G, (float)(h * G1), (float)(h * h * G2), (float)(h * h * h * G3));
-}
-
-int launch_green_table(const MeshGeom& mg, const CellInfo* ci, const GreenPair* gp, const Tables* tab,
-                       void* table, cudaStream_t s) {
-  const int NP = mg.S * (mg.S + 1) / 2;
-  const int total = NP * (kGreenKnots + 1);
-  k_green_table<<<(total + 255) / 256, 256, 0, s>>>(to_dev(mg), ci, gp, tab, reinterpret_cast<float4*>(table));
-  FD3_LAUNCHED();
-  return FD3_OK;
-}
-
 size_t green_table_bytes(int S) { return (size_t)S * (S + 1) / 2 * (kGreenKnots + 1) * sizeof(float4); }
 
 // Up to 8 species: grid-stride thread per k-point; the spectrum is updated in place (H = Gh S).

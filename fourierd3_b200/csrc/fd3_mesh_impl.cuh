@@ -79,38 +79,51 @@ __device__ __forceinline__ void stencil_weights(T x, T* w, T* dw) {
     bspline<P, T>(x, w, dw);
 }
 
-// ------------------------------------------------------------------ stencil records
-// One record per atom in (tile, species)-sorted order: first stencil node + species, the p
-// weights and their x-derivatives per axis, and the rank factors in the mesh precision. The
-// spread and the gather read these instead of recomputing the float64 mesh location per use.
-template <typename T, int P, bool LAG>
-__global__ void __launch_bounds__(256) k_mesh_records(MeshDev g, int n, const double* __restrict__ pos, double ps,
-                                                      const int32_t* __restrict__ species,
-                                                      const double* __restrict__ c6, const CellInfo* __restrict__ ci,
-                                                      const int* __restrict__ order, int4* __restrict__ rb,
-                                                      T* __restrict__ rw, T* __restrict__ rdw, T* __restrict__ rc) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const int atom = order[t];
-  int base[3];
-  T xl[3];
-  mesh_locate<T>(pos, atom, ps, ci, g.n[0], g.n[1], g.n[2], P, base, xl);
-  rb[t] = make_int4(base[0], base[1], base[2], species[atom]);
-  if (c6)
-    for (int r = 0; r < g.R; ++r) rc[(size_t)t * g.R + r] = (T)c6[(size_t)atom * g.R + r];
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    T w[P], dw[P];
-    stencil_weights<P, LAG, T>(xl[a], w, dw);
-#pragma unroll
-    for (int k = 0; k < P; ++k) {
-      rw[((size_t)t * 3 + a) * P + k] = w[k];
-      rdw[((size_t)t * 3 + a) * P + k] = dw[k];
-    }
+// ------------------------------------------------------------------ Green table (mixed form)
+// Entry e of the table: pair e / (kGreenKnots + 1) (X <= Y, index X S - X (X - 1) / 2 + (Y - X)) at
+// knot e mod (kGreenKnots + 1).
+__device__ inline float4 green_table_entry(const MeshDev& g, const double (&rec)[9],
+                                           const GreenPair* __restrict__ gp, const Tables* __restrict__ tab, int e) {
+  const int S = g.S;
+  const int pi = e / (kGreenKnots + 1), j = e - pi * (kGreenKnots + 1);
+  int X = 0;
+  while ((X + 1) * S - (X + 1) * X / 2 <= pi) ++X;
+  const int Y = X + (pi - (X * S - X * (X - 1) / 2));
+  const GreenPair& q = gp[X * S + Y];
+  const int n[3] = {g.n[0], g.n[1], g.n[2]};
+  const double h = green_kmax(rec, n) / kGreenKnots;
+  const double k = j * h;
+  const double s6 = tab->s6, s8 = tab->s8;
+  const double A6 = s6 * q.c6pre, A8 = 3.0 * s8 * q.qq * q.c8pre;
+  double G, G1, G2, G3;
+  if (k * q.R < 1e-15) {
+    // k = 0: the value of the reference's Taylor branch (pair_pot.py:146, G = a), and the
+    // derivatives of the closed form G = F(kR) / k there, G^(m)(0) = F^(m+1)(0) R^(m+1) / (m+1)
+    // with F'(0) = A6 - sqrt2 sin(pi/8) A8, F''(0) = 0, F'''(0) = -2 A6 + sqrt2 sin(pi/8) A8,
+    // F''''(0) = 3 A6. (The reference's k^2 coefficient of the C6 term, pair_pot.py:96, scales as
+    // R where the expansion of the closed form gives 2 pi^2 / (9 R); it multiplies k^2 = 0 there,
+    // so it never enters its results, but the interpolation between knots needs the true G''.)
+    const double a = s6 * q.c6s1 + 3.0 * s8 * q.qq * q.c8s1;
+    const double r2s8 = 0.54119610014619698440;   // sqrt(2) sin(pi/8)
+    const double R3 = q.R * q.R * q.R;
+    G = a;
+    G1 = 0.0;
+    G2 = (-2.0 * A6 + r2s8 * A8) * R3 / 3.0;
+    G3 = 3.0 * A6 * R3 * q.R / 4.0;
+  } else {
+    double n6[4], n8[4];
+    green_n(k * q.R, n6, n8);
+    double F[4];
+    for (int m = 0; m < 4; ++m) F[m] = A6 * n6[m] + A8 * n8[m];
+    G = F[0] / k;
+    G1 = (q.R * F[1] - G) / k;
+    G2 = (q.R * q.R * F[2] - 2.0 * G1) / k;
+    G3 = (q.R * q.R * q.R * F[3] - 3.0 * G2) / k;
   }
+  return make_float4((float)G, (float)(h * G1), (float)(h * h * G2), (float)(h * h * h * G3));
 }
 
-// The records' rank factors alone (sorted order), when the nodes and weights were written earlier.
+// The records' rank factors (sorted order) from values per atom.
 template <typename T>
 __global__ void __launch_bounds__(256) k_rank_factors(int n, int R, const double* __restrict__ c6,
                                                       const int* __restrict__ order, T* __restrict__ rc) {
@@ -675,22 +688,14 @@ inline int spread_zc(const MeshGeom& mg) {
   return zc < 1 ? 0 : zc;
 }
 
-template <typename T, int P, bool LAG>
-static int spread_r(const MeshGeom& mg, dim3 grid, int n, const double* pos, double ps, const int32_t* species,
-                    const double* c6, const CellInfo* ci, const int* ks, const int* order, const MeshRecords& rec,
-                    T* rho, cudaStream_t s, int records) {
+template <typename T, int P>
+static int spread_r(const MeshGeom& mg, dim3 grid, int n, const double* factors, const int* ks, const int* order,
+                    const MeshRecords& rec, T* rho, cudaStream_t s) {
   const MeshDev g = to_dev(mg);
-  if (n > 0) {
-    if (records == 1) {
-      k_rank_factors<T><<<(n + 255) / 256, 256, 0, s>>>(n, mg.R, c6, order, (T*)rec.c);
-    } else {
-      k_mesh_records<T, P, LAG><<<(n + 255) / 256, 256, 0, s>>>(g, n, pos, ps, species,
-                                                                records == kSpreadRecordsOnly ? nullptr : c6, ci,
-                                                                order, rec.b, (T*)rec.w, (T*)rec.dw, (T*)rec.c);
-    }
+  if (n > 0 && factors) {
+    k_rank_factors<T><<<(n + 255) / 256, 256, 0, s>>>(n, mg.R, factors, order, (T*)rec.c);
     FD3_LAUNCHED();
   }
-  if (records == kSpreadRecordsOnly) return FD3_OK;
   const int zc = spread_zc(mg);
   if (zc > 0) {
     // staged atoms per chunk: as many as let 3 (float) or 2 (double) CTAs share an SM
@@ -720,19 +725,15 @@ static int spread_r(const MeshGeom& mg, dim3 grid, int n, const double* pos, dou
 }
 
 template <typename T>
-int launch_spread(const MeshGeom& mg, int n, const double* pos, double pos_scale, const int32_t* species,
-                  const double* c6, const CellInfo* ci, const int* key_start, const int* order,
-                  const MeshRecords& rec, T* rho, cudaStream_t s, int records) {
+int launch_spread(const MeshGeom& mg, int n, const double* factors, const int* key_start, const int* order,
+                  const MeshRecords& rec, T* rho, cudaStream_t s) {
   if (mg.R > FD3_MAX_RANK || mg.order < 1 || mg.order > FD3_MAX_ORDER) return FD3_EINVAL;
   if (mg.t[0] > kSpTX || mg.t[1] > kSpTY || mg.t[2] > kSpTZ || mg.ns[0] * mg.ns[1] * mg.ns[2] > 125)
     return FD3_EINVAL;
   const dim3 grid(mg.nt[0] * mg.nt[1] * mg.nt[2], mg.S);
-#define FD3_SPREAD_CASE(PP)                                                                                  \
-  case PP:                                                                                                   \
-    return mg.lagrange ? spread_r<T, PP, true>(mg, grid, n, pos, pos_scale, species, c6, ci, key_start, order, rec, \
-                                               rho, s, records)                                              \
-                       : spread_r<T, PP, false>(mg, grid, n, pos, pos_scale, species, c6, ci, key_start, order, rec, \
-                                                rho, s, records);
+#define FD3_SPREAD_CASE(PP) \
+  case PP:                  \
+    return spread_r<T, PP>(mg, grid, n, factors, key_start, order, rec, rho, s);
   switch (mg.order) {
     FD3_SPREAD_CASE(1)
     FD3_SPREAD_CASE(2)

@@ -2,7 +2,6 @@
 #include "fd3_mesh_impl.cuh"
 
 namespace fd3 {
-template int launch_spread<double>(const MeshGeom&, int, const double*, double, const int32_t*, const double*,
-                                  const CellInfo*, const int*, const int*, const MeshRecords&, double*, cudaStream_t,
-                                  int);
+template int launch_spread<double>(const MeshGeom&, int, const double*, const int*, const int*, const MeshRecords&, double*,
+                               cudaStream_t);
 }  // namespace fd3

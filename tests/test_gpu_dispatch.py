@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 import torch
 
-from fourierd3_b200 import D3Model, neighbour_list
+from fourierd3_b200 import D3Model, neighbour_list, structures
 from oracle.neighbours import neighbour_list_cells
 from oracle.reference_port import OracleFourierD3
 
@@ -52,3 +52,12 @@ def test_cn_stage_from_image_only_cells_to_bins_beyond_the_stage(cuda_device, ed
     numbers = rng.choice([1, 6, 8], n_atoms)
     _against_oracle(cuda_device, frac @ cell, cell, numbers, precision, TOL[precision], method="spme",
                     mesh_spacing=1.2, interpolation_nodes=4, c6tol=1.0, r_cut=6.0)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n_atoms", [2047, 2048, 2049])
+def test_preparation_in_one_cta_and_in_several_launches(cuda_device, n_atoms, precision):
+    # the one-CTA sort takes up to 2,048 atoms; same density, one atom more or less
+    pos, cell, numbers = structures.hcno_box(seed=5, n_atoms=n_atoms)
+    _against_oracle(cuda_device, pos, cell, numbers, precision, TOL[precision], method="pme", mesh_spacing=1.2,
+                    interpolation_nodes=4, c6tol=1.0, r_cut=6.0)
