@@ -62,6 +62,8 @@ _SIGS = {
                                         ctypes.c_size_t, _vp, _vp, _vp, _vp, _vp]),
     "fd3_energy_forces_stress": (ctypes.c_int, [_vp, _c_int64, _vp, _vp, _dp, _vp, _c_double, _vp,
                                                 ctypes.c_size_t, _vp, _vp, _vp, _vp]),
+    "fd3_energy_forces_stress_hostcell": (ctypes.c_int, [_vp, _c_int64, _vp, _vp, _dp, _c_double, _vp,
+                                                         ctypes.c_size_t, _vp, _vp, _vp, _vp]),
     "fd3_atom_terms": (ctypes.c_int, [_vp, _c_int64, _c_int64, _vp, ctypes.c_size_t, _vp, _vp, _vp]),
     "fd3_direct_workspace_size": (ctypes.c_int, [_vp, _c_int64, _dp, _c_double, _c_double,
                                                  ctypes.POINTER(ctypes.c_size_t)]),

@@ -1033,13 +1033,13 @@ extern "C" int fd3_energy_edges(fd3_plan* p, int64_t n_atoms, const double* d_po
 }
 
 // ------------------------------------------------------------------ fused entry
-extern "C" int fd3_energy_forces_stress(fd3_plan* p, int64_t n_atoms, const double* d_pos_ang,
-                                        const int32_t* d_species, const double* h_cell_ang,
-                                        const double* d_cell_ang, double r_cut_ang, void* d_work,
-                                        size_t work_bytes, double* d_energy, double* d_forces, double* d_stress,
-                                        void* stream) {
-  if (!p || n_atoms < 1 || n_atoms > (int64_t)1 << 30 || !d_pos_ang || !d_species || !h_cell_ang || !d_cell_ang ||
-      !d_energy || !d_forces || !d_stress)
+// d_cell_ang null: the host cell is the call's cell
+static int energy_forces_stress(fd3_plan* p, int64_t n_atoms, const double* d_pos_ang, const int32_t* d_species,
+                                const double* h_cell_ang, const double* d_cell_ang, double r_cut_ang, void* d_work,
+                                size_t work_bytes, double* d_energy, double* d_forces, double* d_stress,
+                                void* stream) {
+  if (!p || n_atoms < 1 || n_atoms > (int64_t)1 << 30 || !d_pos_ang || !d_species || !h_cell_ang || !d_energy ||
+      !d_forces || !d_stress)
     return FD3_EINVAL;
   cudaStream_t s = (cudaStream_t)stream;
   const int N = (int)n_atoms;
@@ -1051,7 +1051,7 @@ extern "C" int fd3_energy_forces_stress(fd3_plan* p, int64_t n_atoms, const doub
   prof_begin(p, s);
   if (p->cnfunc == FD3_CN_D4) {
     // k-space D4 CN: no neighbour search (calculator.py:171-173)
-    FD3_TRY(launch_cellinfo(d_cell_ang, kAngToBohr, w.ci, s));
+    FD3_TRY(launch_cellinfo(d_cell_ang, kAngToBohr, w.ci, s, d_cell_ang ? nullptr : h_cell_ang));
     int n_self = 0, n_kspc = 0, n_mcell = 0, n_cnv = 0;
     FD3_TRY(prepare(p, nullptr, N, d_pos_ang, kAngToBohr, d_species, nullptr, nullptr, w, s));
     FD3_TRY(cn4_forward_any(p, N, d_pos_ang, kAngToBohr, d_species, w, s));
@@ -1089,6 +1089,24 @@ extern "C" int fd3_energy_forces_stress(fd3_plan* p, int64_t n_atoms, const doub
   FD3_TRY(launch_finalize(pa, w.ci, 1, kHartreeToEv, d_energy, d_stress, s));
   prof_mark(p, s, "finalize");
   return FD3_OK;
+}
+
+extern "C" int fd3_energy_forces_stress(fd3_plan* p, int64_t n_atoms, const double* d_pos_ang,
+                                        const int32_t* d_species, const double* h_cell_ang,
+                                        const double* d_cell_ang, double r_cut_ang, void* d_work,
+                                        size_t work_bytes, double* d_energy, double* d_forces, double* d_stress,
+                                        void* stream) {
+  if (!d_cell_ang) return FD3_EINVAL;
+  return energy_forces_stress(p, n_atoms, d_pos_ang, d_species, h_cell_ang, d_cell_ang, r_cut_ang, d_work, work_bytes,
+                              d_energy, d_forces, d_stress, stream);
+}
+
+extern "C" int fd3_energy_forces_stress_hostcell(fd3_plan* p, int64_t n_atoms, const double* d_pos_ang,
+                                                 const int32_t* d_species, const double* h_cell_ang, double r_cut_ang,
+                                                 void* d_work, size_t work_bytes, double* d_energy, double* d_forces,
+                                                 double* d_stress, void* stream) {
+  return energy_forces_stress(p, n_atoms, d_pos_ang, d_species, h_cell_ang, nullptr, r_cut_ang, d_work, work_bytes,
+                              d_energy, d_forces, d_stress, stream);
 }
 
 // ------------------------------------------------------------------ direct pair sum (accuracy oracle)

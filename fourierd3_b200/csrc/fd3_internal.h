@@ -169,7 +169,8 @@ struct MeshGeom {
   const float* win_axes;  // SPME, mixed form: sinc(m/n)^(2p) per axis, [nx | ny | nz/2+1] (null: none)
 };
 // h_expect (optional, host, copied into the launch): the cell the caller's host-side geometry (cell
-// list bins) was built from; a device cell that differs sets ci->stale
+// list bins) was built from; a device cell that differs sets ci->stale. Without a device cell
+// (null) h_expect is the cell.
 int launch_cellinfo(const double* cell, double scale, CellInfo* ci, cudaStream_t s,
                     const double* h_expect = nullptr);
 // energy, forces [n*3] and stress [9] made NaN when ci->stale is set

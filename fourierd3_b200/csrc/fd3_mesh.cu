@@ -28,8 +28,8 @@ __global__ void __launch_bounds__(32) k_cellinfo(const double* __restrict__ cell
   double m[9];
   bool stale = false;
   for (int k = 0; k < 9; ++k) {
-    m[k] = cell[k] * scale;
-    stale |= ex.on && cell[k] != ex.c[k];
+    m[k] = (cell ? cell[k] : ex.c[k]) * scale;   // no device cell: the host's, passed with the launch
+    stale |= cell && ex.on && cell[k] != ex.c[k];
   }
   ci->stale = stale ? 1.0 : 0.0;
   // utils.py:142-167 (adjugate / determinant) and utils.py:130-139 (cofactor determinant)

@@ -27,8 +27,8 @@ void check_rc(int rc, const char* what) {
 
 // pos (N,3) float64 Angstrom on the device; species (N,) int32 compact ids on the device;
 // cell (3,3) float64 Angstrom on the host (sizes the cell list); cell_dev the same cell on the
-// device (copied from cell on the current stream when absent; a device cell that differs from
-// the host cell makes every output NaN); work a uint8 device buffer of at least
+// device (absent: the host cell travels with the launches; a device cell that differs from the
+// host cell makes every output NaN); work a uint8 device buffer of at least
 // fd3_workspace_size bytes.
 std::tuple<at::Tensor, at::Tensor, at::Tensor> energy_forces_stress_cuda(int64_t plan, const at::Tensor& pos,
                                                                          const at::Tensor& species,
@@ -44,18 +44,24 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> energy_forces_stress_cuda(int64_t
               "cell must be a contiguous (3, 3) float64 host tensor");
   const c10::cuda::CUDAGuard guard(pos.device());
   const int64_t n = pos.size(0);
-  at::Tensor cell_dev = cell_dev_in.has_value() ? *cell_dev_in : cell.to(pos.device(), /*non_blocking=*/false);
-  check_cuda(cell_dev, at::kDouble, "cell_dev");
-  TORCH_CHECK(cell_dev.numel() == 9, "cell_dev must be (3, 3)");
+  if (cell_dev_in.has_value()) {
+    check_cuda(*cell_dev_in, at::kDouble, "cell_dev");
+    TORCH_CHECK(cell_dev_in->numel() == 9, "cell_dev must be (3, 3)");
+  }
   at::Tensor e = at::empty({}, pos.options());
   at::Tensor f = at::empty({n, 3}, pos.options());
   at::Tensor s = at::empty({3, 3}, pos.options());
   const cudaStream_t st = c10::cuda::getCurrentCUDAStream(pos.device().index()).stream();
-  check_rc(fd3_energy_forces_stress(reinterpret_cast<fd3_plan*>(plan), n, pos.data_ptr<double>(),
-                                    species.data_ptr<int32_t>(), cell.data_ptr<double>(),
-                                    cell_dev.data_ptr<double>(), r_cut, work.data_ptr(), (size_t)work.numel(),
-                                    e.data_ptr<double>(), f.data_ptr<double>(), s.data_ptr<double>(), st),
-           "fd3_energy_forces_stress");
+  fd3_plan* p = reinterpret_cast<fd3_plan*>(plan);
+  const int rc =
+      cell_dev_in.has_value()
+          ? fd3_energy_forces_stress(p, n, pos.data_ptr<double>(), species.data_ptr<int32_t>(), cell.data_ptr<double>(),
+                                     cell_dev_in->data_ptr<double>(), r_cut, work.data_ptr(), (size_t)work.numel(),
+                                     e.data_ptr<double>(), f.data_ptr<double>(), s.data_ptr<double>(), st)
+          : fd3_energy_forces_stress_hostcell(p, n, pos.data_ptr<double>(), species.data_ptr<int32_t>(),
+                                              cell.data_ptr<double>(), r_cut, work.data_ptr(), (size_t)work.numel(),
+                                              e.data_ptr<double>(), f.data_ptr<double>(), s.data_ptr<double>(), st);
+  check_rc(rc, "fd3_energy_forces_stress");
   return {e, f, s};
 }
 

@@ -135,6 +135,7 @@ class Engine:
             _native.check(lib.fd3_plan_create(ctypes.byref(d), ctypes.byref(self._plan)), "fd3_plan_create")
         self._keep = []
         self._work = None
+        self._fit = None
         self._species_dev = None
 
     def __del__(self):
@@ -298,8 +299,13 @@ class Engine:
         n = pos_ang.shape[0]
         cell_h = np.ascontiguousarray(cell_ang, dtype=np.float64).reshape(9)
         if work is None:
-            (nb, _) = self.cell_grid(cell_h, r_cut_ang)
-            work = self.workspace(n, nb[0] * nb[1] * nb[2])
+            # the workspace's size follows from these values alone: asked for again when one changes
+            fit = (n, float(r_cut_ang), cell_h.tobytes())
+            if fit != self._fit or self._work is None:
+                (nb, _) = self.cell_grid(cell_h, r_cut_ang)
+                self.workspace(n, nb[0] * nb[1] * nb[2])
+                self._fit = fit
+            work = self._work
         if species is None:
             species = self.species_tensor()
         if out is None:

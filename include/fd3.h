@@ -191,6 +191,13 @@ FD3_API int fd3_energy_forces_stress(fd3_plan* plan, int64_t n_atoms, const doub
                              double r_cut_ang, void* d_work, size_t work_bytes, double* d_energy,
                              double* d_forces, double* d_stress, void* stream);
 
+/* The same with the cell from the host alone: it travels with the launches (no copy to the
+ * device, nothing to wait for). Under stream capture the graph keeps the cell of the call. */
+FD3_API int fd3_energy_forces_stress_hostcell(fd3_plan* plan, int64_t n_atoms, const double* d_pos_ang,
+                             const int32_t* d_species, const double* h_cell_ang, double r_cut_ang,
+                             void* d_work, size_t work_bytes, double* d_energy, double* d_forces,
+                             double* d_stress, void* stream);
+
 /*
  * Direct pairwise D3(BJ) lattice sum in float64: the accuracy oracle of the reciprocal-space
  * methods (no reference counterpart; the reference checks its mesh methods against its own
