@@ -673,13 +673,15 @@ void carve(const fd3_plan* p, int64_t N, int64_t K_in, Carver& c, Work& w, int64
   // direct Ewald sum
   if (!mesh) {
     const int64_t nk = (int64_t)p->ens[0] * p->ens[1] * p->ens[2];
-    const int64_t nchunk = ewald_chunks((int)nk);
+    const int64_t nchunk = ewald_chunks(N > 0 ? N : 1, p->ens);
     w.ew.keys = c.take<int>(N);
     w.ew.counts = c.take<int>(p->S);
     w.ew.sp_start = c.take<int>(p->S + 1);
     w.ew.order = c.take<int>(N);
     w.ew.sp_of = c.take<int4>(N);
     w.ew.frac = c.take<double>(3 * N);
+    w.ew.ph_atom = c.take<double2>((size_t)N * (p->ens[0] + p->ens[1] + p->ens[2]));
+    w.ew.ph_m = c.take<double2>((size_t)N * (p->ens[0] + p->ens[1] + p->ens[2]));
     w.ew.spec = c.take<char>((size_t)C * nk * 2 * es);
     w.ew.hspec = c.take<char>((size_t)C * nk * 2 * es);
     w.ew.kpart = w.kspc_part;

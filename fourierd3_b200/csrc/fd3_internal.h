@@ -269,12 +269,13 @@ struct EwaldWork {
   int* order;     // [N] atoms sorted by species
   int4* sp_of;    // [N] species of each sorted slot
   double* frac;   // [N*3] fractional coordinates, sorted order
+  double2 *ph_atom, *ph_m;   // axis phases [N][n0 + n1 + n2] and [n0 + n1 + n2][N]
   void* spec;     // [S*R*nk] structure factors
   void* hspec;    // [S*R*nk] H = G S
   double* kpart;  // filter partials
   double* gpart;  // [N * nchunk * (R+3)] gather partials
 };
-int ewald_chunks(int nk);
+int ewald_chunks(int64_t n, const int* ns);
 template <typename T>
 int launch_ewald(const EwaldGeom& eg, int n, const double* pos, double ps, const int32_t* species,
                  const double* c6, const double* dc6, const CellInfo* ci, const GreenPair* gp, const Tables* tab,

@@ -61,3 +61,12 @@ def test_preparation_in_one_cta_and_in_several_launches(cuda_device, n_atoms, pr
     pos, cell, numbers = structures.hcno_box(seed=5, n_atoms=n_atoms)
     _against_oracle(cuda_device, pos, cell, numbers, precision, TOL[precision], method="pme", mesh_spacing=1.2,
                     interpolation_nodes=4, c6tol=1.0, r_cut=6.0)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n_atoms,z_max,k_cutoff", [(1, 1, 2.0), (33, 8, 3.1), (130, 30, 2.2)])
+def test_ewald_sums_over_tiles_rows_and_many_species(cuda_device, n_atoms, z_max, k_cutoff, precision):
+    # odd and even Miller boxes, one species and dozens (several filter tiles, more than 8 ranks or not)
+    pos, cell, numbers = structures.random_box(seed=n_atoms, n_atoms=n_atoms, z_max=z_max)
+    _against_oracle(cuda_device, pos, cell, numbers, precision, TOL[precision], method="ewald", k_cutoff=k_cutoff,
+                    c6tol=0.05, r_cut=6.0)
