@@ -852,7 +852,7 @@ static int mesh_pipeline(fd3_plan* p, int N, const double* pos, double ps, const
         FD3_CUFFT(cufftExecC2R(p->inv2, (cufftComplex*)w.spec, (cufftReal*)w.rho));
     }
     prof_mark(p, s, "fft_c2r");
-    FD3_TRY(launch_gather<T>(mg, N, pos, ps, species, w.c6, w.dc6, w.ci, p->d_tab, w.morder, w.mstart, w.rec,
+    FD3_TRY(launch_gather<T>(mg, N, pos, ps, w.c6, w.dc6, w.ci, p->d_tab, w.morder, w.mstart, w.rec,
                              (const T*)w.rho, w.gcn, gpos, mcell, n_mcell, s));
     prof_mark(p, s, "gather");
     return FD3_OK;
@@ -877,7 +877,7 @@ static int mesh_pipeline(fd3_plan* p, int N, const double* pos, double ps, const
   else
     FD3_CUFFT(cufftExecC2R(p->inv, (cufftComplex*)hspec, (cufftReal*)w.rho));
   prof_mark(p, s, "fft_c2r");
-  FD3_TRY(launch_gather<T>(mg, N, pos, ps, species, w.c6, w.dc6, w.ci, p->d_tab, w.morder, w.mstart, w.rec,
+  FD3_TRY(launch_gather<T>(mg, N, pos, ps, w.c6, w.dc6, w.ci, p->d_tab, w.morder, w.mstart, w.rec,
                            (const T*)w.rho, w.gcn, gpos, mcell, n_mcell, s));
   prof_mark(p, s, "gather");
   return FD3_OK;

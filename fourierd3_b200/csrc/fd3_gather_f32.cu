@@ -14,7 +14,7 @@ bool gather_tile_applies(const MeshGeom& mg, size_t elem) {
   return (size_t)mg.R * b.x * b.y * b.z * elem + 128 <= kTileGatherSmemCap;
 }
 
-template int launch_gather<float>(const MeshGeom&, int, const double*, double, const int32_t*, const double*,
-                                  const double*, const CellInfo*, const Tables*, const int*, const int*,
+template int launch_gather<float>(const MeshGeom&, int, const double*, double, const double*, const double*,
+                                  const CellInfo*, const Tables*, const int*, const int*,
                                   const MeshRecords&, const float*, double*, double*, double*, int*, cudaStream_t);
 }  // namespace fd3

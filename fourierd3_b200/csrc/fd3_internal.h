@@ -231,8 +231,7 @@ int filter_default_kt(int S, int R, size_t tsize);
 int spread_chunk_in_effect(const MeshGeom& mg, size_t tsize);
 bool filter_kt_valid(int kt, int S, int R, size_t tsize);
 template <typename T>
-int launch_gather(const MeshGeom& mg, int n, const double* pos, double pos_scale, const int32_t* species,
-                  const double* c6, const double* dc6, const CellInfo* ci, const Tables* tab, const int* order,
+int launch_gather(const MeshGeom& mg, int n, const double* pos, double pos_scale, const double* c6, const double* dc6, const CellInfo* ci, const Tables* tab, const int* order,
                   const int* key_start, const MeshRecords& rec, const T* phi, double* gcn, double* gpos,
                   double* mcell_part, int* n_blocks, cudaStream_t s);
 

@@ -755,144 +755,31 @@ namespace fd3 {
 
 constexpr int kGatherWarps = 8;
 
-template <typename T, int P, bool LAG, int MAXR>
-__global__ void __launch_bounds__(32 * kGatherWarps) k_gather(MeshDev g, int n, const double* __restrict__ pos,
-                                                              double ps, const int32_t* __restrict__ species,
-                                                              const double* __restrict__ c6,
-                                                              const double* __restrict__ dc6,
-                                                              const CellInfo* __restrict__ ci,
-                                                              const Tables* __restrict__ tab,
-                                                              const int* __restrict__ order,
-                                                              const int4* __restrict__ rb, const T* __restrict__ rw,
-                                                              const T* __restrict__ rdw,
-                                                              const T* __restrict__ phi, double* __restrict__ gcn,
-                                                              double* __restrict__ gpos,
-                                                              double* __restrict__ mcell_part) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int t = blockIdx.x * kGatherWarps + wid;
-  const int R = g.R;
-  double mc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  if (t < n) {
-    const int i = order[t];
-    const int4 b4 = rb[t];
-    const int s = b4.w;
-    const int base[3] = {b4.x, b4.y, b4.z};
-    T w0[P], dw0[P];
-#pragma unroll
-    for (int k = 0; k < P; ++k) {
-      w0[k] = rw[((size_t)t * 3) * P + k];
-      dw0[k] = rdw[((size_t)t * 3) * P + k];
-    }
-    double cl[MAXR];
-#pragma unroll
-    for (int r = 0; r < MAXR; ++r) cl[r] = r < R ? c6[(size_t)i * R + r] * tab->eigs[r] : 0.0;
-    const size_t M = (size_t)g.n[0] * g.n[1] * g.n[2];
-    double pr[MAXR];
-#pragma unroll
-    for (int r = 0; r < MAXR; ++r) pr[r] = 0.0;
-    double gu0 = 0, gu1 = 0, gu2 = 0;
-    // lanes over the (y, z) stencil nodes, x nodes unrolled: every weight index is static
-    int ixs[P];
-#pragma unroll
-    for (int kx = 0; kx < P; ++kx) {
-      int ix = base[0] + kx;
-      while (ix >= g.n[0]) ix -= g.n[0];
-      ixs[kx] = ix;
-    }
-    for (int q = lane; q < P * P; q += 32) {
-      const int ky = q / P, kz = q - ky * P;
-      const T wy = rw[((size_t)t * 3 + 1) * P + ky], dwy = rdw[((size_t)t * 3 + 1) * P + ky];
-      const T wz = rw[((size_t)t * 3 + 2) * P + kz], dwz = rdw[((size_t)t * 3 + 2) * P + kz];
-      int iy = base[1] + ky;
-      while (iy >= g.n[1]) iy -= g.n[1];
-      int iz = base[2] + kz;
-      while (iz >= g.n[2]) iz -= g.n[2];
-      const T wyz = wy * wz, dyz = dwy * wz, ydz = wy * dwz;
-#pragma unroll
-      for (int kx = 0; kx < P; ++kx) {
-        const size_t m = ((size_t)ixs[kx] * g.n[1] + iy) * g.n[2] + iz;
-        const T W = w0[kx] * wyz;
-        const T Wx = dw0[kx] * wyz;
-        const T Wy = w0[kx] * dyz;
-        const T Wz = w0[kx] * ydz;
-        double cp = 0.0;
-#pragma unroll
-        for (int r = 0; r < MAXR; ++r) {
-          if (r < R) {
-            const double ph = (double)phi[((size_t)s * R + r) * M + m];
-            pr[r] += (double)W * ph;
-            cp += cl[r] * ph;
-          }
-        }
-        gu0 += (double)Wx * cp;
-        gu1 += (double)Wy * cp;
-        gu2 += (double)Wz * cp;
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < MAXR; ++r) pr[r] = warp_sum(pr[r]);
-    gu0 = warp_sum(gu0);
-    gu1 = warp_sum(gu1);
-    gu2 = warp_sum(gu2);
-    const double inv_vol = 1.0 / ci->volume;
-    // dE/dc_r = -(lambda_r / Omega) P_r + lambda_r c_r phi_ss(0); g = sum_r dE/dc_r dc_r/dCN
-    double gsum = 0.0;
-#pragma unroll
-    for (int r = 0; r < MAXR; ++r) {
-      if (r < R) {
-        const double lam = tab->eigs[r];
-        const double c = c6[(size_t)i * R + r];
-        const double dEdc = -lam * inv_vol * pr[r] + lam * c * tab->selfcont[s];
-        gsum += dEdc * dc6[(size_t)i * R + r];
-      }
-    }
-    // dE/du_a = -(1/Omega) sum_r lambda_r c_r sum_m phi dW/du_a; dE/dx_b = sum_a dE/du_a n_a inv[b][a]
-    const double du[3] = {-inv_vol * gu0, -inv_vol * gu1, -inv_vol * gu2};
-    double gx[3];
-#pragma unroll
-    for (int b = 0; b < 3; ++b)
-      gx[b] = du[0] * g.n[0] * ci->inv[3 * b + 0] + du[1] * g.n[1] * ci->inv[3 * b + 1] +
-              du[2] * g.n[2] * ci->inv[3 * b + 2];
-    if (lane == 0) {
-      gcn[i] = gsum;
-      gpos[3 * i] = gx[0];
-      gpos[3 * i + 1] = gx[1];
-      gpos[3 * i + 2] = gx[2];
-      // mesh part of dE/dcell with positions fixed: -sum_i s_iA g_ia (s = fractional coordinate)
-      if (mcell_part) {
-        const double x0 = pos[3 * i] * ps, x1 = pos[3 * i + 1] * ps, x2 = pos[3 * i + 2] * ps;
-        double sf[3];
-#pragma unroll
-        for (int A = 0; A < 3; ++A) sf[A] = x0 * ci->inv[A] + x1 * ci->inv[3 + A] + x2 * ci->inv[6 + A];
-#pragma unroll
-        for (int A = 0; A < 3; ++A)
-#pragma unroll
-          for (int a = 0; a < 3; ++a) mc[3 * A + a] = sf[A] * gx[a];
-      }
-    }
-  }
-  if (mcell_part) block_sum_store<9>(mc, mcell_part + 9 * blockIdx.x);
-}
-
-// Fused-path gather, z-run form: lanes over the (x, y) stencil columns; each lane reads the P
-// z-values of its column from every rank channel with aligned 16-byte vector loads (the column
-// start is rounded down to the vector boundary; a warp-uniform offset O in [0, 16/sizeof(T))
-// selects the run, so every register index stays static) and forms
-//   zr_r = sum_z w_z phi_r,  cp_z = sum_r lambda_r c_r phi_r,  s0 = sum_z w_z cp_z,  s2 = sum_z w'_z cp_z,
-// in T, then accumulates P_r = sum W phi_r and the three spline-gradient sums in float64.
+// Gather, one warp per atom: lanes over the (x, y) stencil columns; each lane reads the P z-values of
+// its column from RC rank channels at a time with aligned 16-byte vector loads (the column start is
+// rounded down to the vector boundary; a warp-uniform offset O in [0, 16/sizeof(T)) selects the run,
+// so every register index stays static) and forms
+//   zr_r = sum_z w_z phi_r,  cp_z = sum_r lambda_r c_r phi_r,  s0 = sum_z w_z cp_z,  s2 = sum_z w'_z cp_z
+// in TA, then accumulates P_r = sum W phi_r and the three spline-gradient sums in float64.
 // A column that wraps the periodic z edge (or a mesh whose nz is not a multiple of the vector
 // width) is read element by element with the offset 0.
-template <typename T, int P, int MAXR, int O, int NE>
-__device__ __forceinline__ void zrun_sums(const T (&v)[MAXR][NE], int R, const T (&wz)[P], const T (&cl)[MAXR],
-                                          T (&zr)[MAXR], T (&cp)[P]) {
+// Ranks go in chunks of RC, so any rank and order runs on registers and vector loads. (Orders above 5
+// and more than 4 or 8 ranks, and every call with cell gradients, took a kernel that read single
+// values and held all ranks: 178 us at 12,000 HCNO atoms, p = 6, 5 ranks, float, now 62; 103 us for the
+// module at 20,736 SiO2 atoms, p = 5, 4 ranks, now 78.)
+// TA: float sums for the orders and ranks of the mixed form that have always had them (launch rule),
+// float64 otherwise.
+template <typename T, typename TA, int P, int RC, int O, int NE>
+__device__ __forceinline__ void zrun_sums(const T (&v)[RC][NE], int nr, const T (&wz)[P], const TA (&cl)[RC],
+                                          TA (&zr)[RC], TA (&cp)[P]) {
 #pragma unroll
-  for (int r = 0; r < MAXR; ++r) {
-    if (r < R) {
-      T a = T(0);
+  for (int r = 0; r < RC; ++r) {
+    if (r < nr) {
+      TA a = TA(0);
 #pragma unroll
       for (int kz = 0; kz < P; ++kz) {
-        const T f = v[r][O + kz];
-        a += wz[kz] * f;
+        const TA f = (TA)v[r][O + kz];
+        a += (TA)wz[kz] * f;
         cp[kz] += cl[r] * f;
       }
       zr[r] = a;
@@ -900,136 +787,155 @@ __device__ __forceinline__ void zrun_sums(const T (&v)[MAXR][NE], int R, const T
   }
 }
 
-template <typename T, int P, int MAXR>
-__global__ void __launch_bounds__(32 * kGatherWarps, (sizeof(T) == 4 && MAXR <= 4 && P <= 5) ? 4 : 1) k_gather_z(MeshDev g, int n, const double* __restrict__ c6,
-                                                                const double* __restrict__ dc6,
-                                                                const CellInfo* __restrict__ ci,
-                                                                const Tables* __restrict__ tab,
-                                                                const int* __restrict__ order,
-                                                                const int4* __restrict__ rb,
-                                                                const T* __restrict__ rw, const T* __restrict__ rdw,
-                                                                const T* __restrict__ phi, double* __restrict__ gcn,
-                                                                double* __restrict__ gpos) {
+// MC: the positions-fixed cell partials of the edge-list path too. ONE: all ranks are one chunk (the
+// loop over chunks costs the common case registers: 139,968 atoms, float, 4 ranks: 205 us without it, 295 us with).
+template <typename T, typename TA, int P, int RC, bool MC, bool ONE>
+__global__ void __launch_bounds__(32 * kGatherWarps, ONE && sizeof(TA) == 4 && P <= 5 ? 4 : 2) k_gather_z(
+    MeshDev g, int n, const double* __restrict__ pos, double ps, const double* __restrict__ c6,
+    const double* __restrict__ dc6, const CellInfo* __restrict__ ci, const Tables* __restrict__ tab,
+    const int* __restrict__ order, const int4* __restrict__ rb, const T* __restrict__ rw, const T* __restrict__ rdw,
+    const T* __restrict__ phi, double* __restrict__ gcn, double* __restrict__ gpos,
+    double* __restrict__ mcell_part) {
   constexpr int VW = 16 / (int)sizeof(T);          // elements per 16-byte vector
   constexpr int NV = (VW - 1 + P + VW - 1) / VW;   // vectors covering a run at any offset
   constexpr int NE = NV * VW;
   using V = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int t = blockIdx.x * kGatherWarps + wid;
-  if (t >= n) return;
-  const int R = g.R;
-  const int i = order[t];
-  const int4 b4 = rb[t];
-  const int s = b4.w;
-  const T* wr = rw + (size_t)t * 3 * P;
-  const T* dwr = rdw + (size_t)t * 3 * P;
-  T wz[P], dwz[P];
+  double mc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  if (t < n) {
+    const int R = g.R;
+    const int i = order[t];
+    const int4 b4 = rb[t];
+    const int s = b4.w;
+    const T* wr = rw + (size_t)t * 3 * P;
+    const T* dwr = rdw + (size_t)t * 3 * P;
+    T wz[P], dwz[P];
 #pragma unroll
-  for (int k = 0; k < P; ++k) {
-    wz[k] = wr[2 * P + k];
-    dwz[k] = dwr[2 * P + k];
-  }
-  T cl[MAXR];
+    for (int k = 0; k < P; ++k) {
+      wz[k] = wr[2 * P + k];
+      dwz[k] = dwr[2 * P + k];
+    }
+    const int n2 = g.n[2];
+    const int iz0 = b4.z;
+    const bool scalar = iz0 + P > n2 || (n2 % VW) != 0;   // warp-uniform
+    const int o = scalar ? 0 : iz0 % VW;
+    const int za = iz0 - o;
+    const int nvec = (o + P + VW - 1) / VW;
+    const size_t M = (size_t)g.n[0] * g.n[1] * n2;
+    const double inv_vol = 1.0 / ci->volume;
+    double gu0 = 0.0, gu1 = 0.0, gu2 = 0.0, gsum = 0.0;
+    for (int rc0 = 0; rc0 < (ONE ? 1 : R); rc0 += RC) {
+      const int nr = ONE || R - rc0 < RC ? R - rc0 : RC;
+      TA cl[RC];
 #pragma unroll
-  for (int r = 0; r < MAXR; ++r) cl[r] = r < R ? (T)(c6[(size_t)i * R + r] * tab->eigs[r]) : T(0);
-  const int n2 = g.n[2];
-  const int iz0 = b4.z;
-  const bool scalar = iz0 + P > n2 || (n2 % VW) != 0;   // warp-uniform
-  const int o = scalar ? 0 : iz0 % VW;
-  const int za = iz0 - o;
-  const int nvec = (o + P + VW - 1) / VW;
-  const size_t M = (size_t)g.n[0] * g.n[1] * n2;
-  double pr[MAXR];
+      for (int r = 0; r < RC; ++r) cl[r] = r < nr ? (TA)(c6[(size_t)i * R + rc0 + r] * tab->eigs[rc0 + r]) : TA(0);
+      double pr[RC];
 #pragma unroll
-  for (int r = 0; r < MAXR; ++r) pr[r] = 0.0;
-  double gu0 = 0.0, gu1 = 0.0, gu2 = 0.0;
-  for (int q = lane; q < P * P; q += 32) {
-    const int kx = q / P, ky = q - kx * P;
-    int ix = b4.x + kx;
-    while (ix >= g.n[0]) ix -= g.n[0];   // a stencil wider than the mesh wraps more than once
-    int iy = b4.y + ky;
-    while (iy >= g.n[1]) iy -= g.n[1];
-    const T wx = wr[kx], dwx = dwr[kx], wy = wr[P + ky], dwy = dwr[P + ky];
-    const T* col = phi + (size_t)s * R * M + ((size_t)ix * g.n[1] + iy) * n2;
-    T v[MAXR][NE];
+      for (int r = 0; r < RC; ++r) pr[r] = 0.0;
+      for (int q = lane; q < P * P; q += 32) {
+        const int kx = q / P, ky = q - kx * P;
+        int ix = b4.x + kx;
+        while (ix >= g.n[0]) ix -= g.n[0];   // a stencil wider than the mesh wraps more than once
+        int iy = b4.y + ky;
+        while (iy >= g.n[1]) iy -= g.n[1];
+        const T wx = wr[kx], dwx = dwr[kx], wy = wr[P + ky], dwy = dwr[P + ky];
+        const T* col = phi + ((size_t)s * R + rc0) * M + ((size_t)ix * g.n[1] + iy) * n2;
+        T v[RC][NE];
 #pragma unroll
-    for (int r = 0; r < MAXR; ++r) {
-      if (r < R) {
-        const T* src = col + (size_t)r * M;
-        if (!scalar) {
-          const V* vs = reinterpret_cast<const V*>(src + za);
+        for (int r = 0; r < RC; ++r) {
+          if (r < nr) {
+            const T* src = col + (size_t)r * M;
+            if (!scalar) {
+              const V* vs = reinterpret_cast<const V*>(src + za);
 #pragma unroll
-          for (int j = 0; j < NV; ++j)
-            if (j < nvec) *reinterpret_cast<V*>(&v[r][j * VW]) = vs[j];
-        } else {
+              for (int j = 0; j < NV; ++j)
+                if (j < nvec) *reinterpret_cast<V*>(&v[r][j * VW]) = vs[j];
+            } else {
 #pragma unroll
-          for (int kz = 0; kz < P; ++kz) {
-            int iz = iz0 + kz;
-            while (iz >= n2) iz -= n2;
-            v[r][kz] = src[iz];
+              for (int kz = 0; kz < P; ++kz) {
+                int iz = iz0 + kz;
+                while (iz >= n2) iz -= n2;
+                v[r][kz] = src[iz];
+              }
+            }
           }
+        }
+        TA zr[RC], cp[P];
+#pragma unroll
+        for (int kz = 0; kz < P; ++kz) cp[kz] = TA(0);
+#pragma unroll
+        for (int r = 0; r < RC; ++r) zr[r] = TA(0);
+        if constexpr (VW == 4) {
+          switch (o) {
+            case 0: zrun_sums<T, TA, P, RC, 0, NE>(v, nr, wz, cl, zr, cp); break;
+            case 1: zrun_sums<T, TA, P, RC, 1, NE>(v, nr, wz, cl, zr, cp); break;
+            case 2: zrun_sums<T, TA, P, RC, 2, NE>(v, nr, wz, cl, zr, cp); break;
+            default: zrun_sums<T, TA, P, RC, 3, NE>(v, nr, wz, cl, zr, cp); break;
+          }
+        } else {
+          if (o == 0)
+            zrun_sums<T, TA, P, RC, 0, NE>(v, nr, wz, cl, zr, cp);
+          else
+            zrun_sums<T, TA, P, RC, 1, NE>(v, nr, wz, cl, zr, cp);
+        }
+        TA s0 = TA(0), s2 = TA(0);
+#pragma unroll
+        for (int kz = 0; kz < P; ++kz) {
+          s0 += (TA)wz[kz] * cp[kz];
+          s2 += (TA)dwz[kz] * cp[kz];
+        }
+        const TA wxy = (TA)wx * (TA)wy;
+#pragma unroll
+        for (int r = 0; r < RC; ++r) pr[r] += (double)(wxy * zr[r]);
+        gu0 += (double)((TA)dwx * (TA)wy * s0);
+        gu1 += (double)((TA)wx * (TA)dwy * s0);
+        gu2 += (double)(wxy * s2);
+      }
+      // dE/dc_r = -(lambda_r / Omega) P_r + lambda_r c_r phi_ss(0); g = sum_r dE/dc_r dc_r/dCN
+#pragma unroll
+      for (int r = 0; r < RC; ++r) {
+        pr[r] = warp_sum(pr[r]);
+        if (r < nr) {
+          const double lam = tab->eigs[rc0 + r];
+          const double c = c6[(size_t)i * R + rc0 + r];
+          const double dEdc = -lam * inv_vol * pr[r] + lam * c * tab->selfcont[s];
+          gsum += dEdc * dc6[(size_t)i * R + rc0 + r];
         }
       }
     }
-    T zr[MAXR], cp[P];
+    gu0 = warp_sum(gu0);
+    gu1 = warp_sum(gu1);
+    gu2 = warp_sum(gu2);
+    if (lane == 0) {
+      // dE/du_a = -(1/Omega) sum_r lambda_r c_r sum_m phi dW/du_a; dE/dx_b = sum_a dE/du_a n_a inv[b][a]
+      const double du[3] = {-inv_vol * gu0, -inv_vol * gu1, -inv_vol * gu2};
+      gcn[i] = gsum;
+      double gx[3];
 #pragma unroll
-    for (int kz = 0; kz < P; ++kz) cp[kz] = T(0);
-#pragma unroll
-    for (int r = 0; r < MAXR; ++r) zr[r] = T(0);
-    if constexpr (VW == 4) {
-      switch (o) {
-        case 0: zrun_sums<T, P, MAXR, 0, NE>(v, R, wz, cl, zr, cp); break;
-        case 1: zrun_sums<T, P, MAXR, 1, NE>(v, R, wz, cl, zr, cp); break;
-        case 2: zrun_sums<T, P, MAXR, 2, NE>(v, R, wz, cl, zr, cp); break;
-        default: zrun_sums<T, P, MAXR, 3, NE>(v, R, wz, cl, zr, cp); break;
+      for (int b = 0; b < 3; ++b) {
+        gx[b] = du[0] * g.n[0] * ci->inv[3 * b + 0] + du[1] * g.n[1] * ci->inv[3 * b + 1] +
+                du[2] * g.n[2] * ci->inv[3 * b + 2];
+        gpos[3 * i + b] = gx[b];
       }
-    } else {
-      if (o == 0)
-        zrun_sums<T, P, MAXR, 0, NE>(v, R, wz, cl, zr, cp);
-      else
-        zrun_sums<T, P, MAXR, 1, NE>(v, R, wz, cl, zr, cp);
-    }
-    T s0 = T(0), s2 = T(0);
+      // mesh part of dE/dcell with positions fixed: -sum_i s_iA g_ia (s = fractional coordinate)
+      if constexpr (MC) {
+        const double x0 = pos[3 * i] * ps, x1 = pos[3 * i + 1] * ps, x2 = pos[3 * i + 2] * ps;
 #pragma unroll
-    for (int kz = 0; kz < P; ++kz) {
-      s0 += wz[kz] * cp[kz];
-      s2 += dwz[kz] * cp[kz];
-    }
-    const T wxy = wx * wy;
+        for (int A = 0; A < 3; ++A) {
+          const double sf = x0 * ci->inv[A] + x1 * ci->inv[3 + A] + x2 * ci->inv[6 + A];
 #pragma unroll
-    for (int r = 0; r < MAXR; ++r) pr[r] += (double)(wxy * zr[r]);
-    gu0 += (double)(dwx * wy * s0);
-    gu1 += (double)(wx * dwy * s0);
-    gu2 += (double)(wxy * s2);
-  }
-#pragma unroll
-  for (int r = 0; r < MAXR; ++r) pr[r] = warp_sum(pr[r]);
-  gu0 = warp_sum(gu0);
-  gu1 = warp_sum(gu1);
-  gu2 = warp_sum(gu2);
-  if (lane != 0) return;
-  const double inv_vol = 1.0 / ci->volume;
-  double gsum = 0.0;
-#pragma unroll
-  for (int r = 0; r < MAXR; ++r) {
-    if (r < R) {
-      const double lam = tab->eigs[r];
-      const double c = c6[(size_t)i * R + r];
-      const double dEdc = -lam * inv_vol * pr[r] + lam * c * tab->selfcont[s];
-      gsum += dEdc * dc6[(size_t)i * R + r];
+          for (int a = 0; a < 3; ++a) mc[3 * A + a] = sf * gx[a];
+        }
+      }
     }
   }
-  const double du[3] = {-inv_vol * gu0, -inv_vol * gu1, -inv_vol * gu2};
-  gcn[i] = gsum;
-#pragma unroll
-  for (int b = 0; b < 3; ++b)
-    gpos[3 * i + b] = du[0] * g.n[0] * ci->inv[3 * b + 0] + du[1] * g.n[1] * ci->inv[3 * b + 1] +
-                      du[2] * g.n[2] * ci->inv[3 * b + 2];
+  if constexpr (MC) block_sum_store<9>(mc, mcell_part + 9 * blockIdx.x);
 }
 
-template <typename T, int P, bool LAG>
-static int gather_r(const MeshGeom& mg, int blocks, int n, const double* pos, double ps, const int32_t* species,
-                    const double* c6, const double* dc6, const CellInfo* ci, const Tables* tab, const int* order,
+template <typename T, int P>
+static int gather_r(const MeshGeom& mg, int blocks, int n, const double* pos, double ps, const double* c6,
+                    const double* dc6, const CellInfo* ci, const Tables* tab, const int* order,
                     const int* key_start, const MeshRecords& rec, const T* phi, double* gcn, double* gpos,
                     double* mcell, int* n_mcell, cudaStream_t s) {
   // tile-staged gather (one CTA per (tile, species) key, the key's mesh box staged once by TMA)
@@ -1040,52 +946,40 @@ static int gather_r(const MeshGeom& mg, int blocks, int n, const double* pos, do
   }
   const MeshDev g = to_dev(mg);
   *n_mcell = mcell ? blocks : 0;
-  const int tb = 32 * kGatherWarps;
-  const int4* rb = rec.b;
-  const T* rw = (const T*)rec.w;
-  const T* rdw = (const T*)rec.dw;
-  // z-run gather where its register arrays (ranks x run) stay small: float up to 4 ranks at any
-  // order or 8 ranks up to order 5; double up to 4 ranks up to order 5
-  constexpr bool z4 = sizeof(T) == 4 || P <= 5;
-  constexpr bool z8 = sizeof(T) == 4 && P <= 5;
-  if (!mcell && ((mg.R <= 4 && z4) || (mg.R <= 8 && z8))) {
-    if (mg.R <= 4)
-      k_gather_z<T, P, 4><<<blocks, tb, 0, s>>>(g, n, c6, dc6, ci, tab, order, rb, rw, rdw, phi, gcn, gpos);
-    else if constexpr (z8)
-      k_gather_z<T, P, 8><<<blocks, tb, 0, s>>>(g, n, c6, dc6, ci, tab, order, rb, rw, rdw, phi, gcn, gpos);
-    FD3_LAUNCHED();
-    return FD3_OK;
+  constexpr int RC = sizeof(T) == 4 || P <= 5 ? 4 : 2;   // rank values in flight per lane: RC (P + 3) or RC (P + 1)
+  auto launch = [&](auto kern) {
+    kern<<<blocks, 32 * kGatherWarps, 0, s>>>(g, n, pos, ps, c6, dc6, ci, tab, order, rec.b, (const T*)rec.w,
+                                              (const T*)rec.dw, phi, gcn, gpos, mcell);
+  };
+#define FD3_GATHER(TA, MC) \
+  (mg.R <= RC ? launch(k_gather_z<T, TA, P, RC, MC, true>) : launch(k_gather_z<T, TA, P, RC, MC, false>))
+  if (mcell) {
+    FD3_GATHER(double, true);
+  } else if constexpr (sizeof(T) == 4) {
+    // float sums: up to 4 ranks at any order, up to 8 ranks up to order 5
+    if (mg.R <= 4 || (mg.R <= 8 && P <= 5))
+      FD3_GATHER(float, false);
+    else
+      FD3_GATHER(double, false);
+  } else {
+    FD3_GATHER(double, false);
   }
-  if (mg.R <= 4)
-    k_gather<T, P, LAG, 4><<<blocks, tb, 0, s>>>(g, n, pos, ps, species, c6, dc6, ci, tab, order, rb, rw, rdw, phi,
-                                                  gcn, gpos, mcell);
-  else if (mg.R <= 8)
-    k_gather<T, P, LAG, 8><<<blocks, tb, 0, s>>>(g, n, pos, ps, species, c6, dc6, ci, tab, order, rb, rw, rdw, phi,
-                                                  gcn, gpos, mcell);
-  else if (mg.R <= 16)
-    k_gather<T, P, LAG, 16><<<blocks, tb, 0, s>>>(g, n, pos, ps, species, c6, dc6, ci, tab, order, rb, rw, rdw, phi,
-                                                   gcn, gpos, mcell);
-  else
-    k_gather<T, P, LAG, 32><<<blocks, tb, 0, s>>>(g, n, pos, ps, species, c6, dc6, ci, tab, order, rb, rw, rdw, phi,
-                                                   gcn, gpos, mcell);
+#undef FD3_GATHER
   FD3_LAUNCHED();
   return FD3_OK;
 }
 
 template <typename T>
-int launch_gather(const MeshGeom& mg, int n, const double* pos, double pos_scale, const int32_t* species,
-                  const double* c6, const double* dc6, const CellInfo* ci, const Tables* tab, const int* order,
+int launch_gather(const MeshGeom& mg, int n, const double* pos, double pos_scale, const double* c6, const double* dc6, const CellInfo* ci, const Tables* tab, const int* order,
                   const int* key_start, const MeshRecords& rec, const T* phi, double* gcn, double* gpos,
                   double* mcell_part, int* n_blocks, cudaStream_t s) {
   const int blocks = (n + kGatherWarps - 1) / kGatherWarps;
   *n_blocks = 0;
   if (blocks == 0) return FD3_OK;
-#define FD3_GATHER_CASE(PP)                                                                                   \
-  case PP:                                                                                                    \
-    return mg.lagrange ? gather_r<T, PP, true>(mg, blocks, n, pos, pos_scale, species, c6, dc6, ci, tab, order, \
-                                               key_start, rec, phi, gcn, gpos, mcell_part, n_blocks, s)       \
-                       : gather_r<T, PP, false>(mg, blocks, n, pos, pos_scale, species, c6, dc6, ci, tab, order, \
-                                                key_start, rec, phi, gcn, gpos, mcell_part, n_blocks, s);
+#define FD3_GATHER_CASE(PP)                                                                                      \
+  case PP:                                                                                                       \
+    return gather_r<T, PP>(mg, blocks, n, pos, pos_scale, c6, dc6, ci, tab, order, key_start, rec, phi, gcn, gpos, \
+                           mcell_part, n_blocks, s);
   switch (mg.order) {
     FD3_GATHER_CASE(1)
     FD3_GATHER_CASE(2)

@@ -70,3 +70,12 @@ def test_ewald_sums_over_tiles_rows_and_many_species(cuda_device, n_atoms, z_max
     pos, cell, numbers = structures.random_box(seed=n_atoms, n_atoms=n_atoms, z_max=z_max)
     _against_oracle(cuda_device, pos, cell, numbers, precision, TOL[precision], method="ewald", k_cutoff=k_cutoff,
                     c6tol=0.05, r_cut=6.0)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("order,z_max,c6tol", [(6, 8, 1.0), (7, 3, 1.0), (5, 40, 0.05), (8, 25, 0.2)])
+def test_gather_of_any_order_and_rank_count(cuda_device, order, z_max, c6tol, precision):
+    # rank chunks with and without a remainder, runs of every offset and the wrapped ones
+    pos, cell, numbers = structures.random_box(seed=order, n_atoms=70, z_max=z_max)
+    _against_oracle(cuda_device, pos, cell, numbers, precision, TOL[precision], method="spme", mesh_spacing=1.2,
+                    interpolation_nodes=order, c6tol=c6tol, r_cut=6.0)
