@@ -681,7 +681,13 @@ inline int spread_zc(const MeshGeom& mg) {
   if (mg.spread_zc == 0 || mg.ns[0] > 2 || mg.ns[1] > 2 || mg.nt[2] < 2 || mg.order > mg.t[2] + 1 ||
       mg.t[2] > kSpTZ)
     return 0;
-  int zc = mg.spread_zc > 0 ? mg.spread_zc : 8;
+  // By default four z-tiles per CTA, fewer while that leaves the chip short of CTAs: staging the
+  // atoms once for longer chunks saves less than an idle SM costs. (648 atoms, 64^3, float64: 8 tiles
+  // 37 us, 1 tile 17; 1,500 HCNO atoms, 64^3, float: 47 -> 21; 12,000, 128^3: 117 -> 99; 139,968,
+  // 256^3: 309 -> 283 with 4, 358 with 1.)
+  int zc = mg.spread_zc;
+  if (zc < 0)
+    for (zc = 4; zc > 1 && mg.nt[0] * mg.nt[1] * ((mg.nt[2] + zc - 1) / zc) * mg.S < 400;) zc >>= 1;
   const int lim = kColMaxSeg / (mg.ns[0] * mg.ns[1]) - 1;
   if (zc > lim) zc = lim;
   if (zc > mg.nt[2]) zc = mg.nt[2];
