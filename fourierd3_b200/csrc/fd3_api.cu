@@ -223,7 +223,7 @@ extern "C" int fd3_plan_create(const fd3_plan_desc* d, fd3_plan** out) {
       m.gather_tile = -1;
       m.fft_yz = -1;
       m.qpitch = 0;
-      m.fft_x = -1;   // default: off (3D cuFFT around the separate filter measured faster on B200)
+      m.fft_x = -1;
       const size_t Mh = (size_t)m.n[0] * m.n[1] * m.nzh;
       m.win_axes = nullptr;
       if (d->method == FD3_METHOD_SPME && d->precision == FD3_PREC_MIXED) {
@@ -360,17 +360,39 @@ extern "C" int fd3_plan_create(const fd3_plan_desc* d, fd3_plan** out) {
   return FD3_OK;
 }
 
-// Unit shape of the TMA x-pass in effect: q values per unit (default 16: one 128-byte line per
-// spectrum row) and ranks per unit (default 1).
+// Unit shape of the TMA x-pass: the knobs, or by default the first of these that fits. Wider units
+// of more ranks share the k-point geometry and the Green lookups; what bounds the width is two units
+// and a working copy in shared memory. Summed transforms and filter, mixed form, 3D cuFFT around the
+// separate filter -> x-pass: 64^3 2 x 4 channels 64 -> 55 us (8 q x 4 ranks), 4 x 5 115 -> 99; 128^3
+// 2 x 4 221 -> 195 (8 x 4), 4 x 5 610 -> 521 (4 x 4); 256 x 256 x 128 827 -> 697 (4 x 4), 256^3 1610 ->
+// 1177 (4 x 4, with the (y, z) transforms of this library).
+static bool xpass_default_shape(const fd3_plan* p, int* Q, int* RG) {
+  static const int wide[][2] = {{8, 4}, {4, 4}, {16, 2}, {8, 2}, {16, 1}};
+  static const int narrow[][2] = {{4, 4}, {8, 2}, {16, 1}};
+  const bool w = p->mg.n[0] <= 128 && (p->mg.n[0] <= 64 || p->S <= 2);
+  const int n = w ? 5 : 3;
+  for (int k = 0; k < n; ++k) {
+    const int* c = w ? wide[k] : narrow[k];
+    if (xpass_applies(p->mg, c[0], c[1])) {
+      *Q = c[0];
+      *RG = c[1];
+      return true;
+    }
+  }
+  return false;
+}
 static void xpass_shape(const fd3_plan* p, int* Q, int* RG) {
+  if (p->mg.xq <= 0 && p->mg.xranks <= 0 && xpass_default_shape(p, Q, RG)) return;
   *Q = p->mg.xq > 0 ? p->mg.xq : 16;
   *RG = p->mg.xranks > 0 ? p->mg.xranks : 1;
 }
+// By default on wherever it applies, unless a knob of the separate filter is set.
 static bool xpass_on(const fd3_plan* p) {
+  if (p->method == FD3_METHOD_EWALD || !p->has_fft2 || p->precision != FD3_PREC_MIXED) return false;
+  if (p->mg.fft_x != 2 && !(p->mg.fft_x == -1 && p->mg.filter_kt < 0 && p->mg.filter_mma != 1)) return false;
   int Q, RG;
   xpass_shape(p, &Q, &RG);
-  return p->method != FD3_METHOD_EWALD && p->has_fft2 && p->precision == FD3_PREC_MIXED && p->mg.fft_x == 2 &&
-         xpass_applies(p->mg, Q, RG);
+  return xpass_applies(p->mg, Q, RG);
 }
 // fused (y, z) transforms in effect: float mesh on a 2D-transform path, ny = nz = 256, asked for
 static bool fft_yz_on(const fd3_plan* p) {

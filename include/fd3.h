@@ -92,7 +92,7 @@ FD3_API int fd3_plan_destroy(fd3_plan* plan);
  *                       or 16 = tiled kernel, -1 = the default for (species, rank).
  *   FD3_TUNE_SPREAD_ZC  z-tiles per column chunk of the mesh spread: 0 = one CTA per
  *                       16x16x8 tile, 1..64 = one CTA per 16x16 column chunk (capped by
- *                       the mesh), -1 = the default (8).
+ *                       the mesh), -1 = the default (4, fewer on small meshes).
  *   FD3_TUNE_SPREAD_CAP staged atoms per column chunk at most: 0 = what shared memory
  *                       holds, >= 256 = a lower bound (denser chunks take the per-tile
  *                       staging path inside the same CTA).
@@ -100,15 +100,15 @@ FD3_API int fd3_plan_destroy(fd3_plan* plan);
  *                       transform, the filter and the inverse x transform per pencil (where
  *                       it applies: at most 4 species and 8 ranks, nx = 64, 128 or 256); 2 =
  *                       the same with units of rank groups moved by TMA (mixed precision); 0 =
- *                       3D cuFFT around a separate filter; -1 = the default (0). Which is
- *                       faster depends on the mesh and precision: time them.
+ *                       3D cuFFT around a separate filter; -1 = the default: 2 where it applies,
+ *                       0 elsewhere and where a knob of the separate filter is set.
  *   FD3_TUNE_XPENCIL    kz values per pencil of the fused x-pass: 1, 2 or 4 (used when the
  *                       pencil fits in shared memory), -1 = the default (the widest that
  *                       leaves three CTAs per SM for float, within 100 KB for double);
  *                       the value in effect is 0 where the fused x-pass does not apply.
  *   FD3_TUNE_XQ         TMA x-pass (FD3_TUNE_FFT_X = 2, mixed precision): flattened (y, kz)
- *                       values per unit, 4, 8, 16 or 32; -1 = the default (16).
- *   FD3_TUNE_XRANKS     TMA x-pass: ranks per unit, 1, 2 or 4; -1 = the default (1).
+ *                       values per unit, 4, 8, 16 or 32; -1 = the default (by mesh and channels).
+ *   FD3_TUNE_XRANKS     TMA x-pass: ranks per unit, 1, 2 or 4; -1 = the default (by mesh and channels).
  *   FD3_TUNE_FILTER_MMA mixed precision, separate filter: 1 = the per-k-point S x S products
  *                       on the tensor cores (tcgen05.mma kind::tf32, operands split into tf32
  *                       high and low parts; at most 64 species and 8 ranks, as shared memory
