@@ -389,7 +389,9 @@ static void xpass_shape(const fd3_plan* p, int* Q, int* RG) {
 // By default on wherever it applies, unless a knob of the separate filter is set.
 static bool xpass_on(const fd3_plan* p) {
   if (p->method == FD3_METHOD_EWALD || !p->has_fft2 || p->precision != FD3_PREC_MIXED) return false;
-  if (p->mg.fft_x != 2 && !(p->mg.fft_x == -1 && p->mg.filter_kt < 0 && p->mg.filter_mma != 1)) return false;
+  if (p->mg.fft_x != 2 &&
+      !(p->mg.fft_x == -1 && p->mg.filter_kt < 0 && p->mg.filter_mma != 1 && tensor_maps_available()))
+    return false;
   int Q, RG;
   xpass_shape(p, &Q, &RG);
   return xpass_applies(p->mg, Q, RG);
@@ -401,9 +403,15 @@ static bool fft_yz_on(const fd3_plan* p) {
 }
 // cluster shape of the fused (y, z) forward transform: the knob, or pairs by default
 static int yz_variant(const fd3_plan* p) { return p->mg.fft_yz > 0 ? p->mg.fft_yz : 1; }
+// The pencil x-pass: asked for, or by default in float64 where this library's plane transforms take
+// the (y, z) part (summed transforms and filter against 3D cuFFT: 64^3, 2 x 4 channels 92 -> 75 us;
+// 128^3, 2 x 4 468 -> 422, 4 x 5 1491 -> 1231; with cuFFT's 2D transforms the pencils lose on larger meshes, 256^3
+// 3191 -> 3326).
 static bool old_xpass_on(const fd3_plan* p) {
-  return p->method != FD3_METHOD_EWALD && p->has_fft2 && p->mg.fft_x == 1 &&
-         xfilter_pencil(p->mg, p->precision == FD3_PREC_FP64 ? 1 : 0) > 0;
+  const bool dp = p->precision == FD3_PREC_FP64;
+  if (p->method == FD3_METHOD_EWALD || !p->has_fft2 || xfilter_pencil(p->mg, dp ? 1 : 0) <= 0) return false;
+  return p->mg.fft_x == 1 || (p->mg.fft_x == -1 && dp && p->mg.filter_kt < 0 && p->mg.fft_yz != 0 &&
+                              plane_applies(p->mg, true));
 }
 
 extern "C" int fd3_plan_set_tuning(fd3_plan* p, int32_t knob, int32_t value) {
@@ -840,8 +848,11 @@ static int mesh_pipeline(fd3_plan* p, int N, const double* pos, double ps, const
     // (y, z) transforms by the fused cluster kernels or cuFFT; x transform, filter and inverse x
     // transform in one kernel
     const bool yz = sizeof(T) == 4 && fft_yz_on(p);
+    const bool plane = mg.fft_yz != 0 && plane_applies(mg, sizeof(T) == 8);
     if (yz) {
       FD3_TRY(launch_yz_forward(mgq, p->S * p->R, yz_variant(p), (const float*)w.rho, w.spec, s));
+    } else if (plane) {
+      FD3_TRY(launch_plane(mg, sizeof(T) == 8, false, p->S * p->R, w.rho, w.spec, s));
     } else {
       FD3_CUFFT(cufftSetStream(p->fwd2, s));
       FD3_CUFFT(cufftSetWorkArea(p->fwd2, w.fftw));
@@ -865,6 +876,8 @@ static int mesh_pipeline(fd3_plan* p, int N, const double* pos, double ps, const
     if (!need_grad) return FD3_OK;
     if (yz) {
       FD3_TRY(launch_yz_inverse(mgq, p->S * p->R, yz_variant(p), w.spec, (float*)w.rho, s));
+    } else if (plane) {
+      FD3_TRY(launch_plane(mg, sizeof(T) == 8, true, p->S * p->R, w.spec, w.rho, s));
     } else {
       FD3_CUFFT(cufftSetStream(p->inv2, s));
       FD3_CUFFT(cufftSetWorkArea(p->inv2, w.fftw));

@@ -197,6 +197,11 @@ int launch_yz_forward(const MeshGeom& mg, int nchannels, int variant, const floa
                       cudaStream_t s);
 int launch_yz_inverse(const MeshGeom& mg, int nchannels, int variant, const void* spec, float* rho,
                       cudaStream_t s);
+// (y, z) plane transforms by single CTAs (planes that fit shared memory; layouts of the batched 2D cuFFT
+// R2C / C2R they replace, qpitch = nzh).
+bool plane_applies(const MeshGeom& mg, bool is_double);
+int launch_plane(const MeshGeom& mg, bool is_double, bool inverse, int nchannels, const void* in, void* out,
+                 cudaStream_t s);
 // Whether the tile-staged (TMA) gather applies to this mesh for elements of `elem` bytes.
 bool gather_tile_applies(const MeshGeom& mg, size_t elem);
 // factors: the records' rank factors are written first, from these values per atom (null: they are
@@ -217,6 +222,7 @@ int launch_xfilter(const MeshGeom& mg, const CellInfo* ci, const GreenPair* gp, 
 int xfilter_pencil(const MeshGeom& mg, int is_double);
 // TMA fused x-pass (float spectrum): units of Q flattened (y, kz) values x all x x RG ranks x S
 bool xpass_applies(const MeshGeom& mg, int Q, int RG);
+bool tensor_maps_available();   // the driver exports the tensor-map encoder
 int launch_xpass(const MeshGeom& mg, int Q, int RG, const CellInfo* ci, const GreenPairF* gpf, const float4* gtab,
                  const Tables* tab, const float* deconv, int spme, void* spec, double* part, int* n_blocks,
                  cudaStream_t s);

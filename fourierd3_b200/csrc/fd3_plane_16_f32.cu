@@ -1,0 +1,4 @@
+#include "fd3_plane.cuh"
+namespace fd3 {
+template int launch_plane_ny<float, 16>(bool, int, int, const void*, void*, cudaStream_t);
+}

@@ -22,6 +22,8 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   return fn;
 }
 
+bool tensor_maps_available() { return tensor_map_encoder() != nullptr; }
+
 // Whether the TMA x-pass can run this mesh with Q q values and RG ranks per unit: nx a tabulated
 // length, at most 4 species, RG <= R, an even number of values per spectrum row block (the TMA
 // strides must be multiples of 16 bytes) and two units in shared memory.

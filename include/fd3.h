@@ -100,8 +100,10 @@ FD3_API int fd3_plan_destroy(fd3_plan* plan);
  *                       transform, the filter and the inverse x transform per pencil (where
  *                       it applies: at most 4 species and 8 ranks, nx = 64, 128 or 256); 2 =
  *                       the same with units of rank groups moved by TMA (mixed precision); 0 =
- *                       3D cuFFT around a separate filter; -1 = the default: 2 where it applies,
- *                       0 elsewhere and where a knob of the separate filter is set.
+ *                       3D cuFFT around a separate filter; -1 = the default: in mixed
+ *                       precision 2 where it applies, in float64 1 where the plane
+ *                       transforms below apply, 0 elsewhere and where a knob of the
+ *                       separate filter is set.
  *   FD3_TUNE_XPENCIL    kz values per pencil of the fused x-pass: 1, 2 or 4 (used when the
  *                       pencil fits in shared memory), -1 = the default (the widest that
  *                       leaves three CTAs per SM for float, within 100 KB for double);
@@ -122,6 +124,9 @@ FD3_API int fd3_plan_destroy(fd3_plan* plan);
  *                       cluster kernels (one pass over the mesh each way instead of cuFFT's
  *                       two; 1: clusters of 2 CTAs, one per SM; 2: the forward transform on
  *                       clusters of 4, two per SM); 0 = cuFFT; -1 = the default (1).
+ *                       Smaller planes (16 to 256 points a side; up to 128 x 256 in mixed
+ *                       precision, 128 x 128 in float64) are transformed by one CTA each
+ *                       unless the value is 0.
  * fd3_plan_get_tuning returns the value in effect (the default resolved). */
 #define FD3_TUNE_FILTER_KT 0
 #define FD3_TUNE_SPREAD_ZC 1

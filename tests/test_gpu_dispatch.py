@@ -79,3 +79,25 @@ def test_gather_of_any_order_and_rank_count(cuda_device, order, z_max, c6tol, pr
     pos, cell, numbers = structures.random_box(seed=order, n_atoms=70, z_max=z_max)
     _against_oracle(cuda_device, pos, cell, numbers, precision, TOL[precision], method="spme", mesh_spacing=1.2,
                     interpolation_nodes=order, c6tol=c6tol, r_cut=6.0)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("lengths", [(24.0, 8.0, 8.0), (24.0, 8.0, 16.0), (24.0, 16.0, 8.0), (24.0, 32.0, 32.0), (36.0, 70.0, 8.0),
+                                     (24.0, 8.0, 70.0), (40.0, 66.0, 32.0), (24.0, 66.0, 67.0), (24.0, 130.0, 24.0),
+                                     (24.0, 24.0, 130.0), (24.0, 130.0, 66.0)])
+def test_plane_transforms_of_every_length_agree_with_cufft(cuda_device, lengths, precision):
+    # planes from 16 x 16 points to the largest that a CTA holds and beyond (cuFFT then), against the 3D transforms
+    rng = np.random.default_rng(int(sum(lengths)))
+    cell = np.diag(lengths)
+    numbers = rng.choice([8, 14], 90)
+    pos = rng.random((90, 3)) @ cell
+    m = D3Model(numbers, cell, precision=precision, device=cuda_device, method="spme", mesh_spacing=1.2,
+                interpolation_nodes=4, r_cut=6.0)
+    m.engine.set_tuning(fft_x=0)
+    e0, f0, s0 = (t.clone() for t in m(pos, cell))
+    m.engine.set_tuning(fft_x=1)
+    e, f, s = m(pos, cell)
+    tol_e, tol_f = (1e-12, 1e-10) if precision == "fp64" else (2e-6, 1e-5)
+    assert abs(float(e) - float(e0)) <= tol_e * abs(float(e0))
+    assert (f - f0).abs().max().item() <= tol_f
+    assert (s - s0).abs().max().item() <= tol_f
