@@ -101,3 +101,25 @@ def test_plane_transforms_of_every_length_agree_with_cufft(cuda_device, lengths,
     assert abs(float(e) - float(e0)) <= tol_e * abs(float(e0))
     assert (f - f0).abs().max().item() <= tol_f
     assert (s - s0).abs().max().item() <= tol_f
+
+
+@pytest.mark.parametrize("lengths,z_max,c6tol", [((8.0, 8.0, 8.0), 4, 1.0), ((8.0, 24.0, 8.0), 1, 1.0),
+                                                 ((16.0, 8.0, 16.0), 2, 1.0), ((32.0, 8.0, 8.0), 4, 0.05),
+                                                 ((66.0, 16.0, 8.0), 3, 1.0), ((130.0, 8.0, 8.0), 4, 1.0)])
+def test_float64_x_pass_of_every_length(cuda_device, lengths, z_max, c6tol):
+    # nx = 16 to 256, one to four species, sheared (the partner of a self-conjugate k has another length),
+    # each pencil width, against the 3D transforms around the separate filter
+    rng = np.random.default_rng(int(sum(lengths)) + z_max)
+    cell = np.diag(lengths) + np.triu(np.full((3, 3), 1.1), 1)
+    numbers = rng.integers(1, z_max + 1, 60)
+    pos = rng.random((60, 3)) @ cell
+    m = D3Model(numbers, cell, precision="fp64", device=cuda_device, method="spme", mesh_spacing=1.2,
+                interpolation_nodes=4, c6tol=c6tol, r_cut=6.0)
+    m.engine.set_tuning(fft_x=0)
+    e0, f0, s0 = (t.clone() for t in m(pos, cell))
+    for kz in (-1, 1, 2, 4):
+        m.engine.set_tuning(fft_x=1, xpencil=kz)
+        e, f, s = m(pos, cell)
+        assert abs(float(e) - float(e0)) <= 1e-12 * abs(float(e0))
+        assert (f - f0).abs().max().item() <= 1e-10 * max(1.0, f0.abs().max().item())
+        assert (s - s0).abs().max().item() <= 1e-10 * max(1.0, s0.abs().max().item())
