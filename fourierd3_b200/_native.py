@@ -74,6 +74,8 @@ _SIGS = {
                                           ctypes.POINTER(_c_int64), _vp]),
     "fd3_neighbor_fill": (ctypes.c_int, [_c_int64, _vp, _dp, _c_double, _vp, ctypes.c_size_t, _c_int64, _vp, _vp,
                                          _vp, ctypes.POINTER(_c_int64), _vp]),
+    "fd3_neighbor_fill_counted": (ctypes.c_int, [_c_int64, _vp, _dp, _c_double, _vp, ctypes.c_size_t, _c_int64, _vp,
+                                                 _vp, _vp, _vp]),
     "fd3_neighbor_fill_static": (ctypes.c_int, [_c_int64, _vp, _dp, _c_double, _c_int64, _vp, _vp, _vp,
                                                 ctypes.POINTER(_c_int64), _vp]),
     "fd3_profile_enable": (ctypes.c_int, [_vp, _c_int32]),

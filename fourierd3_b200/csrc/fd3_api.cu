@@ -404,9 +404,9 @@ static bool fft_yz_on(const fd3_plan* p) {
 // cluster shape of the fused (y, z) forward transform: the knob, or pairs by default
 static int yz_variant(const fd3_plan* p) { return p->mg.fft_yz > 0 ? p->mg.fft_yz : 1; }
 // The pencil x-pass: asked for, or by default in float64 where this library's plane transforms take
-// the (y, z) part (summed transforms and filter against 3D cuFFT: 64^3, 2 x 4 channels 92 -> 75 us;
-// 128^3, 2 x 4 468 -> 422, 4 x 5 1491 -> 1231; with cuFFT's 2D transforms the pencils lose on larger meshes, 256^3
-// 3191 -> 3326).
+// the (y, z) part (summed transforms and filter against 3D cuFFT: 16^3, 4 x 5 channels 64 -> 33 us; 64^3,
+// 2 x 4 92 -> 75, 4 x 5 196 -> 155; 128^3, 2 x 4 468 -> 422, 4 x 5 1491 -> 1102; with cuFFT's 2D transforms the
+// pencils lose on larger meshes, 256^3 3191 -> 3532).
 static bool old_xpass_on(const fd3_plan* p) {
   const bool dp = p->precision == FD3_PREC_FP64;
   if (p->method == FD3_METHOD_EWALD || !p->has_fft2 || xfilter_pencil(p->mg, dp ? 1 : 0) <= 0) return false;
@@ -1276,8 +1276,8 @@ void carve_nbr(int64_t N, int64_t K, Carver& c, NbrWork& w) {
   w.counts = c.take<int>(N);
   w.row_start = c.take<int>(N + 1);
 }
-int nbr_prepare(int64_t n, const double* d_pos, const double* h_cell, double r_cut, void* d_work, size_t bytes,
-                CellGrid& g, NbrWork& w, cudaStream_t s) {
+int nbr_work(int64_t n, const double* d_pos, const double* h_cell, double r_cut, void* d_work, size_t bytes,
+             CellGrid& g, NbrWork& w) {
   if (n < 1 || n > (int64_t)1 << 30 || !d_pos || !h_cell) return FD3_EINVAL;
   FD3_TRY(make_cell_grid(h_cell, r_cut, &g));
   const int64_t K = (int64_t)g.nb[0] * g.nb[1] * g.nb[2];
@@ -1287,8 +1287,13 @@ int nbr_prepare(int64_t n, const double* d_pos, const double* h_cell, double r_c
   Carver c2;
   c2.base = reinterpret_cast<char*>(((uintptr_t)d_work + 255) & ~(uintptr_t)255);
   carve_nbr(n, K, c2, w);
+  return FD3_OK;
+}
+int nbr_prepare(int64_t n, const double* d_pos, const double* h_cell, double r_cut, void* d_work, size_t bytes,
+                CellGrid& g, NbrWork& w, cudaStream_t s) {
+  FD3_TRY(nbr_work(n, d_pos, h_cell, r_cut, d_work, bytes, g, w));
   FD3_TRY(build_cell_list(g, (int)n, d_pos, nullptr, w.cl, s));
-  FD3_TRY(launch_nbr_count(g, (int)n, w.cl, d_pos, w.counts, s));
+  FD3_TRY(launch_nbr_count(g, (int)n, w.cl, w.counts, s));
   FD3_TRY(scan_exclusive(w.counts, (int)n, w.row_start, s));
   return FD3_OK;
 }
@@ -1335,8 +1340,19 @@ extern "C" int fd3_neighbor_fill(int64_t n, const double* d_pos, const double* h
   FD3_CUDA(cudaStreamSynchronize(s));
   *h_count = total;
   if (total > capacity) return FD3_ECAPACITY;
-  FD3_TRY(launch_nbr_fill(g, (int)n, w.cl, d_pos, w.row_start, d_src, d_dst, d_shift, s));
+  FD3_TRY(launch_nbr_fill(g, (int)n, w.cl, w.row_start, d_src, d_dst, d_shift, s));
   return FD3_OK;
+}
+
+extern "C" int fd3_neighbor_fill_counted(int64_t n, const double* d_pos, const double* h_cell, double r_cut,
+                                         void* d_work, size_t bytes, int64_t count, int64_t* d_src, int64_t* d_dst,
+                                         int32_t* d_shift, void* stream) {
+  CellGrid g;
+  NbrWork w;
+  if (count < 0 || (count > 0 && (!d_src || !d_dst || !d_shift))) return FD3_EINVAL;
+  FD3_TRY(nbr_work(n, d_pos, h_cell, r_cut, d_work, bytes, g, w));
+  if (count == 0) return FD3_OK;
+  return launch_nbr_fill(g, (int)n, w.cl, w.row_start, d_src, d_dst, d_shift, (cudaStream_t)stream);
 }
 
 // ------------------------------------------------------------------ profiling

@@ -164,6 +164,19 @@ int build_cell_list(const CellGrid& g, int n, const double* pos_ang, const int32
   return FD3_OK;
 }
 
+// The exact pair predicate (Angstrom, no FMA): d = (x_j - x_i) + S . cell, |d|^2 < r_cut^2.
+__device__ __forceinline__ bool pair_inside(const GridDev& g, double xj0, double xj1, double xj2, double xi0,
+                                            double xi1, double xi2, int S0, int S1, int S2, double& d0, double& d1,
+                                            double& d2) {
+  const double sh0 = dadd(dadd(dmul((double)S0, g.cell[0]), dmul((double)S1, g.cell[3])), dmul((double)S2, g.cell[6]));
+  const double sh1 = dadd(dadd(dmul((double)S0, g.cell[1]), dmul((double)S1, g.cell[4])), dmul((double)S2, g.cell[7]));
+  const double sh2 = dadd(dadd(dmul((double)S0, g.cell[2]), dmul((double)S1, g.cell[5])), dmul((double)S2, g.cell[8]));
+  d0 = dadd(dsub(xj0, xi0), sh0);
+  d1 = dadd(dsub(xj1, xi1), sh1);
+  d2 = dadd(dsub(xj2, xi2), sh2);
+  return dadd(dadd(dmul(d0, d0), dmul(d1, d1)), dmul(d2, d2)) < g.rc2;
+}
+
 // Visit every candidate (j, S) of atom i. All lanes of the warp run the same number of
 // iterations; `fn(hit, u, j, S, d)` gets the exact-predicate result (Angstrom, no FMA).
 template <class Fn>
@@ -205,17 +218,8 @@ __device__ __forceinline__ void visit_neighbors(const GridDev& g, const int* __r
             S0 = sx + offi.x - mj.x;
             S1 = sy + offi.y - mj.y;
             S2 = sz + offi.z - mj.z;
-            const double sh0 = dadd(dadd(dmul((double)S0, g.cell[0]), dmul((double)S1, g.cell[3])),
-                                    dmul((double)S2, g.cell[6]));
-            const double sh1 = dadd(dadd(dmul((double)S0, g.cell[1]), dmul((double)S1, g.cell[4])),
-                                    dmul((double)S2, g.cell[7]));
-            const double sh2 = dadd(dadd(dmul((double)S0, g.cell[2]), dmul((double)S1, g.cell[5])),
-                                    dmul((double)S2, g.cell[8]));
-            d0 = dadd(dsub(xj.x, xi0), sh0);
-            d1 = dadd(dsub(xj.y, xi1), sh1);
-            d2 = dadd(dsub(xj.z, xi2), sh2);
-            const double r2 = dadd(dadd(dmul(d0, d0), dmul(d1, d1)), dmul(d2, d2));
-            hit = r2 < g.rc2 && !(j == i && S0 == 0 && S1 == 0 && S2 == 0);
+            hit = pair_inside(g, xj.x, xj.y, xj.z, xi0, xi1, xi2, S0, S1, S2, d0, d1, d2) &&
+                  !(j == i && S0 == 0 && S1 == 0 && S2 == 0);
           }
           fn(hit, u, j, S0, S1, S2, d0, d1, d2);
         }
@@ -1104,46 +1108,123 @@ int launch_c6_atoms(int n, const int32_t* species, const Tables* tab, const doub
 
 
 // ------------------------------------------------------------------ neighbour export
-__global__ void __launch_bounds__(256) k_nbr_count(GridDev g, int n, const int* __restrict__ bin_start,
-                                                  const double4* __restrict__ xs, const int4* __restrict__ meta,
-                                                  const int4* __restrict__ off, int* __restrict__ counts) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int t = blockIdx.x * kWarpsPerBlock + wid;
-  if (t >= n) return;
-  const double4 xi = xs[t];
-  const int i = meta[t].w;
-  int cnt = 0;
-  visit_neighbors(g, bin_start, xs, meta, i, xi.x, xi.y, xi.z, off[i],
-                  [&](bool hit, int, int, int, int, int, double, double, double) {
-                    cnt += __popc(__ballot_sync(0xffffffffu, hit));
-                  });
-  if (lane == 0) counts[i] = cnt;
+// One warp per atom. The runs of bins around it (two per (dx, dy) at most: a z range that fits the
+// grid wraps once) are laid out at once by the lanes, so that the candidates form one numbered
+// sequence, in the order of visit_neighbors, and every load of a round is independent of the last
+// round's. (Walking the runs one by one waits for bin_start and then for its candidates 18 times per atom.)
+// Grids whose runs do not fit the table (cells narrower than the search) take visit_neighbors.
+constexpr int kNbrRuns = 64;
+struct NbrRuns {
+  int pref[kNbrRuns + 1], a0[kNbrRuns], S0[kNbrRuns], S1[kNbrRuns], S2[kNbrRuns];
+};
+__device__ __forceinline__ bool nbr_runs_fit(const GridDev& g) {
+  return 2 * (2 * g.reach[0] + 1) * (2 * g.reach[1] + 1) <= kNbrRuns && 2 * g.reach[2] + 1 <= g.nb[2];
 }
 
-__global__ void __launch_bounds__(256) k_nbr_fill(GridDev g, int n, const int* __restrict__ bin_start,
-                                                 const double4* __restrict__ xs, const int4* __restrict__ meta,
-                                                 const int4* __restrict__ off, const int* __restrict__ row_start,
-                                                 int64_t* __restrict__ src, int64_t* __restrict__ dst,
-                                                 int32_t* __restrict__ shift) {
+// fn as in visit_neighbors, without the candidate slot and the vector.
+template <class Fn>
+__device__ __forceinline__ void visit_runs(const GridDev& g, const int* __restrict__ bin_start,
+                                           const double4* __restrict__ xs, const int4* __restrict__ meta, int i,
+                                           double4 xi, int4 offi, NbrRuns& rt, Fn&& fn) {
+  const int lane = threadIdx.x & 31;
+  const int ny = 2 * g.reach[1] + 1, npair = (2 * g.reach[0] + 1) * ny;
+  const int bz = offi.w % g.nb[2], by = (offi.w / g.nb[2]) % g.nb[1], bx = offi.w / (g.nb[2] * g.nb[1]);
+  int len0 = 0, len1 = 0;
+  if (lane < npair) {
+    const int cx = bx + lane / ny - g.reach[0], cy = by + lane % ny - g.reach[1];
+    const int sx = floordiv(cx, g.nb[0]), sy = floordiv(cy, g.nb[1]);
+    const int row = ((cx - sx * g.nb[0]) * g.nb[1] + (cy - sy * g.nb[1])) * g.nb[2];
+    const int zs = bz - g.reach[2], nz = 2 * g.reach[2] + 1;
+    const int sz = floordiv(zs, g.nb[2]), wz = zs - sz * g.nb[2];
+    const int n0 = g.nb[2] - wz < nz ? g.nb[2] - wz : nz;   // bins before the wrap
+    const int a = bin_start[row + wz], b = bin_start[row + wz + n0];
+    const int c = n0 < nz ? bin_start[row] : 0, d = n0 < nz ? bin_start[row + nz - n0] : 0;
+    len0 = b - a;
+    len1 = d - c;
+    rt.a0[2 * lane] = a;
+    rt.a0[2 * lane + 1] = c;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      rt.S0[2 * lane + u] = sx + offi.x;
+      rt.S1[2 * lane + u] = sy + offi.y;
+      rt.S2[2 * lane + u] = sz + u + offi.z;
+    }
+  }
+  int incl = len0 + len1;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane < npair) {
+    rt.pref[2 * lane] = incl - len0 - len1;
+    rt.pref[2 * lane + 1] = incl - len1;
+  }
+  const int total = __shfl_sync(0xffffffffu, incl, 31);
+  __syncwarp();
+  const int last = 2 * npair - 1;
+#pragma unroll 2
+  for (int c0 = 0; c0 < total; c0 += 32) {
+    const int c = c0 + lane;
+    bool hit = false;
+    int j = 0, S0 = 0, S1 = 0, S2 = 0;
+    if (c < total) {
+      int lo = 0, hi = last;   // last run with pref <= c
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (rt.pref[mid] <= c) lo = mid; else hi = mid - 1;
+      }
+      const int u = rt.a0[lo] + (c - rt.pref[lo]);
+      const double4 xj = xs[u];
+      const int4 mj = meta[u];
+      j = mj.w;
+      S0 = rt.S0[lo] - mj.x;
+      S1 = rt.S1[lo] - mj.y;
+      S2 = rt.S2[lo] - mj.z;
+      double d0, d1, d2;
+      hit = pair_inside(g, xj.x, xj.y, xj.z, xi.x, xi.y, xi.z, S0, S1, S2, d0, d1, d2) &&
+            !(j == i && S0 == 0 && S1 == 0 && S2 == 0);
+    }
+    fn(hit, j, S0, S1, S2);
+  }
+  __syncwarp();
+}
+
+// Number of neighbours of the warp's atom, and the same traversal writing them from row_start[i].
+template <bool FILL>
+__global__ void __launch_bounds__(256) k_nbr(const __grid_constant__ GridDev g, int n,
+                                            const int* __restrict__ bin_start, const double4* __restrict__ xs,
+                                            const int4* __restrict__ meta, const int4* __restrict__ off,
+                                            int* __restrict__ counts, const int* __restrict__ row_start,
+                                            int64_t* __restrict__ src, int64_t* __restrict__ dst,
+                                            int32_t* __restrict__ shift) {
+  __shared__ NbrRuns runs[kWarpsPerBlock];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int t = blockIdx.x * kWarpsPerBlock + wid;
   if (t >= n) return;
   const double4 xi = xs[t];
   const int i = meta[t].w;
-  int pos = row_start[i];
-  visit_neighbors(g, bin_start, xs, meta, i, xi.x, xi.y, xi.z, off[i],
-                  [&](bool hit, int, int j, int S0, int S1, int S2, double, double, double) {
-                    const unsigned m = __ballot_sync(0xffffffffu, hit);
-                    if (hit) {
-                      const int k = pos + __popc(m & ((1u << lane) - 1u));
-                      src[k] = i;
-                      dst[k] = j;
-                      shift[3 * k] = S0;
-                      shift[3 * k + 1] = S1;
-                      shift[3 * k + 2] = S2;
-                    }
-                    pos += __popc(m);
-                  });
+  int pos = FILL ? row_start[i] : 0;
+  auto take = [&](bool hit, int j, int S0, int S1, int S2) {
+    const unsigned m = __ballot_sync(0xffffffffu, hit);
+    if (FILL && hit) {
+      const int k = pos + __popc(m & ((1u << lane) - 1u));
+      src[k] = i;
+      dst[k] = j;
+      shift[3 * k] = S0;
+      shift[3 * k + 1] = S1;
+      shift[3 * k + 2] = S2;
+    }
+    pos += __popc(m);
+  };
+  if (nbr_runs_fit(g))
+    visit_runs(g, bin_start, xs, meta, i, xi, off[i], runs[wid], take);
+  else
+    visit_neighbors(g, bin_start, xs, meta, i, xi.x, xi.y, xi.z, off[i],
+                    [&](bool hit, int, int j, int S0, int S1, int S2, double, double, double) {
+                      take(hit, j, S0, S1, S2);
+                    });
+  if (!FILL && lane == 0) counts[i] = pos;
 }
 
 // ------------------------------------------------------------------ direct pair sum (float64)
@@ -1243,23 +1324,21 @@ int launch_direct_pairs(const CellGrid& g, int n, const CellList& cl, const doub
   return FD3_OK;
 }
 
-int launch_nbr_count(const CellGrid& g, int n, const CellList& cl, const double* pos_ang, int* counts,
-                     cudaStream_t s) {
-  (void)pos_ang;
+int launch_nbr_count(const CellGrid& g, int n, const CellList& cl, int* counts, cudaStream_t s) {
   const int blocks = (n + kWarpsPerBlock - 1) / kWarpsPerBlock;
   if (blocks == 0) return FD3_OK;
-  k_nbr_count<<<blocks, 32 * kWarpsPerBlock, 0, s>>>(to_dev(g), n, cl.bin_start, cl.xs, cl.meta, cl.off, counts);
+  k_nbr<false><<<blocks, 32 * kWarpsPerBlock, 0, s>>>(to_dev(g), n, cl.bin_start, cl.xs, cl.meta, cl.off, counts,
+                                                      nullptr, nullptr, nullptr, nullptr);
   FD3_LAUNCHED();
   return FD3_OK;
 }
 
-int launch_nbr_fill(const CellGrid& g, int n, const CellList& cl, const double* pos_ang, const int* row_start,
-                    int64_t* src, int64_t* dst, int32_t* shift, cudaStream_t s) {
-  (void)pos_ang;
+int launch_nbr_fill(const CellGrid& g, int n, const CellList& cl, const int* row_start, int64_t* src, int64_t* dst,
+                    int32_t* shift, cudaStream_t s) {
   const int blocks = (n + kWarpsPerBlock - 1) / kWarpsPerBlock;
   if (blocks == 0) return FD3_OK;
-  k_nbr_fill<<<blocks, 32 * kWarpsPerBlock, 0, s>>>(to_dev(g), n, cl.bin_start, cl.xs, cl.meta, cl.off, row_start,
-                                                     src, dst, shift);
+  k_nbr<true><<<blocks, 32 * kWarpsPerBlock, 0, s>>>(to_dev(g), n, cl.bin_start, cl.xs, cl.meta, cl.off, nullptr,
+                                                     row_start, src, dst, shift);
   FD3_LAUNCHED();
   return FD3_OK;
 }

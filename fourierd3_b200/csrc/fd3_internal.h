@@ -139,10 +139,9 @@ int launch_c6_atoms(int n, const int32_t* species, const Tables* tab, const doub
                     int* n_self_blocks, cudaStream_t s);
 
 // neighbour export
-int launch_nbr_count(const CellGrid& g, int n, const CellList& cl, const double* pos_ang, int* counts,
-                     cudaStream_t s);
-int launch_nbr_fill(const CellGrid& g, int n, const CellList& cl, const double* pos_ang, const int* row_start,
-                    int64_t* src, int64_t* dst, int32_t* shift, cudaStream_t s);
+int launch_nbr_count(const CellGrid& g, int n, const CellList& cl, int* counts, cudaStream_t s);
+int launch_nbr_fill(const CellGrid& g, int n, const CellList& cl, const int* row_start, int64_t* src, int64_t* dst,
+                    int32_t* shift, cudaStream_t s);
 
 // ---- mesh ---------------------------------------------------------------------
 struct MeshGeom {

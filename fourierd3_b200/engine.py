@@ -375,14 +375,13 @@ def neighbour_list(positions: torch.Tensor, cell_ang: np.ndarray, r_cut: float):
     _native.check(lib.fd3_neighbor_count(n, ctypes.c_void_p(pos.data_ptr()), _native.dptr(cell_h), float(r_cut),
                                          ctypes.c_void_p(work.data_ptr()), work.numel(), ctypes.byref(count), stream),
                   "fd3_neighbor_count")
-    cap = int(count.value)
-    src = torch.empty(max(cap, 1), dtype=torch.int64, device=pos.device)
-    dst = torch.empty(max(cap, 1), dtype=torch.int64, device=pos.device)
-    sh = torch.empty((max(cap, 1), 3), dtype=torch.int32, device=pos.device)
-    _native.check(lib.fd3_neighbor_fill(n, ctypes.c_void_p(pos.data_ptr()), _native.dptr(cell_h), float(r_cut),
-                                        ctypes.c_void_p(work.data_ptr()), work.numel(), cap,
-                                        ctypes.c_void_p(src.data_ptr()), ctypes.c_void_p(dst.data_ptr()),
-                                        ctypes.c_void_p(sh.data_ptr()), ctypes.byref(count), stream),
-                  "fd3_neighbor_fill")
     m = int(count.value)
-    return src[:m], dst[:m], sh[:m]
+    src = torch.empty(m, dtype=torch.int64, device=pos.device)
+    dst = torch.empty(m, dtype=torch.int64, device=pos.device)
+    sh = torch.empty((m, 3), dtype=torch.int32, device=pos.device)
+    _native.check(lib.fd3_neighbor_fill_counted(n, ctypes.c_void_p(pos.data_ptr()), _native.dptr(cell_h),
+                                                float(r_cut), ctypes.c_void_p(work.data_ptr()), work.numel(), m,
+                                                ctypes.c_void_p(src.data_ptr()), ctypes.c_void_p(dst.data_ptr()),
+                                                ctypes.c_void_p(sh.data_ptr()), stream),
+                  "fd3_neighbor_fill_counted")
+    return src, dst, sh

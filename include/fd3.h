@@ -248,6 +248,13 @@ FD3_API int fd3_neighbor_fill(int64_t n_atoms, const double* d_pos_ang, const do
                       void* d_work, size_t work_bytes, int64_t capacity, int64_t* d_src, int64_t* d_dst,
                       int32_t* d_shift, int64_t* h_count, void* stream);
 
+/* The list that the preceding fd3_neighbor_count on this stream counted: same atoms, positions,
+ * cell, cutoff and workspace, unchanged since; count is what it returned, and the outputs hold that
+ * many pairs. Neither rebuilds the cell list nor synchronises. */
+FD3_API int fd3_neighbor_fill_counted(int64_t n_atoms, const double* d_pos_ang, const double* h_cell_ang,
+                      double r_cut_ang, void* d_work, size_t work_bytes, int64_t count, int64_t* d_src,
+                      int64_t* d_dst, int32_t* d_shift, void* stream);
+
 /*
  * Neighbour list with no allocation and no workspace argument. No counterpart in the
  * reference: it exists for callers that cannot allocate device memory themselves (an MD
