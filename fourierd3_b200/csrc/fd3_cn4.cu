@@ -48,8 +48,11 @@ __device__ __forceinline__ void cn4_green(const CnPair& c, double k, double& G, 
 // Gh = G on every k-point except the self-conjugate-plane Nyquist entries, where it is the mean
 // of G at the entry and at its stored conjugate partner (what the inverse real transform of the
 // reference's G rho amounts to there).
-template <typename T, int MAXS>
-__global__ void __launch_bounds__(256) k_cn4_filter(MeshDev g, int P, int spme, int adjoint,
+// Each pair is used as soon as it is evaluated (H_X += Gh S_Y, H_Y += Gh S_X, its share of the strain
+// term), so that no pair matrix is held: with three of them in registers the float64 kernel ran few
+// warps through long chains (2,592 atoms, 64 x 64 x 128, 4 species: 67 and 71 us).
+template <typename T, int MAXS, bool ADJOINT>
+__global__ void __launch_bounds__(256) k_cn4_filter(MeshDev g, int P, int spme,
                                                    const CellInfo* __restrict__ ci, const CnPair* __restrict__ cp,
                                                    const float* __restrict__ deconv,
                                                    const typename Cplx<T>::type* __restrict__ rhat,
@@ -62,63 +65,50 @@ __global__ void __launch_bounds__(256) k_cn4_filter(MeshDev g, int P, int spme, 
   double acc[7] = {0, 0, 0, 0, 0, 0, 0};
   for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < Mh; k += (size_t)gridDim.x * blockDim.x) {
     const KPoint<T> q = kpoint<T>(g, k, rc, deconv, spme, P);
-    double G[MAXS][MAXS], dG[MAXS][MAXS], Gh[MAXS][MAXS];
-#pragma unroll
-    for (int X = 0; X < MAXS; ++X)
-#pragma unroll
-      for (int Y = X; Y < MAXS; ++Y) {
-        double gv = 0.0, dv = 0.0;
-        if (X < S && Y < S) {
-          cn4_green(cp[X * S + Y], (double)q.knorm, gv, dv);
-          gv *= (double)q.inv_sc;
-          dv *= (double)q.inv_sc;
-        }
-        G[X][Y] = G[Y][X] = gv;
-        dG[X][Y] = dG[Y][X] = dv;
-        Gh[X][Y] = Gh[Y][X] = gv;
-      }
-    if (q.partner) {
-#pragma unroll
-      for (int X = 0; X < MAXS; ++X)
-#pragma unroll
-        for (int Y = X; Y < MAXS; ++Y)
-          if (X < S && Y < S) {
-            double gv, dv;
-            cn4_green(cp[X * S + Y], (double)q.kpart, gv, dv);
-            Gh[X][Y] = Gh[Y][X] = 0.5 * (G[X][Y] + gv * (double)q.inv_sc);
-          }
-    }
     C2 src[MAXS], rh[MAXS];
+    double hre[MAXS], him[MAXS];
 #pragma unroll
     for (int X = 0; X < MAXS; ++X) {
       rh[X] = X < S ? rhat[(size_t)X * Mh + k] : C2{T(0), T(0)};
-      src[X] = adjoint ? (X < S ? out[(size_t)X * Mh + k] : C2{T(0), T(0)}) : rh[X];
+      src[X] = ADJOINT ? (X < S ? out[(size_t)X * Mh + k] : C2{T(0), T(0)}) : rh[X];
+      hre[X] = him[X] = 0.0;
     }
-    if (adjoint) {
-      double dq = 0.0;
+    const double w = (double)q.inv_sc;
+    double dq = 0.0;
 #pragma unroll
-      for (int X = 0; X < MAXS; ++X)
+    for (int X = 0; X < MAXS; ++X)
 #pragma unroll
-        for (int Y = 0; Y < MAXS; ++Y)
-          dq += dG[X][Y] * ((double)rh[Y].x * (double)src[X].x + (double)rh[Y].y * (double)src[X].y);
+      for (int Y = X; Y < MAXS; ++Y)
+        if (Y < S) {
+          double gv, dv;
+          cn4_green(cp[X * S + Y], (double)q.knorm, gv, dv);
+          gv *= w;
+          if (ADJOINT) {
+            const double re = (double)rh[Y].x * (double)src[X].x + (double)rh[Y].y * (double)src[X].y;
+            const double re2 = (double)rh[X].x * (double)src[Y].x + (double)rh[X].y * (double)src[Y].y;
+            dq += dv * w * (X == Y ? re : re + re2);
+          }
+          if (q.partner) {
+            double g2, d2;
+            cn4_green(cp[X * S + Y], (double)q.kpart, g2, d2);
+            gv = 0.5 * (gv + g2 * w);
+          }
+          hre[X] += gv * (double)src[Y].x;
+          him[X] += gv * (double)src[Y].y;
+          if (X != Y) {
+            hre[Y] += gv * (double)src[X].x;
+            him[Y] += gv * (double)src[X].y;
+          }
+        }
+    if (ADJOINT)
       virial_acc<double>(KPoint<double>{{(double)q.kv[0], (double)q.kv[1], (double)q.kv[2]}, (double)q.knorm, 0.0,
                                         (double)q.wk, 0.0, false},
                          dq, acc);
-    }
 #pragma unroll
-    for (int X = 0; X < MAXS; ++X) {
-      if (X < S) {
-        double hre = 0.0, him = 0.0;
-#pragma unroll
-        for (int Y = 0; Y < MAXS; ++Y) {
-          hre += Gh[X][Y] * (double)src[Y].x;
-          him += Gh[X][Y] * (double)src[Y].y;
-        }
-        out[(size_t)X * Mh + k] = C2{(T)hre, (T)him};
-      }
-    }
+    for (int X = 0; X < MAXS; ++X)
+      if (X < S) out[(size_t)X * Mh + k] = C2{(T)hre[X], (T)him[X]};
   }
-  if (adjoint) {
+  if (ADJOINT) {
     // dE/dstrain_ab = -sum_k w dG k_a k_b / |k| Re(conj sigma rho): acc[1..6] holds the sum
     double v[9] = {-acc[1], -acc[4], -acc[5], -acc[4], -acc[2], -acc[6], -acc[5], -acc[6], -acc[3]};
     block_sum_store<9>(v, part + 9 * blockIdx.x);
@@ -246,8 +236,9 @@ int launch_cn4_filter(const MeshGeom& mg, int adjoint, const CellInfo* ci, const
   const MeshDev g = to_dev(mg);
   const C2* r = static_cast<const C2*>(rhat);
   C2* o = static_cast<C2*>(out);
-#define FD3_CN4F(MS) \
-  k_cn4_filter<T, MS><<<(int)blocks, 256, 0, s>>>(g, mg.order, spme, adjoint, ci, cp, deconv, r, o, part)
+#define FD3_CN4F(MS)                                                                                              \
+  (adjoint ? k_cn4_filter<T, MS, true><<<(int)blocks, 256, 0, s>>>(g, mg.order, spme, ci, cp, deconv, r, o, part) \
+           : k_cn4_filter<T, MS, false><<<(int)blocks, 256, 0, s>>>(g, mg.order, spme, ci, cp, deconv, r, o, part))
   if (mg.S <= 1)
     FD3_CN4F(1);
   else if (mg.S <= 2)
