@@ -230,6 +230,10 @@ bool filter_mma_applies(const MeshGeom& mg);
 bool filter_mma_on(const MeshGeom& mg);
 int launch_filter_mma(const MeshGeom& mg, const CellInfo* ci, const float4* gtab, const Tables* tab,
                       const float* deconv, int spme, void* spec, double* part, int* n_blocks, cudaStream_t s);
+// many-species filter (float spectrum, 16 to 64 species, at most 8 ranks, no k-tile asked for)
+bool filter_many_applies(const MeshGeom& mg);
+int launch_filter_many(const MeshGeom& mg, const CellInfo* ci, const float4* gtab, const Tables* tab,
+                       const float* deconv, int spme, void* spec, double* part, int* n_blocks, cudaStream_t s);
 size_t green_table_bytes(int S);
 int filter_max_blocks();
 int filter_default_kt(int S, int R, size_t tsize);

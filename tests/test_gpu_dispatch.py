@@ -123,3 +123,20 @@ def test_float64_x_pass_of_every_length(cuda_device, lengths, z_max, c6tol):
         assert abs(float(e) - float(e0)) <= 1e-12 * abs(float(e0))
         assert (f - f0).abs().max().item() <= 1e-10 * max(1.0, f0.abs().max().item())
         assert (s - s0).abs().max().item() <= 1e-10 * max(1.0, s0.abs().max().item())
+
+
+@pytest.mark.parametrize("n_species,c6tol", [(15, 1.0), (16, 30.0), (17, 1.0), (40, 1.0), (41, 30.0), (43, 1.0)])
+def test_many_species_filter_agrees_with_the_tiled_one(cuda_device, n_species, c6tol):
+    # below its range, whole and ragged 4 x 4 blocks, both tile widths, up to 4 and up to 8 ranks, a sheared cell
+    rng = np.random.default_rng(n_species)
+    numbers = np.concatenate((np.arange(1, n_species + 1), rng.integers(1, n_species + 1, 60)))
+    cell = np.diag([9.0, 12.0, 10.0]) + np.triu(np.full((3, 3), 0.9), 1)
+    pos = rng.random((len(numbers), 3)) @ cell
+    m = D3Model(numbers, cell, precision="mixed", device=cuda_device, method="spme", mesh_spacing=1.2,
+                interpolation_nodes=4, c6tol=c6tol, r_cut=6.0)
+    e, f, s = (t.clone() for t in m(pos, cell))
+    m.engine.set_tuning(filter_kt=4)
+    e0, f0, s0 = m(pos, cell)
+    assert abs(float(e) - float(e0)) <= 2e-6 * abs(float(e0))
+    assert (f - f0).abs().max().item() <= 1e-5 * max(1.0, f0.abs().max().item())
+    assert (s - s0).abs().max().item() <= 1e-5 * max(1.0, s0.abs().max().item())
