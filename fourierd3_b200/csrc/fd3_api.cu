@@ -695,11 +695,14 @@ void carve(const fd3_plan* p, int64_t N, int64_t K_in, Carver& c, Work& w, int64
   w.ei.kd = c.take<int>(E);
   w.ei.ord_s = c.take<int>(E);
   w.ei.ord_d = c.take<int>(E);
-  w.ei.arrival = c.take<int>(E);
-  w.ei.cnt = c.take<int>(N);
+  w.ei.arr_s = c.take<int>(E);
+  w.ei.arr_d = c.take<int>(E);
   w.ei.st_s = c.take<int>(N + 1);
   w.ei.st_d = c.take<int>(N + 1);
-  w.ei.bad = c.take<int>(1);
+  w.ei.bad = c.take<int>(2 + 2 * N);
+  w.ei.unsorted = w.ei.bad + 1;
+  w.ei.cnt_s = w.ei.bad + 2;
+  w.ei.cnt_d = w.ei.cnt_s + N;
   // direct Ewald sum
   if (!mesh) {
     const int64_t nk = (int64_t)p->ens[0] * p->ens[1] * p->ens[2];

@@ -119,10 +119,11 @@ int launch_direct_finalize(const double* pair_part, int n_pair, const double* ta
 struct EdgeIndex {
   int *ks, *kd;         // [E] source / destination keys
   int *ord_s, *ord_d;   // [E] edge ids by source / by destination
-  int* arrival;         // [E] counting-sort scratch
-  int* cnt;             // [N] counting-sort scratch
+  int *arr_s, *arr_d;   // [E] edge ids in arrival order (scratch)
   int *st_s, *st_d;     // [N+1] segment starts
-  int* bad;             // [1] set when an edge index is outside 0..N-1
+  int* bad;             // [1] set when an edge index is outside 0..N-1; followed by
+  int* unsorted;        // [1] set when the sources do not ascend, and
+  int *cnt_s, *cnt_d;   // [N] the counts, one array zeroed at once
 };
 int launch_edge_index(int64_t n_edges, int n, const int64_t* src, const int64_t* dst, const EdgeIndex& ei,
                       cudaStream_t s);

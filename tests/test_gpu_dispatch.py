@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 import torch
 
-from fourierd3_b200 import D3Model, neighbour_list, structures
+from fourierd3_b200 import D3Model, FourierD3, neighbour_list, structures
 from oracle.neighbours import neighbour_list_cells
 from oracle.reference_port import OracleFourierD3
 
@@ -140,3 +140,34 @@ def test_many_species_filter_agrees_with_the_tiled_one(cuda_device, n_species, c
     assert abs(float(e) - float(e0)) <= 2e-6 * abs(float(e0))
     assert (f - f0).abs().max().item() <= 1e-5 * max(1.0, f0.abs().max().item())
     assert (s - s0).abs().max().item() <= 1e-5 * max(1.0, s0.abs().max().item())
+
+
+@pytest.mark.parametrize("n_atoms,n_edges", [(5, 1), (700, 3), (40, 255), (40, 257), (300, 9000)])
+def test_edge_lists_sorted_by_source_or_in_any_order(cuda_device, n_atoms, n_edges):
+    # the two ways to the source segments: atoms without edges first, last and in runs, blocks of 256 edges
+    rng = np.random.default_rng(n_edges)
+    cell = torch.tensor(np.diag([26.0, 30.0, 28.0]), device=cuda_device)
+    numbers = rng.choice([8, 14], n_atoms)
+    pos = torch.tensor(rng.random((n_atoms, 3)) * 26.0, device=cuda_device)
+    active = np.arange(n_atoms // 3, n_atoms - n_atoms // 5)
+    src = torch.tensor(np.sort(rng.choice(active, n_edges)), device=cuda_device)
+    dst = torch.tensor(rng.choice(n_atoms, n_edges), device=cuda_device)
+    shift = torch.tensor(rng.normal(size=(n_edges, 3)) * 3.0, device=cuda_device)
+    m = FourierD3(numbers, cell.cpu().numpy(), dtype=torch.float64, device=cuda_device, verbose=False,
+                  method="spme", mesh_spacing=2.0, interpolation_nodes=4, r_cut=12.0)
+
+    def run(order):
+        p = pos.clone().requires_grad_()
+        sh = shift[order].clone().requires_grad_()
+        e = m(p, torch.stack((src[order], dst[order])), sh)
+        e.backward()
+        g = torch.empty_like(shift)
+        g[order] = sh.grad
+        return e.detach(), p.grad, g
+
+    e0, p0, g0 = run(torch.arange(n_edges, device=cuda_device))
+    for _ in range(2):
+        e, p, g = run(torch.tensor(rng.permutation(n_edges), device=cuda_device))
+        assert abs(float(e - e0)) <= 1e-12 * abs(float(e0))
+        assert (p - p0).abs().max().item() <= 1e-12 * max(1e-3, p0.abs().max().item())
+        assert (g - g0).abs().max().item() <= 1e-12 * max(1e-3, g0.abs().max().item())
