@@ -306,7 +306,8 @@ __global__ void __launch_bounds__(kSpThreads, sizeof(T) == 8 ? 2 : 4) k_spread(M
 }
 
 // Column spread. A CTA owns a column of 16 x 16 points in (x, y) and a chunk of ZC z-tiles of one
-// species; thread (lx, ly) owns the z-row of 8 points of the current z-tile. The atoms whose x and
+// species; a thread owns 16 bytes of z of the current z-tile in 2 (float) or 4 (double) rows adjacent in
+// y, so that neighbouring lanes store one row's 32 or 64 bytes together. The atoms whose x and
 // y stencils reach the column are staged ONCE per chunk, in counting-sorted segment order with the
 // source z-tile outermost, as tile-local x and y weight rows, rank factors, and two z rows: the
 // part of the z stencil inside the atom's own z-tile and the part spilling into the next one
@@ -317,36 +318,56 @@ __global__ void __launch_bounds__(kSpThreads, sizeof(T) == 8 ? 2 : 4) k_spread(M
 // exceeds `cap` falls back, inside the same CTA, to staging per tile in pieces of `cap`. Each
 // mesh value is written exactly once in a fixed summation order (no atomics); results are
 // independent of ZC up to the summation order.
+//
+// The load/store pipe bounds it (256^3, 8 channels, float64: its wavefronts at 75 % of their peak, DRAM at 26 %),
+// so the layouts are chosen for few wavefronts: the stores above (a thread with a whole row stores 16
+// bytes per line), staged rows of 17 or 18 values (a thread stages an atom; rows of 16 put all lanes on
+// the same banks), and per atom one z, one or two y and the rank loads for 32 multiply-adds. 139,968 atoms on
+// 256^3, 2 x 4 channels: float64 497 -> 348 us, float 283 -> 236 (before: a whole row of 8 per thread).
 constexpr int kColMaxSeg = 64;
+
+// what a thread owns of a z-tile: kZL values in each of kRows rows
+template <typename T>
+struct ColOwn {
+  static constexpr int kZL = 16 / sizeof(T);
+  static constexpr int kRows = kSpTZ / kZL;
+  static constexpr int kWx = 17, kWy = 18;            // staged row lengths
+  static constexpr int kWz = sizeof(T) == 4 ? 20 : 18;
+};
 
 template <typename T>
 struct ColSmem {
-  T* wx;      // [cap][16]
-  T* wy;      // [cap][16]
-  T* wzo;     // [cap][8] z row inside the atom's own z-tile
-  T* wzn;     // [cap][8] z row spilling into the next z-tile
+  T* wz;      // [cap][kWz] z row inside the atom's own z-tile (8), then the part spilling into the next (8)
+  T* wy;      // [cap][kWy]
+  T* wx;      // [cap][kWx]
   T* cc;      // [cap][R]
   int* zi;    // [cap] source z-tile (index into the chunk's source range); bit 30: spills
   int* zst;   // [kColMaxSeg + 1] first staged slot of each source z-tile
 };
 
+__host__ __device__ inline size_t col_round16(size_t b) { return (b + 15) & ~(size_t)15; }
+
 template <typename T>
 __host__ __device__ inline size_t col_smem_bytes(int cap, int R) {
-  size_t b = (size_t)cap * (16 + 16 + 2 * kSpTZ + R) * sizeof(T);
-  b += (size_t)cap * sizeof(int) + (kColMaxSeg + 1) * sizeof(int);
-  return (b + 15) & ~(size_t)15;
+  using O = ColOwn<T>;
+  return col_round16((size_t)cap * O::kWz * sizeof(T)) + col_round16((size_t)cap * O::kWy * sizeof(T)) +
+         col_round16((size_t)cap * O::kWx * sizeof(T)) + col_round16((size_t)cap * R * sizeof(T)) +
+         col_round16((size_t)(cap + kColMaxSeg + 1) * sizeof(int));
 }
 
 template <typename T>
 __device__ __forceinline__ ColSmem<T> col_carve(unsigned char* base, int cap, int R) {
+  using O = ColOwn<T>;
   ColSmem<T> m;
-  T* t = reinterpret_cast<T*>(base);
-  m.wx = t;
-  m.wy = m.wx + (size_t)cap * 16;
-  m.wzo = m.wy + (size_t)cap * 16;
-  m.wzn = m.wzo + (size_t)cap * kSpTZ;
-  m.cc = m.wzn + (size_t)cap * kSpTZ;
-  m.zi = reinterpret_cast<int*>(m.cc + (size_t)cap * R);
+  m.wz = reinterpret_cast<T*>(base);
+  base += col_round16((size_t)cap * O::kWz * sizeof(T));
+  m.wy = reinterpret_cast<T*>(base);
+  base += col_round16((size_t)cap * O::kWy * sizeof(T));
+  m.wx = reinterpret_cast<T*>(base);
+  base += col_round16((size_t)cap * O::kWx * sizeof(T));
+  m.cc = reinterpret_cast<T*>(base);
+  base += col_round16((size_t)cap * R * sizeof(T));
+  m.zi = reinterpret_cast<int*>(base);
   m.zst = m.zi + cap;
   return m;
 }
@@ -415,10 +436,10 @@ __device__ int col_stage(const MeshDev& g, const int* s_a0, const int* s_pref, i
     const int slot = staged + block_compact(keep, s_wcnt, &tot);
     if (keep && slot < cap) {
       // tile-local x and y rows (stencil nodes that wrap onto the same point are summed)
-      T* wxr = m.wx + slot * 16;
-      T* wyr = m.wy + slot * 16;
-      T* zo = m.wzo + slot * kSpTZ;
-      T* zn = m.wzn + slot * kSpTZ;
+      T* wxr = m.wx + slot * ColOwn<T>::kWx;
+      T* wyr = m.wy + slot * ColOwn<T>::kWy;
+      T* zo = m.wz + slot * ColOwn<T>::kWz;
+      T* zn = zo + kSpTZ;
 #pragma unroll
       for (int z = 0; z < 16; ++z) {
         wxr[z] = T(0);
@@ -468,89 +489,127 @@ __device__ int col_stage(const MeshDev& g, const int* s_a0, const int* s_pref, i
   return staged < cap ? staged : cap;
 }
 
-// acc[z][r] += w_x(lx) w_y(ly) w_z(z) c_{r0+r} over staged atoms [a0, a1), with their own-tile
-// z rows (spill = false) or spill rows (spill = true). CHECK: the range may hold atoms of other
+// acc[row][z][r] += w_x(lx) w_y(ly0 + row) w_z(z0 + z) c_{r0+r} over staged atoms [a0, a1), with their
+// own-tile z rows (spill = false) or spill rows (spill = true). CHECK: the range may hold atoms of other
 // source z-tiles (per-tile staging), skip those whose source tile is not zsrc. Atoms are taken
-// four at a time so that their x/y weight loads are in flight together; an atom with no spill
+// four at a time so that their x weight loads are in flight together; an atom with no spill
 // has an all-zero spill row and adds exact zeros.
+template <typename T>
+using ColAcc = T[ColOwn<T>::kRows][ColOwn<T>::kZL][kSpRC];
+
 template <typename T, bool CHECK>
-__device__ __forceinline__ void col_atom(const ColSmem<T>& m, const T* zrows, int a, T wxy, int zsrc, int R, int r0,
-                                         T (&acc)[kSpTZ][kSpRC]) {
+__device__ __forceinline__ void col_atom(const ColSmem<T>& m, int a, int z0, T wx, int zsrc, int R, int r0, int ly0,
+                                         ColAcc<T>& acc) {
+  using O = ColOwn<T>;
   if (CHECK && (m.zi[a] & ~kZiSpill) != zsrc) return;
-  T cr[kSpRC];
-  if (sizeof(T) == 4 && kSpRC == 4 && (R & 3) == 0) {
-    // a whole 4-rank group in one 16-byte load (rows of R floats start on 16-byte boundaries)
-    const float4 c4 = *reinterpret_cast<const float4*>(m.cc + a * R + r0);
-    cr[0] = wxy * (T)c4.x;
-    cr[1] = wxy * (T)c4.y;
-    cr[2] = wxy * (T)c4.z;
-    cr[3] = wxy * (T)c4.w;
-  } else {
-#pragma unroll
-    for (int r = 0; r < kSpRC; ++r) cr[r] = r0 + r < R ? wxy * m.cc[a * R + r0 + r] : T(0);
-  }
-  T zr[kSpTZ];
+  T c[kSpRC], zr[O::kZL], wxy[O::kRows];
   if (sizeof(T) == 4) {
-    const float4* v = reinterpret_cast<const float4*>(zrows + a * kSpTZ);
-    const float4 p0 = v[0], p1 = v[1];
-    const float t8[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+    const float2 y = *reinterpret_cast<const float2*>(m.wy + a * O::kWy + ly0);
+    const float4 z = *reinterpret_cast<const float4*>(m.wz + a * O::kWz + z0);
+    const float zz[4] = {z.x, z.y, z.z, z.w};
+    wxy[0] = wx * (T)y.x;
+    wxy[1] = wx * (T)y.y;
 #pragma unroll
-    for (int z = 0; z < kSpTZ; ++z) zr[z] = (T)t8[z];
+    for (int k = 0; k < O::kZL; ++k) zr[k] = (T)zz[k];
+  } else {
+    const double2 ya = *reinterpret_cast<const double2*>(m.wy + a * O::kWy + ly0);
+    const double2 yb = *reinterpret_cast<const double2*>(m.wy + a * O::kWy + ly0 + 2);
+    const double2 z = *reinterpret_cast<const double2*>(m.wz + a * O::kWz + z0);
+    const double yy[4] = {ya.x, ya.y, yb.x, yb.y};
+#pragma unroll
+    for (int k = 0; k < O::kRows; ++k) wxy[k] = wx * (T)yy[k];
+    zr[0] = (T)z.x;
+    zr[1] = (T)z.y;
+  }
+  if (kSpRC == 4 && (R & 3) == 0) {
+    // a whole 4-rank group in 16-byte loads (rows of R values start on 16-byte boundaries)
+    if (sizeof(T) == 4) {
+      const float4 v = *reinterpret_cast<const float4*>(m.cc + a * R + r0);
+      c[0] = (T)v.x;
+      c[1] = (T)v.y;
+      c[2] = (T)v.z;
+      c[3] = (T)v.w;
+    } else {
+      const double2 v0 = *reinterpret_cast<const double2*>(m.cc + a * R + r0);
+      const double2 v1 = *reinterpret_cast<const double2*>(m.cc + a * R + r0 + 2);
+      c[0] = (T)v0.x;
+      c[1] = (T)v0.y;
+      c[2] = (T)v1.x;
+      c[3] = (T)v1.y;
+    }
   } else {
 #pragma unroll
-    for (int z = 0; z < kSpTZ; ++z) zr[z] = zrows[a * kSpTZ + z];
+    for (int r = 0; r < kSpRC; ++r) c[r] = r0 + r < R ? m.cc[a * R + r0 + r] : T(0);
   }
 #pragma unroll
-  for (int z = 0; z < kSpTZ; ++z)
+  for (int k = 0; k < O::kRows; ++k) {
 #pragma unroll
-    for (int r = 0; r < kSpRC; ++r) acc[z][r] += zr[z] * cr[r];
+    for (int r = 0; r < kSpRC; ++r) {
+      const T cr = wxy[k] * c[r];
+#pragma unroll
+      for (int z = 0; z < O::kZL; ++z) acc[k][z][r] += zr[z] * cr;
+    }
+  }
 }
 
 template <typename T, bool CHECK>
 __device__ __forceinline__ void col_accumulate(const ColSmem<T>& m, int a0, int a1, int zsrc, bool spill, int R,
-                                               int r0, int lx, int ly, T (&acc)[kSpTZ][kSpRC]) {
-  const T* zrows = spill ? m.wzn : m.wzo;
+                                               int r0, int lx, int ly0, int zl0, ColAcc<T>& acc) {
+  using O = ColOwn<T>;
+  const int z0 = zl0 + (spill ? kSpTZ : 0);
   int a = a0;
   for (; a + 4 <= a1; a += 4) {
-    T wxy[4];
+    T wx[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) wxy[u] = m.wx[(a + u) * 16 + lx] * m.wy[(a + u) * 16 + ly];
+    for (int u = 0; u < 4; ++u) wx[u] = m.wx[(a + u) * O::kWx + lx];
 #pragma unroll
     for (int u = 0; u < 4; ++u)
-      if (wxy[u] != T(0)) col_atom<T, CHECK>(m, zrows, a + u, wxy[u], zsrc, R, r0, acc);
+      if (wx[u] != T(0)) col_atom<T, CHECK>(m, a + u, z0, wx[u], zsrc, R, r0, ly0, acc);
   }
   for (; a < a1; ++a) {
-    const T wxy = m.wx[a * 16 + lx] * m.wy[a * 16 + ly];
-    if (wxy != T(0)) col_atom<T, CHECK>(m, zrows, a, wxy, zsrc, R, r0, acc);
+    const T wx = m.wx[a * O::kWx + lx];
+    if (wx != T(0)) col_atom<T, CHECK>(m, a, z0, wx, zsrc, R, r0, ly0, acc);
   }
 }
 
 template <typename T>
 __device__ __forceinline__ void col_store(const MeshDev& g, int X, int r0, const int (&t0)[3], int tzt, int lx,
-                                          int ly, const T (&acc)[kSpTZ][kSpRC], T* __restrict__ rho) {
-  if (lx >= g.t[0] || ly >= g.t[1]) return;
+                                          int ly0, int zl0, const ColAcc<T>& acc, T* __restrict__ rho) {
+  using O = ColOwn<T>;
+  if (lx >= g.t[0]) return;
   const size_t M = (size_t)g.n[0] * g.n[1] * g.n[2];
-  const size_t m0 = ((size_t)(t0[0] + lx) * g.n[1] + (t0[1] + ly)) * g.n[2] + (size_t)tzt * g.t[2];
+  const size_t m0 =
+      ((size_t)(t0[0] + lx) * g.n[1] + (t0[1] + ly0)) * g.n[2] + (size_t)tzt * g.t[2] + (size_t)zl0;
 #pragma unroll
   for (int r = 0; r < kSpRC; ++r) {
     if (r0 + r >= g.R) break;
-    T* dst = rho + ((size_t)X * g.R + r0 + r) * M + m0;
-    if (g.t[2] == kSpTZ) {
-      if (sizeof(T) == 4) {
-        float4* v = reinterpret_cast<float4*>(dst);
-        v[0] = make_float4((float)acc[0][r], (float)acc[1][r], (float)acc[2][r], (float)acc[3][r]);
-        v[1] = make_float4((float)acc[4][r], (float)acc[5][r], (float)acc[6][r], (float)acc[7][r]);
+#pragma unroll
+    for (int k = 0; k < O::kRows; ++k) {
+      if (ly0 + k >= g.t[1]) break;
+      T* dst = rho + ((size_t)X * g.R + r0 + r) * M + m0 + (size_t)k * g.n[2];
+      if (g.t[2] == kSpTZ) {
+        if (sizeof(T) == 4)
+          *reinterpret_cast<float4*>(dst) = make_float4((float)acc[k][0][r], (float)acc[k][1 % O::kZL][r],
+                                                        (float)acc[k][2 % O::kZL][r], (float)acc[k][3 % O::kZL][r]);
+        else
+          *reinterpret_cast<double2*>(dst) = make_double2((double)acc[k][0][r], (double)acc[k][1][r]);
       } else {
-        double2* v = reinterpret_cast<double2*>(dst);
 #pragma unroll
-        for (int z = 0; z < kSpTZ; z += 2) v[z / 2] = make_double2((double)acc[z][r], (double)acc[z + 1][r]);
+        for (int z = 0; z < O::kZL; ++z)
+          if (zl0 + z < g.t[2]) dst[z] = acc[k][z][r];
       }
-    } else {
-#pragma unroll
-      for (int z = 0; z < kSpTZ; ++z)
-        if (z < g.t[2]) dst[z] = acc[z][r];
     }
   }
+}
+
+template <typename T>
+__device__ __forceinline__ void col_zero(ColAcc<T>& acc) {
+#pragma unroll
+  for (int k = 0; k < ColOwn<T>::kRows; ++k)
+#pragma unroll
+    for (int z = 0; z < ColOwn<T>::kZL; ++z)
+#pragma unroll
+      for (int r = 0; r < kSpRC; ++r) acc[k][z][r] = T(0);
 }
 
 template <typename T, int P>
@@ -571,7 +630,10 @@ __global__ void __launch_bounds__(kSpThreads, sizeof(T) == 8 ? 2 : 4) k_spread_c
   const int tz0 = zch * zc;
   const int tz1 = tz0 + zc < g.nt[2] ? tz0 + zc : g.nt[2];
   const int t0[3] = {tx * g.t[0], ty * g.t[1], 0};
-  const int lx = tid / kSpTY, ly = tid % kSpTY;
+  // a group of kRows lanes owns kRows rows of its warp's 2 x 16 (x, y) rows; the lane picks the z part
+  using O = ColOwn<T>;
+  const int row0 = (tid >> 5) * 32 + ((tid & 31) / O::kRows) * O::kRows;
+  const int lx = row0 / kSpTY, ly0 = row0 % kSpTY, zl0 = (tid % O::kRows) * O::kZL;
   // source z-tiles of the chunk: tz - 1 and tz for tz in [tz0, tz1), each once
   int nzs = (tz1 - tz0) + 1;
   int zs0 = tz0 - 1;
@@ -627,14 +689,11 @@ __global__ void __launch_bounds__(kSpThreads, sizeof(T) == 8 ? 2 : 4) k_spread_c
       const int zown = nzs == g.nt[2] ? tzt : tzt - zs0;
       const int zprev = nzs == g.nt[2] ? (tzt + g.nt[2] - 1) % g.nt[2] : zown - 1;
       for (int r0 = 0; r0 < g.R; r0 += kSpRC) {
-        T acc[kSpTZ][kSpRC];
-#pragma unroll
-        for (int z = 0; z < kSpTZ; ++z)
-#pragma unroll
-          for (int r = 0; r < kSpRC; ++r) acc[z][r] = T(0);
-        col_accumulate<T, false>(m, m.zst[zprev], m.zst[zprev + 1], zprev, true, g.R, r0, lx, ly, acc);
-        col_accumulate<T, false>(m, m.zst[zown], m.zst[zown + 1], zown, false, g.R, r0, lx, ly, acc);
-        col_store<T>(g, X, r0, t0, tzt, lx, ly, acc, rho);
+        ColAcc<T> acc;
+        col_zero<T>(acc);
+        col_accumulate<T, false>(m, m.zst[zprev], m.zst[zprev + 1], zprev, true, g.R, r0, lx, ly0, zl0, acc);
+        col_accumulate<T, false>(m, m.zst[zown], m.zst[zown + 1], zown, false, g.R, r0, lx, ly0, zl0, acc);
+        col_store<T>(g, X, r0, t0, tzt, lx, ly0, zl0, acc, rho);
       }
     }
     return;
@@ -644,20 +703,17 @@ __global__ void __launch_bounds__(kSpThreads, sizeof(T) == 8 ? 2 : 4) k_spread_c
     const int zown = nzs == g.nt[2] ? tzt : tzt - zs0;
     const int zprev = nzs == g.nt[2] ? (tzt + g.nt[2] - 1) % g.nt[2] : zown - 1;
     for (int r0 = 0; r0 < g.R; r0 += kSpRC) {
-      T acc[kSpTZ][kSpRC];
-#pragma unroll
-      for (int z = 0; z < kSpTZ; ++z)
-#pragma unroll
-        for (int r = 0; r < kSpRC; ++r) acc[z][r] = T(0);
+      ColAcc<T> acc;
+      col_zero<T>(acc);
       int from = 0;
       while (from < total) {
         const int st = col_stage<T, P>(g, s_a0, s_pref, nseg, spz, total, from, t0, tzt, cap, rb, rw, rc, m,
                                        s_wcnt, &s_next, &from);
-        col_accumulate<T, true>(m, 0, st, zprev, true, g.R, r0, lx, ly, acc);
-        col_accumulate<T, true>(m, 0, st, zown, false, g.R, r0, lx, ly, acc);
+        col_accumulate<T, true>(m, 0, st, zprev, true, g.R, r0, lx, ly0, zl0, acc);
+        col_accumulate<T, true>(m, 0, st, zown, false, g.R, r0, lx, ly0, zl0, acc);
         __syncthreads();
       }
-      col_store<T>(g, X, r0, t0, tzt, lx, ly, acc, rho);
+      col_store<T>(g, X, r0, t0, tzt, lx, ly0, zl0, acc, rho);
     }
   }
 }
@@ -682,9 +738,9 @@ inline int spread_zc(const MeshGeom& mg) {
       mg.t[2] > kSpTZ)
     return 0;
   // By default four z-tiles per CTA, fewer while that leaves the chip short of CTAs: staging the
-  // atoms once for longer chunks saves less than an idle SM costs. (648 atoms, 64^3, float64: 8 tiles
-  // 37 us, 1 tile 17; 1,500 HCNO atoms, 64^3, float: 47 -> 21; 12,000, 128^3: 117 -> 99; 139,968,
-  // 256^3: 309 -> 283 with 4, 358 with 1.)
+  // atoms once for longer chunks saves less than an idle SM costs. (With rows of 8 points per thread: 648
+  // atoms, 64^3, float64: 8 tiles 37 us, 1 tile 17; 1,500 HCNO atoms, 64^3, float: 47 -> 21; 12,000,
+  // 128^3: 117 -> 99; 139,968, 256^3: 309 -> 283 with 4, 358 with 1.)
   int zc = mg.spread_zc;
   if (zc < 0)
     for (zc = 4; zc > 1 && mg.nt[0] * mg.nt[1] * ((mg.nt[2] + zc - 1) / zc) * mg.S < 400;) zc >>= 1;
@@ -704,7 +760,6 @@ static int spread_r(const MeshGeom& mg, dim3 grid, int n, const double* factors,
   }
   const int zc = spread_zc(mg);
   if (zc > 0) {
-    // staged atoms per chunk: as many as let 3 (float) or 2 (double) CTAs share an SM
     const int cap = spread_col_cap<T>(mg);
     if (cap >= kColMinCap) {
       const size_t smem = col_smem_bytes<T>(cap, mg.R);
