@@ -816,42 +816,42 @@ namespace fd3 {
 
 constexpr int kGatherWarps = 8;
 
-// Gather, one warp per atom: lanes over the (x, y) stencil columns; each lane reads the P z-values of
-// its column from RC rank channels at a time with aligned 16-byte vector loads (the column start is
-// rounded down to the vector boundary; a warp-uniform offset O in [0, 16/sizeof(T)) selects the run,
-// so every register index stays static) and forms
+// Sums of four values over the warp, 12 shuffles (four butterflies take 40): lanes 8 k .. 8 k + 7 return the
+// k-th sum.
+__device__ __forceinline__ double warp_sum4(double a, double b, double c, double d) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const bool hi = lane & 16;
+  double u = hi ? c : a, v = hi ? d : b;
+  u += __shfl_xor_sync(kAll, hi ? a : c, 16);
+  v += __shfl_xor_sync(kAll, hi ? b : d, 16);
+  const bool odd = lane & 8;
+  double w = odd ? v : u;
+  w += __shfl_xor_sync(kAll, odd ? u : v, 8);
+  w += __shfl_xor_sync(kAll, w, 4);
+  w += __shfl_xor_sync(kAll, w, 2);
+  w += __shfl_xor_sync(kAll, w, 1);
+  return w;
+}
+
+// Gather, one warp per atom. The P z-values of a stencil column lie in NV aligned 16-byte vectors; a lane
+// takes one vector of one column (neighbouring lanes the vectors of one column, so that a load of the warp
+// touches 32 / NV lines) for RC rank channels at a time, with the z weights shifted to the vector (zero
+// outside the stencil), and forms
 //   zr_r = sum_z w_z phi_r,  cp_z = sum_r lambda_r c_r phi_r,  s0 = sum_z w_z cp_z,  s2 = sum_z w'_z cp_z
 // in TA, then accumulates P_r = sum W phi_r and the three spline-gradient sums in float64.
 // A column that wraps the periodic z edge (or a mesh whose nz is not a multiple of the vector
-// width) is read element by element with the offset 0.
-// Ranks go in chunks of RC, so any rank and order runs on registers and vector loads. (Orders above 5
-// and more than 4 or 8 ranks, and every call with cell gradients, took a kernel that read single
-// values and held all ranks: 178 us at 12,000 HCNO atoms, p = 6, 5 ranks, float, now 62; 103 us for the
-// module at 20,736 SiO2 atoms, p = 5, 4 ranks, now 78.)
+// width) is read element by element, from the stencil's first value on.
+// The load/store pipe bounds it (its wavefronts at 89 % of their peak when a lane read a whole column,
+// which is a line per lane and vector, and each rank had a butterfly): 139,968 atoms, p = 5, 4 ranks: float
+// 207 -> 166 us, float64 321 -> 246; 12,000 atoms, p = 6, 5 ranks, float 62 -> 54; 20,736 atoms with the cell
+// partials 78 -> 51. With the loads and reductions of one pass after the other it was a chain of nine memory
+// waits per atom (float 218 us).
 // TA: float sums for the orders and ranks of the mixed form that have always had them (launch rule),
-// float64 otherwise.
-template <typename T, typename TA, int P, int RC, int O, int NE>
-__device__ __forceinline__ void zrun_sums(const T (&v)[RC][NE], int nr, const T (&wz)[P], const TA (&cl)[RC],
-                                          TA (&zr)[RC], TA (&cp)[P]) {
-#pragma unroll
-  for (int r = 0; r < RC; ++r) {
-    if (r < nr) {
-      TA a = TA(0);
-#pragma unroll
-      for (int kz = 0; kz < P; ++kz) {
-        const TA f = (TA)v[r][O + kz];
-        a += (TA)wz[kz] * f;
-        cp[kz] += cl[r] * f;
-      }
-      zr[r] = a;
-    }
-  }
-}
-
-// MC: the positions-fixed cell partials of the edge-list path too. ONE: all ranks are one chunk (the
-// loop over chunks costs the common case registers: 139,968 atoms, float, 4 ranks: 205 us without it, 295 us with).
+// float64 otherwise. MC: the positions-fixed cell partials of the edge-list path too. ONE: all ranks are
+// one chunk.
 template <typename T, typename TA, int P, int RC, bool MC, bool ONE>
-__global__ void __launch_bounds__(32 * kGatherWarps, ONE && sizeof(TA) == 4 && P <= 5 ? 4 : 2) k_gather_z(
+__global__ void __launch_bounds__(32 * kGatherWarps, RC == 8 ? 2 : 3) k_gather_z(
     MeshDev g, int n, const double* __restrict__ pos, double ps, const double* __restrict__ c6,
     const double* __restrict__ dc6, const CellInfo* __restrict__ ci, const Tables* __restrict__ tab,
     const int* __restrict__ order, const int4* __restrict__ rb, const T* __restrict__ rw, const T* __restrict__ rdw,
@@ -859,119 +859,141 @@ __global__ void __launch_bounds__(32 * kGatherWarps, ONE && sizeof(TA) == 4 && P
     double* __restrict__ mcell_part) {
   constexpr int VW = 16 / (int)sizeof(T);          // elements per 16-byte vector
   constexpr int NV = (VW - 1 + P + VW - 1) / VW;   // vectors covering a run at any offset
-  constexpr int NE = NV * VW;
+  constexpr int CPP = 32 / NV;                     // columns per pass
+  constexpr int U = RC == 4 ? 2 : 1;               // passes whose loads are in flight together
   using V = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
+  constexpr unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int t = blockIdx.x * kGatherWarps + wid;
   double mc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   if (t < n) {
+    // two memory waits per atom: the record, then mesh, factors and their derivatives together
     const int R = g.R;
     const int i = order[t];
     const int4 b4 = rb[t];
+    const T wl = lane < 3 * P ? rw[(size_t)t * 3 * P + lane] : T(0);
+    const T dwl = lane < 3 * P ? rdw[(size_t)t * 3 * P + lane] : T(0);
     const int s = b4.w;
-    const T* wr = rw + (size_t)t * 3 * P;
-    const T* dwr = rdw + (size_t)t * 3 * P;
-    T wz[P], dwz[P];
-#pragma unroll
-    for (int k = 0; k < P; ++k) {
-      wz[k] = wr[2 * P + k];
-      dwz[k] = dwr[2 * P + k];
-    }
     const int n2 = g.n[2];
     const int iz0 = b4.z;
     const bool scalar = iz0 + P > n2 || (n2 % VW) != 0;   // warp-uniform
     const int o = scalar ? 0 : iz0 % VW;
-    const int za = iz0 - o;
-    const int nvec = (o + P + VW - 1) / VW;
+    const int c0 = lane / NV, h = lane - c0 * NV;
+    const int k0 = h * VW - o;   // stencil node of the vector's first element
+    const bool mine = c0 < CPP && k0 < P;
     const size_t M = (size_t)g.n[0] * g.n[1] * n2;
     const double inv_vol = 1.0 / ci->volume;
     double gu0 = 0.0, gu1 = 0.0, gu2 = 0.0, gsum = 0.0;
     for (int rc0 = 0; rc0 < (ONE ? 1 : R); rc0 += RC) {
       const int nr = ONE || R - rc0 < RC ? R - rc0 : RC;
-      TA cl[RC];
-#pragma unroll
-      for (int r = 0; r < RC; ++r) cl[r] = r < nr ? (TA)(c6[(size_t)i * R + rc0 + r] * tab->eigs[rc0 + r]) : TA(0);
+      // lane r: lambda_r c_r and the weight of P_r in g (below)
+      double lc = 0.0, gp = 0.0;
+      if (lane < nr) {
+        const double lam = tab->eigs[rc0 + lane], dc = dc6[(size_t)i * R + rc0 + lane];
+        lc = c6[(size_t)i * R + rc0 + lane] * lam;
+        gp = -lam * inv_vol * dc;
+        gsum += lc * tab->selfcont[s] * dc;
+      }
       double pr[RC];
 #pragma unroll
       for (int r = 0; r < RC; ++r) pr[r] = 0.0;
-      for (int q = lane; q < P * P; q += 32) {
-        const int kx = q / P, ky = q - kx * P;
-        int ix = b4.x + kx;
-        while (ix >= g.n[0]) ix -= g.n[0];   // a stencil wider than the mesh wraps more than once
-        int iy = b4.y + ky;
-        while (iy >= g.n[1]) iy -= g.n[1];
-        const T wx = wr[kx], dwx = dwr[kx], wy = wr[P + ky], dwy = dwr[P + ky];
-        const T* col = phi + ((size_t)s * R + rc0) * M + ((size_t)ix * g.n[1] + iy) * n2;
-        T v[RC][NE];
+#pragma unroll 1
+      for (int q0 = 0; q0 < P * P; q0 += U * CPP) {
+        T v[U][RC][VW];
+        int kx[U], ky[U];
 #pragma unroll
-        for (int r = 0; r < RC; ++r) {
-          if (r < nr) {
-            const T* src = col + (size_t)r * M;
-            if (!scalar) {
-              const V* vs = reinterpret_cast<const V*>(src + za);
+        for (int u = 0; u < U; ++u) {
+          int q = q0 + u * CPP + c0;
+          const bool ok = mine && q < P * P;
+          if (!ok) q = 0;
+          kx[u] = q / P;
+          ky[u] = q - kx[u] * P;
+          int ix = b4.x + kx[u];
+          while (ix >= g.n[0]) ix -= g.n[0];   // a stencil wider than the mesh wraps more than once
+          int iy = b4.y + ky[u];
+          while (iy >= g.n[1]) iy -= g.n[1];
+          const T* col = phi + ((size_t)s * R + rc0) * M + ((size_t)ix * g.n[1] + iy) * n2;
 #pragma unroll
-              for (int j = 0; j < NV; ++j)
-                if (j < nvec) *reinterpret_cast<V*>(&v[r][j * VW]) = vs[j];
-            } else {
+          for (int r = 0; r < RC; ++r)
 #pragma unroll
-              for (int kz = 0; kz < P; ++kz) {
-                int iz = iz0 + kz;
-                while (iz >= n2) iz -= n2;
-                v[r][kz] = src[iz];
-              }
+            for (int j = 0; j < VW; ++j) v[u][r][j] = T(0);
+          if (ok && !scalar) {
+            // in the row: iz0 + P <= n2 and n2 is a multiple of VW, so the vector of a node below P is too
+#pragma unroll
+            for (int r = 0; r < RC; ++r)
+              if (r < nr)
+                *reinterpret_cast<V*>(v[u][r]) = *reinterpret_cast<const V*>(col + (size_t)r * M + (iz0 + k0));
+          } else if (ok) {
+#pragma unroll
+            for (int j = 0; j < VW; ++j) {
+              int iz = iz0 + k0 + j;
+              while (iz >= n2) iz -= n2;
+#pragma unroll
+              for (int r = 0; r < RC; ++r)
+                if (r < nr && k0 + j < P) v[u][r][j] = col[(size_t)r * M + iz];
             }
           }
         }
-        TA zr[RC], cp[P];
+        T wz[VW], dwz[VW];
 #pragma unroll
-        for (int kz = 0; kz < P; ++kz) cp[kz] = TA(0);
+        for (int j = 0; j < VW; ++j) {
+          const int k = k0 + j;
+          const T w = __shfl_sync(kAll, wl, (2 * P + k) & 31), dw = __shfl_sync(kAll, dwl, (2 * P + k) & 31);
+          wz[j] = k >= 0 && k < P ? w : T(0);
+          dwz[j] = k >= 0 && k < P ? dw : T(0);
+        }
+        TA cp[U][VW];
 #pragma unroll
-        for (int r = 0; r < RC; ++r) zr[r] = TA(0);
-        if constexpr (VW == 4) {
-          switch (o) {
-            case 0: zrun_sums<T, TA, P, RC, 0, NE>(v, nr, wz, cl, zr, cp); break;
-            case 1: zrun_sums<T, TA, P, RC, 1, NE>(v, nr, wz, cl, zr, cp); break;
-            case 2: zrun_sums<T, TA, P, RC, 2, NE>(v, nr, wz, cl, zr, cp); break;
-            default: zrun_sums<T, TA, P, RC, 3, NE>(v, nr, wz, cl, zr, cp); break;
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+          for (int j = 0; j < VW; ++j) cp[u][j] = TA(0);
+        TA wx[U], wy[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          wx[u] = (TA)__shfl_sync(kAll, wl, kx[u]);
+          wy[u] = (TA)__shfl_sync(kAll, wl, P + ky[u]);
+        }
+#pragma unroll
+        for (int r = 0; r < RC; ++r) {
+          const TA cl = (TA)__shfl_sync(kAll, lc, r);
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            TA zr = TA(0);
+#pragma unroll
+            for (int j = 0; j < VW; ++j) {
+              const TA f = (TA)v[u][r][j];
+              zr += (TA)wz[j] * f;
+              cp[u][j] += cl * f;
+            }
+            pr[r] += (double)(wx[u] * wy[u] * zr);
           }
-        } else {
-          if (o == 0)
-            zrun_sums<T, TA, P, RC, 0, NE>(v, nr, wz, cl, zr, cp);
-          else
-            zrun_sums<T, TA, P, RC, 1, NE>(v, nr, wz, cl, zr, cp);
         }
-        TA s0 = TA(0), s2 = TA(0);
 #pragma unroll
-        for (int kz = 0; kz < P; ++kz) {
-          s0 += (TA)wz[kz] * cp[kz];
-          s2 += (TA)dwz[kz] * cp[kz];
-        }
-        const TA wxy = (TA)wx * (TA)wy;
+        for (int u = 0; u < U; ++u) {
+          TA s0 = TA(0), s2 = TA(0);
 #pragma unroll
-        for (int r = 0; r < RC; ++r) pr[r] += (double)(wxy * zr[r]);
-        gu0 += (double)((TA)dwx * (TA)wy * s0);
-        gu1 += (double)((TA)wx * (TA)dwy * s0);
-        gu2 += (double)(wxy * s2);
-      }
-      // dE/dc_r = -(lambda_r / Omega) P_r + lambda_r c_r phi_ss(0); g = sum_r dE/dc_r dc_r/dCN
-#pragma unroll
-      for (int r = 0; r < RC; ++r) {
-        pr[r] = warp_sum(pr[r]);
-        if (r < nr) {
-          const double lam = tab->eigs[rc0 + r];
-          const double c = c6[(size_t)i * R + rc0 + r];
-          const double dEdc = -lam * inv_vol * pr[r] + lam * c * tab->selfcont[s];
-          gsum += dEdc * dc6[(size_t)i * R + rc0 + r];
+          for (int j = 0; j < VW; ++j) {
+            s0 += (TA)wz[j] * cp[u][j];
+            s2 += (TA)dwz[j] * cp[u][j];
+          }
+          const TA dwx = (TA)__shfl_sync(kAll, dwl, kx[u]), dwy = (TA)__shfl_sync(kAll, dwl, P + ky[u]);
+          gu0 += (double)(dwx * wy[u] * s0);
+          gu1 += (double)(wx[u] * dwy * s0);
+          gu2 += (double)(wx[u] * wy[u] * s2);
         }
       }
+      // dE/dc_r = -(lambda_r / Omega) P_r + lambda_r c_r phi_ss(0); g = sum_r dE/dc_r dc_r/dCN: this lane's part
+#pragma unroll
+      for (int r = 0; r < RC; ++r) gsum += __shfl_sync(kAll, gp, r) * pr[r];
     }
-    gu0 = warp_sum(gu0);
-    gu1 = warp_sum(gu1);
-    gu2 = warp_sum(gu2);
+    const double sum = warp_sum4(gu0, gu1, gu2, gsum);
+    gu0 = __shfl_sync(kAll, sum, 0);
+    gu1 = __shfl_sync(kAll, sum, 8);
+    gu2 = __shfl_sync(kAll, sum, 16);
+    if (lane == 24) gcn[i] = sum;
     if (lane == 0) {
       // dE/du_a = -(1/Omega) sum_r lambda_r c_r sum_m phi dW/du_a; dE/dx_b = sum_a dE/du_a n_a inv[b][a]
       const double du[3] = {-inv_vol * gu0, -inv_vol * gu1, -inv_vol * gu2};
-      gcn[i] = gsum;
       double gx[3];
 #pragma unroll
       for (int b = 0; b < 3; ++b) {
@@ -1007,13 +1029,15 @@ static int gather_r(const MeshGeom& mg, int blocks, int n, const double* pos, do
   }
   const MeshDev g = to_dev(mg);
   *n_mcell = mcell ? blocks : 0;
-  constexpr int RC = sizeof(T) == 4 || P <= 5 ? 4 : 2;   // rank values in flight per lane: RC (P + 3) or RC (P + 1)
   auto launch = [&](auto kern) {
     kern<<<blocks, 32 * kGatherWarps, 0, s>>>(g, n, pos, ps, c6, dc6, ci, tab, order, rec.b, (const T*)rec.w,
                                               (const T*)rec.dw, phi, gcn, gpos, mcell);
   };
-#define FD3_GATHER(TA, MC) \
-  (mg.R <= RC ? launch(k_gather_z<T, TA, P, RC, MC, true>) : launch(k_gather_z<T, TA, P, RC, MC, false>))
+  // 4 or 8 ranks in flight per lane (vectors of 16 bytes), in one chunk where they all fit
+#define FD3_GATHER(TA, MC)                                         \
+  (mg.R <= 4   ? launch(k_gather_z<T, TA, P, 4, MC, true>)         \
+   : mg.R <= 8 ? launch(k_gather_z<T, TA, P, 8, MC, true>)         \
+               : launch(k_gather_z<T, TA, P, 8, MC, false>))
   if (mcell) {
     FD3_GATHER(double, true);
   } else if constexpr (sizeof(T) == 4) {
