@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(kSpThreads, sizeof(T) == 8 ? 2 : 4) k_spread(M
 // so the layouts are chosen for few wavefronts: the stores above (a thread with a whole row stores 16
 // bytes per line), staged rows of 17 or 18 values (a thread stages an atom; rows of 16 put all lanes on
 // the same banks), and per atom one z, one or two y and the rank loads for 32 multiply-adds. 139,968 atoms on
-// 256^3, 2 x 4 channels: float64 497 -> 348 us, float 283 -> 236 (before: a whole row of 8 per thread).
+// 256^3, 2 x 4 channels: float64 497 -> 348 us, float 283 -> 217 (before: a whole row of 8 per thread).
 constexpr int kColMaxSeg = 64;
 
 // what a thread owns of a z-tile: kZL values in each of kRows rows
@@ -541,6 +541,23 @@ __device__ __forceinline__ void col_atom(const ColSmem<T>& m, int a, int z0, T w
 #pragma unroll
     for (int r = 0; r < kSpRC; ++r) c[r] = r0 + r < R ? m.cc[a * R + r0 + r] : T(0);
   }
+  if constexpr (sizeof(T) == 4) {
+    // two ranks per instruction, rounded as two multiply-adds are (instruction issue bounds the float form: 2.7
+    // per cycle and SM, 236 us at the size above, without it)
+#pragma unroll
+    for (int k = 0; k < O::kRows; ++k) {
+#pragma unroll
+      for (int r = 0; r < kSpRC; r += 2) {
+        const float2 cr = make_float2(wxy[k] * c[r], wxy[k] * c[r + 1]);
+#pragma unroll
+        for (int z = 0; z < O::kZL; ++z) {
+          const float2 q = __ffma2_rn(make_float2(zr[z], zr[z]), cr, make_float2(acc[k][z][r], acc[k][z][r + 1]));
+          acc[k][z][r] = q.x;
+          acc[k][z][r + 1] = q.y;
+        }
+      }
+    }
+  } else {
 #pragma unroll
   for (int k = 0; k < O::kRows; ++k) {
 #pragma unroll
@@ -549,6 +566,7 @@ __device__ __forceinline__ void col_atom(const ColSmem<T>& m, int a, int z0, T w
 #pragma unroll
       for (int z = 0; z < O::kZL; ++z) acc[k][z][r] += zr[z] * cr;
     }
+  }
   }
 }
 
@@ -1078,5 +1096,18 @@ int launch_gather(const MeshGeom& mg, int n, const double* pos, double pos_scale
 #undef FD3_GATHER_CASE
   return FD3_EINVAL;
 }
+
+// instantiated once each, in fd3_spread_*.cu and fd3_gather_*.cu
+extern template int launch_spread<float>(const MeshGeom&, int, const double*, const int*, const int*,
+                                         const MeshRecords&, float*, cudaStream_t);
+extern template int launch_spread<double>(const MeshGeom&, int, const double*, const int*, const int*,
+                                          const MeshRecords&, double*, cudaStream_t);
+extern template int launch_gather<float>(const MeshGeom&, int, const double*, double, const double*, const double*,
+                                         const CellInfo*, const Tables*, const int*, const int*, const MeshRecords&,
+                                         const float*, double*, double*, double*, int*, cudaStream_t);
+extern template int launch_gather<double>(const MeshGeom&, int, const double*, double, const double*, const double*,
+                                          const CellInfo*, const Tables*, const int*, const int*,
+                                          const MeshRecords&, const double*, double*, double*, double*, int*,
+                                          cudaStream_t);
 
 }  // namespace fd3
