@@ -139,12 +139,13 @@ __device__ __forceinline__ void virial_acc(const KPoint<T>& q, T dq, double* acc
 
 
 // G, dG and the Hermitian-averaged Gh of every species pair at one k-point (float64 closed
-// form, or the mixed form's table), each divided by the SPME window; unused slots are zero.
+// form on the tables trig, or the mixed form's table), each divided by the SPME window; unused slots are zero.
 template <typename T, int MAXS>
 __device__ __forceinline__ void green_block(const KPoint<T>& q, int S,
                                             const typename GreenPairOf<T>::type* __restrict__ gp,
                                             const float4* __restrict__ gtab, float inv_h, T s6, T s8,
-                                            T (&G)[MAXS][MAXS], T (&dG)[MAXS][MAXS], T (&Gh)[MAXS][MAXS]) {
+                                            T (&G)[MAXS][MAXS], T (&dG)[MAXS][MAXS], T (&Gh)[MAXS][MAXS],
+                                            const double* trig) {
   int tj = 0;
   HermiteF hb{};
   if constexpr (sizeof(T) == 4) table_pos(q.knorm, inv_h, tj, hb);
@@ -158,7 +159,7 @@ __device__ __forceinline__ void green_block(const KPoint<T>& q, int S,
           const int pi = X * S - X * (X - 1) / 2 + (Y - X);
           green_lookup(gtab + (size_t)pi * (kGreenKnots + 1), tj, hb, inv_h, gv, dv);
         } else {
-          green_eval<T>(gp[X * S + Y], q.knorm, s6, s8, gv, dv);
+          green_eval<T>(gp[X * S + Y], q.knorm, s6, s8, gv, dv, TabTrig{trig});
         }
         gv *= q.inv_sc;
         dv *= q.inv_sc;
@@ -181,7 +182,7 @@ __device__ __forceinline__ void green_block(const KPoint<T>& q, int S,
             const int pi = X * S - X * (X - 1) / 2 + (Y - X);
             green_lookup(gtab + (size_t)pi * (kGreenKnots + 1), pj, pb, inv_h, gv, dv);
           } else {
-            green_eval<T>(gp[X * S + Y], q.kpart, s6, s8, gv, dv);
+            green_eval<T>(gp[X * S + Y], q.kpart, s6, s8, gv, dv, TabTrig{trig});
           }
           Gh[X][Y] = Gh[Y][X] = T(0.5) * (G[X][Y] + gv * q.inv_sc);
         }
@@ -198,10 +199,10 @@ __device__ __forceinline__ void filter_point(const KPoint<T>& q, int S, int R,
                                              const typename GreenPairOf<T>::type* __restrict__ gp,
                                              const float4* __restrict__ gtab, float inv_h, T s6, T s8,
                                              const Tables* __restrict__ tab, typename Cplx<T>::type* v, size_t cs,
-                                             double* acc) {
+                                             double* acc, const double* trig) {
   using C2 = typename Cplx<T>::type;
   T G[MAXS][MAXS], dG[MAXS][MAXS], Gh[MAXS][MAXS];
-  green_block<T, MAXS>(q, S, gp, gtab, inv_h, s6, s8, G, dG, Gh);
+  green_block<T, MAXS>(q, S, gp, gtab, inv_h, s6, s8, G, dG, Gh, trig);
   T qq = T(0), dq = T(0);
   const bool full = S == MAXS && R % MAXR == 0;   // every slot holds a channel: no predication
   const size_t xs = (size_t)R * cs;               // channel stride between species

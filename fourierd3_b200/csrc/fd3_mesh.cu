@@ -103,6 +103,11 @@ __global__ void __launch_bounds__(kFilterThreads, sizeof(T) == 8 ? 2 : (MAXS <= 
   load_recip<T>(ci, rc);
   float inv_h = 0.f;
   if constexpr (sizeof(T) == 4) inv_h = green_inv_h(g, ci);
+  __shared__ __align__(16) double trig[sizeof(T) == 8 ? TabTrig::kDoubles : 2];
+  if constexpr (sizeof(T) == 8) {
+    TabTrig::fill(trig);
+    __syncthreads();
+  }
   // the grid stride and the start point decomposed once into (rows of ix, rows of iy, iz);
   // each step then advances (ix, iy, iz) by additions with at most one carry per axis
   const size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -118,7 +123,7 @@ __global__ void __launch_bounds__(kFilterThreads, sizeof(T) == 8 ? 2 : (MAXS <= 
   int ix = (int)k_x;
   for (; k < Mh; k += stride) {
     const KPoint<T> q = kpoint_idx<T>(g, ix, iy, iz, k, rc, deconv, spme, P);
-    filter_point<T, MAXS, MAXR>(q, g.S, g.R, gp, gtab, inv_h, s6, s8, tab, spec + k, Mh, acc);
+    filter_point<T, MAXS, MAXR>(q, g.S, g.R, gp, gtab, inv_h, s6, s8, tab, spec + k, Mh, acc, trig);
     iz += st_z;
     int c = iz >= g.nzh;
     if (c) iz -= g.nzh;

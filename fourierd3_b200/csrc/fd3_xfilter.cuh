@@ -307,8 +307,9 @@ __global__ void __launch_bounds__(kFilterThreads, sizeof(T) == 4 && MAXS * MAXR 
       const int ix = k1 + N1 * k2;
       const size_t k = ((size_t)ix * n1 + y) * nzh + iz;
       const KPoint<T> q = kpoint_idx<T>(g, ix, y, iz, k, rc, deconv, spme, P);
+      static_assert(sizeof(T) == 4);
       filter_point<T, MAXS, MAXR>(q, g.S, g.R, gp, gtab, inv_h, s6, s8, tab,
-                                  buf + ((k1 * L::ROW + k2) << LKZ) + j, (size_t)CSC, acc);
+                                  buf + ((k1 * L::ROW + k2) << LKZ) + j, (size_t)CSC, acc, nullptr);
     }
     __syncthreads();
     xfft_inverse<T, N1, N2>(buf, tw, C, LKZ);
@@ -340,7 +341,7 @@ __global__ void __launch_bounds__(kFilterThreads, sizeof(T) == 4 && MAXS * MAXR 
 
 // kz values per pencil for this plan (0: the fused path does not apply). A requested width
 // (mg.xpencil = 1, 2 or 4) is used when it fits in 200 KB of shared memory; otherwise, and by
-// default, the widest pencil that leaves three CTAs per SM (float) or fits in 100 KB (double).
+// default, the widest pencil that leaves three CTAs per SM. (Float; x64_shape has float64's.)
 // Wider pencils move longer pieces of each spectrum row (measured on the 256^3 x 8-channel
 // float mesh without the L2 prefetch hint: 1.28, 0.675 and 0.568 ms for 1, 2 and 4 kz values).
 template <typename T>
@@ -354,9 +355,8 @@ inline int xfilter_kz(const MeshGeom& mg) {
   else return 0;
   auto bytes = [&](int kz) { return (((size_t)n2 * (n1 + 1)) + (size_t)C * kz * n1 * (n2 + 1)) * 2 * sizeof(T); };
   if ((mg.xpencil == 1 || mg.xpencil == 2 || mg.xpencil == 4) && bytes(mg.xpencil) <= 200 * 1024) return mg.xpencil;
-  const size_t cap = sizeof(T) == 4 ? 74 * 1024 : 100 * 1024;
   for (int kz = 4; kz >= 2; kz >>= 1)
-    if (bytes(kz) <= cap) return kz;
+    if (bytes(kz) <= 74 * 1024) return kz;
   return bytes(1) <= 200 * 1024 ? 1 : 0;
 }
 

@@ -48,7 +48,7 @@ __device__ __forceinline__ void filter_group(const KPoint<float>& q, int S, int 
                                              float inv_h, float s6, float s8, const float (&lam)[RG],
                                              float2* v, int cs, double* acc) {
   float G[MAXS][MAXS], dG[MAXS][MAXS], Gh[MAXS][MAXS];
-  green_block<float, MAXS>(q, S, gp, gtab, inv_h, s6, s8, G, dG, Gh);
+  green_block<float, MAXS>(q, S, gp, gtab, inv_h, s6, s8, G, dG, Gh, nullptr);
   float qq = 0.f, dq = 0.f;
   const bool full = S == MAXS;
 #pragma unroll

@@ -4,15 +4,15 @@
 // (reference: src/fourierd3/kspace_filter_d3.py:29-70, src/fourierd3/pair_pot.py:113-228)
 //
 // In float64 the Green function is the work: three exponentials and three sine-cosine pairs per
-// species pair and k-point, about 300 instructions. A thread that evaluates all pairs of its k-point
-// holds 3 S (S + 1) / 2 values through long chains (255 registers, 8 warps per SM; and on a small mesh
-// the chain is the kernel's time). Here a chunk of kPts points is filtered at a time: geometry once per point,
-// then one (point, pair) evaluation per thread, G, dG and the Hermitian-averaged Gh to shared memory,
-// then one (point, rank) per thread for H = Gh S, the energy and the virial. Two CTAs of 256 threads
-// per SM wherever two pencils fit, so that one loads and stores while the other computes. (One thread
-// for all pairs of a point, one CTA of 256 threads: 128^3, 4 species, 5 ranks 728 us, 64^3 128 us; now 600 and
-// 87. 16^3 and 32^3, which had 3D cuFFT around the separate filter: 64 and 45 us, now 33 and 32 with the
-// plane transforms.)
+// species pair and k-point, about 300 instructions with CUDA's functions, half with TabTrig's. A thread that
+// evaluates all pairs of its k-point holds 3 S (S + 1) / 2 values through long chains (255 registers, 8 warps
+// per SM; and on a small mesh the chain is the kernel's time). Here a chunk of kPts points is filtered
+// at a time: geometry once per point, then one (point, pair) evaluation per thread, G, dG and the
+// Hermitian-averaged Gh to shared memory, then one (point, rank) per thread for H = Gh S, the energy and the
+// virial. Two CTAs of 256 threads per SM wherever two pencils fit, so that one loads and stores while the
+// other computes. (One thread for all pairs of a point, one CTA of 256 threads: 128^3, 4 species, 5 ranks
+// 728 us, 64^3 128 us; with a pair per thread 600 and 87; with TabTrig too 536 and 74. 16^3 and 32^3, which had
+// 3D cuFFT around the separate filter: 64 and 45 us, then 33 and 32 with the plane transforms.)
 #pragma once
 #include "fd3_xfilter.cuh"
 
@@ -33,7 +33,7 @@ template <int N1, int N2>
 __host__ __device__ constexpr size_t x64_smem(int C, int LKZ, int MAXS) {
   using L = XLayout<N1, N2>;
   return ((size_t)L::TW + ((size_t)C * L::PC << LKZ)) * sizeof(double2) +
-         (MAXS <= 2 ? X64Chunk<2>::kDoubles : X64Chunk<4>::kDoubles) * sizeof(double);
+         ((MAXS <= 2 ? X64Chunk<2>::kDoubles : X64Chunk<4>::kDoubles) + TabTrig::kDoubles) * sizeof(double);
 }
 
 template <int N1, int N2, int LKZ, int MAXS, int NT>
@@ -49,7 +49,9 @@ __global__ void __launch_bounds__(NT, 512 / NT)
   double2* buf = tw + L::TW;
   const int S = g.S, R = g.R, C = S * R, NP = S * (S + 1) / 2;
   constexpr int CSC = L::PC << LKZ;
-  double* kn = reinterpret_cast<double*>(buf + (size_t)C * CSC);   // [kPts] each
+  double* trig = reinterpret_cast<double*>(buf + (size_t)C * CSC);
+  TabTrig::fill(trig);
+  double* kn = trig + TabTrig::kDoubles;   // [kPts] each
   double* isc = kn + kPts;
   double* kpart = isc + kPts;          // partner |k|, or -1
   double* sG = kpart + kPts;           // [kPairs][kPts]
@@ -111,13 +113,13 @@ __global__ void __launch_bounds__(NT, 512 / NT)
         while (base + S - X <= pr) base += S - X++;
         const GreenPair& pair = gp[X * S + X + (pr - base)];
         double gv, dv;
-        green_eval<double>(pair, kn[q], s6, s8, gv, dv);
+        green_eval<double>(pair, kn[q], s6, s8, gv, dv, TabTrig{trig});
         const double w = isc[q];
         gv *= w;
         double gh = gv;
         if (kpart[q] >= 0.0) {
           double g2, d2;
-          green_eval<double>(pair, kpart[q], s6, s8, g2, d2);
+          green_eval<double>(pair, kpart[q], s6, s8, g2, d2, TabTrig{trig});
           gh = 0.5 * (gv + g2 * w);
         }
         sG[it] = gv;
@@ -236,15 +238,15 @@ int launch_x64(const X64Args& a, X64Shape sh) {
 
 // Pencil width and CTA shape for this mesh, LKZ = -1 where the x-pass does not apply: the widest pencil
 // of 2 or 4 values that fits twice per SM beside its chunk tables, else the widest that fits once
-// (128^3, 4 species, 5 ranks: 2 values twice 600 us, 4 values once 728; 64^3: 4 values twice 87, 2 values
-// twice 92); narrower where there would be fewer pencils than SMs.
+// (with CUDA's functions, 128^3, 4 species, 5 ranks: 2 values twice 600 us, 4 values once 728; 64^3: 4
+// values twice 87, 2 values twice 92); narrower where there would be fewer pencils than SMs.
 template <int N1, int N2>
 inline X64Shape x64_shape_t(const MeshGeom& mg) {
   const int C = mg.S * mg.R, most = mg.xpencil == 1 ? 0 : mg.xpencil == 2 ? 1 : 2;
   X64Shape sh{-1, 0};
   for (int pass = 0; pass < 2 && sh.LKZ < 0; ++pass)
     for (int l = most; l >= (pass == 0 && most > 0 ? 1 : 0); --l)
-      if (x64_smem<N1, N2>(C, l, mg.S) + 2048 <= (size_t)(pass == 0 ? 112 : 224) * 1024) {
+      if (x64_smem<N1, N2>(C, l, mg.S) + 2048 <= (size_t)(pass == 0 ? 113 : 224) * 1024) {
         sh = X64Shape{l, pass == 0 ? 1 : 0};
         break;
       }

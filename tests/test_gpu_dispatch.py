@@ -171,3 +171,22 @@ def test_edge_lists_sorted_by_source_or_in_any_order(cuda_device, n_atoms, n_edg
         assert abs(float(e - e0)) <= 1e-12 * abs(float(e0))
         assert (p - p0).abs().max().item() <= 1e-12 * max(1e-3, p0.abs().max().item())
         assert (g - g0).abs().max().item() <= 1e-12 * max(1e-3, g0.abs().max().item())
+
+
+@pytest.mark.parametrize("spacing,z", [(0.16, 55), (0.4, 55), (1.2, 1), (1.2, 55), (4.0, 30)])
+def test_float64_green_function_from_tables(cuda_device, spacing, z):
+    # from the smallest |k| R to exponentials below 1e-20: register filter and x-pass (tables) against the tiled filter
+    rng = np.random.default_rng(z)
+    cell = np.diag([7.0, 8.0, 7.5]) + np.triu(np.full((3, 3), 0.6), 1)
+    numbers = rng.choice([1, z], 20)
+    pos = rng.random((20, 3)) @ cell
+    m = D3Model(numbers, cell, precision="fp64", device=cuda_device, method="spme", mesh_spacing=spacing,
+                interpolation_nodes=4, c6tol=1.0, r_cut=6.0)
+    m.engine.set_tuning(fft_x=0, filter_kt=4)
+    e0, f0, s0 = (t.clone() for t in m(pos, cell))
+    for fft_x in (0, 1):
+        m.engine.set_tuning(fft_x=fft_x, filter_kt=-1)
+        e, f, s = m(pos, cell)
+        assert abs(float(e) - float(e0)) <= 1e-12 * abs(float(e0))
+        assert (f - f0).abs().max().item() <= 1e-10 * max(1.0, f0.abs().max().item())
+        assert (s - s0).abs().max().item() <= 1e-10 * max(1.0, s0.abs().max().item())
