@@ -844,7 +844,7 @@ def main():
                         "fft_c2r": (566.8e6 + 493.5e6) if yz_own else None}
     kernel_names = {"filter": {0: "k_filter", 1: "k_xfilter", 2: "k_xpass"}[fx], "spread": "k_spread_col",
                     "gather": "k_gather_z", "fft_r2c": "k_yz_forward", "fft_c2r": "k_yz_inverse",
-                    "cn_c6": "k_cn_bins + k_c6_atoms", "cn_adjoint": "k_cn_adjoint_hits"}
+                    "cn_c6": "k_cn_bins + k_c6_atoms", "cn_adjoint": "k_cn_adjoint"}
     mesh_match = tuple(mesh) == (256, 256, 256) and C == 8 and head == "mixed"
     roof = {"bound": "hbm", "kernel": dom, "kernel_name": kernel_names.get(dom), "achieved": achieved,
             "peak": peak, "peak_kind": peak_kind,

@@ -540,7 +540,7 @@ def autotune_spread(batch: "D3Batch", candidates: Sequence[int] = (0, 2, 4, 8, 1
 def autotune_fft_x(batch: "D3Batch", pencils: Sequence[int] = (1, 2, 4), reps: int = 2,
                    tma_units: Sequence[tuple] = ((16, 1), (8, 2), (8, 4), (4, 4))) -> dict:
     """Choose per plan between the 3D cuFFT transforms around the separate filter ("0") and the
-    (y, z) 2D cuFFT transforms around a fused x-FFT / filter / inverse x-FFT kernel: pencils of
+    (y, z) plane transforms around a fused x-FFT / filter / inverse x-FFT kernel: pencils of
     ``pencils`` kz values of every channel ("1/<kz>"), or TMA-moved units of (q values, ranks)
     from ``tma_units`` ("2/<q>/<ranks>", mixed precision), by the summed time of the forward
     transform, filter and inverse transform stages of the plan's heaviest structure. Plans where

@@ -75,7 +75,8 @@ int scan_exclusive(const int* in, int n, int* out, cudaStream_t s) {
 // there), which makes the order independent of the atomics. Its threads walk the segments in
 // position order, so the lanes of a warp scan the same few segments (broadcast loads): m compares
 // per id for a segment of m ids, all ids at once. (Sorting each segment in one warp, longer ones by
-// insertion in one lane, took 62 us at 12,000 HCNO atoms in 343 bins of 35; this takes 4 us.)
+// insertion in one lane: a call at 12,000 HCNO atoms, 343 bins of 35, 51 us longer; one with 1.2 M edges in
+// segments of 59 380 us longer.)
 __global__ void __launch_bounds__(256) k_key_slots(const int* __restrict__ keys, int n, int* __restrict__ counts,
                                                   int* __restrict__ slot) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;

@@ -98,7 +98,8 @@ FD3_API int fd3_plan_destroy(fd3_plan* plan);
  *                       staging path inside the same CTA).
  *   FD3_TUNE_FFT_X      1 = cuFFT transforms the (y, z) planes and one kernel does the x
  *                       transform, the filter and the inverse x transform per pencil (where
- *                       it applies: at most 4 species and 8 ranks, nx = 64, 128 or 256); 2 =
+ *                       it applies: at most 4 species and 8 ranks, nx = 64, 128 or
+ *                       256, in float64 16 and 32 too); 2 =
  *                       the same with units of rank groups moved by TMA (mixed precision); 0 =
  *                       3D cuFFT around a separate filter; -1 = the default: in mixed
  *                       precision 2 where it applies, in float64 1 where the plane
@@ -106,7 +107,7 @@ FD3_API int fd3_plan_destroy(fd3_plan* plan);
  *                       separate filter is set.
  *   FD3_TUNE_XPENCIL    kz values per pencil of the fused x-pass: 1, 2 or 4 (used when the
  *                       pencil fits in shared memory), -1 = the default (the widest that
- *                       leaves three CTAs per SM for float, within 100 KB for double);
+ *                       leaves three CTAs per SM for float, two for double if two fit);
  *                       the value in effect is 0 where the fused x-pass does not apply.
  *   FD3_TUNE_XQ         TMA x-pass (FD3_TUNE_FFT_X = 2, mixed precision): flattened (y, kz)
  *                       values per unit, 4, 8, 16 or 32; -1 = the default (by mesh and channels).
@@ -274,8 +275,8 @@ FD3_API int fd3_neighbor_fill_static(int64_t n_atoms, const double* d_pos_ang, c
                                      int32_t* d_shift, int64_t* h_count, void* stream);
 
 /* Per-stage timing of the last call on this plan, from CUDA events recorded on the
- * launching stream between stages (cell_list, cn_c6, mesh_sort, spread, fft_r2c,
- * filter, fft_c2r, gather, cn_adjoint, finalize). fd3_profile_read waits for the last
+ * launching stream between stages (cell_list, which includes the mesh sort and the stencil
+ * records, cn_c6, spread, fft_r2c, filter, fft_c2r, gather, cn_adjoint, finalize). fd3_profile_read waits for the last
  * event, writes milliseconds per stage and a comma-separated list of stage names. */
 FD3_API int fd3_profile_enable(fd3_plan* plan, int32_t on);
 FD3_API int fd3_profile_read(fd3_plan* plan, double* ms, int32_t max_stages, char* names, int32_t names_len,
