@@ -404,9 +404,9 @@ static bool fft_yz_on(const fd3_plan* p) {
 // cluster shape of the fused (y, z) forward transform: the knob, or pairs by default
 static int yz_variant(const fd3_plan* p) { return p->mg.fft_yz > 0 ? p->mg.fft_yz : 1; }
 // The pencil x-pass: asked for, or by default in float64 where this library's plane transforms take
-// the (y, z) part (summed transforms and filter against 3D cuFFT: 16^3, 4 x 5 channels 64 -> 33 us; 64^3,
-// 2 x 4 92 -> 75, 4 x 5 196 -> 155; 128^3, 2 x 4 468 -> 422, 4 x 5 1491 -> 1102; with cuFFT's 2D transforms the
-// pencils lose on larger meshes, 256^3 3191 -> 3532).
+// the (y, z) part (summed transforms and filter against 3D cuFFT: 16^3, 4 x 5 channels 56 -> 30 us; 64^3,
+// 2 x 4 89 -> 72, 4 x 5 181 -> 143; 128^3, 2 x 4 446 -> 398, 4 x 5 1237 -> 1040; with cuFFT's 2D transforms the
+// pencils lose: 128 x 128 x 256 815 -> 831, 256^3 3010 -> 3417).
 static bool old_xpass_on(const fd3_plan* p) {
   const bool dp = p->precision == FD3_PREC_FP64;
   if (p->method == FD3_METHOD_EWALD || !p->has_fft2 || xfilter_pencil(p->mg, dp ? 1 : 0) <= 0) return false;

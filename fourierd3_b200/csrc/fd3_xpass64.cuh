@@ -238,8 +238,8 @@ int launch_x64(const X64Args& a, X64Shape sh) {
 
 // Pencil width and CTA shape for this mesh, LKZ = -1 where the x-pass does not apply: the widest pencil
 // of 2 or 4 values that fits twice per SM beside its chunk tables, else the widest that fits once
-// (with CUDA's functions, 128^3, 4 species, 5 ranks: 2 values twice 600 us, 4 values once 728; 64^3: 4
-// values twice 87, 2 values twice 92); narrower where there would be fewer pencils than SMs.
+// (128^3, 4 species, 5 ranks, with CUDA's functions: 2 values twice 600 us, 4 values once 728; with TabTrig
+// 64^3: 4 values twice 76, 2 values twice 82); narrower where there would be fewer pencils than SMs.
 template <int N1, int N2>
 inline X64Shape x64_shape_t(const MeshGeom& mg) {
   const int C = mg.S * mg.R, most = mg.xpencil == 1 ? 0 : mg.xpencil == 2 ? 1 : 2;
