@@ -470,10 +470,11 @@ def _profiled_stage(batch: "D3Batch", i: int, stage, reps: int = 2) -> float:
     raise KeyError(i)
 
 
-def autotune_filter(batch: "D3Batch", candidates: Sequence = (0, 1, 2, 4, 8, 16, "tc"), reps: int = 2) -> dict:
-    """Pick the filter per species-count class from the heaviest structure of each class: a
-    CUDA-core k-tile width (0 = per-thread register kernel) or "tc" (mixed precision: the
-    tensor-core filter, where it applies).
+def autotune_filter(batch: "D3Batch", candidates: Sequence = ("default", 0, 1, 2, 4, 8, 16, "tc"), reps: int = 2) -> dict:
+    """Pick the filter per species-count class from the heaviest structure of each class: the
+    plan's default, a CUDA-core k-tile width (0 = per-thread register kernel) or "tc" (mixed
+    precision: the tensor-core filter, where it applies). The default may be an x-pass, so the
+    transform stages and the filter are timed together.
 
     Classes: up to 8 species, 9-24, 25-64. Each class is timed on its heaviest structure
     (profiled eager calls) and its best choice is set on every engine of that class where it
@@ -489,6 +490,9 @@ def autotune_filter(batch: "D3Batch", candidates: Sequence = (0, 1, 2, 4, 8, 16,
 
     def apply(e, choice) -> bool:
         try:
+            if choice == "default":
+                e.set_tuning(filter_kt=-1, filter_mma=-1)
+                return True
             if choice == "tc":
                 e.set_tuning(filter_kt=-1, filter_mma=1)
                 return e.tuning()["filter_mma"] == 1
@@ -503,7 +507,7 @@ def autotune_filter(batch: "D3Batch", candidates: Sequence = (0, 1, 2, 4, 8, 16,
         times = {}
         for choice in candidates:
             if apply(eng, choice):
-                times[choice] = _profiled_stage(batch, i, "filter", reps)
+                times[choice] = _profiled_stage(batch, i, ("fft_r2c", "filter", "fft_c2r"), reps)
         best = min(times, key=times.get)
         for key, e in batch._engines.items():
             s = len(key[0])
