@@ -346,6 +346,16 @@ __device__ __forceinline__ int nbr_bins(const GridDev& g, int b, const int* __re
   return st.pref[nnb];
 }
 
+// Neighbour bin of candidate c: the last entry with pref[e] <= c.
+__device__ __forceinline__ int nbr_bin_of(const NbrBins& st, int nnb, int c) {
+  int lo = 0, hi = nnb - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (st.pref[mid] <= c) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
+
 // Stage candidates [c0, c1); org is subtracted from the staged positions (zero for double4). The
 // staged w component is the candidate's covalent radius (the CN's only use of the species).
 template <typename P4>
@@ -355,11 +365,7 @@ __device__ __forceinline__ void stage_candidates(const GridDev& g, const NbrBins
                                                  int* j) {
   const int nnb = (2 * g.reach[0] + 1) * (2 * g.reach[1] + 1) * (2 * g.reach[2] + 1);
   for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
-    int lo = 0, hi = nnb - 1;          // last entry with pref[e] <= c
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (st.pref[mid] <= c) lo = mid; else hi = mid - 1;
-    }
+    const int lo = nbr_bin_of(st, nnb, c);
     const int u = st.a0[lo] + (c - st.pref[lo]);
     const double4 xj = xs[u];
     const int4 mj = meta[u];
@@ -388,6 +394,9 @@ __device__ __forceinline__ void wrapped_pos(const GridDev& g, double4 x, int4 m,
 // mixed form), so the adjoint reads a pair with one vector load instead of searching the cell list
 // a second time. An atom with more than `cap` such pairs (or one handled by the global-memory
 // path) is marked n = -1 and the adjoint recomputes it.
+// The dense bins of the mixed form, whose pairs are taken in float64, keep that precision in the same
+// 16 bytes: {f'(r)/r as a double, the neighbour's slot in the bin-sorted atoms, its bin's image}, from
+// which the adjoint forms d again in float64; their atoms are marked n = -2 - (number of pairs).
 template <typename TE> struct Vec4;
 template <> struct Vec4<float> { using type = float4; };
 template <> struct Vec4<double> { using type = double4; };
@@ -399,6 +408,15 @@ struct HitList {
   int* n;
   int cap;
 };
+
+// Image of a neighbour bin in one word: at most 343 bins of 3 or more per axis, so |image| <= 18.
+__device__ __forceinline__ int pack_image(const int (&m)[3]) {
+  return (m[0] + 128) | (m[1] + 128) << 8 | (m[2] + 128) << 16;
+}
+__device__ __forceinline__ float4 exact_record(double a, int u, int image) {
+  return make_float4(__int_as_float(__double2loint(a)), __int_as_float(__double2hiint(a)), __int_as_float(u),
+                     __int_as_float(image));
+}
 
 // C6 weights and factors of one atom by a group of 8 lanes: softmax interpolation over the 7
 // reference CNs (one lane each), the rank-r factors c_r = sum_p w_p V[s, p, r] (core.py:449-478,
@@ -478,9 +496,9 @@ template <typename TC> struct StagePos { using type = double4; };
 template <> struct StagePos<float> { using type = float4; };
 
 template <typename TE, typename TC, typename P4>
-__device__ __forceinline__ void cn_hit(const P4* __restrict__ sp, const int* __restrict__ sj, int c, TC w0, TC w1,
-                                       TC w2, TC rci, TC rc, const HitList<TE>& hl, size_t hb, int h,
-                                       TC& acc) {
+__device__ __forceinline__ void cn_hit(const NbrBins& st, int nnb, int cb, const P4* __restrict__ sp,
+                                       const int* __restrict__ sj, int c, TC w0, TC w1, TC w2, TC rci, TC rc,
+                                       const HitList<TE>& hl, size_t hb, int h, TC& acc) {
   const P4 pj = sp[c];
   const TC v0 = (TC)((pj.x - w0) * (TC)kAngToBohr);
   const TC v1 = (TC)((pj.y - w1) * (TC)kAngToBohr);
@@ -493,7 +511,12 @@ __device__ __forceinline__ void cn_hit(const P4* __restrict__ sp, const int* __r
   }
   if (h < hl.cap) {
     hl.j[hb + h] = sj[c];
-    hl.ad[hb + h] = typename Vec4<TE>::type{(TE)a, (TE)v0, (TE)v1, (TE)v2};
+    if constexpr (sizeof(TE) < sizeof(TC)) {
+      const int e = nbr_bin_of(st, nnb, cb + c);
+      hl.ad[hb + h] = exact_record(a, st.a0[e] + (cb + c - st.pref[e]), pack_image(st.img[e]));
+    } else {
+      hl.ad[hb + h] = typename Vec4<TE>::type{(TE)a, (TE)v0, (TE)v1, (TE)v2};
+    }
   }
 }
 
@@ -520,6 +543,7 @@ __device__ __forceinline__ void cn_bin(const GridDev& g, const NbrBins& st, int 
   const unsigned lt = (1u << lane) - 1u;
   const TC rc = (TC)tab->r_cut;
   const TC rc2 = (TC)g.rc2;
+  const int nnb = (2 * g.reach[0] + 1) * (2 * g.reach[1] + 1) * (2 * g.reach[2] + 1);
   if (ONCE) {
     stage_candidates<P4>(g, st, 0, total, xs, meta, org, tab->rcov, sp, sj);
     __syncthreads();
@@ -565,7 +589,7 @@ __device__ __forceinline__ void cn_bin(const GridDev& g, const NbrBins& st, int 
         __syncwarp();
         if (produced - consumed >= 32) {
           const int h = consumed + lane;
-          cn_hit<TE, TC>(sp, sj, rg[h & (kCnRing - 1)], w0, w1, w2, rci, rc, hl, hb, h, acc);
+          cn_hit<TE, TC>(st, nnb, cb, sp, sj, rg[h & (kCnRing - 1)], w0, w1, w2, rci, rc, hl, hb, h, acc);
           consumed += 32;
           __syncwarp();
         }
@@ -573,21 +597,22 @@ __device__ __forceinline__ void cn_bin(const GridDev& g, const NbrBins& st, int 
       // the ring holds indices into this piece: take the rest of it before the next
       if (consumed + lane < produced) {
         const int h = consumed + lane;
-        cn_hit<TE, TC>(sp, sj, rg[h & (kCnRing - 1)], w0, w1, w2, rci, rc, hl, hb, h, acc);
+        cn_hit<TE, TC>(st, nnb, cb, sp, sj, rg[h & (kCnRing - 1)], w0, w1, w2, rci, rc, hl, hb, h, acc);
       }
       consumed = produced;
       __syncwarp();
     }
     const double cnv = warp_sum((double)acc);
     if (on && lane == 0) {
-      hl.n[t] = produced <= hl.cap ? produced : -1;
+      hl.n[t] = produced > hl.cap ? -1 : sizeof(TE) < sizeof(TC) ? -2 - produced : produced;
       cn[i] = cnv;
     }
   }
 }
 
 // The mixed form (TE = float) takes bins of up to kCnFloat candidates in float and denser ones in
-// float64, so that the sums over more pairs keep the accuracy of the smaller ones.
+// float64, forward and (through their records) backward, so that the sums over more pairs keep the
+// accuracy of the smaller ones.
 constexpr int kCnFloat = 768;
 
 // The other cases, out of line so that the common one keeps its registers (nine CTAs per SM in float):
@@ -662,6 +687,12 @@ __global__ void __launch_bounds__(32 * kCnWarps, sizeof(TE) == 4 ? 9 : 7) k_cn_b
   if constexpr (C6) block_sum_store<1>(self, self_part + blockIdx.x);
 }
 
+static double mean_candidates(const CellGrid& g, int n) {
+  return (double)n / ((double)g.nb[0] * g.nb[1] * g.nb[2]) * (2 * g.reach[0] + 1) * (2 * g.reach[1] + 1) *
+         (2 * g.reach[2] + 1);
+}
+static bool mostly_dense(const CellGrid& g, int n) { return mean_candidates(g, n) + 32 > kCnFloat; }
+
 int64_t cn_max_blocks(int64_t bins) { return 4 * 148 + bins; }   // bins * ceil(4 * 148 / bins) at most
 
 int launch_cn_c6_cells(const CellGrid& g, int n, const CellList& cl, const int32_t* species, const Tables* tab,
@@ -669,9 +700,8 @@ int launch_cn_c6_cells(const CellGrid& g, int n, const CellList& cl, const int32
                        const RankOut& ro, double* self_part, int* n_self_blocks, const HitStore& hs, cudaStream_t s) {
   const int K = g.nb[0] * g.nb[1] * g.nb[2];
   // stage: the mean number of candidates and half as much again, within kCnSmem
-  const double mean = (double)n / K * (2 * g.reach[0] + 1) * (2 * g.reach[1] + 1) * (2 * g.reach[2] + 1);
-  const double want = 1.5 * mean + 64;
-  const int each = !hs.is_double && mean + 32 <= kCnFloat ? 20 : 36;   // float4 or double4, and the id
+  const double want = 1.5 * mean_candidates(g, n) + 64;
+  const int each = hs.is_double || mostly_dense(g, n) ? 36 : 20;   // double4 or float4, and the id
   int stage = want * each < kCnSmem ? ((int)want + 3) / 4 * 4 * each : kCnSmem / (4 * each) * (4 * each);
   if (!hs.is_double && each == 20 && stage > kCnFloat * 20) stage = kCnFloat * 20;
   // few bins: several CTAs share a bin's atoms (each stages the candidates) until the chip has four
@@ -706,21 +736,68 @@ int launch_cn_c6_cells(const CellGrid& g, int n, const CellList& cl, const int32
   return launch_c6_atoms(n, species, tab, eigvecs, R, cn, c6, dc6, ro, self_part, n_self_blocks, s);
 }
 
+// One atom's recorded pairs of a dense bin of the mixed form, in float64; this lane's share.
+__device__ __noinline__ PairSums cn_adjoint_atom_exact(const GridDev& g, const double4* __restrict__ xs,
+                                                       const int4* __restrict__ meta, const double* __restrict__ gcn,
+                                                       const HitList<float>& hl, int t, int nh) {
+  double w0, w1, w2;
+  wrapped_pos(g, xs[t], meta[t], w0, w1, w2);
+  const double gi = gcn[meta[t].w];
+  const size_t hb = (size_t)t * hl.cap;
+  PairSums p{0, 0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll 2
+  for (int e = threadIdx.x & 31; e < nh; e += 32) {
+    const float4 q = hl.ad[hb + e];
+    const double gj = gcn[hl.j[hb + e]];
+    const double a = __hiloint2double(__float_as_int(q.y), __float_as_int(q.x));
+    const int u = __float_as_int(q.z), im = __float_as_int(q.w);
+    const double4 xj = xs[u];
+    const int4 mj = meta[u];
+    const double S0 = (im & 255) - 128 - mj.x, S1 = (im >> 8 & 255) - 128 - mj.y, S2 = (im >> 16) - 128 - mj.z;
+    const double v0 = (xj.x + S0 * g.cell[0] + S1 * g.cell[3] + S2 * g.cell[6] - w0) * kAngToBohr;
+    const double v1 = (xj.y + S0 * g.cell[1] + S1 * g.cell[4] + S2 * g.cell[7] - w1) * kAngToBohr;
+    const double v2 = (xj.z + S0 * g.cell[2] + S1 * g.cell[5] + S2 * g.cell[8] - w2) * kAngToBohr;
+    const double w = (gi + gj) * a;
+    p.f0 -= w * v0;
+    p.f1 -= w * v1;
+    p.f2 -= w * v2;
+    const double b = gi * a;
+    p.xx += b * v0 * v0; p.xy += b * v0 * v1; p.xz += b * v0 * v2;
+    p.yy += b * v1 * v1; p.yz += b * v1 * v2; p.zz += b * v2 * v2;
+  }
+  return p;
+}
+
+// One atom without a float record (hl.n[t] = nh < 0): its float64 records, or the cell list again.
+template <typename TE, bool EXACT>
+__device__ __forceinline__ PairSums cn_adjoint_atom_rest(const GridDev& g, const int* __restrict__ bin_start,
+                                                         const double4* __restrict__ xs,
+                                                         const int4* __restrict__ meta, const int4* __restrict__ off,
+                                                         const Tables* __restrict__ tab,
+                                                         const double* __restrict__ gcn, const HitList<TE>& hl, int t,
+                                                         int nh) {
+  if constexpr (EXACT)
+    if (nh <= -2) return cn_adjoint_atom_exact(g, xs, meta, gcn, hl, t, -2 - nh);
+  return cn_adjoint_atom_global(g, bin_start, xs, meta, off, tab, gcn, t);
+}
+
 // CN adjoint: dE/dx_i = -sum_(j,S) (g_i + g_j) f'(r) d / r  (the list is symmetric), and the
 // strain virial W_ab = sum_i g_i sum_(j,S) f'(r) d_a d_b / r  (Bohr, Hartree). The force written
 // is out_scale * (mesh gradient already in grad + CN gradient). One warp per atom streams the
-// atom's recorded pairs; an atom without a record (n < 0) is traversed again from the cell list.
+// atom's recorded pairs; the others (n < 0, see cn_adjoint_atom_rest) are taken afterwards.
 // A stale cell (ci->stale, see k_cellinfo) makes every force NaN.
 // The kernel is bound by the latency of its dependent loads (count -> atom -> records -> g_j), so
 // a warp fetches the next atom's count and index while it works on this one, issues all of a
 // batch of 96 records' loads before the g_j loads that depend on them, and reads the atom's mesh
 // gradient at the start. Lane l still sums the records l, l + 32, ... in that order.
 //
-// REST: the same kernel takes the unrecorded atoms, for the sizes where another launch costs more
+// REST: the same kernel takes the atoms with n < 0, for the sizes where another launch costs more
 // than the registers of that path (up to kAdjointOne atoms; 5,184: 16 us against 19, 139,968: 104
-// against 78); otherwise k_cn_adjoint_rest follows.
-template <typename TE, bool REST>
-__global__ void __launch_bounds__(256, 4) k_cn_adjoint(const __grid_constant__ GridDev g, int n, const int* __restrict__ bin_start,
+// against 78); otherwise k_cn_adjoint_rest follows. EXACT: from the float64 records,
+// where the mixed form's bins are dense on average (otherwise its few dense ones are traversed again); the work
+// is in the calls then, which spill at four CTAs per SM (12,000 HCNO atoms: call 782 us with four, 776 with three).
+template <typename TE, bool REST, bool EXACT = false>
+__global__ void __launch_bounds__(256, EXACT ? 3 : 4) k_cn_adjoint(const __grid_constant__ GridDev g, int n, const int* __restrict__ bin_start,
                                                         const double4* __restrict__ xs,
                                                         const int4* __restrict__ meta, const int4* __restrict__ off,
                                                         const Tables* __restrict__ tab,
@@ -738,7 +815,7 @@ __global__ void __launch_bounds__(256, 4) k_cn_adjoint(const __grid_constant__ G
   int i_next = t < n ? meta[t].w : 0;
   if (ci->stale != 0.0) out_scale = __longlong_as_double(0x7ff8000000000000LL);
   // grid-stride over atoms: the block's virial is reduced once, after all its atoms
-  bool unrecorded = false;
+  bool rest = false;
   for (; t < n; t += stride) {
     const int nh = nh_next, i = i_next;
     if (t + stride < n) {
@@ -746,7 +823,7 @@ __global__ void __launch_bounds__(256, 4) k_cn_adjoint(const __grid_constant__ G
       i_next = meta[t + stride].w;
     }
     if (nh < 0) {
-      unrecorded = true;
+      rest = true;
     } else {
       const double gi = gcn[i];
       const double gq = lane < 3 ? grad[3 * i + lane] : 0.0;
@@ -794,12 +871,13 @@ __global__ void __launch_bounds__(256, 4) k_cn_adjoint(const __grid_constant__ G
       }
     }
   }
-  // atoms without a record, in a loop of their own: the call would cost the loop above its registers
-  if (REST && unrecorded)
+  // the others in a loop of their own: the calls would cost the loop above its registers
+  if (REST && rest)
     for (t = blockIdx.x * kWarpsPerBlock + wid; t < n; t += stride) {
-      if (hl.n[t] >= 0) continue;
+      const int nh = hl.n[t];
+      if (nh >= 0) continue;
       const int i = meta[t].w;
-      const PairSums p = cn_adjoint_atom_global(g, bin_start, xs, meta, off, tab, gcn, t);
+      const PairSums p = cn_adjoint_atom_rest<TE, EXACT>(g, bin_start, xs, meta, off, tab, gcn, hl, t, nh);
       v[0] += p.xx; v[1] += p.xy; v[2] += p.xz;
       v[4] += p.yy; v[5] += p.yz; v[8] += p.zz;
       const double f0 = warp_sum(p.f0), f1 = warp_sum(p.f1), f2 = warp_sum(p.f2);
@@ -815,8 +893,9 @@ __global__ void __launch_bounds__(256, 4) k_cn_adjoint(const __grid_constant__ G
   block_sum_store<9>(v, vir_part + 9 * blockIdx.x);
 }
 
-// Atoms without a record, after k_cn_adjoint<TE, false>. A warp reads the counts of the 32 atoms that
-// are its own (a grid stride apart) at once: almost always none is unrecorded.
+// The atoms with n < 0, after k_cn_adjoint<TE, false>. A warp reads the counts of the 32 atoms that
+// are its own (a grid stride apart) at once: outside the mixed form's dense boxes almost always none is.
+template <typename TE>
 __global__ void __launch_bounds__(256) k_cn_adjoint_rest(const __grid_constant__ GridDev g, int n,
                                                         const int* __restrict__ bin_start,
                                                         const double4* __restrict__ xs, const int4* __restrict__ meta,
@@ -824,16 +903,18 @@ __global__ void __launch_bounds__(256) k_cn_adjoint_rest(const __grid_constant__
                                                         const CellInfo* __restrict__ ci,
                                                         const double* __restrict__ gcn, double* __restrict__ grad,
                                                         double out_scale, double* __restrict__ vir_part,
-                                                        const int* __restrict__ hit_n) {
+                                                        HitList<TE> hl) {
   const int lane = threadIdx.x & 31, stride = gridDim.x * kWarpsPerBlock;
   double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   if (ci->stale != 0.0) out_scale = __longlong_as_double(0x7ff8000000000000LL);
   for (int64_t t0 = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); t0 < n; t0 += 32 * (int64_t)stride) {
     const int64_t own = t0 + (int64_t)lane * stride;
-    unsigned todo = __ballot_sync(0xffffffffu, own < n && hit_n[own] < 0);
+    const int own_n = own < n ? hl.n[own] : 0;
+    unsigned todo = __ballot_sync(0xffffffffu, own_n < 0);
     for (; todo; todo &= todo - 1) {
-      const int t = (int)(t0 + (int64_t)(__ffs(todo) - 1) * stride), i = meta[t].w;
-      const PairSums p = cn_adjoint_atom_global(g, bin_start, xs, meta, off, tab, gcn, t);
+      const int src = __ffs(todo) - 1, nh = __shfl_sync(0xffffffffu, own_n, src);
+      const int t = (int)(t0 + (int64_t)src * stride), i = meta[t].w;
+      const PairSums p = cn_adjoint_atom_rest<TE, sizeof(TE) == 4>(g, bin_start, xs, meta, off, tab, gcn, hl, t, nh);
       v[0] += p.xx; v[1] += p.xy; v[2] += p.xz;
       v[4] += p.yy; v[5] += p.yz; v[8] += p.zz;
       const double f0 = warp_sum(p.f0), f1 = warp_sum(p.f1), f2 = warp_sum(p.f2);
@@ -862,27 +943,25 @@ int launch_cn_adjoint_cells(const CellGrid& g, int n, const CellList& cl, const 
   if (blocks == 0) return FD3_OK;
   const GridDev gd = to_dev(g);
   const bool one = n <= kAdjointOne;
-  auto launch = [&](auto kern, auto hl) -> int {
-    kern<<<blocks, 32 * kWarpsPerBlock, 0, s>>>(gd, n, cl.bin_start, cl.xs, cl.meta, cl.off, tab, ci, gcn, grad,
-                                                out_scale, vir_part, hl);
+  auto launch = [&](auto kern, int grid, double* part, auto hl) -> int {
+    kern<<<grid, 32 * kWarpsPerBlock, 0, s>>>(gd, n, cl.bin_start, cl.xs, cl.meta, cl.off, tab, ci, gcn, grad,
+                                              out_scale, part, hl);
     FD3_LAUNCHED();
     return FD3_OK;
   };
-  int rc;
-  if (hs.is_double) {
-    const HitList<double> hl{hs.j, (double4*)hs.ad, hs.n, hs.cap};
-    rc = one ? launch(k_cn_adjoint<double, true>, hl) : launch(k_cn_adjoint<double, false>, hl);
-  } else {
-    const HitList<float> hl{hs.j, (float4*)hs.ad, hs.n, hs.cap};
-    rc = one ? launch(k_cn_adjoint<float, true>, hl) : launch(k_cn_adjoint<float, false>, hl);
-  }
-  if (rc || one) return rc;
-  k_cn_adjoint_rest<<<kRestBlocks, 32 * kWarpsPerBlock, 0, s>>>(gd, n, cl.bin_start, cl.xs, cl.meta, cl.off, tab, ci,
-                                                                gcn, grad, out_scale, vir_part + 9 * (size_t)blocks,
-                                                                hs.n);
-  FD3_LAUNCHED();
-  *n_blocks = blocks + kRestBlocks;
-  return FD3_OK;
+  auto both = [&](auto kern_one, auto kern, auto kern_rest, auto hl) -> int {
+    if (one) return launch(kern_one, blocks, vir_part, hl);
+    const int rc = launch(kern, blocks, vir_part, hl);
+    if (rc) return rc;
+    *n_blocks = blocks + kRestBlocks;
+    return launch(kern_rest, kRestBlocks, vir_part + 9 * (size_t)blocks, hl);
+  };
+  if (hs.is_double)
+    return both(k_cn_adjoint<double, true>, k_cn_adjoint<double, false>, k_cn_adjoint_rest<double>,
+                HitList<double>{hs.j, (double4*)hs.ad, hs.n, hs.cap});
+  return both(mostly_dense(g, n) ? k_cn_adjoint<float, true, true> : k_cn_adjoint<float, true>,
+              k_cn_adjoint<float, false>, k_cn_adjoint_rest<float>,
+              HitList<float>{hs.j, (float4*)hs.ad, hs.n, hs.cap});
 }
 
 // ------------------------------------------------------------------ edge-list path

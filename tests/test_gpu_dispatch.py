@@ -190,3 +190,23 @@ def test_float64_green_function_from_tables(cuda_device, spacing, z):
         assert abs(float(e) - float(e0)) <= 1e-12 * abs(float(e0))
         assert (f - f0).abs().max().item() <= 1e-10 * max(1.0, f0.abs().max().item())
         assert (s - s0).abs().max().item() <= 1e-10 * max(1.0, s0.abs().max().item())
+
+
+@pytest.mark.parametrize("n_atoms", [420, 3000, 17000])
+def test_dense_bins_of_the_mixed_form_stay_in_float64(cuda_device, n_atoms):
+    # more than 768 candidates per bin: the mixed form takes such bins in float64, and the direct sum adds
+    # nothing but float64 to them, so that both forms differ by the order of their sums alone: some 1e3 terms of
+    # 1e-16, up to ten times the largest force each, 1e-12. 420 atoms: pieces of the stage, records that overflow;
+    # 17,000: the records in a launch of their own
+    if n_atoms == 420:
+        rng = np.random.default_rng(n_atoms)
+        cell = np.diag([12.2, 12.2, 12.2]) + np.triu(np.full((3, 3), 0.4), 1)
+        grid = rng.permutation(512)[:n_atoms]
+        pos = (np.stack(np.unravel_index(grid, (8, 8, 8)), 1) + rng.uniform(0.4, 0.6, (n_atoms, 3))) / 8 @ cell
+        numbers = rng.choice([1, 6, 8], n_atoms)
+    else:
+        pos, cell, numbers = structures.hcno_box(seed=7, n_atoms=n_atoms)
+    out = [D3Model(numbers, cell, precision=p, device=cuda_device, method="spme", mesh_spacing=2.4,
+                   interpolation_nodes=4, c6tol=1.0, r_cut=6.0).direct(pos, cell, 8.0) for p in ("fp64", "mixed")]
+    for want, got in zip(*out):
+        assert (got - want).abs().max().item() <= 1e-12 * want.abs().max().item()
