@@ -1267,6 +1267,7 @@ struct NbrWork {
   CellList cl;
   int* counts;
   int* row_start;
+  int64_t* total;   // in the bin histogram's slot (256 bytes or more), which the sort has done with
 };
 void carve_nbr(int64_t N, int64_t K, Carver& c, NbrWork& w) {
   w.cl.bin_of = c.take<int>(N);
@@ -1278,6 +1279,7 @@ void carve_nbr(int64_t N, int64_t K, Carver& c, NbrWork& w) {
   w.cl.off = c.take<int4>(N);
   w.counts = c.take<int>(N);
   w.row_start = c.take<int>(N + 1);
+  w.total = reinterpret_cast<int64_t*>(w.cl.bin_count);
 }
 int nbr_work(int64_t n, const double* d_pos, const double* h_cell, double r_cut, void* d_work, size_t bytes,
              CellGrid& g, NbrWork& w) {
@@ -1293,11 +1295,19 @@ int nbr_work(int64_t n, const double* d_pos, const double* h_cell, double r_cut,
   return FD3_OK;
 }
 int nbr_prepare(int64_t n, const double* d_pos, const double* h_cell, double r_cut, void* d_work, size_t bytes,
-                CellGrid& g, NbrWork& w, cudaStream_t s) {
+                CellGrid& g, NbrWork& w, int64_t* h_count, cudaStream_t s) {
   FD3_TRY(nbr_work(n, d_pos, h_cell, r_cut, d_work, bytes, g, w));
   FD3_TRY(build_cell_list(g, (int)n, d_pos, nullptr, w.cl, s));
   FD3_TRY(launch_nbr_count(g, (int)n, w.cl, w.counts, s));
-  FD3_TRY(scan_exclusive(w.counts, (int)n, w.row_start, s));
+  FD3_TRY(launch_nbr_rows(w.counts, (int)n, w.row_start, w.total, s));
+  int64_t total = 0;
+  FD3_CUDA(cudaMemcpyAsync(&total, w.total, sizeof(total), cudaMemcpyDeviceToHost, s));
+  FD3_CUDA(cudaStreamSynchronize(s));
+  *h_count = total;
+  if (total > INT32_MAX) {
+    set_error("neighbour list", "more than 2^31 - 1 pairs");
+    return FD3_ECAPACITY;
+  }
   return FD3_OK;
 }
 }  // namespace
@@ -1322,12 +1332,7 @@ extern "C" int fd3_neighbor_count(int64_t n, const double* d_pos, const double* 
   CellGrid g;
   NbrWork w;
   if (!h_count) return FD3_EINVAL;
-  FD3_TRY(nbr_prepare(n, d_pos, h_cell, r_cut, d_work, bytes, g, w, s));
-  int total = 0;
-  FD3_CUDA(cudaMemcpyAsync(&total, w.row_start + n, sizeof(int), cudaMemcpyDeviceToHost, s));
-  FD3_CUDA(cudaStreamSynchronize(s));
-  *h_count = total;
-  return FD3_OK;
+  return nbr_prepare(n, d_pos, h_cell, r_cut, d_work, bytes, g, w, h_count, s);
 }
 
 extern "C" int fd3_neighbor_fill(int64_t n, const double* d_pos, const double* h_cell, double r_cut, void* d_work,
@@ -1337,12 +1342,8 @@ extern "C" int fd3_neighbor_fill(int64_t n, const double* d_pos, const double* h
   CellGrid g;
   NbrWork w;
   if (!h_count || !d_src || !d_dst || !d_shift) return FD3_EINVAL;
-  FD3_TRY(nbr_prepare(n, d_pos, h_cell, r_cut, d_work, bytes, g, w, s));
-  int total = 0;
-  FD3_CUDA(cudaMemcpyAsync(&total, w.row_start + n, sizeof(int), cudaMemcpyDeviceToHost, s));
-  FD3_CUDA(cudaStreamSynchronize(s));
-  *h_count = total;
-  if (total > capacity) return FD3_ECAPACITY;
+  FD3_TRY(nbr_prepare(n, d_pos, h_cell, r_cut, d_work, bytes, g, w, h_count, s));
+  if (*h_count > capacity) return FD3_ECAPACITY;
   FD3_TRY(launch_nbr_fill(g, (int)n, w.cl, w.row_start, d_src, d_dst, d_shift, s));
   return FD3_OK;
 }
@@ -1352,7 +1353,7 @@ extern "C" int fd3_neighbor_fill_counted(int64_t n, const double* d_pos, const d
                                          int32_t* d_shift, void* stream) {
   CellGrid g;
   NbrWork w;
-  if (count < 0 || (count > 0 && (!d_src || !d_dst || !d_shift))) return FD3_EINVAL;
+  if (count < 0 || count > INT32_MAX || (count > 0 && (!d_src || !d_dst || !d_shift))) return FD3_EINVAL;
   FD3_TRY(nbr_work(n, d_pos, h_cell, r_cut, d_work, bytes, g, w));
   if (count == 0) return FD3_OK;
   return launch_nbr_fill(g, (int)n, w.cl, w.row_start, d_src, d_dst, d_shift, (cudaStream_t)stream);

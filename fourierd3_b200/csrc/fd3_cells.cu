@@ -1359,9 +1359,10 @@ __global__ void __launch_bounds__(256) k_nbr(const __grid_constant__ GridDev g, 
       const int k = pos + __popc(m & ((1u << lane) - 1u));
       src[k] = i;
       dst[k] = j;
-      shift[3 * k] = S0;
-      shift[3 * k + 1] = S1;
-      shift[3 * k + 2] = S2;
+      int32_t* sh = shift + 3 * (size_t)k;
+      sh[0] = S0;
+      sh[1] = S1;
+      sh[2] = S2;
     }
     pos += __popc(m);
   };
@@ -1477,6 +1478,32 @@ int launch_nbr_count(const CellGrid& g, int n, const CellList& cl, int* counts, 
   if (blocks == 0) return FD3_OK;
   k_nbr<false><<<blocks, 32 * kWarpsPerBlock, 0, s>>>(to_dev(g), n, cl.bin_start, cl.xs, cl.meta, cl.off, counts,
                                                       nullptr, nullptr, nullptr, nullptr);
+  FD3_LAUNCHED();
+  return FD3_OK;
+}
+
+// Block 0: row starts; block 1: the total in 64 bits (the row starts hold up to 2^31 - 1 pairs).
+__global__ void __launch_bounds__(kScanThreads) k_nbr_rows(const int* __restrict__ counts, int n,
+                                                          int* __restrict__ row_start, int64_t* __restrict__ total) {
+  if (blockIdx.x == 0) {
+    scan_exclusive_block(counts, n, row_start);
+    return;
+  }
+  __shared__ long long part[32];
+  long long v = 0;
+  for (int i = threadIdx.x; i < n; i += kScanThreads) v += counts[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 32; ++w) v += part[w];
+    *total = v;
+  }
+}
+
+int launch_nbr_rows(const int* counts, int n, int* row_start, int64_t* total, cudaStream_t s) {
+  k_nbr_rows<<<2, kScanThreads, 0, s>>>(counts, n, row_start, total);
   FD3_LAUNCHED();
   return FD3_OK;
 }

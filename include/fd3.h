@@ -240,7 +240,7 @@ FD3_API int fd3_atom_terms(const fd3_plan* plan, int64_t n_atoms, int64_t n_bins
  * |x_j - x_i + S.cell| < r_cut, both directions, self-images included, (i,i,0) excluded.
  * fd3_neighbor_count synchronises the stream and returns the pair count; fd3_neighbor_fill
  * writes rows sorted by i (within a row: cell-list order). h_capacity < count gives
- * FD3_ECAPACITY with the needed count in *h_count.
+ * FD3_ECAPACITY with the needed count in *h_count, as do more than 2^31 - 1 pairs (both functions).
  */
 FD3_API int fd3_neighbor_workspace_size(int64_t n_atoms, const double* h_cell_ang, double r_cut_ang, size_t* bytes);
 FD3_API int fd3_neighbor_count(int64_t n_atoms, const double* d_pos_ang, const double* h_cell_ang, double r_cut_ang,

@@ -1,0 +1,37 @@
+"""The neighbour list at the ends of its index range."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from fourierd3_b200 import _native
+
+
+def test_a_count_beyond_the_row_starts_is_refused():
+    # refused on the host, before the pointers (never read here) reach a launch
+    lib = _native.lib()
+    cell, size = np.eye(3).reshape(9) * 20.0, ctypes.c_size_t()
+    _native.check(lib.fd3_neighbor_workspace_size(10, _native.dptr(cell), 6.0, ctypes.byref(size)), "size")
+    p = ctypes.c_void_p(256)
+    for count in (-1, 2**31, 2**40):
+        assert lib.fd3_neighbor_fill_counted(10, p, _native.dptr(cell), 6.0, p, size.value, count, p, p, p,
+                                             None) == _native.FD3_EINVAL
+
+
+@pytest.mark.gpu
+def test_more_pairs_than_the_row_starts_hold_are_refused_with_their_number(cuda_device):
+    # 66,000 atoms with about half of all others and their images in reach: 2.28e9 pairs
+    import torch
+
+    lib = _native.lib()
+    n, cell = 66000, np.eye(3).reshape(9) * 12.1
+    pos = torch.rand((n, 3), dtype=torch.float64, device=cuda_device, generator=torch.Generator(cuda_device).manual_seed(1)) * 12.1
+    size, count = ctypes.c_size_t(), ctypes.c_int64()
+    _native.check(lib.fd3_neighbor_workspace_size(n, _native.dptr(cell), 6.0, ctypes.byref(size)), "size")
+    work = torch.empty(size.value, dtype=torch.uint8, device=cuda_device)
+    rc = lib.fd3_neighbor_count(n, pos.data_ptr(), _native.dptr(cell), 6.0, work.data_ptr(), size.value,
+                                ctypes.byref(count), torch.cuda.current_stream().cuda_stream)
+    assert rc == _native.FD3_ECAPACITY
+    # pairs of uniform points: n (n - 1) times the sphere's share of the cell, to its statistical error
+    want = n * (n - 1) * 4.0 / 3.0 * np.pi * 6.0**3 / 12.1**3
+    assert count.value > 2**31 and abs(count.value - want) <= 1e-3 * want
