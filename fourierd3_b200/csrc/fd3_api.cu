@@ -1344,7 +1344,7 @@ extern "C" int fd3_neighbor_fill(int64_t n, const double* d_pos, const double* h
   if (!h_count || !d_src || !d_dst || !d_shift) return FD3_EINVAL;
   FD3_TRY(nbr_prepare(n, d_pos, h_cell, r_cut, d_work, bytes, g, w, h_count, s));
   if (*h_count > capacity) return FD3_ECAPACITY;
-  FD3_TRY(launch_nbr_fill(g, (int)n, w.cl, w.row_start, d_src, d_dst, d_shift, s));
+  FD3_TRY(launch_nbr_fill(g, (int)n, w.cl, w.row_start, d_src, d_dst, d_shift, *h_count, s));
   return FD3_OK;
 }
 
@@ -1356,7 +1356,7 @@ extern "C" int fd3_neighbor_fill_counted(int64_t n, const double* d_pos, const d
   if (count < 0 || count > INT32_MAX || (count > 0 && (!d_src || !d_dst || !d_shift))) return FD3_EINVAL;
   FD3_TRY(nbr_work(n, d_pos, h_cell, r_cut, d_work, bytes, g, w));
   if (count == 0) return FD3_OK;
-  return launch_nbr_fill(g, (int)n, w.cl, w.row_start, d_src, d_dst, d_shift, (cudaStream_t)stream);
+  return launch_nbr_fill(g, (int)n, w.cl, w.row_start, d_src, d_dst, d_shift, count, (cudaStream_t)stream);
 }
 
 // ------------------------------------------------------------------ profiling

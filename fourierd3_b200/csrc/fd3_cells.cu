@@ -1338,14 +1338,15 @@ __device__ __forceinline__ void visit_runs(const GridDev& g, const int* __restri
   __syncwarp();
 }
 
-// Number of neighbours of the warp's atom, and the same traversal writing them from row_start[i].
+// Number of neighbours of the warp's atom, and the same traversal writing them from row_start[i]; nothing is
+// written outside the outputs' `room` pairs, whatever the row starts hold.
 template <bool FILL>
 __global__ void __launch_bounds__(256) k_nbr(const __grid_constant__ GridDev g, int n,
                                             const int* __restrict__ bin_start, const double4* __restrict__ xs,
                                             const int4* __restrict__ meta, const int4* __restrict__ off,
                                             int* __restrict__ counts, const int* __restrict__ row_start,
                                             int64_t* __restrict__ src, int64_t* __restrict__ dst,
-                                            int32_t* __restrict__ shift) {
+                                            int32_t* __restrict__ shift, unsigned room) {
   __shared__ NbrRuns runs[kWarpsPerBlock];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int t = blockIdx.x * kWarpsPerBlock + wid;
@@ -1355,8 +1356,8 @@ __global__ void __launch_bounds__(256) k_nbr(const __grid_constant__ GridDev g, 
   int pos = FILL ? row_start[i] : 0;
   auto take = [&](bool hit, int j, int S0, int S1, int S2) {
     const unsigned m = __ballot_sync(0xffffffffu, hit);
-    if (FILL && hit) {
-      const int k = pos + __popc(m & ((1u << lane) - 1u));
+    const int k = pos + __popc(m & ((1u << lane) - 1u));
+    if (FILL && hit && (unsigned)k < room) {
       src[k] = i;
       dst[k] = j;
       int32_t* sh = shift + 3 * (size_t)k;
@@ -1477,7 +1478,7 @@ int launch_nbr_count(const CellGrid& g, int n, const CellList& cl, int* counts, 
   const int blocks = (n + kWarpsPerBlock - 1) / kWarpsPerBlock;
   if (blocks == 0) return FD3_OK;
   k_nbr<false><<<blocks, 32 * kWarpsPerBlock, 0, s>>>(to_dev(g), n, cl.bin_start, cl.xs, cl.meta, cl.off, counts,
-                                                      nullptr, nullptr, nullptr, nullptr);
+                                                      nullptr, nullptr, nullptr, nullptr, 0);
   FD3_LAUNCHED();
   return FD3_OK;
 }
@@ -1509,11 +1510,11 @@ int launch_nbr_rows(const int* counts, int n, int* row_start, int64_t* total, cu
 }
 
 int launch_nbr_fill(const CellGrid& g, int n, const CellList& cl, const int* row_start, int64_t* src, int64_t* dst,
-                    int32_t* shift, cudaStream_t s) {
+                    int32_t* shift, int64_t room, cudaStream_t s) {
   const int blocks = (n + kWarpsPerBlock - 1) / kWarpsPerBlock;
   if (blocks == 0) return FD3_OK;
   k_nbr<true><<<blocks, 32 * kWarpsPerBlock, 0, s>>>(to_dev(g), n, cl.bin_start, cl.xs, cl.meta, cl.off, nullptr,
-                                                     row_start, src, dst, shift);
+                                                     row_start, src, dst, shift, (unsigned)room);
   FD3_LAUNCHED();
   return FD3_OK;
 }

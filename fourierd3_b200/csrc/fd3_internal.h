@@ -143,7 +143,7 @@ int launch_c6_atoms(int n, const int32_t* species, const Tables* tab, const doub
 int launch_nbr_count(const CellGrid& g, int n, const CellList& cl, int* counts, cudaStream_t s);
 int launch_nbr_rows(const int* counts, int n, int* row_start, int64_t* total, cudaStream_t s);
 int launch_nbr_fill(const CellGrid& g, int n, const CellList& cl, const int* row_start, int64_t* src, int64_t* dst,
-                    int32_t* shift, cudaStream_t s);
+                    int32_t* shift, int64_t room, cudaStream_t s);
 
 // ---- mesh ---------------------------------------------------------------------
 struct MeshGeom {

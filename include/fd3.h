@@ -251,7 +251,7 @@ FD3_API int fd3_neighbor_fill(int64_t n_atoms, const double* d_pos_ang, const do
 
 /* The list that the preceding fd3_neighbor_count on this stream counted: same atoms, positions,
  * cell, cutoff and workspace, unchanged since; count is what it returned, and the outputs hold that
- * many pairs. Neither rebuilds the cell list nor synchronises. */
+ * many pairs (nothing is written beyond them). Neither rebuilds the cell list nor synchronises. */
 FD3_API int fd3_neighbor_fill_counted(int64_t n_atoms, const double* d_pos_ang, const double* h_cell_ang,
                       double r_cut_ang, void* d_work, size_t work_bytes, int64_t count, int64_t* d_src,
                       int64_t* d_dst, int32_t* d_shift, void* stream);

@@ -35,3 +35,30 @@ def test_more_pairs_than_the_row_starts_hold_are_refused_with_their_number(cuda_
     # pairs of uniform points: n (n - 1) times the sphere's share of the cell, to its statistical error
     want = n * (n - 1) * 4.0 / 3.0 * np.pi * 6.0**3 / 12.1**3
     assert count.value > 2**31 and abs(count.value - want) <= 1e-3 * want
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("room", [0, 1, 997])
+def test_the_counted_fill_stays_within_the_count_it_is_given(cuda_device, room):
+    # fewer pairs than were counted: the first ones are written, the space behind them is untouched
+    import torch
+
+    from fourierd3_b200 import neighbour_list
+
+    lib = _native.lib()
+    n, cell = 300, np.eye(3).reshape(9) * 13.0
+    pos = torch.rand((n, 3), dtype=torch.float64, device=cuda_device, generator=torch.Generator(cuda_device).manual_seed(2)) * 13.0
+    i, j, s = neighbour_list(pos, cell.reshape(3, 3), 6.0)
+    size, count = ctypes.c_size_t(), ctypes.c_int64()
+    _native.check(lib.fd3_neighbor_workspace_size(n, _native.dptr(cell), 6.0, ctypes.byref(size)), "size")
+    work = torch.empty(size.value, dtype=torch.uint8, device=cuda_device)
+    stream = torch.cuda.current_stream().cuda_stream
+    args = (n, pos.data_ptr(), _native.dptr(cell), 6.0, work.data_ptr(), size.value)
+    _native.check(lib.fd3_neighbor_count(*args, ctypes.byref(count), stream), "count")
+    m = count.value
+    src, dst = (torch.full((m,), -7, dtype=torch.int64, device=cuda_device) for _ in range(2))
+    shift = torch.full((m, 3), -7, dtype=torch.int32, device=cuda_device)
+    _native.check(lib.fd3_neighbor_fill_counted(*args, room, src.data_ptr(), dst.data_ptr(), shift.data_ptr(), stream),
+                  "fill")
+    for got, want in ((src, i), (dst, j), (shift, s)):
+        assert torch.equal(got[:room], want[:room]) and bool((got[room:] == -7).all())
