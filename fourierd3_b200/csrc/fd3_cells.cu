@@ -716,8 +716,8 @@ int launch_cn_c6_cells(const CellGrid& g, int n, const CellList& cl, const int32
   // runs more CTAs per SM without them (139,968 atoms, mixed, both: 226 us with, 189 us without).
   const bool with_c6 = nsplit > 1 || K < 4 * 148;
   auto launch = [&](auto kern, auto hl) -> int {
-    if (stage > kCnSmemPlain)
-      FD3_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kCnSmem));
+    const int rc = stage > kCnSmemPlain ? allow_dynamic_smem(kern, kCnSmem) : FD3_OK;
+    if (rc) return rc;
     kern<<<grid, 32 * kCnWarps, stage, s>>>(to_dev(g), stage, nsplit, cl.bin_start, cl.xs, cl.meta, cl.off, tab,
                                             eigvecs, R, cn, c6, dc6, hl, ro, self_part);
     FD3_LAUNCHED();

@@ -45,6 +45,7 @@ __device__ __forceinline__ float2 unpack2(u64 v) {
 }
 
 constexpr int kManyThreads = 256;
+constexpr int kManyWide = 40;   // species up to which two CTAs' tiles of 16 k-points fit an SM; tiles of 8 beyond
 
 template <int KT, int RP>
 struct Many {
@@ -211,7 +212,8 @@ template <int KT, int RP>
 int launch_many_t(const MeshGeom& mg, const CellInfo* ci, const float4* gtab, const Tables* tab, const float* deconv,
                   int spme, float2* spec, double* part, int* n_blocks, cudaStream_t s) {
   const size_t smem = Many<KT, RP>::smem(mg.S);
-  FD3_CUDA(cudaFuncSetAttribute(k_filter_many<KT, RP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int rc = allow_dynamic_smem(k_filter_many<KT, RP>, Many<KT, RP>::smem(KT == 16 ? kManyWide : FD3_MAX_SPECIES));
+  if (rc) return rc;
   const size_t Mh = (size_t)mg.n[0] * mg.n[1] * mg.nzh, ntile = (Mh + KT - 1) / KT;
   const size_t most = 148 * 2;   // two CTAs per SM, persistent over the tiles
   const int blocks = (int)(ntile < most ? ntile : most);
@@ -231,9 +233,8 @@ bool filter_many_applies(const MeshGeom& mg) {
 int launch_filter_many(const MeshGeom& mg, const CellInfo* ci, const float4* gtab, const Tables* tab,
                        const float* deconv, int spme, void* spec, double* part, int* n_blocks, cudaStream_t s) {
   float2* sp = reinterpret_cast<float2*>(spec);
-  // tiles of 16 k-points while two CTAs' tiles fit an SM (up to 40 species), 8 beyond
 #define FD3_MANY(KT, RP) launch_many_t<KT, RP>(mg, ci, gtab, tab, deconv, spme, sp, part, n_blocks, s)
-  if (mg.S <= 40) return mg.R <= 4 ? FD3_MANY(16, 4) : FD3_MANY(16, 8);
+  if (mg.S <= kManyWide) return mg.R <= 4 ? FD3_MANY(16, 4) : FD3_MANY(16, 8);
   return mg.R <= 4 ? FD3_MANY(8, 4) : FD3_MANY(8, 8);
 #undef FD3_MANY
 }

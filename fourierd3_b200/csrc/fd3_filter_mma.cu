@@ -77,6 +77,7 @@ __host__ __device__ inline int fm_upper_blocks(int S) {
   return n;
 }
 
+constexpr size_t kFmSmem = 225 * 1024;   // of the 227 KB that a CTA may have, 2 KB being static
 __host__ __device__ inline size_t fm_smem_bytes(int S, int R) {
   size_t b = 2 * (size_t)kFmABytes + 2 * (size_t)kFmBBytes;   // A, B: 2 stages
   b += 2 * ((fm_tile_bytes(S, R) + 127) & ~(size_t)127);      // two spectrum tiles
@@ -461,7 +462,7 @@ __global__ void __launch_bounds__(kFmThreads, 1) k_filter_mma(MeshDev g, int P, 
 // species x ranks whose operands and two spectrum tiles fit the 227 KB of a B200 CTA, and whose
 // upper-triangle pair blocks fit kFmMaxBlk per warp
 bool filter_mma_applies(const MeshGeom& mg) {
-  return mg.S >= 1 && mg.S <= kFmMaxS && mg.R >= 1 && mg.R <= 8 && fm_smem_bytes(mg.S, mg.R) <= 225 * 1024 &&
+  return mg.S >= 1 && mg.S <= kFmMaxS && mg.R >= 1 && mg.R <= 8 && fm_smem_bytes(mg.S, mg.R) <= kFmSmem &&
          fm_upper_blocks(mg.S) <= kFmMaxBlk * kFmWarps;
 }
 
@@ -477,24 +478,8 @@ int launch_filter_mma(const MeshGeom& mg, const CellInfo* ci, const float4* gtab
     return FD3_EINVAL;
   }
   const size_t smem = fm_smem_bytes(mg.S, mg.R);
-  static int allowed = -1;
-  if (allowed < 0) {
-    int dev = 0, optin = 0;
-    cudaFuncAttributes fa{};
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
-        cudaFuncGetAttributes(&fa, k_filter_mma) != cudaSuccess ||
-        cudaFuncSetAttribute(k_filter_mma, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             optin - (int)fa.sharedSizeBytes) != cudaSuccess) {
-      set_error("filter", "could not raise the shared-memory limit of the tensor-core filter");
-      return FD3_ECUDA;
-    }
-    allowed = optin - (int)fa.sharedSizeBytes;
-  }
-  if (smem > (size_t)allowed) {
-    set_error("filter", "tensor-core filter tile does not fit in shared memory (too many species x ranks)");
-    return FD3_EINVAL;
-  }
+  const int rc = allow_dynamic_smem(k_filter_mma, kFmSmem);
+  if (rc) return rc;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

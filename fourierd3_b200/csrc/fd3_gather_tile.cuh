@@ -272,18 +272,8 @@ int launch_gather_tile(const MeshGeom& mg, int n, const double* c6, const double
   const long long keys = (long long)mg.nt[0] * mg.nt[1] * mg.nt[2] * mg.S;
   if (keys <= 0 || keys > (1LL << 31) - 1) return FD3_EINVAL;
   auto kern = mg.R <= 4 ? k_gather_tile<T, P, 4> : k_gather_tile<T, P, 8>;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  static unsigned attr_set = 0;   // bit 2 dev + (R > 4) per device (set on every call past 16)
-  const unsigned bit = dev < 16 ? 1u << (2 * dev + (mg.R > 4 ? 1 : 0)) : 0u;
-  if (!bit || !(attr_set & bit)) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileGatherSmemCap) !=
-        cudaSuccess) {
-      set_error("gather", "could not raise the shared-memory limit of the tile-staged gather");
-      return FD3_ECUDA;
-    }
-    attr_set |= bit;
-  }
+  const int rc = allow_dynamic_smem(kern, kTileGatherSmemCap);
+  if (rc) return rc;
   kern<<<(unsigned)keys, 32 * kTileGatherWarps, smem, s>>>(map, to_dev(mg), b.x, b.y, b.z, key_start, c6, dc6, ci,
                                                            tab, order, rec.b, (const T*)rec.w, (const T*)rec.dw, phi,
                                                            gcn, gpos);

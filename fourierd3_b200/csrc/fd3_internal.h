@@ -30,6 +30,16 @@ void count_launch();
     }                                                             \
   } while (0)
 
+// Lets `kern` be launched with up to `most` bytes of dynamic shared memory. The limit belongs to the current
+// device and context, so it is set before every launch; `most` is a constant of the kernel, so that threads
+// that launch it with different sizes at once cannot lower it for one another.
+template <typename F>
+inline int allow_dynamic_smem(F* kern, size_t most) {
+  FD3_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void*>(kern), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)most));
+  return FD3_OK;
+}
+
 // ---- cell list geometry ------------------------------------------------------
 struct CellGrid {
   int nb[3];        // bins per axis

@@ -160,6 +160,7 @@ static int filter_units(int S) {
 // KT modulo 16 complex values: consecutive species then start KT values (one slot's width)
 // apart in the banks and a half-warp's loads do not collide.
 __host__ __device__ inline int tile_pad(int R, int KT) { return (((KT - R * KT) % 16) + 16) % 16; }
+constexpr size_t kFilterTileSmem = 220 * 1024;   // of the 227 KB that a CTA may have, 2 KB being static
 struct FilterTileSmem {
   static size_t bytes(int S, int R, int kt, size_t tsize) {
     const size_t C = (size_t)S * R, np = (size_t)S * (S + 1) / 2;
@@ -390,7 +391,7 @@ int filter_default_kt(int S, int R, size_t tsize) {
 bool filter_kt_valid(int kt, int S, int R, size_t tsize) {
   if (kt == 0) return S <= 8;
   if (kt != 1 && kt != 2 && kt != 4 && kt != 8 && kt != 16) return false;
-  return FilterTileSmem::bytes(S, R, kt, tsize) <= 220 * 1024;
+  return FilterTileSmem::bytes(S, R, kt, tsize) <= kFilterTileSmem;
 }
 
 template <typename T, int KT, int RF>
@@ -399,26 +400,12 @@ static int launch_tiled_r(const MeshDev& g, const MeshGeom& mg, const CellInfo* 
                         const float* deconv, int spme, typename Cplx<T>::type* sp, double* part, int* n_blocks,
                         cudaStream_t s) {
   const size_t smem = FilterTileSmem::bytes(mg.S, mg.R, KT, sizeof(T));
-  // per instantiation, once (outside any stream capture in practice: the first call is eager):
-  // allow the device's whole opt-in shared memory minus the kernel's static part
-  static int allowed = -1;
-  if (allowed < 0) {
-    int dev = 0, optin = 0;
-    cudaFuncAttributes fa{};
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
-        cudaFuncGetAttributes(&fa, k_filter_tiled<T, KT, RF>) != cudaSuccess ||
-        cudaFuncSetAttribute(k_filter_tiled<T, KT, RF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             optin - (int)fa.sharedSizeBytes) != cudaSuccess) {
-      set_error("filter", "could not raise the shared-memory limit of the tiled filter");
-      return FD3_ECUDA;
-    }
-    allowed = optin - (int)fa.sharedSizeBytes;
-  }
-  if (smem > (size_t)allowed) {
+  if (smem > kFilterTileSmem) {
     set_error("filter", "shared-memory tile too large for this device; choose a smaller filter k-tile");
     return FD3_EINVAL;
   }
+  const int rc = allow_dynamic_smem(k_filter_tiled<T, KT, RF>, kFilterTileSmem);
+  if (rc) return rc;
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_filter_tiled<T, KT, RF>, kFilterThreads, smem) !=
           cudaSuccess || per_sm < 1)

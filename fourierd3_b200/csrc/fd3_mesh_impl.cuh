@@ -781,15 +781,8 @@ static int spread_r(const MeshGeom& mg, dim3 grid, int n, const double* factors,
     const int cap = spread_col_cap<T>(mg);
     if (cap >= kColMinCap) {
       const size_t smem = col_smem_bytes<T>(cap, mg.R);
-      static bool attr = false;
-      if (!attr) {
-        if (cudaFuncSetAttribute(k_spread_col<T, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) !=
-            cudaSuccess) {
-          set_error("spread", "could not raise the shared-memory limit of the column spread");
-          return FD3_ECUDA;
-        }
-        attr = true;
-      }
+      const int rc = allow_dynamic_smem(k_spread_col<T, P>, 200 * 1024);
+      if (rc) return rc;
       const int nzc = (mg.nt[2] + zc - 1) / zc;
       const dim3 cgrid(mg.nt[0] * mg.nt[1] * nzc, mg.S);
       k_spread_col<T, P><<<cgrid, kSpThreads, smem, s>>>(g, zc, cap, rec.b, (const T*)rec.w, (const T*)rec.c, ks,

@@ -301,8 +301,10 @@ static int launch_plane_t(bool inverse, int nplanes, const void* in, void* out, 
   static_assert(NY * Cf::A1 % 32 == 0 && NY * Cf::A2 % 32 == 0, "whole warps");
   const void* kern = inverse ? reinterpret_cast<const void*>(k_plane_inverse<T, NY, NZ>)
                              : reinterpret_cast<const void*>(k_plane_forward<T, NY, NZ>);
-  if (Cf::kSmem > 48 * 1024)
-    FD3_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cf::kSmem));
+  if (Cf::kSmem > 48 * 1024) {
+    const int rc = allow_dynamic_smem(kern, Cf::kSmem);
+    if (rc) return rc;
+  }
   const int most = 148 * Cf::kMinBlocks;   // persistent: the twiddles once per CTA
   const int blocks = nplanes < most ? nplanes : most;
   if (inverse)

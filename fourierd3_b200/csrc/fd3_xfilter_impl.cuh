@@ -10,15 +10,8 @@ static int launch_xk(const MeshGeom& mg, const CellInfo* ci, const typename Gree
                      typename Cplx<T>::type* sp, double* part, int* n_blocks, cudaStream_t s) {
   constexpr int KZ = 1 << LKZ;
   const size_t smem = xfilter_smem<T, N1, N2>(mg.S * mg.R, KZ);
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(k_xfilter<T, MAXS, MAXR, N1, N2, LKZ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             200 * 1024) != cudaSuccess) {
-      set_error("filter", "could not raise the shared-memory limit of the fused x-pass filter");
-      return FD3_ECUDA;
-    }
-    attr = true;
-  }
+  const int rc = allow_dynamic_smem(k_xfilter<T, MAXS, MAXR, N1, N2, LKZ>, 200 * 1024);
+  if (rc) return rc;
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_xfilter<T, MAXS, MAXR, N1, N2, LKZ>, kFilterThreads,
                                                     smem) != cudaSuccess || per_sm < 1)

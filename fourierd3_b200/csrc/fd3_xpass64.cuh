@@ -18,6 +18,8 @@
 
 namespace fd3 {
 
+constexpr size_t kX64Smem = 224 * 1024;   // of the 227 KB that a CTA may have, 2 KB being static
+
 struct X64Shape {
   int LKZ, two;   // pencil width 2^LKZ; two CTAs of 256 threads per SM, else one of 512
 };
@@ -211,8 +213,10 @@ static int launch_x64_t(const X64Args& a) {
   const MeshGeom& mg = *a.mg;
   const size_t smem = x64_smem<N1, N2>(mg.S * mg.R, LKZ, MAXS);
   auto kern = k_xpass64<N1, N2, LKZ, MAXS, NT>;
-  if (smem > 40 * 1024)   // (a few KB are static)
-    FD3_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem > 40 * 1024) {   // (a few KB are static)
+    const int rc = allow_dynamic_smem(kern, kX64Smem);
+    if (rc) return rc;
+  }
   const long long ngroups = (long long)mg.n[1] * ((mg.nzh + (1 << LKZ) - 1) >> LKZ);
   long long blocks = 148LL * (512 / NT);
   if (blocks > ngroups) blocks = ngroups;
@@ -246,7 +250,7 @@ inline X64Shape x64_shape_t(const MeshGeom& mg) {
   X64Shape sh{-1, 0};
   for (int pass = 0; pass < 2 && sh.LKZ < 0; ++pass)
     for (int l = most; l >= (pass == 0 && most > 0 ? 1 : 0); --l)
-      if (x64_smem<N1, N2>(C, l, mg.S) + 2048 <= (size_t)(pass == 0 ? 113 : 224) * 1024) {
+      if (x64_smem<N1, N2>(C, l, mg.S) + 2048 <= (pass == 0 ? (size_t)113 * 1024 : kX64Smem)) {
         sh = X64Shape{l, pass == 0 ? 1 : 0};
         break;
       }

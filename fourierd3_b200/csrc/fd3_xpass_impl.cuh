@@ -45,15 +45,8 @@ int launch_xpass_t(const XpassArgs& a) {
     return FD3_EINVAL;
   }
   const size_t smem = kXpAlignPad + kXpTwBytes + (size_t)nstage * unit + work;
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(k_xpass<N1, N2, Q, RG, MAXS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)kXpSmemCap) != cudaSuccess) {
-      set_error("filter", "could not raise the shared-memory limit of the fused x-pass");
-      return FD3_ECUDA;
-    }
-    attr = true;
-  }
+  const int rc = allow_dynamic_smem(k_xpass<N1, N2, Q, RG, MAXS>, kXpSmemCap);
+  if (rc) return rc;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;

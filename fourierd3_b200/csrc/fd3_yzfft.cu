@@ -636,19 +636,10 @@ __global__ void __launch_bounds__(YzInvT::kThreads, 1)
 }
 
 template <int CL>
-int launch_yz(const void* kern, int which, int threads, size_t smem, void** args, int nplanes, cudaStream_t s,
+int launch_yz(const void* kern, int threads, size_t smem, void** args, int nplanes, cudaStream_t s,
               const char* what) {
-  static unsigned attr_set[3] = {0, 0, 0};   // per kernel, one bit per device (set every call past 32)
-  int dev = 0;
-  cudaGetDevice(&dev);
-  const unsigned bit = dev < 32 ? 1u << dev : 0u;
-  if (!bit || !(attr_set[which] & bit)) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-      set_error(what, "could not raise the shared-memory limit of the (y, z) transform");
-      return FD3_ECUDA;
-    }
-    attr_set[which] |= bit;
-  }
+  const int rc = allow_dynamic_smem(kern, smem);   // a constant of each kernel
+  if (rc) return rc;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -696,9 +687,9 @@ int launch_yz_forward(const MeshGeom& mg, int nchannels, int variant, const floa
   if (qp != kYzH && qp != kYzH + 1) return FD3_EINVAL;
   void* args[4] = {&in, &out, &n, &qp};
   if (variant == 1)
-    return launch_yz<2>(reinterpret_cast<const void*>(k_yz_forward<2>), 0, YzCfg<2>::kThreads,
+    return launch_yz<2>(reinterpret_cast<const void*>(k_yz_forward<2>), YzCfg<2>::kThreads,
                         sizeof(YzSmem<2>) + 128, args, n, s, "fft_r2c");
-  return launch_yz<4>(reinterpret_cast<const void*>(k_yz_forward<4>), 0, YzCfg<4>::kThreads, sizeof(YzSmem<4>) + 128,
+  return launch_yz<4>(reinterpret_cast<const void*>(k_yz_forward<4>), YzCfg<4>::kThreads, sizeof(YzSmem<4>) + 128,
                       args, n, s, "fft_r2c");
 }
 
@@ -714,7 +705,7 @@ int launch_yz_inverse(const MeshGeom& mg, int nchannels, int variant, const void
   int n = (int)np;
   if (qp == kYzH) {
     void* args[3] = {&in, &out, &n};
-    return launch_yz<2>(reinterpret_cast<const void*>(k_yz_inverse<2>), 1, YzCfg<2>::kThreads,
+    return launch_yz<2>(reinterpret_cast<const void*>(k_yz_inverse<2>), YzCfg<2>::kThreads,
                         sizeof(YzSmem<2>) + 128, args, n, s, "fft_c2r");
   }
   if (qp != kYzH + 1) return FD3_EINVAL;
@@ -741,7 +732,7 @@ int launch_yz_inverse(const MeshGeom& mg, int nchannels, int variant, const void
     }
   }
   void* args[5] = {&tcols, &tnyq, &in, &out, &n};
-  return launch_yz<2>(reinterpret_cast<const void*>(k_yz_inverse_tma), 2, YzInvT::kThreads, sizeof(YzInvTSmem) + 128,
+  return launch_yz<2>(reinterpret_cast<const void*>(k_yz_inverse_tma), YzInvT::kThreads, sizeof(YzInvTSmem) + 128,
                       args, n, s, "fft_c2r");
 }
 

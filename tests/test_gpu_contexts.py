@@ -41,7 +41,8 @@ def upload(a):
 
 ok(cu.cuInit(0))
 lib = _native.lib()
-boxes = {"few": structures.random_box(seed=1, n_atoms=90, z_max=2), "many": structures.random_box(seed=2, n_atoms=90, z_max=30)}
+boxes = {"few": (structures.random_box(seed=1, n_atoms=90, z_max=2), 0.3),    # 64^3: the x-passes apply
+         "many": (structures.random_box(seed=2, n_atoms=90, z_max=30), 0.9)}
 forms = [("few", "mixed", {}), ("few", "mixed", dict(fft_x=1)), ("few", "mixed", dict(gather_tile=1)),
          ("few", "fp64", {}), ("many", "mixed", {}), ("many", "mixed", dict(filter_kt=8)),
          ("many", "mixed", dict(filter_mma=1)), ("many", "fp64", {})]
@@ -49,13 +50,14 @@ for turn in range(2):
     ctx = vp()
     ok(cu.cuCtxCreate_v2(ctypes.byref(ctx), 0, 0))
     for box, precision, knobs in forms:
-        pos, cell, numbers = boxes[box]
+        (pos, cell, numbers), spacing = boxes[box]
         h = np.ascontiguousarray(cell, dtype=np.float64).reshape(9)
-        mesh = geometry.ns_mesh(np.asarray(cell) * geometry.ANGSTROM_TO_BOHR, 0.5 * geometry.ANGSTROM_TO_BOHR)
+        mesh = geometry.ns_mesh(np.asarray(cell) * geometry.ANGSTROM_TO_BOHR, spacing * geometry.ANGSTROM_TO_BOHR)
         eng = engine.Engine(engine.species_setup(np.asarray(numbers), 1.0), method="spme", order=4, mesh=mesh,
                             ewald_ns=(0, 0, 0), precision=precision, r_cut_bohr=6.0 * geometry.ANGSTROM_TO_BOHR,
                             params=engine.PBE_BJ, device=torch.device("cuda:0"))
         eng.set_tuning(**knobs)
+        assert box == "many" or eng.tuning()["fft_x"] == knobs.get("fft_x", 2 if precision == "mixed" else 1)
         n = len(numbers)
         size = eng.workspace_bytes(n, h, 6.0)
         out, species = alloc(8 * (1 + 3 * n + 9)), upload(np.ascontiguousarray(eng.setup.species, dtype=np.int32))
