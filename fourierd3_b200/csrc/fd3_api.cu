@@ -706,7 +706,6 @@ void carve(const fd3_plan* p, int64_t N, int64_t K_in, Carver& c, Work& w, int64
   // direct Ewald sum
   if (!mesh) {
     const int64_t nk = (int64_t)p->ens[0] * p->ens[1] * p->ens[2];
-    const int64_t nchunk = ewald_chunks(N > 0 ? N : 1, p->ens);
     w.ew.keys = c.take<int>(N);
     w.ew.counts = c.take<int>(p->S);
     w.ew.sp_start = c.take<int>(p->S + 1);
@@ -718,7 +717,7 @@ void carve(const fd3_plan* p, int64_t N, int64_t K_in, Carver& c, Work& w, int64
     w.ew.spec = c.take<char>((size_t)C * nk * 2 * es);
     w.ew.hspec = c.take<char>((size_t)C * nk * 2 * es);
     w.ew.kpart = w.kspc_part;
-    w.ew.gpart = c.take<double>((size_t)N * nchunk * (p->R + 3));
+    w.ew.gpart = c.take<double>((size_t)ewald_gather_slots(N, p->ens) * (p->R + 3));
   }
 }
 }  // namespace

@@ -347,6 +347,13 @@ int ewald_chunks(int64_t n, const int* ns) {
   return (int)((nrow + rows - 1) / rows);
 }
 
+// (atom, chunk) pairs that the workspace holds for n atoms: no fewer than n ewald_chunks(n), and no fewer
+// than for any smaller n, so that a workspace made for more atoms serves fewer.
+int64_t ewald_gather_slots(int64_t n, const int* ns) {
+  const int64_t by_rows = n * (((int64_t)ns[0] * ns[1] + 3) / 4), by_chip = 148 * 1024 + n;
+  return by_rows < by_chip ? by_rows : by_chip;
+}
+
 template <typename T>
 int launch_ewald(const EwaldGeom& eg, int n, const double* pos, double ps, const int32_t* species,
                  const double* c6, const double* dc6, const CellInfo* ci, const GreenPair* gp, const Tables* tab,

@@ -293,9 +293,10 @@ struct EwaldWork {
   void* spec;     // [S*R*nk] structure factors
   void* hspec;    // [S*R*nk] H = G S
   double* kpart;  // filter partials
-  double* gpart;  // [N * nchunk * (R+3)] gather partials
+  double* gpart;  // [ewald_gather_slots * (R+3)] gather partials
 };
 int ewald_chunks(int64_t n, const int* ns);
+int64_t ewald_gather_slots(int64_t n, const int* ns);
 template <typename T>
 int launch_ewald(const EwaldGeom& eg, int n, const double* pos, double ps, const int32_t* species,
                  const double* c6, const double* dc6, const CellInfo* ci, const GreenPair* gp, const Tables* tab,

@@ -210,3 +210,16 @@ def test_dense_bins_of_the_mixed_form_stay_in_float64(cuda_device, n_atoms):
                    interpolation_nodes=4, c6tol=1.0, r_cut=6.0).direct(pos, cell, 8.0) for p in ("fp64", "mixed")]
     for want, got in zip(*out):
         assert (got - want).abs().max().item() <= 1e-12 * want.abs().max().item()
+
+
+@pytest.mark.parametrize("k_cutoff", [1.0, 4.0, 10.0])
+def test_an_ewald_workspace_made_for_more_atoms_serves_fewer(cuda_device, k_cutoff):
+    # through the counts at which the sums change their number of chunks, and one call in a workspace for more
+    pos, cell, numbers = structures.random_box(seed=3, n_atoms=40, z_max=8)
+    m = D3Model(numbers, cell, precision="fp64", device=cuda_device, method="ewald", k_cutoff=k_cutoff, r_cut=6.0)
+    size = [m.engine.workspace_bytes(n, cell, 6.0) for n in (*range(1, 1500), *range(74000, 77000), 151551, 151552, 151553)]
+    assert all(a <= b for a, b in zip(size, size[1:]))
+    e, f, s = (t.clone() for t in m(pos, cell))
+    work = torch.empty(m.engine.workspace_bytes(41, cell, 6.0), dtype=torch.uint8, device=cuda_device)
+    got = m.engine.energy_forces_stress(torch.tensor(pos, device=cuda_device), cell, 6.0, work=work)
+    assert all(torch.equal(a, b) for a, b in zip(got, (e, f, s)))
