@@ -410,8 +410,7 @@ static int yz_variant(const fd3_plan* p) { return p->mg.fft_yz > 0 ? p->mg.fft_y
 static bool old_xpass_on(const fd3_plan* p) {
   const bool dp = p->precision == FD3_PREC_FP64;
   if (p->method == FD3_METHOD_EWALD || !p->has_fft2 || xfilter_pencil(p->mg, dp ? 1 : 0) <= 0) return false;
-  return p->mg.fft_x == 1 || (p->mg.fft_x == -1 && dp && p->mg.filter_kt < 0 && p->mg.fft_yz != 0 &&
-                              plane_applies(p->mg, true));
+  return p->mg.fft_x == 1 || (p->mg.fft_x == -1 && dp && p->mg.filter_kt < 0 && plane_applies(p->mg, true));
 }
 
 extern "C" int fd3_plan_set_tuning(fd3_plan* p, int32_t knob, int32_t value) {
@@ -850,7 +849,7 @@ static int mesh_pipeline(fd3_plan* p, int N, const double* pos, double ps, const
     // (y, z) transforms by the fused cluster kernels or cuFFT; x transform, filter and inverse x
     // transform in one kernel
     const bool yz = sizeof(T) == 4 && fft_yz_on(p);
-    const bool plane = mg.fft_yz != 0 && plane_applies(mg, sizeof(T) == 8);
+    const bool plane = plane_applies(mg, sizeof(T) == 8);
     if (yz) {
       FD3_TRY(launch_yz_forward(mgq, p->S * p->R, yz_variant(p), (const float*)w.rho, w.spec, s));
     } else if (plane) {

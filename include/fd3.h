@@ -126,8 +126,8 @@ FD3_API int fd3_plan_destroy(fd3_plan* plan);
  *                       two; 1: clusters of 2 CTAs, one per SM; 2: the forward transform on
  *                       clusters of 4, two per SM); 0 = cuFFT; -1 = the default (1).
  *                       Smaller planes (16 to 256 points a side; up to 128 x 256 in mixed
- *                       precision, 128 x 128 in float64) are transformed by one CTA each
- *                       unless the value is 0.
+ *                       precision, 128 x 128 in float64) are transformed by one CTA each,
+ *                       whatever the value (in effect it is 0 there).
  * fd3_plan_get_tuning returns the value in effect (the default resolved). */
 #define FD3_TUNE_FILTER_KT 0
 #define FD3_TUNE_SPREAD_ZC 1

@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 import torch
 
-from fourierd3_b200 import D3Model, FourierD3, neighbour_list, structures
+from fourierd3_b200 import D3Model, FourierD3, _native, neighbour_list, structures
 from oracle.neighbours import neighbour_list_cells
 from oracle.reference_port import OracleFourierD3
 
@@ -223,3 +223,37 @@ def test_an_ewald_workspace_made_for_more_atoms_serves_fewer(cuda_device, k_cuto
     work = torch.empty(m.engine.workspace_bytes(41, cell, 6.0), dtype=torch.uint8, device=cuda_device)
     got = m.engine.energy_forces_stress(torch.tensor(pos, device=cuda_device), cell, 6.0, work=work)
     assert all(torch.equal(a, b) for a, b in zip(got, (e, f, s)))
+
+
+def _box(lengths, numbers, seed):
+    rng = np.random.default_rng(seed)
+    cell = np.diag(lengths) + np.triu(np.full((3, 3), 0.3), 1)
+    return rng.random((len(numbers), 3)) @ cell, cell
+
+
+def _settable(t):
+    # 0 stands for "does not apply" in these, and is not a setting
+    return {k: v for k, v in t.items() if v != 0 or k not in ("xpencil", "xq", "xranks")}
+
+
+@pytest.mark.parametrize("precision,method,lengths,n_species", [
+    ("fp64", "spme", (36.0, 36.0, 36.0), 2), ("fp64", "spme", (8.0, 16.0, 8.0), 3), ("fp64", "pme", (24.0, 8.0, 140.0), 2),
+    ("mixed", "spme", (36.0, 36.0, 36.0), 2), ("mixed", "spme", (36.0, 8.0, 36.0), 4), ("mixed", "pme", (16.0, 16.0, 16.0), 2),
+    ("mixed", "spme", (36.0, 140.0, 140.0), 1), ("mixed", "ewald", (9.0, 9.0, 9.0), 2)])
+def test_settings_read_back_and_set_again_change_no_kernel(cuda_device, precision, method, lengths, n_species):
+    numbers = np.concatenate((np.arange(1, n_species + 1), np.random.default_rng(4).integers(1, n_species + 1, 60)))
+    pos, cell = _box(lengths, numbers, 5)
+
+    def run(tuning):
+        m = D3Model(numbers, cell, precision=precision, device=cuda_device, method=method, mesh_spacing=1.2,
+                    interpolation_nodes=4, r_cut=6.0)
+        if tuning is not None:
+            m.engine.set_tuning(**_settable(tuning))
+        launches = _native.launch_count()
+        out = [t.clone() for t in m(pos, cell)]
+        return m.engine.tuning(), _native.launch_count() - launches, out
+
+    tuning, launches, out = run(None)
+    again = run(tuning)
+    assert again[0] == tuning and again[1] == launches
+    assert all(torch.equal(a, b) for a, b in zip(again[2], out))
