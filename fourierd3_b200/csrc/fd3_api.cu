@@ -29,8 +29,8 @@ struct fd3_plan {
   float* d_win_axes = nullptr;
   cufftHandle fwd = 0, inv = 0;
   bool has_fft = false;
-  cufftHandle fwd2 = 0, inv2 = 0;   // (y, z) 2D transforms of the fused x-pass path
-  bool has_fft2 = false;
+  cufftHandle fwd2 = 0, inv2 = 0;   // cuFFT's (y, z) 2D transforms of the fused x-pass path
+  bool xpass_possible = false;      // some fused x-pass applies to this mesh, species and rank count
   size_t fft_ws = 0;
   // optional per-stage CUDA-event timing (fd3_profile_enable / fd3_profile_read)
   static constexpr int kMaxMarks = 24;
@@ -282,8 +282,9 @@ extern "C" int fd3_plan_create(const fd3_plan_desc* d, fd3_plan** out) {
       }
       p->has_fft = true;
       p->fft_ws = ws1 > ws2 ? ws1 : ws2;
-      // (y, z) planes for the fused x-pass: batch over the C channels and nx planes
-      if (xfilter_pencil(m, dp ? 1 : 0) > 0 || (!dp && xpass_applies(m, 8, 1))) {
+      // (y, z) planes for the fused x-pass, where they may be cuFFT's: batch over the C channels and nx planes
+      p->xpass_possible = xfilter_pencil(m, dp ? 1 : 0) > 0 || (!dp && xpass_applies(m, 8, 1));
+      if (p->xpass_possible && !plane_applies(m, dp)) {
         long long n2d[2] = {m.n[1], m.n[2]};
         const long long pr = (long long)m.n[1] * m.n[2], pc = (long long)m.n[1] * m.nzh;
         size_t ws3 = 0, ws4 = 0;
@@ -300,7 +301,6 @@ extern "C" int fd3_plan_create(const fd3_plan_desc* d, fd3_plan** out) {
           rc = FD3_ECUFFT;
           break;
         }
-        p->has_fft2 = true;
         if (ws3 > p->fft_ws) p->fft_ws = ws3;
         if (ws4 > p->fft_ws) p->fft_ws = ws4;
       }
@@ -388,7 +388,7 @@ static void xpass_shape(const fd3_plan* p, int* Q, int* RG) {
 }
 // By default on wherever it applies, unless a knob of the separate filter is set.
 static bool xpass_on(const fd3_plan* p) {
-  if (p->method == FD3_METHOD_EWALD || !p->has_fft2 || p->precision != FD3_PREC_MIXED) return false;
+  if (p->method == FD3_METHOD_EWALD || !p->xpass_possible || p->precision != FD3_PREC_MIXED) return false;
   if (p->mg.fft_x != 2 &&
       !(p->mg.fft_x == -1 && p->mg.filter_kt < 0 && p->mg.filter_mma != 1 && tensor_maps_available()))
     return false;
@@ -409,7 +409,7 @@ static int yz_variant(const fd3_plan* p) { return p->mg.fft_yz > 0 ? p->mg.fft_y
 // pencils lose: 128 x 128 x 256 815 -> 831, 256^3 3010 -> 3417).
 static bool old_xpass_on(const fd3_plan* p) {
   const bool dp = p->precision == FD3_PREC_FP64;
-  if (p->method == FD3_METHOD_EWALD || !p->has_fft2 || xfilter_pencil(p->mg, dp ? 1 : 0) <= 0) return false;
+  if (p->method == FD3_METHOD_EWALD || !p->xpass_possible || xfilter_pencil(p->mg, dp ? 1 : 0) <= 0) return false;
   return p->mg.fft_x == 1 || (p->mg.fft_x == -1 && dp && p->mg.filter_kt < 0 && plane_applies(p->mg, true));
 }
 
@@ -526,7 +526,7 @@ extern "C" int fd3_plan_get_tuning(const fd3_plan* p, int32_t knob, int32_t* val
   if (knob == FD3_TUNE_XQ || knob == FD3_TUNE_XRANKS) {
     int Q = 0, RG = 0;
     xpass_shape(p, &Q, &RG);
-    const bool ok = p->has_fft2 && p->precision == FD3_PREC_MIXED && xpass_applies(p->mg, Q, RG);
+    const bool ok = p->xpass_possible && p->precision == FD3_PREC_MIXED && xpass_applies(p->mg, Q, RG);
     *value = ok ? (knob == FD3_TUNE_XQ ? Q : RG) : 0;
     return FD3_OK;
   }
@@ -538,7 +538,7 @@ extern "C" int fd3_plan_get_tuning(const fd3_plan* p, int32_t knob, int32_t* val
     return FD3_OK;
   }
   if (knob == FD3_TUNE_XPENCIL) {
-    *value = p->has_fft2 ? xfilter_pencil(p->mg, p->precision == FD3_PREC_FP64 ? 1 : 0) : 0;
+    *value = p->xpass_possible ? xfilter_pencil(p->mg, p->precision == FD3_PREC_FP64 ? 1 : 0) : 0;
     return FD3_OK;
   }
   if (knob == FD3_TUNE_FFT_YZ) {
