@@ -505,8 +505,12 @@ extern "C" int fd3_plan_get_tuning(const fd3_plan* p, int32_t knob, int32_t* val
   if (!p || !value) return FD3_EINVAL;
   if (knob == FD3_TUNE_FILTER_KT) {
     const size_t ts = p->precision == FD3_PREC_FP64 ? 8 : 4;
+    // unset and another kernel does the filter: -1, which asks for that kernel when set again
+    const bool other = xpass_on(p) || old_xpass_on(p) ||
+                       (ts == 4 && (filter_mma_on(p->mg) || filter_many_applies(p->mg)));
     *value = p->method == FD3_METHOD_EWALD ? -1
              : p->mg.filter_kt >= 0        ? p->mg.filter_kt
+             : other                       ? -1
                                            : filter_default_kt(p->S, p->R, ts);
     return FD3_OK;
   }

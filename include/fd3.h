@@ -128,7 +128,8 @@ FD3_API int fd3_plan_destroy(fd3_plan* plan);
  *                       Smaller planes (16 to 256 points a side; up to 128 x 256 in mixed
  *                       precision, 128 x 128 in float64) are transformed by one CTA each,
  *                       whatever the value (in effect it is 0 there).
- * fd3_plan_get_tuning returns the value in effect (the default resolved). */
+ * fd3_plan_get_tuning returns the value in effect (the default resolved; FILTER_KT -1 where no k-tile
+ * is set and another kernel does the filter: an x-pass, the many-species or the tensor-core filter). */
 #define FD3_TUNE_FILTER_KT 0
 #define FD3_TUNE_SPREAD_ZC 1
 #define FD3_TUNE_SPREAD_CAP 2

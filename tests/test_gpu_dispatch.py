@@ -239,7 +239,8 @@ def _settable(t):
 @pytest.mark.parametrize("precision,method,lengths,n_species", [
     ("fp64", "spme", (36.0, 36.0, 36.0), 2), ("fp64", "spme", (8.0, 16.0, 8.0), 3), ("fp64", "pme", (24.0, 8.0, 140.0), 2),
     ("mixed", "spme", (36.0, 36.0, 36.0), 2), ("mixed", "spme", (36.0, 8.0, 36.0), 4), ("mixed", "pme", (16.0, 16.0, 16.0), 2),
-    ("mixed", "spme", (36.0, 140.0, 140.0), 1), ("mixed", "ewald", (9.0, 9.0, 9.0), 2)])
+    ("mixed", "spme", (36.0, 140.0, 140.0), 1), ("mixed", "ewald", (9.0, 9.0, 9.0), 2), ("mixed", "spme", (9.0, 12.0, 10.0), 20),
+    ("mixed", "spme", (9.0, 12.0, 10.0), 10), ("fp64", "spme", (9.0, 12.0, 10.0), 20)])
 def test_settings_read_back_and_set_again_change_no_kernel(cuda_device, precision, method, lengths, n_species):
     numbers = np.concatenate((np.arange(1, n_species + 1), np.random.default_rng(4).integers(1, n_species + 1, 60)))
     pos, cell = _box(lengths, numbers, 5)
