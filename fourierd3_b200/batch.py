@@ -519,8 +519,8 @@ def autotune_filter(batch: "D3Batch", candidates: Sequence = ("default", 0, 1, 2
 
 def autotune_spread(batch: "D3Batch", candidates: Sequence[int] = (0, 2, 4, 8, 15), reps: int = 2) -> dict:
     """Pick the spread's z-chunk length (0 = per-tile kernel) from the heaviest structure of each
-    plan: every candidate is timed (profiled eager calls) and the fastest is set on that plan.
-    Returns {plan index: (chunk, {chunk: ms})}. Drops a captured graph."""
+    plan: every candidate and the plan's default are timed (profiled eager calls) and the fastest
+    is set on that plan. Returns {plan index: (chunk, {chunk: ms})}. Drops a captured graph."""
     batch.drop_captures()
     heaviest: dict = {}
     for i, key in enumerate(batch._keys):
@@ -530,7 +530,9 @@ def autotune_spread(batch: "D3Batch", candidates: Sequence[int] = (0, 2, 4, 8, 1
     for n, (key, i) in enumerate(heaviest.items()):
         eng = batch._engines[key]
         times = {}
-        for zc in candidates:
+        eng.set_tuning(spread_zc=-1)
+        default = eng.tuning()["spread_zc"]
+        for zc in (*candidates, *([] if default in candidates else [default])):
             eng.set_tuning(spread_zc=zc)
             if eng.tuning()["spread_zc"] != zc and zc != 0:
                 continue   # capped by the mesh: the same as a smaller chunk
@@ -546,7 +548,7 @@ def autotune_fft_x(batch: "D3Batch", pencils: Sequence[int] = (1, 2, 4), reps: i
     """Choose per plan between the 3D cuFFT transforms around the separate filter ("0") and the
     (y, z) plane transforms around a fused x-FFT / filter / inverse x-FFT kernel: pencils of
     ``pencils`` kz values of every channel ("1/<kz>"), or TMA-moved units of (q values, ranks)
-    from ``tma_units`` ("2/<q>/<ranks>", mixed precision), by the summed time of the forward
+    from ``tma_units`` and the plan's default unit ("2/<q>/<ranks>", mixed precision), by the summed time of the forward
     transform, filter and inverse transform stages of the plan's heaviest structure. Plans where
     no fused path applies keep "0". On an x-pass path with 256 x 256 (y, z) planes it then times
     the (y, z) transforms as cluster kernels on pairs (the default), with the forward on quads
@@ -569,7 +571,10 @@ def autotune_fft_x(batch: "D3Batch", pencils: Sequence[int] = (1, 2, 4), reps: i
             if t["fft_x"] != 1 or t["xpencil"] != kz:
                 continue   # no fused kernel for this mesh, species or rank count, or too wide
             times[f"1/{kz}"] = _profiled_stage(batch, i, stages, reps)
-        for xq, xr in tma_units:
+        eng.set_tuning(fft_x=2, xq=-1, xranks=-1)
+        t = eng.tuning()
+        default = (t["xq"], t["xranks"])
+        for xq, xr in (*tma_units, *([] if t["fft_x"] != 2 or default in tma_units else [default])):
             eng.set_tuning(fft_x=2, xq=xq, xranks=xr)
             t = eng.tuning()
             if t["fft_x"] != 2 or (t["xq"], t["xranks"]) != (xq, xr):

@@ -191,3 +191,20 @@ def test_forward_batch_surface(cuda_device):
     for (pos, cell, z), (e, f, s) in zip(structs, res):
         e1, f1, s1 = D3Model(z, cell, precision="fp64", device=cuda_device, **KW)(pos, cell)
         assert torch.equal(e, e1) and torch.equal(f, f1) and torch.equal(s, s1)
+
+
+def test_autotuners_time_the_plans_own_defaults(cuda_device):
+    """The default chunk of a small box's spread (1) and the default x-pass unit at three ranks
+    ((16, 2)) are not among the fixed candidates: both are timed all the same."""
+    from fourierd3_b200.batch import D3Batch, autotune_fft_x, autotune_spread
+
+    rng = np.random.default_rng(6)
+    cell = np.diag([36.0, 20.0, 20.0])
+    numbers = np.concatenate(([1, 2], rng.integers(1, 3, 60)))
+    b = D3Batch([(rng.random((len(numbers), 3)) @ cell, cell, numbers)], precision="mixed", device=cuda_device,
+                method="spme", mesh_spacing=1.2, interpolation_nodes=5, c6tol=0.05, r_cut=6.0)
+    t = next(iter(b._engines.values())).tuning()
+    assert t["spread_zc"] not in (0, 2, 4, 8, 15) and t["fft_x"] == 2
+    assert (t["xq"], t["xranks"]) not in ((16, 1), (8, 2), (8, 4), (4, 4))
+    assert t["spread_zc"] in autotune_spread(b, reps=1)[0][1]
+    assert f"2/{t['xq']}/{t['xranks']}" in autotune_fft_x(b, reps=1)[0][1]
