@@ -258,3 +258,30 @@ def test_settings_read_back_and_set_again_change_no_kernel(cuda_device, precisio
     again = run(tuning)
     assert again[0] == tuning and again[1] == launches
     assert all(torch.equal(a, b) for a, b in zip(again[2], out))
+
+
+@pytest.mark.parametrize("sources", [(100000, 100009), (0, 1), (199998, 199999)])
+def test_sorted_edges_on_a_few_of_many_atoms(cuda_device, sources):
+    # 200,000 atoms, two of them with edges: the same results as in descending order, and no slower (the segment
+    # starts of the atoms without edges are one run of stores; half as long again is left for the timer)
+    n = 200000
+    rng = np.random.default_rng(8)
+    cell = torch.tensor(np.diag([230.0] * 3), device=cuda_device)
+    numbers = rng.choice([8, 14], n)
+    pos = torch.tensor(rng.random((n, 3)) * 230.0, device=cuda_device)
+    m = FourierD3(numbers, cell.cpu().numpy(), dtype=torch.float64, device=cuda_device, verbose=False, method="spme",
+                  mesh_spacing=8.0, interpolation_nodes=4, r_cut=12.0)
+    edges = torch.tensor([sources, sources[::-1]], device=cuda_device)
+    shift = torch.tensor([[1.0, 2.0, 3.0], [-1.0, -2.0, -3.0]], dtype=torch.float64, device=cuda_device)
+    shift -= pos[edges[1]] - pos[edges[0]]
+    m._eng.profile(True)
+    out, ms = [], []
+    for order in ([0, 1], [1, 0]):
+        times = []
+        for _ in range(6):
+            got = m._eng.energy_edges(pos, cell, edges[:, order], shift[order], True)
+            times.append(m._eng.stage_times()["cn_c6"])
+        out.append((got[0].clone(), got[1].clone(), got[2][order].clone(), got[3].clone()))
+        ms.append(np.median(times[1:]))
+    assert all(torch.equal(a, b) for a, b in zip(*out))
+    assert ms[0] <= 1.5 * ms[1]
