@@ -139,6 +139,7 @@ extern "C" int fd3_plan_create(const fd3_plan_desc* d, fd3_plan** out) {
 
   Tables& t = p->h_tab;
   memset(&t, 0, sizeof(t));
+  TabTrig::make(t.trig);
   t.n_species = S;
   t.n_rank = R;
   t.s6 = d->params[0];

@@ -15,6 +15,7 @@ namespace fd3 {
 
 constexpr double kPi = 3.14159265358979323846;
 constexpr double kAngToBohr = 1.0 / 0.52917726;   // core.py:120
+constexpr int kTrigDoubles = 6 * 64;
 constexpr double kHartreeToEv = 27.21138505;      // calculator.py:54
 
 // Cell-derived quantities, computed on the device from the (possibly strained) cell.
@@ -47,6 +48,7 @@ struct Tables {
   double eigs[FD3_MAX_RANK];
   double s6, s8, r_cut;
   int n_species, n_rank, has_cncorr, pad;
+  alignas(16) double trig[kTrigDoubles];     // TabTrig::make
   // eigvecs (S,7,r) and the (S,S) GreenPair matrix follow in separate device arrays
 };
 
@@ -240,12 +242,15 @@ __device__ __forceinline__ void lagrange(T x, T* w, T* dw) {
 
 // The exponentials and sine-cosine pairs of the Green function: CUDA's, or in float64 from tables in
 // shared memory (table-driven reduction as in Tang, ACM TOMS 15 (1989) 144, and angle addition):
-//   exp(x) = 2^(m / 64) e^r, |r| <= ln 2 / 128, Taylor to r^5 (remainder 4e-17), for x <= 0;
-//   sin, cos(pi a) by rotating entry m of 128 by pi (a - m / 64), |.| <= pi / 128, Taylor to r^7, r^6 (4e-18).
-// Measured against 128-bit arithmetic on [-60, 0] and [0.3, 40]: exp 1.02 ulp, sine and cosine 1.2e-16.
+//   exp(x) = 2^(m / 64) e^r, |r| <= ln 2 / 128, Taylor to r^6 (remainder 3e-20), for x <= 0;
+//   sin, cos(pi a) by rotating entry m of 64 by pi (a - m / 32), |.| <= pi / 64, Taylor to r^7, r^8 (5e-18).
+// The entries are in two parts, so that a result is rounded once at full size (with entries of one part, from
+// CUDA's functions, the exponential was up to 2.05 x 2^-53 of its value off, 0.60 in the root mean square).
+// Measured against 128-bit arithmetic on [-600, 0] and [0.25, 600], largest and root mean square: exp
+// 1.00 and 0.42 x 2^-53 of its value (CUDA's 1.24 and 0.44), sine and cosine 7.2e-17 and 3.5e-17 (1.3e-16, 4.1e-17).
 // About 45 instructions for an exponential and a pair, where the library's, which serve every argument, take
-// about 100: they bound the float64 filters. 256^3, 2 species, 4 ranks 690 -> 528 us, 128^3, 4 x 5 397 -> 280;
-// x-pass of 128^3, 4 x 5 598 -> 536, 64^3, 4 x 5 89 -> 74.
+// about 100: they bound the float64 filters. 256^3, 2 species, 4 ranks 690 -> 545 us (entries of one part: 523);
+// x-pass of 128^3, 4 x 5 598 -> 557, 64^3, 4 x 5 89 -> 76.
 struct LibTrig {
   template <typename T>
   __device__ __forceinline__ T expv(T x) const {
@@ -257,12 +262,23 @@ struct LibTrig {
   }
 };
 struct TabTrig {
-  static constexpr int kExp = 64, kArc = 128, kDoubles = 2 * kArc + kExp;
-  const double* t;   // [kArc] (sin, cos), then [kExp] powers of two; 16-byte aligned
-  __device__ __forceinline__ static void fill(double* t) {
-    for (int i = threadIdx.x; i < kArc; i += blockDim.x) sincospi(i / 64.0, t + 2 * i, t + 2 * i + 1);
-    for (int i = threadIdx.x; i < kExp; i += blockDim.x) t[2 * kArc + i] = exp2(i / 64.0);
+  static constexpr int kN = 64, kDoubles = kTrigDoubles;
+  const double* t;   // [kN] (sin, cos), [kN] their second parts, [kN] (power of two, second part); 16-byte aligned
+  // The table, on the host: sin, cos(pi i / 32) and 2^(i / 64) rounded to double, and what is left of them.
+  static void make(double* t) {
+    auto put = [t](int k, long double v) { t[k] = (double)v, t[k + (k < 2 * kN ? 2 * kN : 1)] = (double)(v - (double)v); };
+    for (int i = 0; i < kN; ++i) {
+      const long double x = 3.14159265358979323846264338327950288L * (i % 16) / 32, s = sinl(x), c = cosl(x);
+      const long double q[5] = {s, c, -s, -c, s};   // a quarter turn on: (s, c) -> (c, -s)
+      put(2 * i, q[i / 16]);
+      put(2 * i + 1, q[i / 16 + 1]);
+      put(4 * kN + 2 * i, exp2l(i / 64.0L));
+    }
   }
+  __device__ __forceinline__ static void fill(double* t, const Tables* __restrict__ tab) {
+    for (int i = threadIdx.x; i < kDoubles; i += blockDim.x) t[i] = tab->trig[i];
+  }
+  __device__ __forceinline__ double2 entry(int i) const { return reinterpret_cast<const double2*>(t)[i]; }
   __device__ __forceinline__ double expv(double x) const {
     constexpr double kRound = 6755399441055744.0;   // 1.5 * 2^52: the sum's low word is the nearest integer
     x = x < -700.0 ? -700.0 : x;
@@ -271,22 +287,24 @@ struct TabTrig {
     const double md = q - kRound;
     double r = fma(md, -0.010830424696249145, x);     // ln 2 / 64 in two parts
     r = fma(md, -3.623510646634843e-19, r);
-    double p = fma(fma(fma(r, 1.0 / 120.0, 1.0 / 24.0), r, 1.0 / 6.0), r, 0.5);
+    double p = fma(fma(fma(fma(r, 1.0 / 720.0, 1.0 / 120.0), r, 1.0 / 24.0), r, 1.0 / 6.0), r, 0.5);
     p = fma(p * r, r, r);
-    const double e = t[2 * kArc + (m & (kExp - 1))];
-    const double v = fma(e, p, e);
+    const double2 e = entry(2 * kN + (m & (kN - 1)));
+    const double v = e.x + fma(e.x, p, e.y);
     return __hiloint2double(__double2hiint(v) + ((m >> 6) << 20), __double2loint(v));
   }
   __device__ __forceinline__ void sincospiv(double a, double* s, double* c) const {
     constexpr double kRound = 6755399441055744.0;
-    const double q = fma(a, 64.0, kRound);
-    const int m = __double2loint(q);
-    const double r = fma(q - kRound, -1.0 / 64.0, a) * kPi, r2 = r * r;
-    const double sr = fma(r * r2, fma(r2, fma(r2, -1.0 / 5040.0, 1.0 / 120.0), -1.0 / 6.0), r);
-    const double cr = r2 * fma(r2, fma(r2, -1.0 / 720.0, 1.0 / 24.0), -0.5);
-    const double2 e = *reinterpret_cast<const double2*>(t + 2 * (m & (kArc - 1)));
-    *s = e.x + fma(e.x, cr, e.y * sr);
-    *c = e.y + fma(e.y, cr, -(e.x * sr));
+    const double q = fma(a, 32.0, kRound);
+    const int m = __double2loint(q) & (kN - 1);
+    const double r = fma(q - kRound, -1.0 / 32.0, a), r2 = r * r;   // powers of pi are in the coefficients
+    constexpr double p2 = kPi * kPi, p4 = p2 * p2;
+    const double sr =
+        r * fma(r2, fma(r2, fma(r2, -p4 * p2 * kPi / 5040.0, p4 * kPi / 120.0), -p2 * kPi / 6.0), kPi);
+    const double cr = r2 * fma(r2, fma(r2, fma(r2, p4 * p4 / 40320.0, -p4 * p2 / 720.0), p4 / 24.0), -p2 / 2.0);
+    const double2 e = entry(m), l = entry(kN + m);
+    *s = e.x + fma(e.x, cr, fma(e.y, sr, l.x));
+    *c = e.y + fma(e.y, cr, fma(-e.x, sr, l.y));
   }
 };
 

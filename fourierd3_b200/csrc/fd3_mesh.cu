@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(kFilterThreads, sizeof(T) == 8 ? 2 : (MAXS <= 
   if constexpr (sizeof(T) == 4) inv_h = green_inv_h(g, ci);
   __shared__ __align__(16) double trig[sizeof(T) == 8 ? TabTrig::kDoubles : 2];
   if constexpr (sizeof(T) == 8) {
-    TabTrig::fill(trig);
+    TabTrig::fill(trig, tab);
     __syncthreads();
   }
   // the grid stride and the start point decomposed once into (rows of ix, rows of iy, iz);

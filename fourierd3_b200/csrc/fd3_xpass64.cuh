@@ -11,7 +11,7 @@
 // Hermitian-averaged Gh to shared memory, then one (point, rank) per thread for H = Gh S, the energy and the
 // virial. Two CTAs of 256 threads per SM wherever two pencils fit, so that one loads and stores while the
 // other computes. (One thread for all pairs of a point, one CTA of 256 threads: 128^3, 4 species, 5 ranks
-// 728 us, 64^3 128 us; with a pair per thread 600 and 87; with TabTrig too 536 and 74. 16^3 and 32^3, which had
+// 728 us, 64^3 128 us; with a pair per thread 600 and 87; with TabTrig too 557 and 76. 16^3 and 32^3, which had
 // 3D cuFFT around the separate filter: 64 and 45 us, then 33 and 32 with the plane transforms.)
 #pragma once
 #include "fd3_xfilter.cuh"
@@ -52,7 +52,8 @@ __global__ void __launch_bounds__(NT, 512 / NT)
   const int S = g.S, R = g.R, C = S * R, NP = S * (S + 1) / 2;
   constexpr int CSC = L::PC << LKZ;
   double* trig = reinterpret_cast<double*>(buf + (size_t)C * CSC);
-  TabTrig::fill(trig);
+  for (int i = threadIdx.x; i < TabTrig::kDoubles / 2; i += NT)   // waited for with the first pencil
+    copy_async16(trig + 2 * i, tab->trig + 2 * i);
   double* kn = trig + TabTrig::kDoubles;   // [kPts] each
   double* isc = kn + kPts;
   double* kpart = isc + kPts;          // partner |k|, or -1
