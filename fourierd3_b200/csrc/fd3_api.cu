@@ -407,11 +407,16 @@ static int yz_variant(const fd3_plan* p) { return p->mg.fft_yz > 0 ? p->mg.fft_y
 // The pencil x-pass: asked for, or by default in float64 where this library's plane transforms take
 // the (y, z) part (summed transforms and filter against 3D cuFFT: 16^3, 4 x 5 channels 56 -> 30 us; 64^3,
 // 2 x 4 89 -> 72, 4 x 5 181 -> 143; 128^3, 2 x 4 446 -> 398, 4 x 5 1237 -> 1040; with cuFFT's 2D transforms the
-// pencils lose: 128 x 128 x 256 815 -> 831, 256^3 3010 -> 3417).
+// pencils lose: 128 x 128 x 256 815 -> 831, 256^3 3010 -> 3417), and its pencils fit an SM twice: one at a time they
+// win up to nx = 128 and 64 x 64 planes alone (4 x 8, whole calls of 64 atoms: 128 x 64 x 64 543 -> 487 us,
+// 128^3 1750 -> 1827; 4 x 5, 256 x 64 x 64 671 -> 681, 256 x 128 x 128 2253 -> 2537). Over all planes of 16 to
+// 256 a side and nx = 16 to 256 the default is 1.08 times as fast as 3D cuFFT, at worst 0.95 (16 x 256 x 32).
 static bool old_xpass_on(const fd3_plan* p) {
   const bool dp = p->precision == FD3_PREC_FP64;
   if (p->method == FD3_METHOD_EWALD || !p->xpass_possible || xfilter_pencil(p->mg, dp ? 1 : 0) <= 0) return false;
-  return p->mg.fft_x == 1 || (p->mg.fft_x == -1 && dp && p->mg.filter_kt < 0 && plane_applies(p->mg, true));
+  return p->mg.fft_x == 1 || (p->mg.fft_x == -1 && dp && p->mg.filter_kt < 0 && plane_applies(p->mg, true) &&
+                              (xpass64_twice_per_sm(p->mg) ||
+                               (p->mg.n[0] <= 128 && p->mg.n[1] * p->mg.n[2] <= 64 * 64)));
 }
 
 extern "C" int fd3_plan_set_tuning(fd3_plan* p, int32_t knob, int32_t value) {

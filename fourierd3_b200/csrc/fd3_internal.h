@@ -231,6 +231,7 @@ int launch_xfilter(const MeshGeom& mg, const CellInfo* ci, const GreenPair* gp, 
                    int* n_blocks, cudaStream_t s);
 // kz width of the fused x-pass pencils for this mesh (0: the fused path does not apply)
 int xfilter_pencil(const MeshGeom& mg, int is_double);
+bool xpass64_twice_per_sm(const MeshGeom& mg);   // two of the float64 x-pass's pencils fit an SM
 // TMA fused x-pass (float spectrum): units of Q flattened (y, kz) values x all x x RG ranks x S
 bool xpass_applies(const MeshGeom& mg, int Q, int RG);
 bool tensor_maps_available();   // the driver exports the tensor-map encoder

@@ -28,6 +28,8 @@ int launch_xfilter<double>(const MeshGeom& mg, const CellInfo* ci, const GreenPa
   }
 }
 
+bool xpass64_twice_per_sm(const MeshGeom& mg) { return x64_shape(mg).two != 0; }
+
 int xfilter_pencil(const MeshGeom& mg, int is_double) {
   if (!is_double) return xfilter_kz<float>(mg);
   const X64Shape sh = x64_shape(mg);

@@ -244,7 +244,10 @@ int launch_x64(const X64Args& a, X64Shape sh) {
 // Pencil width and CTA shape for this mesh, LKZ = -1 where the x-pass does not apply: the widest pencil
 // of 2 or 4 values that fits twice per SM beside its chunk tables, else the widest that fits once
 // (128^3, 4 species, 5 ranks, with CUDA's functions: 2 values twice 600 us, 4 values once 728; with TabTrig
-// 64^3: 4 values twice 76, 2 values twice 82); narrower where there would be fewer pencils than SMs.
+// 64^3: 4 values twice 76, 2 values twice 82); from there on the width that makes the rounds of the chip the
+// shortest: a pencil costs its kz values and about 1200 / (C nx) of one more. (A narrower one only below 148
+// pencils left half of the chip idle: whole calls of 64 atoms, 4 species, 5 ranks, 64 x 64 x 32 128 -> 111 us,
+// 128 x 64 x 16 134 -> 116; 2 species, 4 ranks, 256 x 32 x 16 85 -> 73.)
 template <int N1, int N2>
 inline X64Shape x64_shape_t(const MeshGeom& mg) {
   const int C = mg.S * mg.R, most = mg.xpencil == 1 ? 0 : mg.xpencil == 2 ? 1 : 2;
@@ -255,7 +258,18 @@ inline X64Shape x64_shape_t(const MeshGeom& mg) {
         sh = X64Shape{l, pass == 0 ? 1 : 0};
         break;
       }
-  while (mg.xpencil < 0 && sh.LKZ > 0 && (long long)mg.n[1] * ((mg.nzh + (1 << sh.LKZ) - 1) >> sh.LKZ) < 148) --sh.LKZ;
+  if (mg.xpencil < 0) {
+    const long long slots = sh.two ? 2 * 148 : 148;
+    double least = 0.0;
+    for (int l = sh.LKZ, widest = sh.LKZ; l >= 0; --l) {
+      const long long pencils = (long long)mg.n[1] * ((mg.nzh + (1 << l) - 1) >> l);
+      const double cost = (double)((pencils + slots - 1) / slots) * ((1 << l) + 1200.0 / (C * mg.n[0]));
+      if (l == widest || cost < least) {
+        least = cost;
+        sh.LKZ = l;
+      }
+    }
+  }
   return sh;
 }
 

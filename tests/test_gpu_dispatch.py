@@ -285,3 +285,19 @@ def test_sorted_edges_on_a_few_of_many_atoms(cuda_device, sources):
         ms.append(np.median(times[1:]))
     assert all(torch.equal(a, b) for a, b in zip(*out))
     assert ms[0] <= 1.5 * ms[1]
+
+
+@pytest.mark.parametrize("mesh,z_max,c6tol,want", [
+    ((64, 64, 64), 4, 1.0, (1, 4)), ((64, 64, 32), 4, 1.0, (1, 2)), ((128, 64, 16), 4, 1.0, (1, 1)),
+    ((32, 256, 32), 2, 1.0, (1, 4)), ((256, 32, 16), 2, 1.0, (1, 1)),
+    ((256, 64, 64), 8, 1.0, (0, None)), ((64, 256, 256), 2, 1.0, (0, None))])
+def test_float64_x_pass_by_default_where_it_was_measured_faster(cuda_device, mesh, z_max, c6tol, want):
+    # the pencil width that fills the chip, and the separate filter where one pencil at a time fits an SM or the planes
+    # are cuFFT's
+    lengths = [(0.8 * n - 1.0) * 0.6 for n in mesh]
+    numbers = np.concatenate(([1, 6, 7, 8] if z_max == 8 else np.arange(1, z_max + 1), [1] * 20))
+    m = D3Model(numbers, np.diag(lengths), precision="fp64", device=cuda_device, method="spme", mesh_spacing=1.2,
+                interpolation_nodes=4, c6tol=c6tol, r_cut=6.0)
+    assert tuple(m.mesh) == mesh
+    t = m.engine.tuning()
+    assert t["fft_x"] == want[0] and (want[1] is None or t["xpencil"] == want[1]), (t, m.setup.n_rank)
