@@ -301,3 +301,108 @@ def test_float64_x_pass_by_default_where_it_was_measured_faster(cuda_device, mes
     assert tuple(m.mesh) == mesh
     t = m.engine.tuning()
     assert t["fft_x"] == want[0] and (want[1] is None or t["xpencil"] == want[1]), (t, m.setup.n_rank)
+
+
+def _launches(m, pos, cell, **knobs):
+    m.engine.set_tuning(**knobs)
+    before = _native.launch_count()
+    m(pos, cell)
+    return _native.launch_count() - before
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("mesh", [(64, 16, 16), (64, 16, 32), (64, 32, 16), (64, 64, 64), (64, 128, 16), (64, 16, 128),
+                                  (128, 128, 64), (64, 128, 128), (64, 256, 64), (64, 64, 256), (64, 256, 128),
+                                  (64, 8, 16)])
+def test_planes_that_fit_a_cta_are_the_librarys_own(cuda_device, mesh, precision):
+    # the x-pass in place of the filter, and a launch each way for the planes unless they are cuFFT's
+    lengths = [(0.8 * n - 1.0) * 0.6 for n in mesh]
+    numbers = np.array([8, 14] * 20)
+    pos, _ = _box(lengths, numbers, 9)
+    cell = np.diag(lengths)
+    m = D3Model(numbers, cell, precision=precision, device=cuda_device, method="spme", mesh_spacing=1.2,
+                interpolation_nodes=4, r_cut=6.0)
+    assert tuple(m.mesh) == mesh
+    separate = _launches(m, pos, cell, fft_x=0)
+    fused = _launches(m, pos, cell, fft_x=1)
+    assert m.engine.tuning()["fft_x"] == 1
+    own = min(mesh[1:]) >= 16 and mesh[1] * mesh[2] <= (128 * 128 if precision == "fp64" else 128 * 256)
+    assert fused - separate == (2 if own else 0)
+
+
+@pytest.mark.parametrize("lengths,z_max,c6tol", [((8.0, 8.0, 8.0), 4, 1.0), ((8.0, 24.0, 8.0), 1, 1.0),
+                                                 ((16.0, 8.0, 16.0), 2, 1.0), ((32.0, 8.0, 8.0), 4, 0.05),
+                                                 ((66.0, 16.0, 8.0), 3, 1.0), ((130.0, 8.0, 8.0), 4, 1.0)])
+def test_float64_x_pass_takes_every_length_and_width(cuda_device, lengths, z_max, c6tol):
+    # the cases of test_float64_x_pass_of_every_length run the x-pass, at the width asked for or the widest that fits
+    rng = np.random.default_rng(int(sum(lengths)) + z_max)
+    cell = np.diag(lengths) + np.triu(np.full((3, 3), 1.1), 1)
+    m = D3Model(rng.integers(1, z_max + 1, 60), cell, precision="fp64", device=cuda_device, method="spme",
+                mesh_spacing=1.2, interpolation_nodes=4, c6tol=c6tol, r_cut=6.0)
+    got = []
+    for kz in (1, 2, 4):
+        m.engine.set_tuning(fft_x=1, xpencil=kz)
+        t = m.engine.tuning()
+        assert t["fft_x"] == 1 and t["xpencil"] <= kz
+        got.append(t["xpencil"])
+    assert got == [min(kz, got[2]) for kz in (1, 2, 4)] and got[2] >= 2
+
+
+def test_float64_green_function_of_a_coarse_mesh_in_the_x_pass(cuda_device):
+    # the longest spacing of test_float64_green_function_from_tables on a mesh that the x-pass takes (16^3)
+    rng = np.random.default_rng(30)
+    cell = np.diag([15.0, 16.0, 15.5]) + np.triu(np.full((3, 3), 0.6), 1)
+    numbers = rng.choice([1, 30], 60)
+    pos = rng.random((60, 3)) @ cell
+    m = D3Model(numbers, cell, precision="fp64", device=cuda_device, method="spme", mesh_spacing=4.0,
+                interpolation_nodes=4, c6tol=1.0, r_cut=6.0)
+    m.engine.set_tuning(fft_x=0, filter_kt=4)
+    e0, f0, s0 = (t.clone() for t in m(pos, cell))
+    m.engine.set_tuning(fft_x=1, filter_kt=-1)
+    assert m.engine.tuning()["fft_x"] == 1
+    e, f, s = m(pos, cell)
+    assert abs(float(e) - float(e0)) <= 1e-12 * abs(float(e0))
+    assert (f - f0).abs().max().item() <= 1e-10 * max(1.0, f0.abs().max().item())
+    assert (s - s0).abs().max().item() <= 1e-10 * max(1.0, s0.abs().max().item())
+
+
+@pytest.mark.parametrize("n_species,c6tol,runs", [(15, 1.0, False), (16, 30.0, True), (40, 1.0, True), (41, 1.0, True),
+                                                  (64, 30.0, True), (64, 1.0, True)])
+def test_many_species_filter_up_to_the_most_it_takes(cuda_device, n_species, c6tol, runs):
+    # which kernel filters by default (no k-tile in effect: the many-species one), and 64 species against the tiled one
+    rng = np.random.default_rng(n_species)
+    numbers = np.concatenate((np.arange(1, n_species + 1), rng.integers(1, n_species + 1, 60)))
+    cell = np.diag([9.0, 12.0, 10.0]) + np.triu(np.full((3, 3), 0.9), 1)
+    pos = rng.random((len(numbers), 3)) @ cell
+    m = D3Model(numbers, cell, precision="mixed", device=cuda_device, method="spme", mesh_spacing=1.2,
+                interpolation_nodes=4, c6tol=c6tol, r_cut=6.0)
+    assert m.setup.n_rank <= 8 and (m.engine.tuning()["filter_kt"] == -1) == runs
+    e, f, s = (t.clone() for t in m(pos, cell))
+    m.engine.set_tuning(filter_kt=2)
+    assert m.engine.tuning()["filter_kt"] == 2
+    e0, f0, s0 = m(pos, cell)
+    assert abs(float(e) - float(e0)) <= 2e-6 * abs(float(e0))
+    assert (f - f0).abs().max().item() <= 1e-5 * max(1.0, f0.abs().max().item())
+    assert (s - s0).abs().max().item() <= 1e-5 * max(1.0, s0.abs().max().item())
+
+
+@pytest.mark.parametrize("precision,method,cnfunc", [("fp64", "spme", "smooth_cut"), ("mixed", "spme", "smooth_cut"),
+                                                     ("fp64", "pme", "d4"), ("mixed", "ewald", "smooth_cut")])
+def test_a_captured_call_keeps_its_host_cell_and_takes_new_positions(cuda_device, precision, method, cnfunc):
+    # without a device copy of the cell it travels with the launches, so that a graph holds the cell of its capture
+    pos, cell, numbers = structures.hcno_box(seed=9, n_atoms=120)
+    m = D3Model(numbers, cell, precision=precision, device=cuda_device, method=method, cnfunc=cnfunc, mesh_spacing=1.2,
+                interpolation_nodes=4, c6tol=1.0, r_cut=6.0)
+    x = torch.tensor(pos, device=cuda_device)
+    moved = torch.tensor(pos + 0.1 * np.random.default_rng(1).normal(size=pos.shape), device=cuda_device)
+    want = [[t.clone() for t in m.engine.energy_forces_stress(p, cell, 6.0)] for p in (x, moved)]
+    host_cell = np.array(cell)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = m.engine.energy_forces_stress(x, host_cell, 6.0)
+    host_cell *= 1.1
+    for p, w in zip((torch.tensor(pos, device=cuda_device), moved), want):
+        x.copy_(p)
+        graph.replay()
+        assert all(torch.equal(a, b) for a, b in zip(got, w))

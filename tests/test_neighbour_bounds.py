@@ -18,6 +18,22 @@ def test_a_count_beyond_the_row_starts_is_refused():
                                              None) == _native.FD3_EINVAL
 
 
+def test_the_counted_fill_checks_its_arguments_on_the_host():
+    # no list to build: nothing is launched, and outputs may be absent; each bad argument by itself is refused
+    lib = _native.lib()
+    cell, size, p = np.eye(3).reshape(9) * 20.0, ctypes.c_size_t(), ctypes.c_void_p(256)
+    _native.check(lib.fd3_neighbor_workspace_size(10, _native.dptr(cell), 6.0, ctypes.byref(size)), "size")
+
+    def fill(n=10, pos=p, h=_native.dptr(cell), r=6.0, work=p, room=size.value, count=5, src=p, dst=p, shift=p):
+        return lib.fd3_neighbor_fill_counted(n, pos, h, r, work, room, count, src, dst, shift, None)
+
+    assert fill(count=0, src=None, dst=None, shift=None) == _native.FD3_OK
+    for bad in (dict(n=0), dict(n=2**30 + 1), dict(pos=None), dict(h=None), dict(r=0.0), dict(src=None), dict(dst=None),
+                dict(shift=None), dict(h=_native.dptr(np.zeros(9)))):
+        assert fill(**bad) == _native.FD3_EINVAL, bad
+    assert fill(work=None) == fill(room=size.value - 1) == _native.FD3_ENOMEM
+
+
 @pytest.mark.gpu
 def test_more_pairs_than_the_row_starts_hold_are_refused_with_their_number(cuda_device):
     # 66,000 atoms with about half of all others and their images in reach: 2.28e9 pairs
