@@ -313,6 +313,18 @@ def touched_mesh_values(pos, cell, numbers, mesh, order: int, R: int) -> int:
     return int(total) * R
 
 
+def own_plane_kernels(tuning, mesh, precision):
+    """The library's kernels of the two (y, z) transform stages for settings in effect, or None where cuFFT runs
+    them: with an x-pass the clusters' where they are in effect, one CTA's for planes that fit it."""
+    if tuning["fft_x"] < 1:
+        return None
+    if tuning["fft_yz"] > 0:
+        return "k_yz_forward", "k_yz_inverse"
+    ny, nz = mesh[1:]
+    fits = ny * nz <= (128 * 128 if precision == "fp64" else 128 * 256)
+    return ("k_plane_forward", "k_plane_inverse") if fits and {ny, nz} <= {16, 32, 64, 128, 256} else None
+
+
 def stage_bytes(stage: str, n: int, mesh, C: int, R: int, b: int, touched: int = 0) -> float:
     """Algorithmic HBM bytes of one launch of a pipeline stage: mesh terms per mesh point and
     channel (b bytes real, 2b complex), atom terms per atom. The gather reads only the mesh
@@ -816,9 +828,10 @@ def main():
 
     b = 4 if head == "mixed" else 8
     st_mixed = stages[head]
-    # this library's stages: the (y, z) transform stages count when the fused cluster kernels run
-    # them (otherwise they are cuFFT's)
-    yz_own = int(models[head].engine.tuning().get("fft_yz", 0)) > 0
+    # this library's stages: the (y, z) transform stages count when its own kernels run them
+    # (otherwise they are cuFFT's)
+    plane_kernels = own_plane_kernels(models[head].engine.tuning(), mesh, head)
+    yz_own = plane_kernels is not None
     ours = {k: v for k, v in st_mixed.items() if yz_own or not k.startswith("fft")}
     dom = max(ours, key=ours.get)
     peak, peak_kind = measured_peaks()
@@ -843,7 +856,7 @@ def main():
                         "fft_r2c": (545.1e6 + 488.7e6) if yz_own else None,
                         "fft_c2r": (566.8e6 + 493.5e6) if yz_own else None}
     kernel_names = {"filter": {0: "k_filter", 1: "k_xfilter", 2: "k_xpass"}[fx], "spread": "k_spread_col",
-                    "gather": "k_gather_z", "fft_r2c": "k_yz_forward", "fft_c2r": "k_yz_inverse",
+                    "gather": "k_gather_z", "fft_r2c": yz_own and plane_kernels[0], "fft_c2r": yz_own and plane_kernels[1],
                     "cn_c6": "k_cn_bins + k_c6_atoms", "cn_adjoint": "k_cn_adjoint"}
     mesh_match = tuple(mesh) == (256, 256, 256) and C == 8 and head == "mixed"
     roof = {"bound": "hbm", "kernel": dom, "kernel_name": kernel_names.get(dom), "achieved": achieved,

@@ -52,3 +52,16 @@ def test_stage_bytes_formulas():
     assert bench.stage_bytes("gather", n, mesh, C, R, 4, touched=100) == 400 + n * (60 + 16 * R)
     assert bench.stage_bytes("gather", n, mesh, C, R, 4) == C * M * 4 + n * (60 + 16 * R)
     assert bench.stage_bytes("unknown", n, mesh, C, R, 4) == 0.0
+
+
+def test_own_plane_kernels_of_each_route():
+    import bench
+
+    cluster, single = ("k_yz_forward", "k_yz_inverse"), ("k_plane_forward", "k_plane_inverse")
+    for fft_x, fft_yz, mesh, precision, want in (
+            (2, 1, (256, 256, 256), "mixed", cluster), (1, 2, (64, 256, 256), "mixed", cluster),
+            (2, 0, (256, 256, 256), "mixed", None), (2, 0, (64, 64, 64), "mixed", single),
+            (2, 0, (64, 256, 128), "mixed", single), (1, 0, (64, 256, 128), "fp64", None),
+            (1, 0, (16, 128, 128), "fp64", single), (2, 0, (64, 8, 64), "mixed", None),
+            (0, 0, (64, 64, 64), "mixed", None)):
+        assert bench.own_plane_kernels(dict(fft_x=fft_x, fft_yz=fft_yz), mesh, precision) == want
