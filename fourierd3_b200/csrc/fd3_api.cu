@@ -387,7 +387,11 @@ static void xpass_shape(const fd3_plan* p, int* Q, int* RG) {
   *Q = p->mg.xq > 0 ? p->mg.xq : 16;
   *RG = p->mg.xranks > 0 ? p->mg.xranks : 1;
 }
-// By default on wherever it applies, unless a knob of the separate filter is set.
+// By default on wherever it applies, unless a knob of the separate filter is set; planes left to 2D cuFFT
+// included (125 meshes of 8 to 512 a side with 2 x 4 and 4 x 5 channels: none slower by more than the 2 us of
+// the timer). The exception is one species whose ranks do not fill the units, from 2^21 points on: it shares
+// nothing but the padding (3 ranks, whole calls of 64 atoms: 128^3 138 -> 131 us, but 256 x 128 x 128 217 -> 224,
+// 64 x 256 x 256 218 -> 240, 64 x 256 x 512 406 -> 456).
 static bool xpass_on(const fd3_plan* p) {
   if (p->method == FD3_METHOD_EWALD || !p->xpass_possible || p->precision != FD3_PREC_MIXED) return false;
   if (p->mg.fft_x != 2 &&
@@ -395,6 +399,9 @@ static bool xpass_on(const fd3_plan* p) {
     return false;
   int Q, RG;
   xpass_shape(p, &Q, &RG);
+  if (p->mg.fft_x == -1 && p->S == 1 && p->R % RG != 0 &&
+      (long long)p->mg.n[0] * p->mg.n[1] * p->mg.n[2] > 1 << 21)
+    return false;
   return xpass_applies(p->mg, Q, RG);
 }
 // fused (y, z) transforms in effect: float mesh on a 2D-transform path, ny = nz = 256, asked for
@@ -407,16 +414,22 @@ static int yz_variant(const fd3_plan* p) { return p->mg.fft_yz > 0 ? p->mg.fft_y
 // The pencil x-pass: asked for, or by default in float64 where this library's plane transforms take
 // the (y, z) part (summed transforms and filter against 3D cuFFT: 16^3, 4 x 5 channels 56 -> 30 us; 64^3,
 // 2 x 4 89 -> 72, 4 x 5 181 -> 143; 128^3, 2 x 4 446 -> 398, 4 x 5 1237 -> 1040; with cuFFT's 2D transforms the
-// pencils lose: 128 x 128 x 256 815 -> 831, 256^3 3010 -> 3417), and its pencils fit an SM twice: one at a time they
-// win up to nx = 128 and 64 x 64 planes alone (4 x 8, whole calls of 64 atoms: 128 x 64 x 64 543 -> 487 us,
-// 128^3 1750 -> 1827; 4 x 5, 256 x 64 x 64 671 -> 681, 256 x 128 x 128 2253 -> 2537). Over all planes of 16 to
-// 256 a side and nx = 16 to 256 the default is 1.08 times as fast as 3D cuFFT, at worst 0.95 (16 x 256 x 32).
+// pencils lose: 128 x 128 x 256 815 -> 831, 256^3 3010 -> 3417), and
+// - its pencils fit an SM twice: one at a time they win up to nx = 128 and planes of 64 x 64 points alone (4 x 8, whole
+//   calls of 64 atoms: 128 x 64 x 64 543 -> 487 us, 128^3 1750 -> 1827; 4 x 5, 256 x 64 x 64 671 -> 681, 256 x 128 x
+//   128 2253 -> 2537);
+// - there are two species or more, beyond planes of 128 x 64 points: with one the separate filter has little to do
+//   (1 x 3: 64 x 128 x 64 101 -> 95, 64 x 128 x 128 134 -> 146, 128^3 224 -> 236).
+// Over all planes of 16 to 256 a side and nx = 16 to 256 the default is 1.08 times as fast as 3D cuFFT with 2 x 4 and
+// 4 x 5 channels, at worst 0.95 (16 x 256 x 32).
 static bool old_xpass_on(const fd3_plan* p) {
   const bool dp = p->precision == FD3_PREC_FP64;
   if (p->method == FD3_METHOD_EWALD || !p->xpass_possible || xfilter_pencil(p->mg, dp ? 1 : 0) <= 0) return false;
-  return p->mg.fft_x == 1 || (p->mg.fft_x == -1 && dp && p->mg.filter_kt < 0 && plane_applies(p->mg, true) &&
-                              (xpass64_twice_per_sm(p->mg) ||
-                               (p->mg.n[0] <= 128 && p->mg.n[1] * p->mg.n[2] <= 64 * 64)));
+  if (p->mg.fft_x != -1) return p->mg.fft_x == 1;
+  if (!dp || p->mg.filter_kt >= 0 || !plane_applies(p->mg, true)) return false;
+  const bool twice = xpass64_twice_per_sm(p->mg);
+  const int plane = p->mg.n[1] * p->mg.n[2];
+  return plane <= 64 * 64 ? twice || p->mg.n[0] <= 128 : twice && (p->S >= 2 || plane <= 128 * 64);
 }
 
 extern "C" int fd3_plan_set_tuning(fd3_plan* p, int32_t knob, int32_t value) {

@@ -103,8 +103,8 @@ FD3_API int fd3_plan_destroy(fd3_plan* plan);
  *                       the same with units of rank groups moved by TMA (mixed precision); 0 =
  *                       3D cuFFT around a separate filter; -1 = the default: in mixed
  *                       precision 2 where it applies, in float64 1 where the plane
- *                       transforms below apply, 0 elsewhere and where a knob of the
- *                       separate filter is set.
+ *                       transforms below apply, either only where it was measured
+ *                       faster; 0 elsewhere and where a knob of the separate filter is set.
  *   FD3_TUNE_XPENCIL    kz values per pencil of the fused x-pass: 1, 2 or 4 (used when the
  *                       pencil fits in shared memory), -1 = the default (the widest that
  *                       leaves three CTAs per SM for float, two for double if two fit);

@@ -406,3 +406,15 @@ def test_a_captured_call_keeps_its_host_cell_and_takes_new_positions(cuda_device
         x.copy_(p)
         graph.replay()
         assert all(torch.equal(a, b) for a, b in zip(got, w))
+
+
+@pytest.mark.parametrize("precision,element,mesh,want", [
+    ("mixed", 8, (128, 128, 128), 2), ("mixed", 8, (64, 256, 256), 0), ("mixed", 1, (64, 256, 256), 2),
+    ("fp64", 8, (64, 64, 64), 1), ("fp64", 8, (64, 128, 64), 1), ("fp64", 8, (64, 64, 256), 0), ("fp64", 1, (256, 64, 64), 1)])
+def test_x_pass_by_default_with_one_species(cuda_device, precision, element, mesh, want):
+    # three ranks (oxygen) leave a rank group partly empty, two (hydrogen) do not; large planes in float64
+    lengths = [(0.8 * n - 1.0) * 0.6 for n in mesh]
+    m = D3Model(np.full(20, element), np.diag(lengths), precision=precision, device=cuda_device, method="spme",
+                mesh_spacing=1.2, interpolation_nodes=4, c6tol=0.01 if element == 8 else 1.0, r_cut=6.0)
+    assert tuple(m.mesh) == mesh and m.setup.n_rank == (3 if element == 8 else 2)
+    assert m.engine.tuning()["fft_x"] == want
