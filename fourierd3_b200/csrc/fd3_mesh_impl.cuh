@@ -323,7 +323,8 @@ __global__ void __launch_bounds__(kSpThreads, sizeof(T) == 8 ? 2 : 4) k_spread(M
 // so the layouts are chosen for few wavefronts: the stores above (a thread with a whole row stores 16
 // bytes per line), staged rows of 17 or 18 values (a thread stages an atom; rows of 16 put all lanes on
 // the same banks), and per atom one z, one or two y and the rank loads for 32 multiply-adds. 139,968 atoms on
-// 256^3, 2 x 4 channels: float64 497 -> 348 us, float 283 -> 217 (before: a whole row of 8 per thread).
+// 256^3, 2 x 4 channels: float64 497 -> 348 us, float 283 -> 217 (before: a whole row of 8 per thread); with the
+// ranks in the rows' padding (kColPadRanks) 320 and 200.
 constexpr int kColMaxSeg = 64;
 
 // what a thread owns of a z-tile: kZL values in each of kRows rows
@@ -335,24 +336,34 @@ struct ColOwn {
   static constexpr int kWz = sizeof(T) == 4 ? 20 : 18;
 };
 
+// The words that pad a row off the bank period hold the atom's first four ranks (float: after wz; double: two after
+// wz, two after wy) and its source z-tile (after wx), so that padded rows hold as many atoms as rows of 16 did: 256
+// float or 270 double with 4 ranks. (226 and 238 with the ranks in rows of their own: chunks of 8 tiles of 128^3 with
+// 30,840 atoms, 2 species, float, took 121 us, 70 with rows of 16 and now 52; all sizes gain by the shared address.)
+constexpr int kColPadRanks = 4;
+
 template <typename T>
 struct ColSmem {
   T* wz;      // [cap][kWz] z row inside the atom's own z-tile (8), then the part spilling into the next (8)
   T* wy;      // [cap][kWy]
   T* wx;      // [cap][kWx]
-  T* cc;      // [cap][R]
-  int* zi;    // [cap] source z-tile (index into the chunk's source range); bit 30: spills
+  T* cc;      // [cap][max(R - kColPadRanks, 0)] the other ranks
   int* zst;   // [kColMaxSeg + 1] first staged slot of each source z-tile
+  // source z-tile (index into the chunk's source range) of a slot; bit 30: spills
+  __device__ __forceinline__ int& zi(int a) const {
+    return *reinterpret_cast<int*>(wx + a * ColOwn<T>::kWx + 16);
+  }
 };
 
 __host__ __device__ inline size_t col_round16(size_t b) { return (b + 15) & ~(size_t)15; }
+__host__ __device__ inline int col_more_ranks(int R) { return R > kColPadRanks ? R - kColPadRanks : 0; }
 
 template <typename T>
 __host__ __device__ inline size_t col_smem_bytes(int cap, int R) {
   using O = ColOwn<T>;
   return col_round16((size_t)cap * O::kWz * sizeof(T)) + col_round16((size_t)cap * O::kWy * sizeof(T)) +
-         col_round16((size_t)cap * O::kWx * sizeof(T)) + col_round16((size_t)cap * R * sizeof(T)) +
-         col_round16((size_t)(cap + kColMaxSeg + 1) * sizeof(int));
+         col_round16((size_t)cap * O::kWx * sizeof(T)) + col_round16((size_t)cap * col_more_ranks(R) * sizeof(T)) +
+         col_round16((size_t)(kColMaxSeg + 1) * sizeof(int));
 }
 
 template <typename T>
@@ -366,11 +377,25 @@ __device__ __forceinline__ ColSmem<T> col_carve(unsigned char* base, int cap, in
   m.wx = reinterpret_cast<T*>(base);
   base += col_round16((size_t)cap * O::kWx * sizeof(T));
   m.cc = reinterpret_cast<T*>(base);
-  base += col_round16((size_t)cap * R * sizeof(T));
-  m.zi = reinterpret_cast<int*>(base);
-  m.zst = m.zi + cap;
+  base += col_round16((size_t)cap * col_more_ranks(R) * sizeof(T));
+  m.zst = reinterpret_cast<int*>(base);
   return m;
 }
+
+// The first four ranks of slot a (FIRST), or ranks r0 .. r0 + 3 of a later group: two at lo(a), two at hi(a).
+template <typename T, bool FIRST>
+struct ColRanks {
+  const ColSmem<T>& m;
+  int R, r0;
+  __device__ __forceinline__ T* lo(int a) const {
+    using O = ColOwn<T>;
+    static_assert(O::kWz >= 16 + (sizeof(T) == 4 ? 4 : 2) && O::kWy >= 18);
+    return FIRST ? m.wz + a * O::kWz + 16 : m.cc + a * (R - kColPadRanks) + (r0 - kColPadRanks);
+  }
+  __device__ __forceinline__ T* hi(int a) const {
+    return FIRST && sizeof(T) == 8 ? m.wy + a * ColOwn<T>::kWy + 16 : lo(a) + 2;
+  }
+};
 
 constexpr int kZiSpill = 1 << 30;
 
@@ -471,8 +496,13 @@ __device__ int col_stage(const MeshDev& g, const int* s_a0, const int* s_pref, i
           spill = true;
         }
       }
-      m.zi[slot] = seg / seg_per_z + (spill ? kZiSpill : 0);
-      for (int r = 0; r < R; ++r) m.cc[slot * R + r] = rc[(size_t)u * R + r];
+      m.zi(slot) = seg / seg_per_z + (spill ? kZiSpill : 0);
+      const ColRanks<T, true> first{m, R, 0};
+#pragma unroll
+      for (int r = 0; r < kColPadRanks; ++r)
+        (r < 2 ? first.lo(slot) : first.hi(slot))[r & 1] = r < R ? rc[(size_t)u * R + r] : T(0);
+      for (int r = kColPadRanks; r < R; ++r)
+        m.cc[slot * (R - kColPadRanks) + r - kColPadRanks] = rc[(size_t)u * R + r];
     }
     if (keep && slot >= cap) atomicMin(s_next, ca);
     staged += tot;
@@ -497,11 +527,12 @@ __device__ int col_stage(const MeshDev& g, const int* s_a0, const int* s_pref, i
 template <typename T>
 using ColAcc = T[ColOwn<T>::kRows][ColOwn<T>::kZL][kSpRC];
 
-template <typename T, bool CHECK>
+template <typename T, bool CHECK, bool FIRST>
 __device__ __forceinline__ void col_atom(const ColSmem<T>& m, int a, int z0, T wx, int zsrc, int R, int r0, int ly0,
                                          ColAcc<T>& acc) {
   using O = ColOwn<T>;
-  if (CHECK && (m.zi[a] & ~kZiSpill) != zsrc) return;
+  const ColRanks<T, FIRST> cr4{m, R, r0};
+  if (CHECK && (m.zi(a) & ~kZiSpill) != zsrc) return;
   T c[kSpRC], zr[O::kZL], wxy[O::kRows];
   if (sizeof(T) == 4) {
     const float2 y = *reinterpret_cast<const float2*>(m.wy + a * O::kWy + ly0);
@@ -521,17 +552,18 @@ __device__ __forceinline__ void col_atom(const ColSmem<T>& m, int a, int z0, T w
     zr[0] = (T)z.x;
     zr[1] = (T)z.y;
   }
-  if (kSpRC == 4 && (R & 3) == 0) {
-    // a whole 4-rank group in 16-byte loads (rows of R values start on 16-byte boundaries)
+  static_assert(kSpRC == 4 && kColPadRanks == 4);
+  if (FIRST || (R & 3) == 0) {
+    // a whole 4-rank group in 16-byte loads (the first four, zero beyond R, and groups of rows of 4 n values)
     if (sizeof(T) == 4) {
-      const float4 v = *reinterpret_cast<const float4*>(m.cc + a * R + r0);
+      const float4 v = *reinterpret_cast<const float4*>(cr4.lo(a));
       c[0] = (T)v.x;
       c[1] = (T)v.y;
       c[2] = (T)v.z;
       c[3] = (T)v.w;
     } else {
-      const double2 v0 = *reinterpret_cast<const double2*>(m.cc + a * R + r0);
-      const double2 v1 = *reinterpret_cast<const double2*>(m.cc + a * R + r0 + 2);
+      const double2 v0 = *reinterpret_cast<const double2*>(cr4.lo(a));
+      const double2 v1 = *reinterpret_cast<const double2*>(cr4.hi(a));
       c[0] = (T)v0.x;
       c[1] = (T)v0.y;
       c[2] = (T)v1.x;
@@ -539,7 +571,7 @@ __device__ __forceinline__ void col_atom(const ColSmem<T>& m, int a, int z0, T w
     }
   } else {
 #pragma unroll
-    for (int r = 0; r < kSpRC; ++r) c[r] = r0 + r < R ? m.cc[a * R + r0 + r] : T(0);
+    for (int r = 0; r < kSpRC; ++r) c[r] = r0 + r < R ? cr4.lo(a)[r] : T(0);
   }
   if constexpr (sizeof(T) == 4) {
     // two ranks per instruction, rounded as two multiply-adds are (instruction issue bounds the float form: 2.7
@@ -570,9 +602,9 @@ __device__ __forceinline__ void col_atom(const ColSmem<T>& m, int a, int z0, T w
   }
 }
 
-template <typename T, bool CHECK>
-__device__ __forceinline__ void col_accumulate(const ColSmem<T>& m, int a0, int a1, int zsrc, bool spill, int R,
-                                               int r0, int lx, int ly0, int zl0, ColAcc<T>& acc) {
+template <typename T, bool CHECK, bool FIRST>
+__device__ __forceinline__ void col_range(const ColSmem<T>& m, int a0, int a1, int zsrc, bool spill, int R, int r0,
+                                          int lx, int ly0, int zl0, ColAcc<T>& acc) {
   using O = ColOwn<T>;
   const int z0 = zl0 + (spill ? kSpTZ : 0);
   int a = a0;
@@ -582,12 +614,21 @@ __device__ __forceinline__ void col_accumulate(const ColSmem<T>& m, int a0, int 
     for (int u = 0; u < 4; ++u) wx[u] = m.wx[(a + u) * O::kWx + lx];
 #pragma unroll
     for (int u = 0; u < 4; ++u)
-      if (wx[u] != T(0)) col_atom<T, CHECK>(m, a + u, z0, wx[u], zsrc, R, r0, ly0, acc);
+      if (wx[u] != T(0)) col_atom<T, CHECK, FIRST>(m, a + u, z0, wx[u], zsrc, R, r0, ly0, acc);
   }
   for (; a < a1; ++a) {
     const T wx = m.wx[a * O::kWx + lx];
-    if (wx != T(0)) col_atom<T, CHECK>(m, a, z0, wx, zsrc, R, r0, ly0, acc);
+    if (wx != T(0)) col_atom<T, CHECK, FIRST>(m, a, z0, wx, zsrc, R, r0, ly0, acc);
   }
+}
+
+template <typename T, bool CHECK>
+__device__ __forceinline__ void col_accumulate(const ColSmem<T>& m, int a0, int a1, int zsrc, bool spill, int R,
+                                               int r0, int lx, int ly0, int zl0, ColAcc<T>& acc) {
+  if (r0 == 0)
+    col_range<T, CHECK, true>(m, a0, a1, zsrc, spill, R, r0, lx, ly0, zl0, acc);
+  else
+    col_range<T, CHECK, false>(m, a0, a1, zsrc, spill, R, r0, lx, ly0, zl0, acc);
 }
 
 template <typename T>
@@ -698,7 +739,7 @@ __global__ void __launch_bounds__(kSpThreads, sizeof(T) == 8 ? 2 : 4) k_spread_c
       int lo = 0, hi = staged;
       while (lo < hi) {
         const int mid = (lo + hi) >> 1;
-        if ((m.zi[mid] & ~kZiSpill) < zi) lo = mid + 1; else hi = mid;
+        if ((m.zi(mid) & ~kZiSpill) < zi) lo = mid + 1; else hi = mid;
       }
       m.zst[zi] = lo;
     }
@@ -736,13 +777,14 @@ __global__ void __launch_bounds__(kSpThreads, sizeof(T) == 8 ? 2 : 4) k_spread_c
   }
 }
 
-// Staged atoms per column chunk: as many as let 4 (float) or 2 (double) CTAs share an SM.
+// Staged atoms per column chunk: as many as let 4 (float) or 2 (double) CTAs share an SM's 228 KB, of which each
+// has 1 KB reserved and 560 bytes static.
 template <typename T>
 inline int spread_col_cap(const MeshGeom& mg) {
   constexpr int per_sm = sizeof(T) == 8 ? 2 : 4;
   const size_t fixed = col_smem_bytes<T>(0, mg.R);
-  const size_t per_atom = col_smem_bytes<T>(64, mg.R) / 64;
-  int cap = (int)((size_t)(220 * 1024 / per_sm - 2048 - fixed) / per_atom);
+  const size_t per_atom = (col_smem_bytes<T>(64, mg.R) - fixed) / 64;
+  int cap = (int)((size_t)(228 * 1024 / per_sm - 1024 - 704 - fixed) / per_atom);
   if (cap > 1024) cap = 1024;
   if (mg.spread_cap > 0 && mg.spread_cap < cap) cap = mg.spread_cap;
   return cap;

@@ -418,3 +418,38 @@ def test_x_pass_by_default_with_one_species(cuda_device, precision, element, mes
                 mesh_spacing=1.2, interpolation_nodes=4, c6tol=0.01 if element == 8 else 1.0, r_cut=6.0)
     assert tuple(m.mesh) == mesh and m.setup.n_rank == (3 if element == 8 else 2)
     assert m.engine.tuning()["fft_x"] == want
+
+
+@pytest.mark.parametrize("precision,n_atoms", [("mixed", 32000), ("mixed", 90000), ("mixed", 400000), ("fp64", 37000),
+                                               ("fp64", 400000)])
+def test_column_spread_of_full_and_overfull_chunks(cuda_device, precision, n_atoms):
+    # 128^3, chunks of 8 z-tiles: nearly as full as the stage, several times as full, and with single tiles that
+    # overflow it. The results of chunks of one tile and of the per-tile kernel, to rounding; where the stage holds the
+    # chunk, in about the time of chunks of one tile (a stage of 226 float atoms, of 250 before, did not: 2.1 times)
+    lengths = [(n_atoms / 0.07) ** (1 / 3)] * 3
+    rng = np.random.default_rng(n_atoms)
+    m1 = int(np.ceil(n_atoms ** (1 / 3)))
+    grid = np.stack(np.unravel_index(np.sort(rng.permutation(m1**3)[:n_atoms]), (m1,) * 3), 1)
+    cell = np.diag(lengths)
+    pos = torch.tensor((grid + rng.uniform(0.2, 0.8, grid.shape)) / m1 @ cell, device=cuda_device)
+    numbers = np.where(grid.sum(1) % 2 == 0, 8, 14)
+    m = D3Model(numbers, cell, precision=precision, device=cuda_device, method="spme", mesh_spacing=lengths[0] / 51.2,
+                interpolation_nodes=5, c6tol=1.0, r_cut=6.0)
+    assert tuple(m.mesh) == (128, 128, 128) and m.setup.n_rank == 4
+    m.engine.profile(True)
+    out, ms = {}, {}
+    for zc in (8, 1, 0):
+        m.engine.set_tuning(spread_zc=zc)
+        assert m.engine.tuning()["spread_zc"] == zc
+        times = []
+        for _ in range(6):
+            out[zc] = [t.clone() for t in m(pos, cell)]
+            times.append(m.engine.stage_times()["spread"])
+        ms[zc] = np.median(times[1:])
+    e_tol, f_tol = (1e-12, 1e-10) if precision == "fp64" else (2e-6, 1e-5)
+    for zc in (1, 0):
+        for k, tol in enumerate((e_tol, f_tol, f_tol)):
+            scale = out[zc][k].abs().max().item()
+            assert (out[8][k] - out[zc][k]).abs().max().item() <= tol * (scale if k == 0 else max(1.0, scale))
+    if n_atoms == 32000:
+        assert ms[8] <= 1.5 * ms[1]
