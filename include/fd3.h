@@ -89,14 +89,16 @@ FD3_API int fd3_plan_destroy(fd3_plan* plan);
  * summation order), and every value is checked against the plan's sizes.
  *   FD3_TUNE_FILTER_KT  k-points per shared-memory tile of the reciprocal-space filter:
  *                       0 = per-thread register kernel (at most 8 species), 1, 2, 4, 8
- *                       or 16 = tiled kernel, -1 = the default for (species, rank).
+ *                       or 16 = tiled kernel, -1 = the default: an x-pass where it applies, in mixed
+ *                       precision the many-species filter (16 to 64 species), else by (species, rank).
  *   FD3_TUNE_SPREAD_ZC  z-tiles per column chunk of the mesh spread: 0 = one CTA per
  *                       16x16x8 tile, 1..64 = one CTA per 16x16 column chunk (capped by
  *                       the mesh), -1 = the default (4, fewer on small meshes).
  *   FD3_TUNE_SPREAD_CAP staged atoms per column chunk at most: 0 = what shared memory
- *                       holds, >= 256 = a lower bound (denser chunks take the per-tile
- *                       staging path inside the same CTA).
- *   FD3_TUNE_FFT_X      1 = cuFFT transforms the (y, z) planes and one kernel does the x
+ *                       holds, >= 256 = a lower bound (a CTA takes denser chunks in
+ *                       shorter runs of z-tiles, a denser tile in pieces).
+ *   FD3_TUNE_FFT_X      1 = plane transforms of (y, z) (this library's or cuFFT's, see
+ *                       FD3_TUNE_FFT_YZ) and one kernel that does the x
  *                       transform, the filter and the inverse x transform per pencil (where
  *                       it applies: at most 4 species and 8 ranks, nx = 64, 128 or
  *                       256, in float64 16 and 32 too); 2 =
@@ -107,7 +109,7 @@ FD3_API int fd3_plan_destroy(fd3_plan* plan);
  *                       faster; 0 elsewhere and where a knob of the separate filter is set.
  *   FD3_TUNE_XPENCIL    kz values per pencil of the fused x-pass: 1, 2 or 4 (used when the
  *                       pencil fits in shared memory), -1 = the default (the widest that
- *                       leaves three CTAs per SM for float, two for double if two fit);
+ *                       leaves three CTAs per SM for float, by the rounds of the chip for double);
  *                       the value in effect is 0 where the fused x-pass does not apply.
  *   FD3_TUNE_XQ         TMA x-pass (FD3_TUNE_FFT_X = 2, mixed precision): flattened (y, kz)
  *                       values per unit, 4, 8, 16 or 32; -1 = the default (by mesh and channels).
